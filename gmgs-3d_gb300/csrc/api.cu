@@ -186,12 +186,12 @@ int64_t model_bytes(const gmgs::Model& M) {
     int64_t b = 0;
     for (const auto& lv : M.levels)
         for (const gmgs::DevBuf* d : {&lv.emask, &lv.nflag, &lv.etype, &lv.escale64, &lv.escale32, &lv.Ks64, &lv.Ks32,
-                                      &lv.kslot, &lv.diag64, &lv.diag32, &lv.wdinv32, &lv.emask8, &lv.perel_nodes, &lv.node_slot, &lv.elem_slot,
-                                      &lv.vr, &lv.vrp, &lv.vdx, &lv.vx, &lv.vy, &lv.tile_occ, &lv.tc_occ})
+                                      &lv.kslot, &lv.diag64, &lv.wdinv32, &lv.wdinv64, &lv.bnd_nodes, &lv.emask8, &lv.perel_nodes, &lv.node_slot, &lv.elem_slot,
+                                      &lv.vr, &lv.vrp, &lv.vx, &lv.tile_occ, &lv.tc_occ})
             b += (int64_t)d->bytes;
     for (const gmgs::DevBuf* d : {&M.ke0_dev, &M.rho, &M.F, &M.U, &M.free_idx, &M.cb.sinv, &M.cb.g, &M.cb.partial, &M.cb.ticket, &M.cvec_in, &M.cvec_out,
-                                  &M.cg_x, &M.cg_r, &M.cg_p, &M.cg_dx, &M.cg_q64, &M.cg_y64, &M.cg_z64, &M.cg_q32,
-                                  &M.cg_y32, &M.cg_z32, &M.cg_r32, &M.cg_r32b, &M.cg_pa, &M.cg_pb, &M.scal, &M.dot_partials, &M.dot_ticket, &M.tc_err})
+                                  &M.cg_x, &M.cg_r, &M.cg_rb, &M.cg_p, &M.cg_p2, &M.cg_q64, &M.cg_z64, &M.mask_stencil, &M.cg_q32,
+                                  &M.cg_z32, &M.cg_r32, &M.cg_r32b, &M.cg_pa, &M.cg_pb, &M.scal, &M.dot_partials, &M.dot_ticket, &M.tc_err})
         b += (int64_t)d->bytes;
     return b;
 }
@@ -245,8 +245,8 @@ const char* site_name(int site) {
         "k_up32 coarse values", "k_up32 output", "k_perel_vdown node list", "k_perel_vdown element data",
         "k_perel_vdown vectors", "k_perel_vdown element matrices", "k_perel_vdown output", "k_tc_vdown field staging",
         "k_tc_vdown element data", "k_tc_vdown node operands", "k_tc_vdown shared ring",
-        "k_tc_vdown element-output buffer", "k_tc_vdown output", "k_matvec input gather", "k_matvec element data",
-        "k_matvec output", "k_restrict", "k_prolong_post", "stress displacement gather", "stress outputs",
+        "k_tc_vdown element-output buffer", "k_tc_vdown output", "FP64 operator field", "FP64 operator node lists",
+        "FP64 operator tile buffers", "FP64 operator outputs", "k_restrict", "stress displacement gather", "stress outputs",
         "k_grad"};
     return site > 0 && site < SITE_COUNT ? names[site] : "unknown site";
 }
@@ -563,7 +563,7 @@ int gmgs_apply_preconditioner(gmgs_handle* h, const double* r, double* z) {
         GMGS_CUDA(cudaMemsetAsync(xd.p, 0, 3 * S * sizeof(double), M.ctx.stream));
         GMGS_CUDA(cudaMemsetAsync(yd.p, 0, 3 * S * sizeof(double), M.ctx.stream));
         gmgs::launch_compact_to_dense<double>(M.ctx, nn, S, lv.node_slot.as<int32_t>(), xc.as<double>(), xd.as<double>());
-        gmgs::vcycle_apply_fp64(M, xd.as<double>(), yd.as<double>());
+        gmgs::vcycle_apply(M, xd.as<double>(), yd.as<double>());
         gmgs::launch_dense_to_compact<double>(M.ctx, nn, S, lv.node_slot.as<int32_t>(), yd.as<double>(), xc.as<double>());
         GMGS_CUDA(cudaMemcpyAsync(z, xc.p, 3 * nn * sizeof(double), cudaMemcpyDeviceToHost, M.ctx.stream));
         GMGS_CUDA(cudaStreamSynchronize(M.ctx.stream));
@@ -603,7 +603,7 @@ int gmgs_apply_preconditioner_dev(gmgs_handle* h, const double* r, double* z) {
         GMGS_CUDA(cudaMemsetAsync(xd.p, 0, 3 * S * sizeof(double), M.ctx.stream));
         GMGS_CUDA(cudaMemsetAsync(yd.p, 0, 3 * S * sizeof(double), M.ctx.stream));
         gmgs::launch_compact_to_dense<double>(M.ctx, nn, S, lv.node_slot.as<int32_t>(), r, xd.as<double>());
-        gmgs::vcycle_apply_fp64(M, xd.as<double>(), yd.as<double>());
+        gmgs::vcycle_apply(M, xd.as<double>(), yd.as<double>());
         gmgs::launch_dense_to_compact<double>(M.ctx, nn, S, lv.node_slot.as<int32_t>(), yd.as<double>(), z);
         GMGS_CUDA(cudaStreamSynchronize(M.ctx.stream));
         return GMGS_OK;

@@ -1,0 +1,924 @@
+// FP64 streaming operator kernels of the default path.
+//
+// GB300 issues FP64 arithmetic at about 2 lanes per clock per SM, 1/64 of its
+// FP32 rate: every FP64 operation per node costs as much time as moving 11
+// bytes per node through HBM, so these kernels are organised to spend as few
+// FP64 operations as possible and to let everything else (loads, shared
+// memory, integer work) hide behind that pipe.
+//
+// K x on interior nodes of a uniform level: the trilinear box element's
+// stencil is a sum of tensor products of 1-D operators (Coef64), so it is
+// applied axis by axis (z in registers, x and y through shared memory), 66
+// operations per node instead of the 117 of the assembled 27-point pairs or
+// the 576 of the element form.  The 1-D second differences annihilate
+// constants exactly, so the result is also more accurate than the assembled
+// sum (2.6e-14 against 3.8e-14 relative on a smooth field, where |K x| is
+// small against |K||x|).
+//
+// Solid nodes with void elements around them take the assembled stencil of
+// their own set of solid elements (256 precomputed sets), nodes on elements
+// with stored matrices the element sum, both from compact node lists, 8 lanes
+// per node; a level with an element scale (density) takes the element form in
+// modal coordinates (k_modal64).  All parts of one K x run in one launch: the
+// list blocks first, then the tiles.
+//
+// The vector operations around K x (Jacobi step, CG direction, CG update,
+// residuals, dot products) are fused into it as in the mixed path (fine.cu).
+//
+// Measured at 6.4M nodes (169 x 147 x 256 elements): K x alone took 4.1 ms as
+// a thread per node on the assembled pairs and eight element rows; with the
+// Jacobi step and the residual in the same launch it takes 1.44 ms, with the
+// CG direction 1.54 ms, with the CG update 1.80 ms, at 78 to 83 % of the FP64
+// pipe (12 % of the issue slots).  A PCG iteration went from 16.9 to 6.2 ms.
+#include <algorithm>
+#include <atomic>
+
+#include "element_host.h"
+#include "fine.cuh"
+#include "fine64.cuh"
+
+namespace gmgs {
+
+namespace {
+
+constexpr int TY = 32, TX = 8;
+constexpr int NT = TY * TX;
+constexpr int HY = TY + 2, HX = TX + 2;
+constexpr int NP = HY * HX;          // points of a tile plane with its one-node halo
+constexpr int NHALO = NP - NT;       // 84
+constexpr int NXP = HY * TX;         // points of the x stage: the tile's columns with the y halo
+constexpr int LANES = 8;             // lanes per list node
+
+__host__ __device__ constexpr int field_arrays64(int mode) {
+    return mode == M64_PLAIN ? 1 : (mode == M64_CG_UPDATE_JACOBI ? 3 : 2);
+}
+__host__ __device__ constexpr bool has_dot(int mode) { return mode == M64_CG_UPDATE_JACOBI || mode == M64_CG_DIRECTION; }
+
+// input arrays of the field, in the order form() takes them
+template <int MODE>
+__device__ __forceinline__ const double* field_array(const Args64& a, int j) {
+    if (MODE == M64_PLAIN) return a.v;
+    if (MODE == M64_VCYCLE_DOWN) return j == 0 ? a.r : a.w;
+    if (MODE == M64_CG_UPDATE_JACOBI) return j == 0 ? a.r : (j == 1 ? a.w : a.q);
+    return j == 0 ? a.z : a.pold;
+}
+
+// one component of the field from its inputs; s: what the epilogue needs of
+// them at the node itself (r of the down-sweep, r_m of the update)
+template <int MODE>
+__device__ __forceinline__ void form(double f0, double f1, double f2, double ab, int first, double& v, double& s) {
+    s = 0.0;
+    if (MODE == M64_PLAIN) {
+        v = f0;
+    } else if (MODE == M64_VCYCLE_DOWN) {
+        s = f0;
+        v = f0 * f1;
+    } else if (MODE == M64_CG_UPDATE_JACOBI) {
+        s = first ? f0 : fma(-ab, f2, f0);
+        v = s * f1;
+    } else {
+        v = first ? f0 : fma(ab, f1, f0);
+    }
+}
+template <int MODE>
+__device__ __forceinline__ void form_at(const Args64& a, int64_t i, int64_t n3, double ab, double& v, double& s) {
+    constexpr int F = chk::F64_FIELD;
+    const double f0 = chk::ld(field_array<MODE>(a, 0), i, n3, F);
+    double f1 = 0.0, f2 = 0.0;
+    const bool need1 = MODE == M64_VCYCLE_DOWN || MODE == M64_CG_UPDATE_JACOBI || (MODE == M64_CG_DIRECTION && !a.first);
+    if (need1) f1 = chk::ld(field_array<MODE>(a, 1), i, n3, F);
+    if (MODE == M64_CG_UPDATE_JACOBI && !a.first) f2 = chk::ld(field_array<MODE>(a, 2), i, n3, F);
+    form<MODE>(f0, f1, f2, ab, a.first, v, s);
+}
+
+// outputs of one DOF from y = (A v), already zeroed on fixed DOFs; px, xx: p
+// and x of the node (update only)
+template <int MODE>
+__device__ __forceinline__ void finish_dof(const Args64& a, int64_t i, int64_t n3, double y, double v, double s, double px,
+                                           double xx, double ab, double& dot) {
+    constexpr int O = chk::F64_OUT;
+    if (MODE == M64_PLAIN) {
+        chk::st(a.out, i, n3, O, y);
+    } else if (MODE == M64_VCYCLE_DOWN) {
+        chk::st(a.out, i, n3, O, s - y);
+    } else if (MODE == M64_CG_UPDATE_JACOBI) {
+        // x += alpha p + dx; r = r_m - A dx; the caller removes the last dx
+        // (of an iteration that does not run) when the solve stops
+        chk::st(a.x, i, n3, O, xx + (a.first ? v : fma(ab, px, v)));
+        chk::st(a.out, i, n3, O, s - y);
+        dot = fma(s, s, dot);
+    } else {
+        chk::st(a.pout, i, n3, O, v);
+        chk::st(a.out, i, n3, O, y);
+        dot = fma(v, y, dot);
+    }
+}
+
+__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// sum over the 8 lanes of a list node
+__device__ __forceinline__ double lanes_sum(double v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
+    return v;
+}
+
+// one list node (8 lanes, j = lane): bnd: the assembled stencil of its solid
+// elements, lane j taking the offsets j, j + 8, ...; else the element sum,
+// lane j taking the coupling to element node j
+template <int MODE>
+__device__ void list_node(const Level64& L, const Args64& a, bool bnd, int at, int j, double ab, double& dot) {
+    const Grid& g = L.g;
+    const int64_t S = g.slots, n3 = 3 * S, sx = g.sx(), sz = g.sz();
+    const int count = bnd ? L.n_bnd : L.n_perel;
+    const bool active = at < count;
+    const int64_t n = active ? chk::ld(bnd ? L.bnd : L.perel, at, count, chk::F64_LIST) : 0;
+    double y[3] = {0.0, 0.0, 0.0};
+    if (active && bnd) {
+        uint32_t mask = 0;
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (chk::ld(L.emask, n - (e & 1) - ((e >> 1) & 1) * sx - (e >> 2) * sz, S, chk::F64_LIST)) mask |= 1u << e;
+        const double* T = L.mask_stencil + (int64_t)mask * MASK_STENCIL;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const int k = j + t * LANES;
+            if (k < 27) {
+                const int64_t m = n + off_y(k) + off_x(k) * sx + off_z(k) * sz;
+                double v[3], s;
+#pragma unroll
+                for (int b = 0; b < 3; ++b) form_at<MODE>(a, m + b * S, n3, ab, v[b], s);
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+#pragma unroll
+                    for (int b = 0; b < 3; ++b) y[c] = fma(T[9 * k + 3 * c + b], v[b], y[c]);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) y[c] *= L.kscale;
+    } else if (active) {
+#pragma unroll 2
+        for (int e = 0; e < 8; ++e) {
+            const int A = e & 1, B = (e >> 1) & 1, C = e >> 2;
+            const int64_t es = n - A - B * sx - C * sz;
+            if (!chk::ld(L.emask, es, S, chk::F64_LIST)) continue;      // uniform across the node's lanes
+            const int t = L.etype ? chk::ld(L.etype, es, S, chk::F64_LIST) : 0;
+            if (t > 0 && !chk::ok(t - 1, L.nK, chk::F64_LIST)) continue;
+            const int64_t m = es + corner_y(j) + corner_x(j) * sx + corner_z(j) * sz;
+            const double* K = (t > 0 ? L.Ks + (int64_t)(t - 1) * KE : L.ke0) + 3 * corner_of(A, B, C) * 24 + 3 * j;
+            const double k = t > 0 ? 1.0 : L.kscale;
+            double v[3], s;
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                form_at<MODE>(a, m + b * S, n3, ab, v[b], s);
+                v[b] *= k;
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+#pragma unroll
+                for (int b = 0; b < 3; ++b) y[c] = fma(K[24 * c + b], v[b], y[c]);
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) y[c] = lanes_sum(y[c]);
+    if (active && j < 3) {
+        const uint32_t f = chk::ld(L.nflag, n, S, chk::F64_LIST);
+        const int64_t i = n + j * S;
+        double v, s, px = 0.0, xx = 0.0;
+        form_at<MODE>(a, i, n3, ab, v, s);
+        if (MODE == M64_CG_UPDATE_JACOBI) {
+            xx = chk::ld((const double*)a.x, i, n3, chk::F64_FIELD);
+            if (!a.first) px = chk::ld(a.pold, i, n3, chk::F64_FIELD);
+        }
+        double yj = j == 0 ? y[0] : (j == 1 ? y[1] : y[2]);
+        if (f & (NF_FIX_X << j)) yj = 0.0;
+        finish_dof<MODE>(a, i, n3, yj, v, s, px, xx, ab, dot);
+    }
+}
+
+// beta = r.z / r_old.z_old of the direction, alpha = r.z / p.q of the update:
+// one division per CTA
+template <int MODE>
+__device__ __forceinline__ double step_length(const Args64& a) {
+    if (!has_dot(MODE) || a.first) return 0.0;
+    __shared__ double s_ab;
+    if (threadIdx.x == 0) s_ab = a.scal[a.cur] / a.scal[MODE == M64_CG_DIRECTION ? (a.cur ^ 1) : 2];
+    __syncthreads();
+    return s_ab;
+}
+
+template <int MODE>
+__device__ __forceinline__ void dot_finish(double dot, const Args64& a, double* sh) {
+    if (has_dot(MODE)) grid_dot_finish(dot, DotOut{a.dot.partials, a.dot.ticket, a.dot.out}, sh);
+}
+
+// this thread's points of a tile plane: its own node and, for the first
+// NHALO threads, one point of the one-node halo
+struct Points {
+    int pc, ph;             // index in the (HX x HY) plane
+    int64_t cbase, hbase;   // slot at z = 0
+    bool cok, hok;          // inside the allocated grid
+    int cy, cx;
+    __device__ Points(const Grid& g, int y0, int x0, int tid) {
+        const int ly = tid & (TY - 1), lx = tid / TY;
+        cy = y0 + ly;
+        cx = x0 + lx;
+        pc = (ly + 1) + (lx + 1) * HY;
+        cok = cy <= g.ny + 1 && cx <= g.nx + 1;
+        cbase = g.slot(cy, cx, 0);
+        ph = 0;
+        hbase = 0;
+        hok = false;
+        if (tid < NHALO) {
+            int hy, hx;
+            if (tid < 2 * TY) { hx = tid < TY ? 0 : HX - 1; hy = 1 + (tid & (TY - 1)); }      // x faces: whole rows
+            else { const int k = tid - 2 * TY; hy = (k & 1) ? HY - 1 : 0; hx = k >> 1; }      // y faces with the corners
+            ph = hy + hx * HY;
+            const int gy = y0 - 1 + hy, gx = x0 - 1 + hx;
+            hok = gy <= g.ny + 1 && gx <= g.nx + 1;
+            hbase = g.slot(gy, gx, 0);
+        }
+    }
+};
+
+template <int MODE>
+constexpr size_t fine64_smem() {
+    return sizeof(double) * (9 * NP + 9 * NXP + 2 * 3 * field_arrays64(MODE) * NP);
+}
+
+// ---------------------------------------------------------------------------
+// K x with the uniform matrix, axis by axis.  A CTA owns a 32 (y, lanes) x 8
+// (x) column of nodes and walks a chunk of z planes.  Per plane:
+//   - the field of plane z + 1 is formed from its inputs, which cp.async has
+//     brought to this thread's own places in shared memory one plane ahead
+//     (each thread reads back only what it copied: no barrier)
+//   - z stage: m, k and d along z at the tile's nodes and halo, from the three
+//     planes in registers                                  (12 operations, 11/8 warps)
+//   - x stage: sums P, Q, R of the y operators m, k, d at the tile's columns
+//     and their y halo                                     (33 operations, 9/8 warps)
+//   - y stage and the mode's vector updates at the interior nodes
+// Two barriers per plane; two CTAs per SM keep the FP64 pipe fed across them.
+// ---------------------------------------------------------------------------
+template <int MODE>
+__global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_constant__ Coef64 cf, Args64 a, int zc, int nb_bnd,
+                                                  int nb_list, int tiles_y, int tiles_x) {
+    __shared__ double sh[32];
+    extern __shared__ double dyn[];
+    const int tid = threadIdx.x;
+    const Grid& g = L.g;
+    const double ab = step_length<MODE>(a);
+    double dot = 0.0;
+    if ((int)blockIdx.x < nb_list) {
+        const bool bnd = (int)blockIdx.x < nb_bnd;
+        const int at = ((int)blockIdx.x - (bnd ? 0 : nb_bnd)) * (NT / LANES) + tid / LANES;
+        list_node<MODE>(L, a, bnd, at, tid % LANES, ab, dot);
+        dot_finish<MODE>(dot, a, sh);
+        return;
+    }
+    const int bid = (int)blockIdx.x - nb_list;
+    const int bty = bid % tiles_y, btx = bid / tiles_y % tiles_x, btz = bid / (tiles_y * tiles_x);
+    const int y0 = bty * TY, x0 = btx * TX;
+    const int zb = btz * zc, ze = min(zb + zc, g.nz + 1);       // node planes [zb, ze)
+    auto occ = [&](int iz) { return L.tile_occ[((int64_t)iz * tiles_x + btx) * tiles_y + bty] != 0; };
+    {
+        bool any = false;
+        for (int iz = zb; iz < ze; ++iz) any |= occ(iz);
+        if (!any) {                                             // uniform across the CTA
+            dot_finish<MODE>(0.0, a, sh);
+            return;
+        }
+    }
+    const int64_t S = g.slots, n3 = 3 * S, sz = g.sz();
+    const Points p(g, y0, x0, tid);
+    const bool own = p.cy <= g.ny && p.cx <= g.nx;
+    constexpr int NA = field_arrays64(MODE);
+    constexpr int R = chk::F64_TILE;
+    double* const Zb = dyn;                       // 9 fields of the z stage: m, k, d of the three components
+    double* const Xb = Zb + 9 * NP;               // 9 fields of the x stage: P, Q, R
+    double* const stage = Xb + 9 * NXP;           // [2][NA * 3][NP] field inputs of two planes
+    const int narr = ((MODE == M64_CG_UPDATE_JACOBI || MODE == M64_CG_DIRECTION) && a.first) ? NA - 1 : NA;
+
+    // field inputs of plane iz to this thread's places of buffer iz & 1
+    auto issue = [&](int iz) {
+        double* st = stage + ((iz + 1) & 1) * (NA * 3 * NP);
+#pragma unroll
+        for (int j = 0; j < NA; ++j) {
+            if (j >= narr) break;
+            const double* src = field_array<MODE>(a, j);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const int64_t ic = p.cbase + iz * sz + c * S, ih = p.hbase + iz * sz + c * S;
+                if (p.cok && chk::ok(ic, n3, chk::F64_FIELD)) cp_async8(st + (j * 3 + c) * NP + p.pc, src + ic);
+                if (p.hok && chk::ok(ih, n3, chk::F64_FIELD)) cp_async8(st + (j * 3 + c) * NP + p.ph, src + ih);
+            }
+        }
+    };
+    auto formed = [&](int iz, int pt, bool ok, double v[3], double s[3]) {
+        const double* st = stage + ((iz + 1) & 1) * (NA * 3 * NP);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            v[c] = s[c] = 0.0;
+            if (ok) {
+                const double f0 = chk::ld(st, c * NP + pt, NA * 3 * NP, R);
+                double f1 = 0.0, f2 = 0.0;
+                if (NA > 1 && narr > 1) f1 = chk::ld(st, (3 + c) * NP + pt, NA * 3 * NP, R);
+                if (NA > 2 && narr > 2) f2 = chk::ld(st, (6 + c) * NP + pt, NA * 3 * NP, R);
+                form<MODE>(f0, f1, f2, ab, a.first, v[c], s[c]);
+            }
+        }
+    };
+    double vm[3], vc[3], vp[3], hm[3], hc[3], hp[3], sc[3], sp[3], unused[3];
+    issue(zb - 1);
+    cp_async_commit();
+    issue(zb);
+    cp_async_commit();
+    cp_async_wait<1>();
+    formed(zb - 1, p.pc, p.cok, vm, unused);
+    formed(zb - 1, p.ph, p.hok, hm, unused);
+    issue(zb + 1);
+    cp_async_commit();
+    cp_async_wait<1>();
+    formed(zb, p.pc, p.cok, vc, sc);
+    formed(zb, p.ph, p.hok, hc, unused);
+
+    auto z_stage = [&](int pt, const double* um, const double* u, const double* up) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double s = um[c] + up[c];
+            chk::st(Zb, c * NP + pt, 9 * NP, R, fma(4.0, u[c], s));
+            chk::st(Zb, (3 + c) * NP + pt, 9 * NP, R, fma(2.0, u[c], -s));
+            chk::st(Zb, (6 + c) * NP + pt, 9 * NP, R, up[c] - um[c]);
+        }
+    };
+    // P, Q, R at plane point (yy, x column): operands at pt - HY, pt, pt + HY
+    auto x_stage = [&](int pt, double P[3], double Q[3], double Rr[3]) {
+        auto zf = [&](int f, int o) { return chk::ld((const double*)Zb, f * NP + pt + o * HY, 9 * NP, R); };
+        auto mx = [&](int f) { return fma(4.0, zf(f, 0), zf(f, -1) + zf(f, 1)); };
+        double kM[3], dM[2];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double l = zf(c, -1), u = zf(c, 0), r = zf(c, 1), s = l + r;
+            Q[c] = fma(4.0, u, s);
+            kM[c] = fma(2.0, u, -s);
+            if (c < 2) dM[c] = r - l;
+        }
+        const double dDz = zf(8, 1) - zf(8, -1), dDx = zf(6, 1) - zf(6, -1);
+        P[0] = fma(cf.gxz, dDz, fma(cf.az[0], mx(3), cf.ax[0] * kM[0]));
+        P[1] = fma(cf.az[1], mx(4), cf.ax[1] * kM[1]);
+        P[2] = fma(cf.gxz, dDx, fma(cf.az[2], mx(5), cf.ax[2] * kM[2]));
+        Rr[0] = dM[1];
+        Rr[1] = fma(cf.gyz, mx(8), cf.gxy * dM[0]);
+        Rr[2] = mx(7);
+    };
+    const int xc = (p.pc % HY) + (tid / TY) * HY;                // own point of the x stage
+    const int hxc = tid & 15, hyy = (hxc & 1) ? HY - 1 : 0;      // the y halo's points: 16 threads
+    const int hz_pt = hyy + ((hxc >> 1) + 1) * HY, hx_pt = hyy + (hxc >> 1) * HY;
+
+#pragma unroll 1
+    for (int iz = zb; iz < ze; ++iz) {
+        if (iz + 1 < ze) issue(iz + 2);
+        cp_async_commit();
+        const int64_t n = p.cbase + iz * sz;
+        const uint32_t f = own ? chk::ld(L.nflag, n, S, chk::F64_FIELD) : 0u;
+        const bool node = (f & NF_INTERIOR) != 0;
+        double xx[3] = {0.0, 0.0, 0.0}, px[3] = {0.0, 0.0, 0.0};
+        if (MODE == M64_CG_UPDATE_JACOBI && node) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                xx[c] = chk::ld((const double*)a.x, n + c * S, n3, chk::F64_FIELD);
+                if (!a.first) px[c] = chk::ld(a.pold, n + c * S, n3, chk::F64_FIELD);
+            }
+        }
+        cp_async_wait<1>();
+        formed(iz + 1, p.pc, p.cok, vp, sp);
+        formed(iz + 1, p.ph, p.hok, hp, unused);
+        if (occ(iz)) {                                           // uniform across the CTA
+            z_stage(p.pc, vm, vc, vp);
+            if (tid < NHALO) z_stage(p.ph, hm, hc, hp);
+            __syncthreads();
+            double P[3], Q[3], Rr[3];
+            if (tid < 16) {
+                x_stage(hz_pt, P, Q, Rr);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    chk::st(Xb, c * NXP + hx_pt, 9 * NXP, R, P[c]);
+                    chk::st(Xb, (3 + c) * NXP + hx_pt, 9 * NXP, R, Q[c]);
+                    chk::st(Xb, (6 + c) * NXP + hx_pt, 9 * NXP, R, Rr[c]);
+                }
+            }
+            x_stage(p.pc, P, Q, Rr);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                chk::st(Xb, c * NXP + xc, 9 * NXP, R, P[c]);
+                chk::st(Xb, (3 + c) * NXP + xc, 9 * NXP, R, Q[c]);
+                chk::st(Xb, (6 + c) * NXP + xc, 9 * NXP, R, Rr[c]);
+            }
+            __syncthreads();
+            if (node) {
+                const double gr[3] = {cf.gxy, 1.0, cf.gyz};
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    auto xf = [&](int k, int o) { return chk::ld((const double*)Xb, (3 * k + c) * NXP + xc + o, 9 * NXP, R); };
+                    const double mP = fma(4.0, P[c], xf(0, -1) + xf(0, 1));
+                    const double kQ = fma(2.0, Q[c], -(xf(1, -1) + xf(1, 1)));
+                    const double dR = xf(2, 1) - xf(2, -1);
+                    double y = fma(cf.ay[c], kQ, mP);
+                    y = c == 1 ? y + dR : fma(gr[c], dR, y);
+                    if (f & (NF_FIX_X << c)) y = 0.0;
+                    finish_dof<MODE>(a, n + c * S, n3, y, vc[c], sc[c], px[c], xx[c], ab, dot);
+                }
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            vm[c] = vc[c];
+            vc[c] = vp[c];
+            hm[c] = hc[c];
+            hc[c] = hp[c];
+            sc[c] = sp[c];
+        }
+    }
+    cp_async_wait<0>();
+    dot_finish<MODE>(dot, a, sh);
+}
+
+// ---------------------------------------------------------------------------
+// K x with a scale per element (density), element form in modal coordinates.
+// With the sums s = u0 + u1 and differences e = u1 - u0 along each axis, the
+// 1-D element operators are diagonal or have one entry (mass: h/4 s s' +
+// h/12 e e'; stiffness: e e'/h; derivative: e s'/2), so the 24 x 24 element
+// matrix becomes 45 multiplications, and the transforms along z and their
+// sums at the nodes are shared between neighbouring elements: about 235
+// operations per node against 600 for eight elements' rows.  Rigid
+// translations (the all-s modes) drop out exactly.
+// Walk as in k_fine64; layer l lies between the node planes l and l + 1.
+// ---------------------------------------------------------------------------
+constexpr int EY = TY + 1, EX = TX + 1, NE = EY * EX;      // elements of a layer that touch the tile
+constexpr size_t MODAL_SMEM = sizeof(double) * (6 * NP + 24 * NE);
+
+// coefficients of the modal element matrix
+struct Modal {
+    double m[3][2];           // mass per axis (x, y, z): [0] sum mode, [1] difference mode
+    double k[3];              // stiffness per axis on the difference mode
+    double lam4, mu4, lam, mu, sgn_xy, sgn_xz, sgn_yz;
+};
+__device__ __forceinline__ Modal modal_coefs(const Coef64& cf) {
+    Modal c;
+    const double h[3] = {cf.hx, cf.hy, cf.hz};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        c.m[d][0] = 0.25 * h[d];
+        c.m[d][1] = h[d] / 12.0;
+        c.k[d] = 1.0 / h[d];
+    }
+    c.lam = cf.lam;
+    c.mu = cf.mu;
+    c.lam4 = 0.25 * cf.lam;
+    c.mu4 = 0.25 * cf.mu;
+    c.sgn_xy = -1.0;          // physical y runs against the node index
+    c.sgn_xz = 1.0;
+    c.sgn_yz = -1.0;
+    return c;
+}
+
+// the constants of the 45 products, formed once per thread
+struct ModalK {
+    double d[3][8];           // diagonal, component c, mode bits x = 1, y = 2, z = 4
+    double l_xy[2], u_xy[2];  // lambda and mu couplings of the axes (x, y) by the third axis' mode
+    double l_xz[2], u_xz[2];
+    double l_yz[2], u_yz[2];
+};
+__device__ __forceinline__ void modal_k(const Coef64& cf, double* out) {
+    const Modal c = modal_coefs(cf);
+    ModalK k;
+#pragma unroll
+    for (int comp = 0; comp < 3; ++comp)
+#pragma unroll
+        for (int md = 0; md < 8; ++md) {
+            double v = 0.0;
+#pragma unroll
+            for (int ax = 0; ax < 3; ++ax) {
+                const int o1 = ax == 0 ? 1 : 0, o2 = ax == 2 ? 1 : 2;
+                if (!((md >> ax) & 1)) continue;
+                const double e = ax == comp ? c.lam + 2.0 * c.mu : c.mu;
+                v += e * c.k[ax] * c.m[o1][(md >> o1) & 1] * c.m[o2][(md >> o2) & 1];
+            }
+            k.d[comp][md] = v;
+        }
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        k.l_xy[t] = c.sgn_xy * c.lam4 * c.m[2][t];
+        k.u_xy[t] = c.sgn_xy * c.mu4 * c.m[2][t];
+        k.l_xz[t] = c.sgn_xz * c.lam4 * c.m[1][t];
+        k.u_xz[t] = c.sgn_xz * c.mu4 * c.m[1][t];
+        k.l_yz[t] = c.sgn_yz * c.lam4 * c.m[0][t];
+        k.u_yz[t] = c.sgn_yz * c.mu4 * c.m[0][t];
+    }
+    double* o = out;
+    for (int comp = 0; comp < 3; ++comp)
+        for (int md = 0; md < 8; ++md) *o++ = k.d[comp][md];
+    for (int t = 0; t < 2; ++t) {
+        *o++ = k.l_xy[t]; *o++ = k.u_xy[t];
+        *o++ = k.l_xz[t]; *o++ = k.u_xz[t];
+        *o++ = k.l_yz[t]; *o++ = k.u_yz[t];
+    }
+}
+constexpr int NMODAL = 36;
+
+template <int MODE>
+__global__ void __launch_bounds__(NT, 2) k_modal64(Level64 L, const __grid_constant__ Coef64 cf, Args64 a, int zc, int tiles_y,
+                                                   int tiles_x) {
+    __shared__ double sh[32], mk[NMODAL];
+    extern __shared__ double dyn[];
+    const int tid = threadIdx.x;
+    const Grid& g = L.g;
+    const double ab = step_length<MODE>(a);
+    const int bty = blockIdx.x % tiles_y, btx = blockIdx.x / tiles_y % tiles_x, btz = blockIdx.x / (tiles_y * tiles_x);
+    const int y0 = bty * TY, x0 = btx * TX;
+    const int zb = btz * zc, ze = min(zb + zc, g.nz + 1);
+    double dot = 0.0;
+    {
+        bool any = false;
+        for (int iz = zb; iz < ze; ++iz) any |= L.tile_occ[((int64_t)iz * tiles_x + btx) * tiles_y + bty] != 0;
+        if (!any) {
+            dot_finish<MODE>(0.0, a, sh);
+            return;
+        }
+    }
+    if (tid == 0) modal_k(cf, mk);
+    const int64_t S = g.slots, n3 = 3 * S, sx = g.sx(), sz = g.sz();
+    const Points p(g, y0, x0, tid);
+    const bool own = p.cy <= g.ny && p.cx <= g.nx;
+    constexpr int R = chk::F64_TILE;
+    double* const Zb = dyn;               // s (0..2) and e (3..5) along z of the three components
+    double* const Eb = Zb + 6 * NP;       // per element: component, z mode, (y, x) corner
+    auto field = [&](int iz, int64_t base, bool ok, double v[3], double s[3]) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            v[c] = s[c] = 0.0;
+            if (ok) form_at<MODE>(a, base + iz * sz + c * S, n3, ab, v[c], s[c]);
+        }
+    };
+    double vc[3], vp[3], hc[3], hp[3], sc[3], sp[3], unused[3];
+    double carry[3] = {0.0, 0.0, 0.0};    // A v at plane l from layer l - 1
+    const int l0 = max(zb - 1, 0);
+    field(l0, p.cbase, p.cok, vc, sc);
+    field(l0, p.hbase, p.hok, hc, unused);
+#pragma unroll 1
+    for (int l = l0; l < ze; ++l) {       // layer l, then node plane l
+        double y[3] = {carry[0], carry[1], carry[2]};
+        const int64_t n = p.cbase + l * sz;
+        const uint32_t f = own && l >= zb ? chk::ld(L.nflag, n, S, chk::F64_FIELD) : 0u;
+        double xx[3] = {0.0, 0.0, 0.0}, px[3] = {0.0, 0.0, 0.0};
+        if (MODE == M64_CG_UPDATE_JACOBI && (f & NF_SOLID)) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                xx[c] = chk::ld((const double*)a.x, n + c * S, n3, chk::F64_FIELD);
+                if (!a.first) px[c] = chk::ld(a.pold, n + c * S, n3, chk::F64_FIELD);
+            }
+        }
+        if (l < g.nz) {
+            field(l + 1, p.cbase, p.cok, vp, sp);
+            field(l + 1, p.hbase, p.hok, hp, unused);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                chk::st(Zb, c * NP + p.pc, 6 * NP, R, vp[c] + vc[c]);
+                chk::st(Zb, (3 + c) * NP + p.pc, 6 * NP, R, vp[c] - vc[c]);
+                if (tid < NHALO) {
+                    chk::st(Zb, c * NP + p.ph, 6 * NP, R, hp[c] + hc[c]);
+                    chk::st(Zb, (3 + c) * NP + p.ph, 6 * NP, R, hp[c] - hc[c]);
+                }
+            }
+            __syncthreads();
+            for (int e = tid; e < NE; e += NT) {
+                const int ey = e % EY, ex = e / EY, gy = y0 - 1 + ey, gx = x0 - 1 + ex;
+                double sc_e = 0.0;
+                if (gy >= 0 && gx >= 0 && gy < g.ny && gx < g.nx) {
+                    const int64_t es = g.slot(gy, gx, l);
+                    if (chk::ld(L.emask, es, S, chk::F64_FIELD)) sc_e = L.kscale * chk::ld(L.escale, es, S, chk::F64_FIELD);
+                }
+                if (sc_e != 0.0) {
+                    // modes u[c][mode], bits x = 1, y = 2, z = 4
+                    double u[3][8];
+                    const int pt = ey + ex * HY;
+#pragma unroll
+                    for (int c = 0; c < 3; ++c)
+#pragma unroll
+                        for (int zm = 0; zm < 2; ++zm) {
+                            auto zf = [&](int o) { return chk::ld((const double*)Zb, (3 * zm + c) * NP + pt + o, 6 * NP, R); };
+                            const double a00 = zf(0), a10 = zf(1), a01 = zf(HY), a11 = zf(HY + 1);   // (y, x)
+                            const double s0 = a10 + a00, e0 = a10 - a00, s1 = a11 + a01, e1 = a11 - a01;
+                            u[c][4 * zm + 0] = s1 + s0;
+                            u[c][4 * zm + 1] = s1 - s0;
+                            u[c][4 * zm + 2] = e1 + e0;
+                            u[c][4 * zm + 3] = e1 - e0;
+                        }
+                    const double* D = mk;
+                    const double *c0 = mk + 24, *c1 = mk + 30;   // couplings by the third axis' mode: l_xy u_xy l_xz u_xz l_yz u_yz
+                    double t[3][8];
+                    t[0][1] = fma(c0[2], u[2][4], fma(c0[0], u[1][2], D[1] * u[0][1]));
+                    t[0][2] = fma(c0[1], u[1][1], D[2] * u[0][2]);
+                    t[0][4] = fma(c0[3], u[2][1], D[4] * u[0][4]);
+                    t[0][3] = fma(c1[2], u[2][6], D[3] * u[0][3]);
+                    t[0][5] = fma(c1[0], u[1][6], D[5] * u[0][5]);
+                    t[0][6] = fma(c1[3], u[2][3], fma(c1[1], u[1][5], D[6] * u[0][6]));
+                    t[0][7] = D[7] * u[0][7];
+                    t[1][2] = fma(c0[4], u[2][4], fma(c0[0], u[0][1], D[8 + 2] * u[1][2]));
+                    t[1][1] = fma(c0[1], u[0][2], D[8 + 1] * u[1][1]);
+                    t[1][4] = fma(c0[5], u[2][2], D[8 + 4] * u[1][4]);
+                    t[1][3] = fma(c1[4], u[2][5], D[8 + 3] * u[1][3]);
+                    t[1][6] = fma(c1[0], u[0][5], D[8 + 6] * u[1][6]);
+                    t[1][5] = fma(c1[5], u[2][3], fma(c1[1], u[0][6], D[8 + 5] * u[1][5]));
+                    t[1][7] = D[8 + 7] * u[1][7];
+                    t[2][4] = fma(c0[4], u[1][2], fma(c0[2], u[0][1], D[16 + 4] * u[2][4]));
+                    t[2][1] = fma(c0[3], u[0][4], D[16 + 1] * u[2][1]);
+                    t[2][2] = fma(c0[5], u[1][4], D[16 + 2] * u[2][2]);
+                    t[2][5] = fma(c1[4], u[1][3], D[16 + 5] * u[2][5]);
+                    t[2][6] = fma(c1[2], u[0][3], D[16 + 6] * u[2][6]);
+                    t[2][3] = fma(c1[5], u[1][5], fma(c1[3], u[0][6], D[16 + 3] * u[2][3]));
+                    t[2][7] = D[16 + 7] * u[2][7];
+#pragma unroll
+                    for (int c = 0; c < 3; ++c)
+#pragma unroll
+                        for (int zm = 0; zm < 2; ++zm) {
+                            // transposed transforms along x and y; mode 0 carries no force
+                            const double m0 = zm ? sc_e * t[c][4] : 0.0, m1 = sc_e * t[c][4 * zm + 1],
+                                         m2 = sc_e * t[c][4 * zm + 2], m3 = sc_e * t[c][4 * zm + 3];
+                            const double s0 = m0 - m1, s1 = m0 + m1, e0 = m2 - m3, e1 = m2 + m3;   // x = 0, 1
+                            double* o = Eb + ((c * 2 + zm) * 4) * NE + e;
+                            constexpr int N = 24 * NE;
+                            const int b = ((c * 2 + zm) * 4) * NE + e;
+                            (void)o;
+                            chk::st(Eb, b, N, R, s0 - e0);                // (y, x) = (0, 0)
+                            chk::st(Eb, b + NE, N, R, s0 + e0);           // (1, 0)
+                            chk::st(Eb, b + 2 * NE, N, R, s1 - e1);       // (0, 1)
+                            chk::st(Eb, b + 3 * NE, N, R, s1 + e1);       // (1, 1)
+                        }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 24; ++k) chk::st(Eb, k * NE + e, 24 * NE, R, 0.0);
+                }
+            }
+            __syncthreads();
+            const int ly = tid & (TY - 1), lx = tid / TY;
+            const int e00 = ly + lx * EY;      // the element with this node at its (1, 1) corner
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                double fz[2];
+#pragma unroll
+                for (int zm = 0; zm < 2; ++zm) {
+                    const int b = ((c * 2 + zm) * 4) * NE + e00;
+                    auto E = [&](int i) { return chk::ld((const double*)Eb, b + i, 24 * NE, R); };
+                    fz[zm] = (E(3 * NE) + E(2 * NE + 1)) + (E(NE + EY) + E(EY + 1));
+                }
+                y[c] += fz[0] - fz[1];
+                carry[c] = fz[0] + fz[1];
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) carry[c] = vp[c] = hp[c] = sp[c] = 0.0;
+        }
+        if (f & NF_SOLID) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                finish_dof<MODE>(a, n + c * S, n3, (f & (NF_FIX_X << c)) ? 0.0 : y[c], vc[c], sc[c], px[c], xx[c], ab, dot);
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            vc[c] = vp[c];
+            hc[c] = hp[c];
+            sc[c] = sp[c];
+        }
+    }
+    dot_finish<MODE>(dot, a, sh);
+}
+
+// z planes per CTA: about 12 waves of two resident CTAs per SM on large grids,
+// at least 4 planes there (each chunk forms two planes beyond its own), down
+// to 2 where the grid would otherwise leave SMs without a CTA
+int pick_zc64(const Grid& g, const Ctx& c, int zmin) {
+    const int64_t cols = (int64_t)((g.ny + 1 + TY - 1) / TY) * ((g.nx + 1 + TX - 1) / TX);
+    const int64_t want = (int64_t)c.num_sms * 2 * 12;
+    int64_t zc = (cols * (g.nz + 1) + want - 1) / want;
+    if (zc < 4) zc = cols * ((g.nz + 1 + 3) / 4) >= 4 * (int64_t)c.num_sms ? 4 : zmin;
+    return (int)std::min<int64_t>(zc, 32);
+}
+
+template <typename K>
+void opt_in_smem(K kernel, size_t bytes, std::atomic<unsigned long long>& opted) {
+    if (bytes <= 48 * 1024) return;
+    int dev = 0;
+    GMGS_CUDA(cudaGetDevice(&dev));
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (opted.load() & bit) return;
+    GMGS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    opted.fetch_or(bit);
+}
+
+}  // namespace
+
+Coef64 make_coef64(double E, double nu, const double ele[3]) {
+    double D[6][6];
+    hooke(E, nu, D);
+    const double a = D[0][0], lam = D[0][1], mu = D[3][3];
+    const double x = ele[0], y = ele[1], z = ele[2];
+    const double cx = y * z / (36.0 * x), cy = x * z / (36.0 * y), cz = x * y / (36.0 * z);
+    Coef64 c;
+    for (int k = 0; k < 3; ++k) {
+        c.ax[k] = (k == 0 ? a : mu) * cx;
+        c.ay[k] = (k == 1 ? a : mu) * cy;
+        c.az[k] = (k == 2 ? a : mu) * cz;
+    }
+    c.gxy = (lam + mu) * z / 24.0;       // physical y runs against the node index: the sign of the
+    c.gxz = -(lam + mu) * y / 24.0;      // (x, y) and (y, z) terms is the opposite of (x, z)'s
+    c.gyz = (lam + mu) * x / 24.0;
+    c.lam = lam;
+    c.mu = mu;
+    c.hx = x;
+    c.hy = y;
+    c.hz = z;
+    return c;
+}
+
+__global__ void k_mask_stencils(const double* __restrict__ ke0, double* __restrict__ table) {
+    const int mask = blockIdx.x;
+    for (int i = threadIdx.x; i < MASK_STENCIL; i += blockDim.x) {
+        const int k = i / 9, a = i % 9 / 3, b = i % 3;
+        double v = 0.0;
+        for (int e = 0; e < 8; ++e) {
+            if (!((mask >> e) & 1)) continue;
+            const int A = e & 1, B = (e >> 1) & 1, C = e >> 2;                  // node = element origin + (A, B, C)
+            const int my = A + off_y(k), mx = B + off_x(k), mz = C + off_z(k);  // neighbour relative to the origin
+            if (my < 0 || my > 1 || mx < 0 || mx > 1 || mz < 0 || mz > 1) continue;
+            v += ke0[(3 * corner_of(A, B, C) + a) * 24 + 3 * corner_of(my, mx, mz) + b];
+        }
+        table[(int64_t)mask * MASK_STENCIL + i] = v;
+    }
+}
+void launch_mask_stencils(Ctx& c, const double* ke0, double* table) {
+    k_mask_stencils<<<256, 256, 0, c.stream>>>(ke0, table);
+    GMGS_LAUNCHED(c);
+}
+
+template <int MODE>
+void launch_fine64(Ctx& c, const Level64& L, const Coef64& cf0, const Args64& a) {
+    const int ty = (L.g.ny + 1 + TY - 1) / TY, tx = (L.g.nx + 1 + TX - 1) / TX;
+    static std::atomic<unsigned long long> opted_m{0}, opted_f{0};
+    if (L.escale) {
+        opt_in_smem(k_modal64<MODE>, MODAL_SMEM, opted_m);
+        const int zc = pick_zc64(L.g, c, 3);
+        const int blocks = ty * tx * ((L.g.nz + 1 + zc - 1) / zc);
+        k_modal64<MODE><<<blocks, NT, MODAL_SMEM, c.stream>>>(L, cf0, a, zc, ty, tx);
+        GMGS_LAUNCHED(c);
+        return;
+    }
+    Coef64 cf = cf0;
+    for (int k = 0; k < 3; ++k) {
+        cf.ax[k] *= L.kscale;
+        cf.ay[k] *= L.kscale;
+        cf.az[k] *= L.kscale;
+    }
+    cf.gxy *= L.kscale;
+    cf.gxz *= L.kscale;
+    cf.gyz *= L.kscale;
+    opt_in_smem(k_fine64<MODE>, fine64_smem<MODE>(), opted_f);
+    const int per = NT / LANES;
+    const int nb_bnd = (L.n_bnd + per - 1) / per, nb_list = nb_bnd + (L.n_perel + per - 1) / per;
+    const int zc = pick_zc64(L.g, c, 2);
+    // a level whose nodes are all on the lists has no tiles to walk
+    const int tiles = L.n_bnd + (int64_t)L.n_perel < L.n_node ? ty * tx * ((L.g.nz + 1 + zc - 1) / zc) : 0;
+    k_fine64<MODE><<<nb_list + tiles, NT, fine64_smem<MODE>(), c.stream>>>(L, cf, a, zc, nb_bnd, nb_list, ty, tx);
+    GMGS_LAUNCHED(c);
+}
+template void launch_fine64<M64_PLAIN>(Ctx&, const Level64&, const Coef64&, const Args64&);
+template void launch_fine64<M64_VCYCLE_DOWN>(Ctx&, const Level64&, const Coef64&, const Args64&);
+template void launch_fine64<M64_CG_UPDATE_JACOBI>(Ctx&, const Level64&, const Coef64&, const Args64&);
+template void launch_fine64<M64_CG_DIRECTION>(Ctx&, const Level64&, const Coef64&, const Args64&);
+
+int dot64_blocks(const Grid& g, int64_t n_list) {
+    const int64_t tiles = (int64_t)((g.ny + 1 + TY - 1) / TY) * ((g.nx + 1 + TX - 1) / TX) * ((g.nz + 1 + 1) / 2);
+    return (int)(tiles + n_list / (NT / LANES) + 2);
+}
+
+// ---------------------------------------------------------------------------
+// up-sweep (Vcycle.m:27-32): one thread per (y, x) column of a 32 x 8 tile,
+// walking a chunk of z planes.  The trilinear sum adds the coarse planes
+// first, then x, then y (3.5 additions per DOF on average instead of up to 7
+// weighted terms), and omega / diagonal is stored, so no division is left.
+// ---------------------------------------------------------------------------
+template <bool DOT>
+__global__ void __launch_bounds__(NT, 2) k_up64(Grid gf, Grid gc, const uint8_t* __restrict__ nflag,
+                                                const uint8_t* __restrict__ tile_occ, int zc, const double* __restrict__ w,
+                                                const double* __restrict__ r, const double* __restrict__ rp,
+                                                const double* __restrict__ xc, double* __restrict__ xf, int zero_fixed,
+                                                DotOut64 dout) {
+    __shared__ double sh[32];
+    const int64_t Sf = gf.slots, Sc = gc.slots, csx = gc.sx(), csz = gc.sz(), fsz = gf.sz();
+    const int iy = blockIdx.x * TY + threadIdx.x, ix = blockIdx.y * TX + threadIdx.y;
+    const int zb = blockIdx.z * zc, ze = min(zb + zc, gf.nz + 1);
+    double dot = 0.0;
+    if (iy <= gf.ny && ix <= gf.nx) {
+        const bool oy = iy & 1, ox = ix & 1;            // ox is uniform across a warp
+        const double wyx = (oy ? 0.5 : 1.0) * (ox ? 0.5 : 1.0);
+        const int64_t fcol = gf.slot(iy, ix, 0), ccol = gc.slot(iy >> 1, ix >> 1, 0);
+        const int64_t trow = (int64_t)gridDim.y * gridDim.x, tcol = (int64_t)blockIdx.y * gridDim.x + blockIdx.x;
+        constexpr int U = chk::UP_FINE, UC = chk::UP_COARSE;
+        double qa[3][4], qb[3][4];
+        int qa_z = -1;
+        auto load_q = [&](int Z, double (&q)[3][4]) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const int64_t x = c * Sc + ccol + Z * csz;
+                q[c][0] = chk::ld(xc, x, 3 * Sc, UC);
+                q[c][1] = chk::ld(xc, x + 1, 3 * Sc, UC);
+                q[c][2] = ox ? chk::ld(xc, x + csx, 3 * Sc, UC) : 0.0;
+                q[c][3] = ox ? chk::ld(xc, x + csx + 1, 3 * Sc, UC) : 0.0;
+            }
+        };
+        for (int iz = zb; iz < ze; ++iz) {
+            if (tile_occ && !tile_occ[iz * trow + tcol]) continue;
+            const int64_t fs = fcol + iz * fsz;
+            const uint32_t fl = chk::ld(nflag, fs, Sf, U);
+            if (!(fl & NF_SOLID)) continue;
+            double wv[3], rv[3], pv[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                wv[c] = chk::ld(w, fs + c * Sf, 3 * Sf, U);
+                rv[c] = chk::ld(r, fs + c * Sf, 3 * Sf, U);
+                pv[c] = chk::ld(rp, fs + c * Sf, 3 * Sf, U);
+            }
+            const int Iz = iz >> 1;
+            const bool oz = iz & 1;                     // uniform across the CTA
+            if (qa_z != Iz) load_q(Iz, qa);
+            if (oz) load_q(Iz + 1, qb);
+            const double wt = wyx * (oz ? 0.5 : 1.0);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                double e0 = qa[c][0], e1 = qa[c][1], e2 = qa[c][2], e3 = qa[c][3];
+                if (oz) {
+                    e0 += qb[c][0];
+                    e1 += qb[c][1];
+                    if (ox) { e2 += qb[c][2]; e3 += qb[c][3]; }
+                }
+                if (ox) { e0 += e2; e1 += e3; }
+                const double t = oy ? e0 + e1 : e0;
+                double out = fma(wt, t, wv[c] * (rv[c] + pv[c]));
+                if (zero_fixed && (fl & (NF_FIX_X << c))) out = 0.0;
+                chk::st(xf, fs + c * Sf, 3 * Sf, chk::UP_OUT, out);
+                if (DOT) dot = fma(rv[c], out, dot);
+            }
+            qa_z = Iz;
+            if (oz) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) qa[c][k] = qb[c][k];
+                qa_z = Iz + 1;
+            }
+        }
+    }
+    if (DOT) grid_dot_finish(dot, DotOut{dout.partials, dout.ticket, dout.out}, sh);
+}
+
+void launch_up64(Ctx& c, const Grid& gf, const Grid& gc, const uint8_t* nflag, const uint8_t* tile_occ, const double* w,
+                 const double* r, const double* rp, const double* xc, double* xf, bool zero_fixed, const DotOut64* dot) {
+    const int zc = pick_zc64(gf, c, 2);
+    const dim3 grid((gf.ny + 1 + TY - 1) / TY, (gf.nx + 1 + TX - 1) / TX, (gf.nz + 1 + zc - 1) / zc);
+    const dim3 blk(TY, TX, 1);
+    if (dot) k_up64<true><<<grid, blk, 0, c.stream>>>(gf, gc, nflag, tile_occ, zc, w, r, rp, xc, xf, zero_fixed, *dot);
+    else k_up64<false><<<grid, blk, 0, c.stream>>>(gf, gc, nflag, tile_occ, zc, w, r, rp, xc, xf, zero_fixed, DotOut64{});
+    GMGS_LAUNCHED(c);
+}
+
+// x -= dx, dx = w (r - alpha q) as the fused update added it
+__global__ void k_drop_last_dx64(int64_t n, double* __restrict__ x, const double* __restrict__ r, const double* __restrict__ q,
+                                 const double* __restrict__ w, const double* __restrict__ scal, int cur) {
+    const double alpha = scal[cur] / scal[2];
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        x[i] -= fma(-alpha, q[i], r[i]) * w[i];
+}
+void launch_drop_last_dx64(Ctx& c, int64_t n, double* x, const double* r, const double* q, const double* w,
+                           const double* scal, int cur) {
+    const int blocks = (int)std::min<int64_t>((n + 255) / 256, (int64_t)c.num_sms * 16);
+    k_drop_last_dx64<<<blocks, 256, 0, c.stream>>>(n, x, r, q, w, scal, cur);
+    GMGS_LAUNCHED(c);
+}
+
+__global__ void k_wdinv64(int64_t n, const double* __restrict__ d, double omega, double* __restrict__ w) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        w[i] = d[i] != 0.0 ? omega / d[i] : 0.0;
+}
+void launch_wdinv64(Ctx& c, int64_t n, const double* d, double omega, double* w) {
+    const int blocks = (int)std::min<int64_t>((n + 255) / 256, (int64_t)c.num_sms * 16);
+    k_wdinv64<<<blocks, 256, 0, c.stream>>>(n, d, omega, w);
+    GMGS_LAUNCHED(c);
+}
+
+}  // namespace gmgs

@@ -71,7 +71,7 @@ enum Site : int {
     FINE_FIELD = 1, FINE_EPI, FINE_FLAGS, FINE_ELEM, FINE_KS, FINE_RING, FINE_OUT,
     UP_FINE, UP_COARSE, UP_OUT, PEREL_NODE, PEREL_ELEM, PEREL_VEC, PEREL_KS, PEREL_OUT,
     TC_FIELD, TC_ELEM, TC_NODE, TC_RING, TC_EOUT, TC_OUT,
-    MV_X, MV_ELEM, MV_Y, RESTRICT, PROLONG, STRESS_U, STRESS_OUT, GRAD,
+    F64_FIELD, F64_LIST, F64_TILE, F64_OUT, RESTRICT, STRESS_U, STRESS_OUT, GRAD,
     SITE_COUNT
 };
 const char* site_name(int site);
@@ -214,22 +214,6 @@ enum : uint8_t { NF_SOLID = 1, NF_FIX_X = 2, NF_FIX_Y = 4, NF_FIX_Z = 8 };
 constexpr uint8_t NF_INTERIOR = 16;  // all 8 surrounding elements carry the level's kscale * Ke0
 
 // ---------------------------------------------------------------------------
-// device-side views passed to kernels by value
-// ---------------------------------------------------------------------------
-template <typename T>
-struct LevelView {
-    Grid g;
-    const uint8_t* emask;    // element solid / non-empty
-    const uint8_t* nflag;    // node flags
-    const int32_t* etype;    // -1 void, 0 universal (Kc), k>0 -> Ks[k-1]; null = all universal
-    const T* Ks;             // per-element matrices, 576 each, row = output DOF
-    int64_t nK;              // matrices held in Ks
-    const T* escale;         // finest-level element scale (density extension) or null
-    const T* diag;           // 3 planes
-    T omega;
-};
-
-// ---------------------------------------------------------------------------
 // host-side level storage
 // ---------------------------------------------------------------------------
 // Device bytes held by every DevBuf in the process, and the high-water mark.
@@ -270,12 +254,15 @@ struct Level {
     DevBuf emask, nflag, etype, escale64, escale32;
     DevBuf Ks64, Ks32;
     DevBuf kslot;             // slot of the coarse element owning Ks[k]
-    DevBuf diag64, diag32;
+    DevBuf diag64;
     DevBuf node_slot;         // compact node id -> slot (int32), reference nodMapBack order
     DevBuf elem_slot;         // compact element id -> slot (int32), eleMapBack order
     // V-cycle work vectors (3 planes each), precision of the V-cycle
-    DevBuf vr, vrp, vdx, vx, vy;
-    DevBuf tile_occ;          // mixed path: per 32x8 node tile and z plane, 1 if it holds a solid node
+    DevBuf vr, vrp, vx;
+    DevBuf tile_occ;          // per 32x8 node tile and z plane, 1 if it holds a solid node
+    DevBuf wdinv64;           // FP64 path: omega / diag
+    DevBuf bnd_nodes;         // FP64 operator: slots of solid nodes with void elements around them and no stored matrix
+    int64_t n_bnd = -1;       // -1: the list is not built yet
     DevBuf wdinv32;           // mixed path: omega / diag in FP32
     DevBuf emask8;            // mixed path: per-node mask of the 8 surrounding solid elements
     DevBuf perel_nodes;       // slots of nodes touching an element with its own stored matrix
@@ -340,65 +327,20 @@ struct Ctx {
 // ---------------------------------------------------------------------------
 constexpr int KE = 576;
 
-// uniform element matrices in constant memory: [0] = Ke0 (FP64), [1] = Ke0 (FP32)
-// Element matrix Ke0 (row = output DOF) and the assembled 27-point interior
-// stencil (3x3 block per offset k, offsets (k%3-1, k/3%3-1, k/9-1) in (y,x,z)),
-// passed to the operator kernels as a __grid_constant__ parameter so that
-// every handle carries its own material and voxel size.
-template <typename T>
-struct MatCoef {
-    T K[KE];
-    T S[243];
-};
-void make_mat_coef(const double* ke_rows, MatCoef<double>& c64, MatCoef<float>& c32);
-
-template <typename T> LevelView<T> view(const Level& L, double omega);
-
-// y = K_l x, fixed rows zeroed (AtX.m:1-58).  Tin/Tout let the mixed path read
-// FP64 CG vectors and compute in FP32.
-template <typename Tc, typename Tin, typename Tout>
-void launch_matvec(Ctx& c, const LevelView<Tc>& lv, const MatCoef<Tc>& cf, const Tin* x, Tout* y, double kscale);
-
-// dx = (omega r) / d  (JacobiSmoother.m:5)
-template <typename Tr, typename Td, typename Tx>
-void launch_jacobi_dx(Ctx& c, const Grid& g, const Td* diag, double omega, const Tr* r, Tx* dx);
-// x += dx (elementwise over 3 planes)
-template <typename T, typename U>
-void launch_add(Ctx& c, int64_t n, T* x, const U* dx);
-// r -= y
-template <typename T, typename U>
-void launch_sub(Ctx& c, int64_t n, T* r, const U* y);
-// out = a (conversion copy)
+// conversion copy out = a
 template <typename T, typename U>
 void launch_copy(Ctx& c, int64_t n, T* out, const U* a);
-// out = a - b
-template <typename T>
-void launch_diff(Ctx& c, int64_t n, T* out, const T* a, const T* b);
 
-// restriction r_c = P^T r_f (RestrictResidual.m) and prolongation with the
-// post-smoothing term x_f = (dx + P x_c) + (omega r') / d (Vcycle.m:29-32)
+// restriction r_c = P^T r_f (RestrictResidual.m)
 template <typename T>
 void launch_restrict(Ctx& c, const Grid& gf, const Grid& gc, const uint8_t* nflag_c,
                      const T* rf, T* rc);
-template <typename T>
-void launch_prolong_post(Ctx& c, const Grid& gf, const Grid& gc, const uint8_t* nflag_f,
-                         const T* diag_f, double omega, const T* xc, const T* dx,
-                         const T* rp, T* xf, bool zero_fixed);
-
 // deterministic dot product: out[0] = sum a*b over n entries (FP64 accumulate)
 struct DotScratch { double* partials; unsigned int* ticket; int blocks; };
 template <typename Ta, typename Tb>
 void launch_dot(Ctx& c, const DotScratch& s, int64_t n, const Ta* a, const Tb* b, double* out);
 
-// CG updates.  scal: device scalars (see solver.cu)
-// cur_first = (r.z slot) | (first iteration << 1)
-template <typename Tz>
-void launch_p_update(Ctx& c, int64_t n, const Tz* z, double* p, const double* scal, int cur_first);
-template <typename Tq>
-void launch_xr_update(Ctx& c, int64_t n, double* x, double* r, const double* p, const Tq* q,
-                      const double* scal, int cur);
-
-// coarsest level: gather free DOFs, dense GEMV with the inverse, scatter back
+// coarsest level: gather free DOFs, scatter back
 template <typename T>
 void launch_gather(Ctx& c, int64_t n, const int32_t* idx, const T* src, double* dst);
 template <typename T>

@@ -758,6 +758,8 @@ void set_density_dev(Model& M, const double* rho_dev) {
                                                              M.penal, l0.escale64.as<double>());
     GMGS_LAUNCHED(c);
     l0.escale32.release();
+    l0.bnd_nodes.release();
+    l0.n_bnd = -1;
     M.has_density = true;
     build_levels(M, nullptr);
     build_operators(M);
@@ -771,7 +773,7 @@ void build_operators(Model& M) {
     for (int i = 0; i < 24; ++i)
         for (int j = 0; j < 24; ++j) KeT[i * 24 + j] = Ke[j * 24 + i];   // row = output DOF
     std::copy(KeT, KeT + KE, M.ke0_rows);
-    make_mat_coef(KeT, M.mc64, M.mc32);
+    M.coef64 = make_coef64(M.prm.youngs_modulus, M.prm.poisson_ratio, M.ele);
     make_stencil(KeT, M.coef);
     make_tc_coef(KeT, M.tcoef);
     for (int l = 0; l < L; ++l) {
@@ -910,12 +912,6 @@ void build_operators(Model& M) {
                                                                              lv.Ks32.as<float>());
                 GMGS_LAUNCHED(c);
             }
-            if (l < L - 1) {
-                lv.diag32 = dalloc(3 * lv.g.slots * sizeof(float));
-                k_to_float<<<blocks_for(c, 3 * lv.g.slots), 256, 0, c.stream>>>(3 * lv.g.slots, lv.diag64.as<double>(),
-                                                                                 lv.diag32.as<float>());
-                GMGS_LAUNCHED(c);
-            }
             if (l == 0 && lv.escale64.p) {
                 lv.escale32 = dalloc(lv.g.slots * sizeof(float));
                 k_to_float<<<blocks_for(c, lv.g.slots), 256, 0, c.stream>>>(lv.g.slots, lv.escale64.as<double>(),
@@ -926,6 +922,29 @@ void build_operators(Model& M) {
     }
     GMGS_CUDA(cudaStreamSynchronize(c.stream));
     c.trace_point("create: diagonals + FP32 copies");
+}
+
+// nodes of a uniform level that are neither interior nor on a stored matrix
+__global__ void k_boundary_count(int64_t n, const uint8_t* __restrict__ f, int32_t* __restrict__ cnt) {
+    GRID_STRIDE(i, n) cnt[i] = (f[i] & (NF_SOLID | NF_INTERIOR | NF_PEREL)) == NF_SOLID;
+}
+__global__ void k_boundary_list(int64_t n, const uint8_t* __restrict__ f, const int32_t* __restrict__ scan,
+                                int32_t* __restrict__ list) {
+    GRID_STRIDE(i, n) if ((f[i] & (NF_SOLID | NF_INTERIOR | NF_PEREL)) == NF_SOLID) list[scan[i]] = (int32_t)i;
+}
+void build_boundary_list(Model& M, int l) {
+    Ctx& c = M.ctx;
+    Level& lv = M.levels[l];
+    DevBuf cnt = dalloc(lv.g.slots * sizeof(int32_t));
+    k_boundary_count<<<blocks_for(c, lv.g.slots), 256, 0, c.stream>>>(lv.g.slots, lv.nflag.as<uint8_t>(), cnt.as<int32_t>());
+    GMGS_LAUNCHED(c);
+    const int64_t n = exclusive_scan(c, cnt.as<int32_t>(), lv.g.slots);
+    lv.bnd_nodes = dalloc(std::max<int64_t>(1, n) * sizeof(int32_t));
+    k_boundary_list<<<blocks_for(c, lv.g.slots), 256, 0, c.stream>>>(lv.g.slots, lv.nflag.as<uint8_t>(), cnt.as<int32_t>(),
+                                                                     lv.bnd_nodes.as<int32_t>());
+    GMGS_LAUNCHED(c);
+    GMGS_CUDA(cudaStreamSynchronize(c.stream));   // the counts go out of scope
+    lv.n_bnd = n;
 }
 
 void apply_bc(Model& M, const int32_t* fixed, int64_t nfixed, const double* loads, int64_t nload) {

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "fine.cuh"
+#include "fine64.cuh"
 #include "gmgs_internal.cuh"
 
 namespace gmgs {
@@ -22,19 +23,19 @@ struct Model {
     DevBuf ke0_dev;
     DevBuf galerkin_child; // 8 x 24x24: P_j^T Ke0 P_j per child position j
     bool lean_level1 = false; // level-2 (index 1) matrices kept in FP32 only (mixed precision + density)
-    MatCoef<double> mc64;  // Ke0 and the interior stencil of this handle's material and voxel
-    MatCoef<float> mc32;
+    Coef64 coef64{};       // factorised FP64 stencil of this handle's material and voxel
+    DevBuf mask_stencil;   // its 256 boundary stencils
     DevBuf rho;            // compact density (double), extension
     // boundary conditions and solution (finest level, FP64, 3 planes)
     DevBuf F, U;
-    double normF = 0;
     // coarsest level
     int nfree = 0;
     DevBuf free_idx, cvec_in, cvec_out;   // free DOF slots; coarse vectors (cb.nb * cb.B long)
     CoarseBlocks cb;
     // outer CG work vectors
-    DevBuf cg_x, cg_r, cg_p, cg_dx, cg_q64, cg_y64, cg_z64;   // FP64 path
-    DevBuf cg_q32, cg_y32, cg_z32, cg_r32;                     // mixed path
+    DevBuf cg_x, cg_r;                                         // mixed path: hi / lo parts; cg_r also FP64
+    DevBuf cg_rb, cg_p, cg_p2, cg_q64, cg_z64;                 // FP64 path (r and p double-buffered)
+    DevBuf cg_q32, cg_z32, cg_r32;                             // mixed path
     DevBuf cg_r32b, cg_pa, cg_pb;                              // mixed path double buffers
     Coef32 coef{};                                             // FP32 stencil + element matrix
     TcCoef tcoef{};                                            // Ke as the tensor cores' B operand
@@ -64,15 +65,12 @@ int64_t exclusive_scan(Ctx& c, int32_t* d, int64_t n);
 void element_stiffness(double E, double nu, const double ele[3], double Ke[KE]);
 // Isotropic Hooke coefficients (d11, d12, d44) and reciprocal element edges
 // (1/dx, 1/dy, 1/dz) for the stress kernels.
-template <typename T> inline const MatCoef<T>& mat_coef(const Model& M);
-template <> inline const MatCoef<double>& mat_coef<double>(const Model& M) { return M.mc64; }
-template <> inline const MatCoef<float>& mat_coef<float>(const Model& M) { return M.mc32; }
-
 void stress_coefficients(double E, double nu, const double ele[3], double c[6]);
 
 // setup.cu
 void build_levels(Model& M, const int32_t* occ_dev);
 void build_operators(Model& M);
+void build_boundary_list(Model& M, int l);
 void apply_bc(Model& M, const int32_t* fixed, int64_t nfixed, const double* loads, int64_t nload);
 // overlap: see factor_coarse
 void build_coarse_bc(Model& M, const std::function<void()>& overlap = {});
@@ -82,7 +80,7 @@ void set_density_dev(Model& M, const double* rho_dev);
 void alloc_work(Model& M);
 void reset_graphs(Model& M);   // destroy the captured PCG iteration graphs
 int pcg_solve(Model& M, const double* b_dense, double* x_dense, int32_t* iters, double* relres, double* hist);
-void vcycle_apply_fp64(Model& M, const double* r_dense, double* z_dense);
+void vcycle_apply(Model& M, const double* r_dense, double* z_dense);
 void apply_operator_dense(Model& M, int level, const double* x_dense, double* y_dense);
 
 // post.cu

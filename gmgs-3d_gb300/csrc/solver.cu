@@ -1,10 +1,10 @@
 // V-cycle preconditioner and the outer PCG (src/kernel/Vcycle.m:1-36,
 // src/kernel/CG_solver.m:1-56, src/kernel/JacobiSmoother.m:1-10).
 //
-// The FP64 path runs every vector and operator in double precision.  The
-// mixed path keeps x, r, p, the dot products and the coarsest solve in FP64
-// and runs the V-cycle (smoothers, transfers, level matvecs) in FP32; the
-// CG's own matvecs read FP64 vectors and compute in FP32.
+// The FP64 path runs every vector and operator in double precision on the
+// kernels of fine64.cu.  The mixed path keeps x and r as double-float vectors
+// and the coarsest solve in FP64 and runs everything else in FP32 on the
+// kernels of fine.cu.  Both fuse the vector updates into the operator.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -21,15 +21,42 @@ static void zalloc(Ctx& c, DevBuf& b, size_t bytes) {
     GMGS_CUDA(cudaMemsetAsync(b.p, 0, bytes, c.stream));
 }
 
-// level-0 matvec with optional event timing; algorithmic bytes: read x and
-// write y at every solid node, one mask byte per solid element and node
-template <typename Tc, typename Tin, typename Tout>
-static void fine_matvec(Model& M, const Tin* x, Tout* y) {
-    Level& l0 = M.levels[0];
-    const double bytes = (double)l0.n_node * (3.0 * sizeof(Tin) + 3.0 * sizeof(Tout) + 1.0) + (double)l0.n_elem;
-    M.ctx.mark(PK_FINE_MATVEC, false);
-    launch_matvec<Tc, Tin, Tout>(M.ctx, view<Tc>(l0, M.prm.omega), mat_coef<Tc>(M), x, y, l0.kscale);
-    M.ctx.mark(PK_FINE_MATVEC, true, bytes);
+// what the FP64 operator needs of a level beyond the hierarchy: the occupied
+// tiles and the list of its boundary nodes (an FP64 handle builds them with
+// its work buffers, a mixed one when an FP64 operator is first applied)
+static void prepare_fp64_level(Model& M, int l) {
+    Ctx& c = M.ctx;
+    Level& lv = M.levels[l];
+    if (!M.mask_stencil.p) {
+        M.mask_stencil = dalloc(256 * MASK_STENCIL * sizeof(double));
+        launch_mask_stencils(c, M.ke0_dev.as<double>(), M.mask_stencil.as<double>());
+    }
+    if (lv.n_bnd >= 0) return;
+    if (lv.tile_occ.bytes < tile_occ_bytes(lv.g)) lv.tile_occ = dalloc(tile_occ_bytes(lv.g));
+    launch_tile_occ(c, lv.g, lv.nflag.as<uint8_t>(), lv.tile_occ.as<uint8_t>());
+    if (l == 0 && lv.escale64.p) lv.n_bnd = 0;   // every node takes the scaled elements
+    else build_boundary_list(M, l);
+}
+
+static Level64 level64(const Model& M, const Level& lv) {
+    Level64 f;
+    f.g = lv.g;
+    f.emask = lv.emask.as<uint8_t>();
+    f.nflag = lv.nflag.as<uint8_t>();
+    f.tile_occ = lv.tile_occ.as<uint8_t>();
+    f.etype = lv.etype.as<int32_t>();
+    f.Ks = lv.Ks64.as<double>();
+    f.nK = lv.Ks64.p ? lv.nK : 0;
+    f.ke0 = M.ke0_dev.as<double>();
+    f.kscale = lv.kscale;
+    f.escale = lv.escale64.as<double>();
+    f.mask_stencil = M.mask_stencil.as<double>();
+    f.bnd = lv.bnd_nodes.as<int32_t>();
+    f.n_bnd = (int)lv.n_bnd;
+    f.perel = lv.perel_nodes.as<int32_t>();
+    f.n_perel = (int)lv.n_perel;
+    f.n_node = lv.n_node;
+    return f;
 }
 
 void alloc_work(Model& M) {
@@ -42,12 +69,13 @@ void alloc_work(Model& M) {
         Level& lv = M.levels[l];
         const size_t n3 = 3 * (size_t)lv.g.slots;
         if (l > 0) zalloc(c, lv.vr, n3 * T);
-        if (l > 0 || !mixed) zalloc(c, lv.vx, n3 * T);
+        if (l > 0) zalloc(c, lv.vx, n3 * T);
+        if (!mixed) prepare_fp64_level(M, l);
         if (l < L - 1) {
             zalloc(c, lv.vrp, n3 * T);
             if (!mixed) {
-                zalloc(c, lv.vdx, n3 * T);
-                zalloc(c, lv.vy, n3 * T);
+                if (lv.wdinv64.bytes < n3 * 8) lv.wdinv64 = dalloc(n3 * 8);
+                launch_wdinv64(c, (int64_t)n3, lv.diag64.as<double>(), M.prm.omega, lv.wdinv64.as<double>());
             } else {
                 if (lv.wdinv32.bytes < n3 * 4) lv.wdinv32 = dalloc(n3 * 4);
                 launch_wdinv(c, (int64_t)n3, lv.diag64.as<double>(), M.prm.omega, lv.wdinv32.as<float>());
@@ -61,9 +89,9 @@ void alloc_work(Model& M) {
         }
     }
     const size_t n3 = 3 * (size_t)M.levels[0].g.slots;
-    zalloc(c, M.cg_x, n3 * 8);
     zalloc(c, M.cg_r, n3 * 8);
     if (mixed) {
+        zalloc(c, M.cg_x, n3 * 8);
         zalloc(c, M.cg_r32b, n3 * 4);
         zalloc(c, M.cg_pa, n3 * 4);
         zalloc(c, M.cg_pb, n3 * 4);
@@ -71,16 +99,18 @@ void alloc_work(Model& M) {
         zalloc(c, M.cg_z32, n3 * 4);
         zalloc(c, M.cg_r32, n3 * 4);
     } else {
+        zalloc(c, M.cg_rb, n3 * 8);
         zalloc(c, M.cg_p, n3 * 8);
-        zalloc(c, M.cg_dx, n3 * 8);
+        zalloc(c, M.cg_p2, n3 * 8);
         zalloc(c, M.cg_q64, n3 * 8);
-        zalloc(c, M.cg_y64, n3 * 8);
         zalloc(c, M.cg_z64, n3 * 8);
     }
     zalloc(c, M.scal, SC_N * sizeof(double));
     if (mixed) zalloc(c, M.tc_err, sizeof(int));
     M.dot_blocks = M.ctx.num_sms * 4;
-    const int maxb = std::max({M.dot_blocks, fine_grid_blocks(M.levels[0].g), up32_grid_blocks(M.levels[0].g)});
+    const Level& l0 = M.levels[0];
+    const int maxb = mixed ? std::max({M.dot_blocks, fine_grid_blocks(l0.g), up32_grid_blocks(l0.g)})
+                           : std::max(M.dot_blocks, dot64_blocks(l0.g, l0.n_bnd + l0.n_perel));
     zalloc(c, M.dot_partials, (size_t)maxb * sizeof(double));
     zalloc(c, M.dot_ticket, sizeof(unsigned int));
     if (!M.scal_host) GMGS_CUDA(cudaMallocHost(&M.scal_host, SC_N * sizeof(double)));
@@ -112,37 +142,44 @@ static void check_tc(Model& M) {
     }
 }
 
-// One V(1,1) cycle, Vcycle.m:1-36: down-sweep Jacobi with residual update and
-// restriction, coarsest direct solve, up-sweep prolongation + Jacobi with the
-// pre-smoothing residual, fixed DOFs of the finest level zeroed.
-template <typename T>
-static void vcycle(Model& M, const T* r0, T* z) {
+static DotOut64 dot_out64(Model& M, int slot) {
+    DotOut64 d;
+    d.partials = M.dot_partials.as<double>();
+    d.ticket = M.dot_ticket.as<unsigned int>();
+    d.out = M.scal.as<double>() + slot;
+    return d;
+}
+
+// One V(1,1) cycle in FP64, Vcycle.m:1-36: down-sweep Jacobi with residual
+// update and restriction, coarsest direct solve, up-sweep prolongation +
+// Jacobi with the pre-smoothing residual, fixed DOFs of the finest level
+// zeroed.  The finest up-sweep also accumulates r . z into scal[dot_slot].
+static void vcycle64(Model& M, const double* r0, double* z, bool with_dot, int dot_slot) {
     Ctx& c = M.ctx;
     c.mark(PK_VCYCLE, false);
     const int L = M.num_levels;
-    const double om = M.prm.omega;
     for (int l = 0; l < L - 1; ++l) {
         Level& lv = M.levels[l];
         Level& lc = M.levels[l + 1];
-        const T* r = l == 0 ? r0 : lv.vr.as<T>();
-        const LevelView<T> v = view<T>(lv, om);
-        const int64_t n3 = 3 * lv.g.slots;
-        launch_jacobi_dx<T, T, T>(c, lv.g, v.diag, om, r, lv.vdx.as<T>());
-        if (l == 0) fine_matvec<T, T, T>(M, lv.vdx.as<T>(), lv.vy.as<T>());
-        else launch_matvec<T, T, T>(c, v, mat_coef<T>(M), lv.vdx.as<T>(), lv.vy.as<T>(), lv.kscale);
-        launch_diff<T>(c, n3, lv.vrp.as<T>(), r, lv.vy.as<T>());
-        launch_restrict<T>(c, lv.g, lc.g, lc.nflag.as<uint8_t>(), lv.vrp.as<T>(), lc.vr.as<T>());
+        Args64 a;
+        a.r = l == 0 ? r0 : lv.vr.as<double>();
+        a.w = lv.wdinv64.as<double>();
+        a.out = lv.vrp.as<double>();
+        if (l == 0) c.mark(PK_FINE_MATVEC, false);
+        launch_fine64<M64_VCYCLE_DOWN>(c, level64(M, lv), M.coef64, a);
+        if (l == 0) c.mark(PK_FINE_MATVEC, true, (double)lv.n_node * 3 * 24 + (double)lv.n_elem);
+        launch_restrict<double>(c, lv.g, lc.g, lc.nflag.as<uint8_t>(), lv.vrp.as<double>(), lc.vr.as<double>());
     }
     Level& lc = M.levels[L - 1];
-    launch_gather<T>(c, M.nfree, M.free_idx.as<int32_t>(), lc.vr.as<T>(), M.cvec_in.as<double>());
+    launch_gather<double>(c, M.nfree, M.free_idx.as<int32_t>(), lc.vr.as<double>(), M.cvec_in.as<double>());
     launch_coarse_solve(c, M.cb, M.cvec_in.as<double>(), M.cvec_out.as<double>());
-    launch_scatter<T>(c, M.nfree, M.free_idx.as<int32_t>(), M.cvec_out.as<double>(), lc.vx.as<T>());
+    launch_scatter<double>(c, M.nfree, M.free_idx.as<int32_t>(), M.cvec_out.as<double>(), lc.vx.as<double>());
     for (int l = L - 2; l >= 0; --l) {
         Level& lv = M.levels[l];
-        T* out = l == 0 ? z : lv.vx.as<T>();
-        const LevelView<T> v = view<T>(lv, om);
-        launch_prolong_post<T>(c, lv.g, M.levels[l + 1].g, lv.nflag.as<uint8_t>(), v.diag, om,
-                               M.levels[l + 1].vx.as<T>(), lv.vdx.as<T>(), lv.vrp.as<T>(), out, l == 0);
+        const DotOut64 d = dot_out64(M, dot_slot);
+        launch_up64(c, lv.g, M.levels[l + 1].g, lv.nflag.as<uint8_t>(), lv.tile_occ.as<uint8_t>(), lv.wdinv64.as<double>(),
+                    l == 0 ? r0 : lv.vr.as<double>(), lv.vrp.as<double>(), M.levels[l + 1].vx.as<double>(),
+                    l == 0 ? z : lv.vx.as<double>(), l == 0, (l == 0 && with_dot) ? &d : nullptr);
     }
     c.mark(PK_VCYCLE, true);
 }
@@ -158,15 +195,16 @@ void vcycle_apply(Model& M, const double* r, double* z) {
         launch_copy<double, float>(M.ctx, n3, z, M.cg_z32.as<float>());
         check_tc(M);
     } else {
-        vcycle<double>(M, r, z);
+        vcycle64(M, r, z, false, 0);
     }
 }
 
-void vcycle_apply_fp64(Model& M, const double* r, double* z) { vcycle_apply(M, r, z); }
-
 void apply_operator_dense(Model& M, int level, const double* x, double* y) {
-    Level& lv = M.levels[level];
-    launch_matvec<double, double, double>(M.ctx, view<double>(lv, M.prm.omega), M.mc64, x, y, lv.kscale);
+    prepare_fp64_level(M, level);
+    Args64 a;
+    a.v = x;
+    a.out = y;
+    launch_fine64<M64_PLAIN>(M.ctx, level64(M, M.levels[level]), M.coef64, a);
 }
 
 
@@ -478,23 +516,25 @@ static int pcg_mixed(Model& M, const double* b, double* x, int32_t* iters_out, d
 }
 
 // CG_solver.m:1-56 with the Jacobi step before each preconditioner call.
-int pcg_solve(Model& M, const double* b, double* x, int32_t* iters_out, double* relres_out, double* hist) {
-    if (M.prm.precision == GMGS_MIXED) return pcg_mixed(M, b, x, iters_out, relres_out, hist);
+static int pcg_fp64(Model& M, const double* b, double* x, int32_t* iters_out, double* relres_out, double* hist) {
     Ctx& c = M.ctx;
     Level& l0 = M.levels[0];
     const int64_t n3 = 3 * l0.g.slots;
-    const bool mixed = M.prm.precision == GMGS_MIXED;
-    const double om = M.prm.omega;
     double* scal = M.scal.as<double>();
     const DotScratch ds = dots(M);
-    double* r = M.cg_r.as<double>();
-    double* p = M.cg_p.as<double>();
-    double* dx = M.cg_dx.as<double>();
+    const double* r = b;                      // r = b - A*0; then alternately in the two buffers
+    double* rbuf[2] = {M.cg_r.as<double>(), M.cg_rb.as<double>()};
+    int rnext = 0;
+    double* pa = M.cg_p.as<double>();
+    double* pb = M.cg_p2.as<double>();
+    double* q = M.cg_q64.as<double>();
+    double* z = M.cg_z64.as<double>();
+    const double* w = l0.wdinv64.as<double>();
+    const Level64 f0 = level64(M, l0);
 
     launch_dot<double, double>(c, ds, n3, b, b, scal + SC_BB);
     GMGS_CUDA(cudaMemcpyAsync(M.scal_host + SC_BB, scal + SC_BB, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
     GMGS_CUDA(cudaMemsetAsync(x, 0, n3 * sizeof(double), c.stream));
-    GMGS_CUDA(cudaMemcpyAsync(r, b, n3 * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));  // r = b - A*0
     GMGS_CUDA(cudaStreamSynchronize(c.stream));
     const double normB = std::sqrt(M.scal_host[SC_BB]);
     if (normB == 0.0) {
@@ -506,44 +546,62 @@ int pcg_solve(Model& M, const double* b, double* x, int32_t* iters_out, double* 
         return GMGS_OK;
     }
     if (!std::isfinite(normB)) throw Error(GMGS_ERR_NONFINITE, "non-finite load vector");
+    // algorithmic bytes per node: r read and written, x read and written, q, p, w; z, p read, p, q written
+    const double jbytes = (double)l0.n_node * 3 * 8 * 7 + 2.0 * (double)l0.n_node;
+    const double pbytes = (double)l0.n_node * 3 * 8 * 4 + 2.0 * (double)l0.n_node;
+    const double* r_read = b;
+    // the previous iteration's update and the next iteration's Jacobi step in
+    // one pass, as in the mixed path
+    auto update_jacobi = [&](int first, int cur) {
+        Args64 a;
+        a.r = r;
+        a.w = w;
+        a.q = q;
+        a.pold = pa;
+        a.x = x;
+        a.out = rbuf[rnext];
+        a.scal = scal;
+        a.cur = cur;
+        a.first = first;
+        a.dot = dot_out64(M, SC_RR);
+        c.mark(PK_FINE_MATVEC, false);
+        c.mark(PK_UPDATE_JACOBI, false);
+        launch_fine64<M64_CG_UPDATE_JACOBI>(c, f0, M.coef64, a);
+        c.mark(PK_FINE_MATVEC, true, jbytes);
+        c.mark(PK_UPDATE_JACOBI, true, jbytes);
+        r_read = r;
+        r = rbuf[rnext];
+        rnext ^= 1;
+    };
 
     const auto t0 = std::chrono::steady_clock::now();
-    int its = 0;
+    int its = 0, nhist = 0;
     double resnorm = INFINITY;
     int status = GMGS_ERR_MAX_ITERATIONS;
-    const int max_it = M.prm.max_it;
-    int nhist = 0;
-    while (its <= max_it) {
+    update_jacobi(1, 0);          // [x, r1] = JacobiSmoother(var) of the first iteration (CG_solver.m:18-19)
+    while (its <= M.prm.max_it) {
         c.mark(PK_CG_ITER, false);
-        // [x, r1] = JacobiSmoother(var)   (CG_solver.m:18-19)
-        launch_jacobi_dx<double, double, double>(c, l0.g, l0.diag64.as<double>(), om, r, dx);
-        launch_add<double, double>(c, n3, x, dx);
-        if (mixed) {
-            fine_matvec<float, double, float>(M, dx, M.cg_y32.as<float>());
-            launch_sub<double, float>(c, n3, r, M.cg_y32.as<float>());
-            launch_copy<float, double>(c, n3, M.cg_r32.as<float>(), r);
-            vcycle<float>(M, M.cg_r32.as<float>(), M.cg_z32.as<float>());
-        } else {
-            fine_matvec<double, double, double>(M, dx, M.cg_y64.as<double>());
-            launch_sub<double, double>(c, n3, r, M.cg_y64.as<double>());
-            vcycle<double>(M, r, M.cg_z64.as<double>());
-        }
         ++its;
         const int cur = its & 1;
-        if (mixed) {
-            launch_dot<double, float>(c, ds, n3, r, M.cg_z32.as<float>(), scal + cur);
-            launch_p_update<float>(c, n3, M.cg_z32.as<float>(), p, scal, cur | ((its == 1) << 1));
-            fine_matvec<float, double, float>(M, p, M.cg_q32.as<float>());
-            launch_dot<double, float>(c, ds, n3, p, M.cg_q32.as<float>(), scal + SC_PQ);
-            launch_xr_update<float>(c, n3, x, r, p, M.cg_q32.as<float>(), scal, cur);
-        } else {
-            launch_dot<double, double>(c, ds, n3, r, M.cg_z64.as<double>(), scal + cur);
-            launch_p_update<double>(c, n3, M.cg_z64.as<double>(), p, scal, cur | ((its == 1) << 1));
-            fine_matvec<double, double, double>(M, p, M.cg_q64.as<double>());
-            launch_dot<double, double>(c, ds, n3, p, M.cg_q64.as<double>(), scal + SC_PQ);
-            launch_xr_update<double>(c, n3, x, r, p, M.cg_q64.as<double>(), scal, cur);
+        vcycle64(M, r, z, true, cur);      // z2 = PtV(r1), r1'z2   (CG_solver.m:21,26)
+        {   // p2 = z2 + beta p1; q = A p2; p2'q   (CG_solver.m:23-31)
+            Args64 a;
+            a.z = z;
+            a.pold = pa;
+            a.pout = pb;
+            a.out = q;
+            a.scal = scal;
+            a.cur = cur;
+            a.first = its == 1;
+            a.dot = dot_out64(M, SC_PQ);
+            c.mark(PK_FINE_MATVEC, false);
+            c.mark(PK_DIRECTION, false);
+            launch_fine64<M64_CG_DIRECTION>(c, f0, M.coef64, a);
+            c.mark(PK_FINE_MATVEC, true, pbytes);
+            c.mark(PK_DIRECTION, true, pbytes);
+            std::swap(pa, pb);
         }
-        launch_dot<double, double>(c, ds, n3, r, r, scal + SC_RR);
+        update_jacobi(0, cur);    // x += alpha p2; r2 = r1 - alpha q; |r2|; next Jacobi step
         c.mark(PK_CG_ITER, true);
         GMGS_CUDA(cudaMemcpyAsync(M.scal_host + SC_RR, scal + SC_RR, sizeof(double), cudaMemcpyDeviceToHost,
                                   c.stream));
@@ -569,13 +627,19 @@ int pcg_solve(Model& M, const double* b, double* x, int32_t* iters_out, double* 
         }
         ++nhist;
     }
-    if (status == GMGS_ERR_MAX_ITERATIONS && M.prm.verbose)
-        std::printf("Exceed the maximum iterate numbers\n");
+    launch_drop_last_dx64(c, n3, x, r_read, q, w, scal, its & 1);
+    GMGS_CUDA(cudaStreamSynchronize(c.stream));
+    if (status == GMGS_ERR_MAX_ITERATIONS && M.prm.verbose) std::printf("Exceed the maximum iterate numbers\n");
     if (iters_out) *iters_out = its;
     if (relres_out) *relres_out = resnorm;
     M.last_iters = its;
     M.last_relres = resnorm;
     return status;
+}
+
+int pcg_solve(Model& M, const double* b, double* x, int32_t* iters_out, double* relres_out, double* hist) {
+    return M.prm.precision == GMGS_MIXED ? pcg_mixed(M, b, x, iters_out, relres_out, hist)
+                                         : pcg_fp64(M, b, x, iters_out, relres_out, hist);
 }
 
 }  // namespace gmgs
