@@ -16,328 +16,369 @@
 //     x_i = D_i^-1 c_i for every block (D = S, T or M)
 //     x_i -= G_(i+1)^T x_(i+1) (i = k-1..0),  x_i -= H_(i-1)^T x_(i-1) (i = k+1..nb-1)
 // so both sequential sweeps run as two independent chains of about nb/2
-// steps, and the two halves of the factorisation run on two streams.  The
-// factors take 2 nb B^2 doubles (the D_i^-1 and the couplings G_i / H_i)
-// instead of the n^2 of a dense inverse factor.  Each D_i^-1 comes from a
-// recursive blocked Cholesky that also forms L^-1 (no pivoting: every D_i is
-// SPD), then D^-1 = L^-T L^-1.
+// steps, and the two halves of the factorisation run on two streams.
 //
-// Everything runs in FP64 in this file's own kernels, launched in stream
-// order: a tiled DGEMM with triangle-aware k-ranges, a one-CTA Cholesky +
-// inverse of 32 x 32 diagonal tiles, and block matrix-vector products whose
-// last CTA per output block (arrival ticket, no spinning) sums the
-// reduction-tile partial sums in a fixed order.
+// Everything runs in FP64 (about 2 lanes per clock per SM on GB300), so the
+// factorisation is organised to do few operations on many SMs:
+//   - each D_i^-1 by symmetric block sweeps (Gauss-Jordan on the lower
+//     triangle, 32 pivots at a time, no pivoting: every D_i is SPD), B^3 / 2
+//     multiply-adds in B/32 pairs of launches.  A recursive Cholesky with the
+//     inverse factor and L^-T L^-1 took B^3 and spent 43 us in each of its
+//     B/32 single-CTA leaves: 1.45 ms per block of order 448
+//   - the couplings A_(i,i-1) hold about 20 non-zeros per row (27-point
+//     coupling), so the products with them are sparse: 5 % of the dense ones'
+//     operations (172 and 118 us per block)
+// Measured for 15 blocks of order 448: factorisation 14 -> 5 ms, solve 15
+// launches of a 64 x 64-tile product with partial sums and arrival counters
+// (about 8 us each in the stream) -> 15 launches of a warp per row.
+// The errors of the solve are the same (5.9e-15 for both on a 6315-DOF
+// coarsest level, 1.5e-10 against 2.2e-10 on a long column of condition 2e7).
 #include "setup.cuh"
 
 namespace gmgs {
 
 namespace {
 
-constexpr int GT = 16;       // DGEMM output tile (one output per thread)
-constexpr int MT = 64;       // block matrix-vector tile
+constexpr int PB = 32;       // pivots per sweep
+constexpr int PR = 16;       // rows per panel CTA
 
-enum : int { TRI_A_LOWER = 1, TRI_A_UPPER = 2, TRI_B_LOWER = 4, TRI_B_UPPER = 8 };
-
-// C = alpha op(A) op(B) + beta C, column-major, m, n, k multiples of 16.
-// TRI marks operands known to be triangular so the k-loop skips their zero
-// tiles (the skipped products are exact zeros); LOWER_OUT skips output tiles
-// strictly above the diagonal (their values are never read).
-template <bool TA, bool TB, int TRI, bool LOWER_OUT>
-__global__ void __launch_bounds__(256) k_dgemm(int k, double alpha, const double* __restrict__ A, int lda,
-                                               const double* __restrict__ B, int ldb, double beta,
-                                               double* __restrict__ C, int ldc) {
-    const int r0 = blockIdx.x * GT, c0 = blockIdx.y * GT;
-    if (LOWER_OUT && r0 + GT <= c0) return;
-    __shared__ double As[GT][GT + 1];   // As[l][i] = op(A)(r0 + i, k0 + l)
-    __shared__ double Bs[GT][GT + 1];   // Bs[l][j] = op(B)(k0 + l, c0 + j)
-    const int tx = threadIdx.x & (GT - 1), ty = threadIdx.x / GT;
-    int kb = 0, ke = k;
-    if (TRI & TRI_A_LOWER) ke = min(ke, r0 + GT);
-    if (TRI & TRI_A_UPPER) kb = max(kb, r0);
-    if (TRI & TRI_B_LOWER) kb = max(kb, c0);
-    if (TRI & TRI_B_UPPER) ke = min(ke, c0 + GT);
-    double acc = 0.0;
-    for (int k0 = kb; k0 < ke; k0 += GT) {
-        if (!TA) As[ty][tx] = A[(int64_t)(k0 + ty) * lda + r0 + tx];
-        else     As[tx][ty] = A[(int64_t)(r0 + ty) * lda + k0 + tx];
-        if (!TB) Bs[tx][ty] = B[(int64_t)(c0 + ty) * ldb + k0 + tx];
-        else     Bs[ty][tx] = B[(int64_t)(k0 + ty) * ldb + c0 + tx];
-        __syncthreads();
-#pragma unroll
-        for (int l = 0; l < GT; ++l) acc = fma(As[l][tx], Bs[l][ty], acc);
-        __syncthreads();
+// Inverse P of the 32 x 32 pivot block and W = C P for 16 rows of the panel C
+// (the pivot columns of the symmetric matrix, of which D holds the lower
+// triangle).  Every CTA inverts the pivot block for itself: the 32 scalar
+// sweeps are a dependent chain, so sharing one inverse would only add a launch
+// between it and the panel.  Elements of the lower triangle stay in registers,
+// the current pivot column goes through shared memory, one barrier per sweep.
+// A pivot that is not positive sets *info and is replaced by 1 so the
+// arithmetic stays finite.
+__global__ void __launch_bounds__(256) k_sweep_panel(int B, const double* __restrict__ D, int k0, double* __restrict__ W,
+                                                     double* __restrict__ C, double* __restrict__ P, int* __restrict__ info) {
+    __shared__ double col[2][PB], rp[2];
+    __shared__ double Ps[PB][PB + 1], Cs[PR][PB + 1];
+    const int t = threadIdx.x;
+    constexpr int NL = PB * (PB + 1) / 2, NQ = (NL + 255) / 256;
+    const int r0 = blockIdx.x * PR;
+    const bool pivot_rows = r0 >= k0 && r0 < k0 + PB;
+    if (!pivot_rows) {
+        for (int e = t; e < PR * PB; e += 256) {
+            // above the pivot block the column is held as a row of the lower triangle
+            const int rr = r0 > k0 ? e % PR : e / PB, c = r0 > k0 ? e / PR : e % PB;
+            Cs[rr][c] = r0 > k0 ? D[(int64_t)(k0 + c) * B + r0 + rr] : D[(int64_t)(r0 + rr) * B + k0 + c];
+        }
     }
-    double* cp = C + (int64_t)(c0 + ty) * ldc + r0 + tx;
-    *cp = beta == 0.0 ? alpha * acc : fma(alpha, acc, beta * *cp);
+    int ei[NQ], ej[NQ];
+    double a[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const int e = t + 256 * q;
+        int i = (int)((sqrtf(8.f * (float)e + 1.f) - 1.f) * 0.5f);
+        while ((i + 1) * (i + 2) / 2 <= e) ++i;
+        while (i * (i + 1) / 2 > e) --i;
+        ei[q] = e < NL ? i : -1;
+        ej[q] = e < NL ? e - i * (i + 1) / 2 : -1;
+        a[q] = e < NL ? D[(int64_t)(k0 + ej[q]) * B + k0 + i] : 0.0;
+    }
+    auto publish = [&](int s) {     // the pivot column of sweep s and its reciprocal
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            if (ei[q] == s || ej[q] == s) col[s & 1][ei[q] == s ? ej[q] : ei[q]] = a[q];
+            if (ei[q] == s && ej[q] == s) {
+                const bool ok = a[q] > 0.0 && a[q] < INFINITY;
+                if (!ok) atomicExch(info, 1);
+                rp[s & 1] = ok ? 1.0 / a[q] : 1.0;
+            }
+        }
+    };
+    publish(0);
+#pragma unroll 1
+    for (int s = 0; s < PB; ++s) {
+        __syncthreads();
+        const double* c = col[s & 1];
+        const double r = rp[s & 1];
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const int i = ei[q], j = ej[q];
+            if (i < 0) continue;
+            if (i == s || j == s) a[q] = i == j ? -r : c[i == s ? j : i] * r;
+            else a[q] = fma(-(c[i] * r), c[j], a[q]);
+        }
+        if (s + 1 < PB) publish(s + 1);
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        if (ei[q] < 0) continue;
+        Ps[ei[q]][ej[q]] = -a[q];
+        Ps[ej[q]][ei[q]] = -a[q];
+    }
+    __syncthreads();
+    if (pivot_rows) {
+        for (int e = t; e < PR * PB; e += 256) P[(e % PR + r0 - k0) * PB + e / PR] = Ps[e % PR + r0 - k0][e / PR];
+        return;
+    }
+#pragma unroll
+    for (int q = 0; q < PR * PB / 256; ++q) {
+        const int rr = t % PR, c = t / PR + q * (256 / PR);
+        double w0 = 0.0, w1 = 0.0;
+#pragma unroll 8
+        for (int m = 0; m < PB; m += 2) {
+            w0 = fma(Cs[rr][m], Ps[m][c], w0);
+            w1 = fma(Cs[rr][m + 1], Ps[m + 1][c], w1);
+        }
+        W[(int64_t)c * B + r0 + rr] = w0 + w1;
+        C[(int64_t)c * B + r0 + rr] = Cs[rr][c];
+    }
 }
 
-enum class Op { N, T };
+// The sweep's update of one 32 x 32 tile of the lower triangle: A_ij -= W_i
+// C_j^T off the pivots, A_ik = W_i, A_kk = -P.  After the last pivots the
+// matrix is -D^-1: that launch changes the sign and fills both triangles.
+__global__ void __launch_bounds__(256) k_sweep_update(int B, double* __restrict__ D, int k0, const double* __restrict__ W,
+                                                      const double* __restrict__ C, const double* __restrict__ P, int last) {
+    __shared__ double Ws[PB][PB + 1], Cs[PB][PB + 1];   // [pivot][row], [pivot][column]
+    int ti = (int)((sqrtf(8.f * (float)blockIdx.x + 1.f) - 1.f) * 0.5f);
+    while ((ti + 1) * (ti + 2) / 2 <= (int)blockIdx.x) ++ti;
+    while (ti * (ti + 1) / 2 > (int)blockIdx.x) --ti;
+    const int tj = (int)blockIdx.x - ti * (ti + 1) / 2, kt = k0 / PB;
+    const int t = threadIdx.x, x = t & 15, y = t >> 4, ri = ti * PB, cj = tj * PB;
+    double v[2][2];
+    if (ti == kt || tj == kt) {
+#pragma unroll
+        for (int p = 0; p < 2; ++p)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int r = x + 16 * p, c = y + 16 * q;
+                v[p][q] = ti == tj ? -P[r * PB + c] : (tj == kt ? W[(int64_t)c * B + ri + r] : W[(int64_t)r * B + cj + c]);
+            }
+    } else {
+#pragma unroll
+        for (int q = 0; q < PB * PB / 256; ++q) {
+            const int e = t + q * 256, m = e / PB, r = e % PB;
+            Ws[m][r] = W[(int64_t)m * B + ri + r];
+            Cs[m][r] = C[(int64_t)m * B + cj + r];
+        }
+#pragma unroll
+        for (int p = 0; p < 2; ++p)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) v[p][q] = D[(int64_t)(cj + y + 16 * q) * B + ri + x + 16 * p];
+        __syncthreads();
+#pragma unroll 8
+        for (int m = 0; m < PB; ++m) {
+            const double w0 = Ws[m][x], w1 = Ws[m][x + 16], c0 = Cs[m][y], c1 = Cs[m][y + 16];
+            v[0][0] = fma(-w0, c0, v[0][0]);
+            v[1][0] = fma(-w1, c0, v[1][0]);
+            v[0][1] = fma(-w0, c1, v[0][1]);
+            v[1][1] = fma(-w1, c1, v[1][1]);
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int r = ri + x + 16 * p, c = cj + y + 16 * q;
+            if (!last) {
+                D[(int64_t)c * B + r] = v[p][q];
+            } else if (ti != tj || r >= c) {        // a diagonal tile's lower half, mirrored
+                D[(int64_t)c * B + r] = -v[p][q];
+                D[(int64_t)r * B + c] = -v[p][q];
+            }
+        }
+}
 
-struct Gemm {
-    Op ta = Op::N, tb = Op::N;
-    int tri = 0;
-    bool lower_out = false;
+// The non-zeros E'(row, c0 .. c0 + 255) of one row of E' (E, or its transpose)
+// into shared memory in column order; returns their number.  E column-major.
+__device__ __forceinline__ int row_nonzeros(int B, const double* __restrict__ E, bool trans, int row, int c0, double* val,
+                                            int* idx, int* cnt) {
+    const int t = threadIdx.x, c = c0 + t;
+    double v = 0.0;
+    if (c < B) v = trans ? E[(int64_t)row * B + c] : E[(int64_t)c * B + row];
+    const unsigned m = __ballot_sync(0xffffffffu, v != 0.0);
+    __syncthreads();                                  // the previous chunk's readers are done
+    if ((t & 31) == 0) cnt[t >> 5] = __popc(m);
+    __syncthreads();
+    int at = 0, n = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+        if (w == (t >> 5)) at = n;
+        n += cnt[w];
+    }
+    if (v != 0.0) {
+        at += __popc(m & ((1u << (t & 31)) - 1u));
+        val[at] = v;
+        idx[at] = c;
+    }
+    __syncthreads();
+    return n;
+}
+
+// G = E' X with X symmetric (both triangles): one CTA per row and 256 columns;
+// G row-major to gt, column-major to gc
+__global__ void __launch_bounds__(256) k_sparse_left(int B, const double* __restrict__ E, int trans, const double* __restrict__ X,
+                                                     double* __restrict__ gt, double* __restrict__ gc) {
+    __shared__ double val[256];
+    __shared__ int idx[256], cnt[8];
+    const int row = blockIdx.x, j = blockIdx.y * 256 + threadIdx.x;
+    double acc = 0.0;
+    for (int c0 = 0; c0 < B; c0 += 256) {
+        const int n = row_nonzeros(B, E, trans != 0, row, c0, val, idx, cnt);
+        if (j < B)
+            for (int q = 0; q < n; ++q) acc = fma(val[q], X[(int64_t)idx[q] * B + j], acc);
+    }
+    if (j < B) {
+        gt[(int64_t)row * B + j] = acc;
+        gc[(int64_t)j * B + row] = acc;
+    }
+}
+
+// D -= G E'^T on the lower triangle, G column-major: one CTA per column of D
+// and 256 rows
+__global__ void __launch_bounds__(256) k_sparse_update(int B, const double* __restrict__ E, int trans,
+                                                       const double* __restrict__ gc, double* __restrict__ D) {
+    __shared__ double val[256];
+    __shared__ int idx[256], cnt[8];
+    const int j = blockIdx.x, i = blockIdx.y * 256 + threadIdx.x;
+    if ((int)blockIdx.y * 256 + 255 < j) return;      // above the diagonal, uniform across the CTA
+    double acc = 0.0;
+    for (int c0 = 0; c0 < B; c0 += 256) {
+        const int n = row_nonzeros(B, E, trans != 0, j, c0, val, idx, cnt);
+        if (i < B)
+            for (int q = 0; q < n; ++q) acc = fma(val[q], gc[(int64_t)idx[q] * B + i], acc);
+    }
+    if (i < B && i >= j) D[(int64_t)j * B + i] -= acc;
+}
+
+// scratch of one chain of the factorisation
+struct Chain {
+    DevBuf w, c, p, g;      // panels W and C (32 x B), pivot inverse, G column-major
+    void alloc(int B) {
+        w = dalloc((size_t)PB * B * sizeof(double));
+        c = dalloc((size_t)PB * B * sizeof(double));
+        p = dalloc((size_t)PB * PB * sizeof(double));
+        g = dalloc((size_t)B * B * sizeof(double));
+    }
 };
 
-template <bool TA, bool TB, int TRI, bool LO>
-void run_gemm(Ctx& c, int m, int n, int k, double alpha, const double* A, int lda, const double* B, int ldb,
-              double beta, double* C, int ldc) {
-    const dim3 grid(m / GT, n / GT);
-    k_dgemm<TA, TB, TRI, LO><<<grid, GT * GT, 0, c.stream>>>(k, alpha, A, lda, B, ldb, beta, C, ldc);
+// D^-1 of the SPD block D (lower triangle in, both triangles out)
+void inv_spd(Ctx& c, double* D, int B, Chain& s, int* info) {
+    const int tiles = B / PB;
+    for (int k0 = 0; k0 < B; k0 += PB) {
+        k_sweep_panel<<<B / PR, 256, 0, c.stream>>>(B, D, k0, s.w.as<double>(), s.c.as<double>(), s.p.as<double>(), info);
+        GMGS_LAUNCHED(c);
+        k_sweep_update<<<tiles * (tiles + 1) / 2, 256, 0, c.stream>>>(B, D, k0, s.w.as<double>(), s.c.as<double>(),
+                                                                      s.p.as<double>(), k0 + PB == B);
+        GMGS_LAUNCHED(c);
+    }
+}
+void sparse_left(Ctx& c, int B, const double* E, bool trans, const double* X, double* gt, double* gc) {
+    k_sparse_left<<<dim3(B, (B + 255) / 256), 256, 0, c.stream>>>(B, E, trans, X, gt, gc);
+    GMGS_LAUNCHED(c);
+}
+void sparse_update(Ctx& c, int B, const double* E, bool trans, const double* gc, double* D) {
+    k_sparse_update<<<dim3(B, (B + 255) / 256), 256, 0, c.stream>>>(B, E, trans, gc, D);
     GMGS_LAUNCHED(c);
 }
 
-// the operand forms the factorisation uses
-void gemm(Ctx& c, const Gemm& g, int m, int n, int k, double alpha, const double* A, int lda, const double* B,
-          int ldb, double beta, double* C, int ldc) {
-    if (m <= 0 || n <= 0) return;
-    if (g.ta == Op::N && g.tb == Op::T && g.tri == TRI_B_UPPER && !g.lower_out)
-        run_gemm<false, true, TRI_B_UPPER, false>(c, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
-    else if (g.ta == Op::N && g.tb == Op::T && g.tri == 0 && g.lower_out)
-        run_gemm<false, true, 0, true>(c, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
-    else if (g.ta == Op::N && g.tb == Op::N && g.tri == TRI_B_LOWER && !g.lower_out)
-        run_gemm<false, false, TRI_B_LOWER, false>(c, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
-    else if (g.ta == Op::N && g.tb == Op::N && g.tri == TRI_A_LOWER && !g.lower_out)
-        run_gemm<false, false, TRI_A_LOWER, false>(c, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
-    else if (g.ta == Op::T && g.tb == Op::N && g.tri == (TRI_A_UPPER | TRI_B_LOWER) && !g.lower_out)
-        run_gemm<true, false, TRI_A_UPPER | TRI_B_LOWER, false>(c, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
-    else if (g.ta == Op::N && g.tb == Op::N && g.tri == 0 && !g.lower_out)
-        run_gemm<false, false, 0, false>(c, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
-    else if (g.ta == Op::N && g.tb == Op::N && g.tri == 0 && g.lower_out)
-        run_gemm<false, false, 0, true>(c, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
-    else if (g.ta == Op::T && g.tb == Op::N && g.tri == 0 && !g.lower_out)
-        run_gemm<true, false, 0, false>(c, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
-    else
-        throw Error(GMGS_ERR_CUDA, "internal: unsupported DGEMM form");
-}
-
-// Cholesky of a 32 x 32 SPD tile (lower triangle of A, in place) and the
-// inverse of its factor into Li (zeros above the diagonal), one column per
-// step: the pivot's square root and reciprocal, column j of L, row j of L^-1
-// (forward substitution of L X = I carried along: X(j, c) is final once
-// scaled by 1/L(j,j)), then the rank-1 updates of the trailing part of A and
-// of the rows of X below j.  A pivot that is not positive sets *info and is
-// replaced by 1 so the arithmetic stays finite.
-__global__ void __launch_bounds__(256) k_chol_inv32(double* __restrict__ A, int lda, double* __restrict__ Li,
-                                                    int ldl, int* __restrict__ info) {
-    __shared__ double a[32][33];   // a[c][r] = A(r, c), becomes L
-    __shared__ double x[32][33];   // x[c][r] = X(r, c), becomes L^-1
-    __shared__ double dinv;
-    const int t = threadIdx.x;
-    for (int e = t; e < 1024; e += 256) {
-        const int cc = e >> 5, r = e & 31;
-        a[cc][r] = A[(int64_t)cc * lda + r];
-        x[cc][r] = r == cc ? 1.0 : 0.0;
-    }
-    __syncthreads();
-    for (int j = 0; j < 32; ++j) {
-        if (t == 0) {
-            const double d = a[j][j];
-            const bool ok = d > 0.0 && d < INFINITY;
-            if (!ok) atomicExch(info, 1);
-            const double piv = ok ? sqrt(d) : 1.0;
-            a[j][j] = piv;
-            dinv = 1.0 / piv;
-        }
-        __syncthreads();
-        if (t > j && t < 32) a[j][t] *= dinv;                  // L(t, j)
-        if (t >= 32 && t - 32 <= j) x[t - 32][j] *= dinv;      // X(j, c), c <= j
-        __syncthreads();
-        // only rows r > j change: (31 - j) rows x 32 columns, column cc of row r
-        // of A (j < cc <= r) or of X (cc <= j); the same update per element as a
-        // full sweep, in the same column order
-        for (int e = t; e < 32 * (31 - j); e += 256) {
-            const int r = j + 1 + (e >> 5), cc = e & 31;
-            if (cc > j) {
-                if (r >= cc) a[cc][r] = fma(-a[j][r], a[j][cc], a[cc][r]);
-            } else {
-                x[cc][r] = fma(-a[j][r], x[cc][j], x[cc][r]);
-            }
-        }
-        __syncthreads();
-    }
-    for (int e = t; e < 1024; e += 256) {
-        const int cc = e >> 5, r = e & 31;
-        if (r >= cc) A[(int64_t)cc * lda + r] = a[cc][r];
-        Li[(int64_t)cc * ldl + r] = x[cc][r];
-    }
-}
-
-// L (in place of the lower triangle of A) and L^-1 (into Li, whose part above
-// the diagonal must be zero on entry) of an n x n SPD matrix, n a multiple of
-// 32, by halves:  L11 = chol(A11), L21 = A21 L11^-T, L22 = chol(A22 - L21 L21^T),
-// L^-1_21 = -L22^-1 L21 L11^-1.  T: scratch of at least n * n / 2 doubles.
-void chol_inv(Ctx& c, double* A, double* Li, int n, int ld, double* T, int* info) {
-    if (n == 32) {
-        k_chol_inv32<<<1, 256, 0, c.stream>>>(A, ld, Li, ld, info);
-        GMGS_LAUNCHED(c);
-        return;
-    }
-    const int n1 = 32 * ((n / 32) / 2), n2 = n - n1;
-    double* A21 = A + n1;
-    double* A22 = A + (int64_t)n1 * ld + n1;
-    const double* Li11 = Li;
-    double* Li21 = Li + n1;
-    double* Li22 = Li + (int64_t)n1 * ld + n1;
-    chol_inv(c, A, Li, n1, ld, T, info);
-    gemm(c, {Op::N, Op::T, TRI_B_UPPER, false}, n2, n1, n1, 1.0, A21, ld, Li11, ld, 0.0, T, n2);   // L21
-    GMGS_CUDA(cudaMemcpy2DAsync(A21, (size_t)ld * sizeof(double), T, (size_t)n2 * sizeof(double),
-                                (size_t)n2 * sizeof(double), n1, cudaMemcpyDeviceToDevice, c.stream));
-    gemm(c, {Op::N, Op::T, 0, true}, n2, n2, n1, -1.0, A21, ld, A21, ld, 1.0, A22, ld);         // A22 - L21 L21^T
-    chol_inv(c, A22, Li22, n2, ld, T, info);
-    gemm(c, {Op::N, Op::N, TRI_B_LOWER, false}, n2, n1, n1, 1.0, A21, ld, Li11, ld, 0.0, T, n2);   // L21 L11^-1
-    gemm(c, {Op::N, Op::N, TRI_A_LOWER, false}, n2, n1, n2, -1.0, Li22, ld, T, n2, 0.0, Li21, ld);
-}
-
-// one 64 x 64 tile of op(M) times v: the tile into shared memory, 64 partial
-// sums (4 threads per output, 16 terms each, fixed order) returned in the
-// threads with (t & 3) == 0
-__device__ __forceinline__ double tile_mv(int Bn, const double* __restrict__ M, bool trans, int r0, int c0,
-                                          const double* v, double (*tile)[MT + 1], double* vs, bool wait_first) {
-    const int t = threadIdx.x;
-    constexpr int PER = MT * MT / 256;
-    double reg[PER];
-#pragma unroll
-    for (int j = 0; j < PER; ++j) {
-        const int e = t + j * 256;
-        reg[j] = M[(int64_t)(c0 + e / MT) * Bn + r0 + e % MT];
-    }
-#pragma unroll
-    for (int j = 0; j < PER; ++j) {
-        const int e = t + j * 256;
-        tile[e / MT][e % MT] = reg[j];
-    }
-    if (wait_first) asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (t < MT) vs[t] = v[(trans ? r0 : c0) + t];
-    __syncthreads();
-    const int o = t >> 2, q = t & 3;
-    double s = 0.0;
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-        const int w = q * 16 + u;
-        s = fma(trans ? tile[o][w] : tile[w][o], vs[w], s);
-    }
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    return s;
-}
-
-// Partial sums of one output block are stored, and the last CTA of that
-// output block to arrive adds them up in reduction-tile order:
-// y[i] = base[i] - sum (or the sum alone when base is null).
-__device__ __forceinline__ void finish_partials(int Bn, int nred, int rt, int out0, double s, double* partial,
-                                                unsigned int* ticket, const double* base, double* y) {
-    __shared__ bool last;
-    const int t = threadIdx.x;
-    if ((t & 3) == 0) partial[(int64_t)rt * Bn + out0 + (t >> 2)] = s;
-    __threadfence();
-    __syncthreads();
-    if (t == 0) last = atomicAdd(ticket, 1u) == (unsigned)(nred * (Bn / MT) - 1);
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    for (int i = t; i < Bn; i += 256) {
-        double acc = 0.0;
-        int k = 0;
-        for (; k + 8 <= nred; k += 8) {
-            double p[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) p[j] = __ldcg(partial + (int64_t)(k + j) * Bn + i);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) acc += p[j];
-        }
-        for (; k < nred; ++k) acc += __ldcg(partial + (int64_t)k * Bn + i);
-        y[i] = base ? base[i] - acc : acc;
-    }
-    if (t == 0) *ticket = 0;
-}
-
-// y_b = M_b v_b for the blocks b of the grid's z dimension (M_b: Bn x Bn,
-// column-major, stride sM; vectors stride Bn)
-__global__ void __launch_bounds__(256) k_blk_mv(int Bn, const double* __restrict__ M, int64_t sM, const double* v,
-                                                double* y, double* partial, unsigned int* ticket) {
-    __shared__ double tile[MT][MT + 1];
-    __shared__ double vs[MT];
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int b = blockIdx.z, ntiles = Bn / MT;
-    const double s = tile_mv(Bn, M + b * sM, false, blockIdx.x * MT, blockIdx.y * MT, v + (int64_t)b * Bn, tile, vs,
-                             true);
-    finish_partials(Bn, ntiles, blockIdx.y, blockIdx.x * MT, s, partial + (int64_t)b * ntiles * Bn, ticket + b,
-                    nullptr, y + (int64_t)b * Bn);
-}
-
-// up to two independent jobs (grid z), each y = base - sum_s op(M_s) v_s over
-// one or two segments s; grid y runs over (segment, reduction tile)
+// ---------------------------------------------------------------------------
+// the solve: launches of independent jobs y = base - sum_s M_s v_s (base null:
+// the sum itself), M_s B x B with its rows contiguous
+// ---------------------------------------------------------------------------
+constexpr int STEP_ROWS = 4;      // rows (warps) per CTA
+constexpr int MAX_JOBS = 4;
 struct StepJob {
     const double* M[2];
     const double* v[2];
-    int trans[2];
     const double* base;
     double* y;
-};
-struct StepJobs {
-    StepJob j[2];
     int nseg;
 };
+struct StepJobs {
+    StepJob j[MAX_JOBS];
+    int n = 0;
+    void add(double* y, const double* base, const double* M0, const double* v0, const double* M1 = nullptr,
+             const double* v1 = nullptr) {
+        j[n++] = {{M0, M1}, {v0, v1}, base, y, M1 ? 2 : 1};
+    }
+};
 
-__global__ void __launch_bounds__(256) k_blk_step(int Bn, const __grid_constant__ StepJobs jobs, double* partial,
-                                                  unsigned int* ticket) {
-    __shared__ double tile[MT][MT + 1];
-    __shared__ double vs[MT];
+// One warp per row, four rows per CTA: at 2 FP64 lanes per clock per SM a
+// matrix-vector product has to be spread over all SMs, and a row per warp
+// needs no partial sums through memory.  Launched as a programmatic dependent
+// of the previous kernel in the stream: the first 16 entries per lane (rows of
+// up to 512) are loaded while that kernel finishes, then the hardware grid
+// dependency is waited for, and only then are vectors read or written.
+__global__ void __launch_bounds__(32 * STEP_ROWS) k_rows(int B, const __grid_constant__ StepJobs jobs) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const StepJob& J = jobs.j[blockIdx.z];
-    const int ntiles = Bn / MT;
-    const int seg = blockIdx.y / ntiles, red = blockIdx.y % ntiles;
-    const bool tr = J.trans[seg] != 0;
-    const int r0 = (tr ? red : blockIdx.x) * MT, c0 = (tr ? blockIdx.x : red) * MT;
-    const double s = tile_mv(Bn, J.M[seg], tr, r0, c0, J.v[seg], tile, vs, true);
-    const int nred = jobs.nseg * ntiles;
-    finish_partials(Bn, nred, blockIdx.y, blockIdx.x * MT, s, partial + (int64_t)blockIdx.z * nred * Bn,
-                    ticket + blockIdx.z, J.base, J.y);
+    const StepJob& J = jobs.j[blockIdx.y];
+    const int lane = threadIdx.x & 31, row = blockIdx.x * STEP_ROWS + (threadIdx.x >> 5);
+    constexpr int PRE = 8;        // double2 per lane
+    double2 m[2][PRE];
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+        if (s < J.nseg) {
+            const double2* r = reinterpret_cast<const double2*>(J.M[s] + (int64_t)row * B);
+#pragma unroll
+            for (int q = 0; q < PRE; ++q)
+                if (64 * q < B) m[s][q] = r[32 * q + lane];
+        }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const double b = (lane == 0 && J.base) ? J.base[row] : 0.0;
+    double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+        if (s < J.nseg) {
+            const double2* v = reinterpret_cast<const double2*>(J.v[s]);
+#pragma unroll
+            for (int q = 0; q < PRE; ++q)
+                if (64 * q < B) {
+                    const double2 u = v[32 * q + lane];
+                    s0 = fma(m[s][q].x, u.x, s0);
+                    s1 = fma(m[s][q].y, u.y, s1);
+                }
+            const double2* r = reinterpret_cast<const double2*>(J.M[s] + (int64_t)row * B);
+            for (int q = PRE; 64 * q < B; ++q) {
+                const double2 u = v[32 * q + lane], w = r[32 * q + lane];
+                s0 = fma(w.x, u.x, s0);
+                s1 = fma(w.y, u.y, s1);
+            }
+        }
+    double s = s0 + s1;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) J.y[row] = J.base ? b - s : s;
 }
 
-// launched as a programmatic dependent of the previous kernel in the stream:
-// its CTAs load their matrix tiles while that kernel finishes, then wait
-// (griddepcontrol.wait, the hardware grid dependency) before they read the
-// vector it writes and touch the shared partial sums and arrival counters
-void launch_step(Ctx& c, int B, const StepJobs& jobs, int njobs, double* part, unsigned int* tk) {
+void launch_step(Ctx& c, int B, const StepJobs& jobs) {
+    if (jobs.n == 0) return;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(B / MT, jobs.nseg * (B / MT), njobs);
-    cfg.blockDim = dim3(256, 1, 1);
+    cfg.gridDim = dim3(B / STEP_ROWS, jobs.n, 1);
+    cfg.blockDim = dim3(32 * STEP_ROWS, 1, 1);
     cfg.stream = c.stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    GMGS_CUDA(cudaLaunchKernelEx(&cfg, k_blk_step, B, jobs, part, tk));
+    GMGS_CUDA(cudaLaunchKernelEx(&cfg, k_rows, B, jobs));
     GMGS_LAUNCHED(c);
 }
 
-// D^-1 of the SPD block D (in place): Cholesky + inverse factor, L^-T L^-1
-void inv_spd(Ctx& c, double* D, int B, double* li, double* t, int* info) {
-    const int64_t B2 = (int64_t)B * B;
-    GMGS_CUDA(cudaMemsetAsync(li, 0, B2 * sizeof(double), c.stream));
-    chol_inv(c, D, li, B, B, t, info);
-    gemm(c, {Op::T, Op::N, TRI_A_UPPER | TRI_B_LOWER, false}, B, B, B, 1.0, li, B, li, B, 0.0, D, B);
-}
+int coarse_middle(int nb) { return (nb - 1) / 2; }
 
 }  // namespace
 
 int coarse_block_order(int n, int half_bandwidth) {
+    constexpr int Q = 64;         // a lane of k_rows reads double2: rows of 64 entries
     const int want = std::max(half_bandwidth, 1);
-    return std::max(MT, (std::min(want, n) + MT - 1) / MT * MT);
+    return std::max(Q, (std::min(want, n) + Q - 1) / Q * Q);
 }
-
-int coarse_middle(int nb) { return (nb - 1) / 2; }
 
 void factor_coarse(Ctx& c, CoarseBlocks& cb, const std::function<void()>& overlap) {
     const int B = cb.B, nb = cb.nb, k = coarse_middle(nb);
     const int64_t B2 = (int64_t)B * B;
     double* D = cb.sinv.as<double>();   // A_ii on entry
     double* E = cb.g.as<double>();      // E_i = A_(i,i-1) on entry (i >= 1)
+    cb.gt = dalloc((size_t)nb * B2 * sizeof(double));
     auto Db = [&](int i) { return D + i * B2; };
     auto Eb = [&](int i) { return E + i * B2; };
+    auto Gt = [&](int i) { return cb.gt.as<double>() + i * B2; };
     // the two halves run on their own streams, forked from and joined to c.stream
     cudaStream_t st[2] = {nullptr, nullptr};
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
@@ -352,12 +393,8 @@ void factor_coarse(Ctx& c, CoarseBlocks& cb, const std::function<void()>& overla
     for (int i = 0; i < 3; ++i) GMGS_CUDA(cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming));
     DevBuf info = dalloc(2 * sizeof(int));
     GMGS_CUDA(cudaMemsetAsync(info.p, 0, 2 * sizeof(int), c.stream));
-    DevBuf li[2], tt[2], t2[2];
-    for (int h = 0; h < 2; ++h) {
-        li[h] = dalloc(B2 * sizeof(double));
-        tt[h] = dalloc(B2 * sizeof(double));
-        t2[h] = dalloc(B2 * sizeof(double));
-    }
+    Chain chain[2];
+    for (int h = 0; h < 2; ++h) chain[h].alloc(B);
     GMGS_CUDA(cudaEventRecord(ev[0], c.stream));
     Ctx half[2] = {c, c};
     for (int h = 0; h < 2; ++h) {
@@ -368,31 +405,38 @@ void factor_coarse(Ctx& c, CoarseBlocks& cb, const std::function<void()>& overla
         GMGS_CUDA(cudaStreamWaitEvent(st[h], ev[0], 0));
     }
     int* inf = info.as<int>();
-    {   // top: S_i^-1 (i < k), G_i (i = 1..k-1), and G_k into t2[0]
-        Ctx& h = half[0];
-        for (int i = 0; i < k; ++i) {
-            if (i > 0) {
-                gemm(h, {Op::N, Op::N, 0, false}, B, B, B, 1.0, Eb(i), B, Db(i - 1), B, 0.0, t2[0].as<double>(), B);
-                gemm(h, {Op::N, Op::T, 0, true}, B, B, B, -1.0, t2[0].as<double>(), B, Eb(i), B, 1.0, Db(i), B);
-                GMGS_CUDA(cudaMemcpyAsync(Eb(i), t2[0].p, B2 * sizeof(double), cudaMemcpyDeviceToDevice, h.stream));
+    auto keep_g = [&](Ctx& h, Chain& s, int i) {     // G column-major takes the coupling's place
+        GMGS_CUDA(cudaMemcpyAsync(Eb(i), s.g.p, B2 * sizeof(double), cudaMemcpyDeviceToDevice, h.stream));
+    };
+    // block by block from both ends (interleaved, so both streams have work
+    // from the start): top S_i^-1 (i < k) with G_i, then G_k; bottom T_i^-1
+    // (i > k) with H_i in the place of E_(i+1), then H_k.  The middle block's
+    // couplings stay in place until both have reached it.
+    for (int step = 0; step <= std::max(k, nb - 1 - k); ++step) {
+        if (step <= k) {
+            const int i = step;
+            Ctx& h = half[0];
+            if (i > 0) sparse_left(h, B, Eb(i), false, Db(i - 1), Gt(i), chain[0].g.as<double>());
+            if (i < k) {
+                if (i > 0) {
+                    sparse_update(h, B, Eb(i), false, chain[0].g.as<double>(), Db(i));
+                    keep_g(h, chain[0], i);
+                }
+                inv_spd(h, Db(i), B, chain[0], inf);
             }
-            inv_spd(h, Db(i), B, li[0].as<double>(), tt[0].as<double>(), inf);
         }
-        if (k >= 1)
-            gemm(h, {Op::N, Op::N, 0, false}, B, B, B, 1.0, Eb(k), B, Db(k - 1), B, 0.0, t2[0].as<double>(), B);
-    }
-    {   // bottom: T_i^-1 (i > k), H_i = E_(i+1) (i = k+1..nb-2), and H_k into t2[1]
-        Ctx& h = half[1];
-        for (int i = nb - 1; i > k; --i) {
-            if (i < nb - 1) {
-                gemm(h, {Op::T, Op::N, 0, false}, B, B, B, 1.0, Eb(i + 1), B, Db(i + 1), B, 0.0, t2[1].as<double>(), B);
-                gemm(h, {Op::N, Op::N, 0, true}, B, B, B, -1.0, t2[1].as<double>(), B, Eb(i + 1), B, 1.0, Db(i), B);
-                GMGS_CUDA(cudaMemcpyAsync(Eb(i + 1), t2[1].p, B2 * sizeof(double), cudaMemcpyDeviceToDevice, h.stream));
+        if (nb - 1 - step >= k) {
+            const int i = nb - 1 - step;
+            Ctx& h = half[1];
+            if (i < nb - 1) sparse_left(h, B, Eb(i + 1), true, Db(i + 1), Gt(i + 1), chain[1].g.as<double>());
+            if (i > k) {
+                if (i < nb - 1) {
+                    sparse_update(h, B, Eb(i + 1), true, chain[1].g.as<double>(), Db(i));
+                    keep_g(h, chain[1], i + 1);
+                }
+                inv_spd(h, Db(i), B, chain[1], inf + 1);
             }
-            inv_spd(h, Db(i), B, li[1].as<double>(), tt[1].as<double>(), inf + 1);
         }
-        if (k + 1 <= nb - 1)
-            gemm(h, {Op::T, Op::N, 0, false}, B, B, B, 1.0, Eb(k + 1), B, Db(k + 1), B, 0.0, t2[1].as<double>(), B);
     }
     if (overlap) overlap();
     c.trace_point("bc: work buffers (beside the factorisation)");
@@ -403,83 +447,64 @@ void factor_coarse(Ctx& c, CoarseBlocks& cb, const std::function<void()>& overla
     }
     // the middle block: M = A_kk - G_k A_(k,k-1)^T - H_k A_(k+1,k), then M^-1
     if (k >= 1) {
-        gemm(c, {Op::N, Op::T, 0, true}, B, B, B, -1.0, t2[0].as<double>(), B, Eb(k), B, 1.0, Db(k), B);
-        GMGS_CUDA(cudaMemcpyAsync(Eb(k), t2[0].p, B2 * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
+        sparse_update(c, B, Eb(k), false, chain[0].g.as<double>(), Db(k));
+        keep_g(c, chain[0], k);
     }
     if (k + 1 <= nb - 1) {
-        gemm(c, {Op::N, Op::N, 0, true}, B, B, B, -1.0, t2[1].as<double>(), B, Eb(k + 1), B, 1.0, Db(k), B);
-        GMGS_CUDA(cudaMemcpyAsync(Eb(k + 1), t2[1].p, B2 * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
+        sparse_update(c, B, Eb(k + 1), true, chain[1].g.as<double>(), Db(k));
+        keep_g(c, chain[1], k + 1);
     }
-    inv_spd(c, Db(k), B, li[0].as<double>(), tt[0].as<double>(), inf);
+    inv_spd(c, Db(k), B, chain[0], inf);
     c.trace_point("bc: coarsest block LDL^T");
     int h_info[2] = {0, 0};
     GMGS_CUDA(cudaMemcpyAsync(h_info, info.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
     GMGS_CUDA(cudaStreamSynchronize(c.stream));
     if (h_info[0] || h_info[1]) throw Error(GMGS_ERR_NOT_SPD, "coarsest-level matrix is not positive definite");
-    const int nslot = std::max(nb, 4);
-    cb.partial = dalloc((size_t)nslot * (B / MT) * B * sizeof(double));
-    cb.ticket = dalloc((size_t)nslot * sizeof(unsigned int));
-    GMGS_CUDA(cudaMemsetAsync(cb.ticket.p, 0, (size_t)nslot * sizeof(unsigned int), c.stream));
-    GMGS_CUDA(cudaStreamSynchronize(c.stream));
 }
 
 void launch_coarse_solve(Ctx& c, const CoarseBlocks& cb, double* cvec, double* x) {
     const int B = cb.B, nb = cb.nb, k = coarse_middle(nb);
     if (nb <= 0) return;
     const int64_t B2 = (int64_t)B * B;
-    const double* D = cb.sinv.as<double>();
-    const double* E = cb.g.as<double>();
-    double* part = cb.partial.as<double>();
-    unsigned int* tk = cb.ticket.as<unsigned int>();
-    auto Eb = [&](int i) { return E + i * B2; };
-    auto vb = [&](double* v, int i) { return v + (int64_t)i * B; };
-    // forward chains, in place on cvec: top i = 1..k-1, bottom i = nb-2..k+1
-    const int top_steps = std::max(0, k - 1), bot_steps = std::max(0, nb - 2 - k);
-    for (int s = 0; s < std::max(top_steps, bot_steps); ++s) {
-        StepJobs J = {};
-        J.nseg = 1;
-        int nj = 0;
-        if (s < top_steps) {
-            const int i = 1 + s;
-            J.j[nj++] = {{Eb(i), nullptr}, {vb(cvec, i - 1), nullptr}, {0, 0}, vb(cvec, i), vb(cvec, i)};
+    auto Db = [&](int i) { return cb.sinv.as<double>() + i * B2; };    // symmetric
+    auto G = [&](int i) { return cb.gt.as<double>() + i * B2; };       // rows of G
+    auto GT = [&](int i) { return cb.g.as<double>() + i * B2; };       // rows of G^T
+    auto cv = [&](int i) { return cvec + (int64_t)i * B; };
+    auto xv = [&](int i) { return x + (int64_t)i * B; };
+    // Forward chains, in place on cvec: top i = 1..k-1, bottom i = nb-2..k+1.
+    // x_i = D_i^-1 c_i of the blocks that the previous launch finished rides
+    // along (one launch of its own for all blocks would wait for them all and
+    // read every D_i^-1 at once).
+    const int top = k, bot = nb - 1 - k;      // blocks above and below the middle
+    const int steps = std::max(top, bot);
+    for (int step = 0; step < steps; ++step) {
+        StepJobs J;
+        if (step == steps - 1) {              // the middle block's right-hand side: both chains have ended
+            if (top > 0 && bot > 0) J.add(cv(k), cv(k), G(k), cv(k - 1), G(k + 1), cv(k + 1));
+            else J.add(cv(k), cv(k), G(bot > 0 ? k + 1 : k), cv(bot > 0 ? k + 1 : k - 1));
         }
-        if (s < bot_steps) {
-            const int i = nb - 2 - s;
-            J.j[nj++] = {{Eb(i + 1), nullptr}, {vb(cvec, i + 1), nullptr}, {0, 0}, vb(cvec, i), vb(cvec, i)};
+        if (step < top) {
+            J.add(xv(step), nullptr, Db(step), cv(step));
+            if (step + 1 < top) J.add(cv(step + 1), cv(step + 1), G(step + 1), cv(step));
         }
-        launch_step(c, B, J, nj, part, tk);
+        if (step < bot) {
+            const int i = nb - 1 - step;
+            J.add(xv(i), nullptr, Db(i), cv(i));
+            if (step + 1 < bot) J.add(cv(i - 1), cv(i - 1), G(i), cv(i));
+        }
+        launch_step(c, B, J);
     }
-    {   // the middle block's right-hand side
-        StepJobs J = {};
-        int ns = 0;
-        StepJob& m = J.j[0];
-        if (k >= 1) { m.M[ns] = Eb(k); m.v[ns] = vb(cvec, k - 1); m.trans[ns] = 0; ++ns; }
-        if (k + 1 <= nb - 1) { m.M[ns] = Eb(k + 1); m.v[ns] = vb(cvec, k + 1); m.trans[ns] = 0; ++ns; }
-        if (ns > 0) {
-            m.base = vb(cvec, k);
-            m.y = vb(cvec, k);
-            J.nseg = ns;
-            launch_step(c, B, J, 1, part, tk);
-        }
+    {
+        StepJobs J;
+        J.add(xv(k), nullptr, Db(k), cv(k));
+        launch_step(c, B, J);
     }
-    // x_i = D_i^-1 c_i for all blocks
-    k_blk_mv<<<dim3(B / MT, B / MT, nb), 256, 0, c.stream>>>(B, D, B2, cvec, x, part, tk);
-    GMGS_LAUNCHED(c);
     // backward chains, in place on x: top i = k-1..0, bottom i = k+1..nb-1
-    const int tb = k, bb = nb - 1 - k;
-    for (int s = 0; s < std::max(tb, bb); ++s) {
-        StepJobs J = {};
-        J.nseg = 1;
-        int nj = 0;
-        if (s < tb) {
-            const int i = k - 1 - s;
-            J.j[nj++] = {{Eb(i + 1), nullptr}, {vb(x, i + 1), nullptr}, {1, 0}, vb(x, i), vb(x, i)};
-        }
-        if (s < bb) {
-            const int i = k + 1 + s;
-            J.j[nj++] = {{Eb(i), nullptr}, {vb(x, i - 1), nullptr}, {1, 0}, vb(x, i), vb(x, i)};
-        }
-        launch_step(c, B, J, nj, part, tk);
+    for (int s = 0; s < steps; ++s) {
+        StepJobs J;
+        if (s < top) J.add(xv(k - 1 - s), xv(k - 1 - s), GT(k - s), xv(k - s));
+        if (s < bot) J.add(xv(k + 1 + s), xv(k + 1 + s), GT(k + 1 + s), xv(k + s));
+        launch_step(c, B, J);
     }
 }
 

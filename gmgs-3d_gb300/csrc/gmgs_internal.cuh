@@ -351,10 +351,9 @@ struct CoarseBlocks {
     int n = 0;        // free DOFs
     int B = 0;        // block order: a multiple of 64, at least the half bandwidth
     int nb = 0;       // blocks; rows n..nb*B-1 are identity padding
-    DevBuf sinv;      // nb x (B x B) column-major: A_ii on entry, D_i^-1 after factor_coarse
-    DevBuf g;         // nb x (B x B): A_(i,i-1) on entry, the coupling G_i or H_(i-1) after
-    DevBuf partial;   // max(nb, 4) x (B/64) x B partial sums of the block matrix-vector products
-    DevBuf ticket;    // max(nb, 4) arrival counters (zero between launches)
+    DevBuf sinv;      // nb x (B x B) column-major: A_ii on entry, D_i^-1 (symmetric) after factor_coarse
+    DevBuf g;         // nb x (B x B) column-major: A_(i,i-1) on entry, the coupling G_i or H_(i-1) after
+    DevBuf gt;        // the couplings row-major
 };
 int coarse_block_order(int n, int half_bandwidth);
 // overlap: host work run while the two halves factor on their own streams
