@@ -533,17 +533,12 @@ int gmgs_apply_operator(gmgs_handle* h, int32_t level, const double* x, double* 
             fail(GMGS_ERR_STATE, "level 2 keeps only FP32 element matrices on a mixed-precision handle with a density "
                                  "field; use an FP64 handle to apply it");
         ensure_coarse(h);
-        gmgs::Level& lv = M.levels[level - 1];
-        const int64_t nn = lv.n_node, S = lv.g.slots;
-        gmgs::DevBuf xc = gmgs::dalloc(3 * nn * sizeof(double)), xd = gmgs::dalloc(3 * S * sizeof(double)),
-                     yd = gmgs::dalloc(3 * S * sizeof(double));
-        HostPin pin_in(x, 3 * nn * sizeof(double), true), pin_out(y, 3 * nn * sizeof(double), false);
-        GMGS_CUDA(cudaMemcpyAsync(xc.p, x, 3 * nn * sizeof(double), cudaMemcpyHostToDevice, M.ctx.stream));
-        GMGS_CUDA(cudaMemsetAsync(xd.p, 0, 3 * S * sizeof(double), M.ctx.stream));
-        gmgs::launch_compact_to_dense<double>(M.ctx, nn, S, lv.node_slot.as<int32_t>(), xc.as<double>(), xd.as<double>());
-        gmgs::apply_operator_dense(M, level - 1, xd.as<double>(), yd.as<double>());
-        gmgs::launch_dense_to_compact<double>(M.ctx, nn, S, lv.node_slot.as<int32_t>(), yd.as<double>(), xc.as<double>());
-        GMGS_CUDA(cudaMemcpyAsync(y, xc.p, 3 * nn * sizeof(double), cudaMemcpyDeviceToHost, M.ctx.stream));
+        const size_t bytes = 3 * (size_t)M.levels[level - 1].n_node * sizeof(double);
+        gmgs::DevBuf xc = gmgs::dalloc(bytes);
+        HostPin pin_in(x, bytes, true), pin_out(y, bytes, false);
+        GMGS_CUDA(cudaMemcpyAsync(xc.p, x, bytes, cudaMemcpyHostToDevice, M.ctx.stream));
+        gmgs::operator_apply(M, level - 1, xc.as<double>(), xc.as<double>());
+        GMGS_CUDA(cudaMemcpyAsync(y, xc.p, bytes, cudaMemcpyDeviceToHost, M.ctx.stream));
         GMGS_CUDA(cudaStreamSynchronize(M.ctx.stream));
         return GMGS_OK;
     });
@@ -554,18 +549,12 @@ int gmgs_apply_preconditioner(gmgs_handle* h, const double* r, double* z) {
         if (!h || !r || !z) fail(GMGS_ERR_INVALID_ARGUMENT, "NULL argument");
         gmgs::Model& M = h->M;
         ensure_coarse(h);
-        gmgs::Level& lv = M.levels[0];
-        const int64_t nn = lv.n_node, S = lv.g.slots;
-        gmgs::DevBuf xc = gmgs::dalloc(3 * nn * sizeof(double)), xd = gmgs::dalloc(3 * S * sizeof(double)),
-                     yd = gmgs::dalloc(3 * S * sizeof(double));
-        HostPin pin_in(r, 3 * nn * sizeof(double), true), pin_out(z, 3 * nn * sizeof(double), false);
-        GMGS_CUDA(cudaMemcpyAsync(xc.p, r, 3 * nn * sizeof(double), cudaMemcpyHostToDevice, M.ctx.stream));
-        GMGS_CUDA(cudaMemsetAsync(xd.p, 0, 3 * S * sizeof(double), M.ctx.stream));
-        GMGS_CUDA(cudaMemsetAsync(yd.p, 0, 3 * S * sizeof(double), M.ctx.stream));
-        gmgs::launch_compact_to_dense<double>(M.ctx, nn, S, lv.node_slot.as<int32_t>(), xc.as<double>(), xd.as<double>());
-        gmgs::vcycle_apply(M, xd.as<double>(), yd.as<double>());
-        gmgs::launch_dense_to_compact<double>(M.ctx, nn, S, lv.node_slot.as<int32_t>(), yd.as<double>(), xc.as<double>());
-        GMGS_CUDA(cudaMemcpyAsync(z, xc.p, 3 * nn * sizeof(double), cudaMemcpyDeviceToHost, M.ctx.stream));
+        const size_t bytes = 3 * (size_t)M.levels[0].n_node * sizeof(double);
+        gmgs::DevBuf xc = gmgs::dalloc(bytes);
+        HostPin pin_in(r, bytes, true), pin_out(z, bytes, false);
+        GMGS_CUDA(cudaMemcpyAsync(xc.p, r, bytes, cudaMemcpyHostToDevice, M.ctx.stream));
+        gmgs::vcycle_apply(M, xc.as<double>(), xc.as<double>());
+        GMGS_CUDA(cudaMemcpyAsync(z, xc.p, bytes, cudaMemcpyDeviceToHost, M.ctx.stream));
         GMGS_CUDA(cudaStreamSynchronize(M.ctx.stream));
         return GMGS_OK;
     });
@@ -580,13 +569,7 @@ int gmgs_apply_operator_dev(gmgs_handle* h, int32_t level, const double* x, doub
             fail(GMGS_ERR_STATE, "level 2 keeps only FP32 element matrices on a mixed-precision handle with a density "
                                  "field; use an FP64 handle to apply it");
         ensure_coarse(h);
-        gmgs::Level& lv = M.levels[level - 1];
-        const int64_t nn = lv.n_node, S = lv.g.slots;
-        gmgs::DevBuf xd = gmgs::dalloc(3 * S * sizeof(double)), yd = gmgs::dalloc(3 * S * sizeof(double));
-        GMGS_CUDA(cudaMemsetAsync(xd.p, 0, 3 * S * sizeof(double), M.ctx.stream));
-        gmgs::launch_compact_to_dense<double>(M.ctx, nn, S, lv.node_slot.as<int32_t>(), x, xd.as<double>());
-        gmgs::apply_operator_dense(M, level - 1, xd.as<double>(), yd.as<double>());
-        gmgs::launch_dense_to_compact<double>(M.ctx, nn, S, lv.node_slot.as<int32_t>(), yd.as<double>(), y);
+        gmgs::operator_apply(M, level - 1, x, y);
         GMGS_CUDA(cudaStreamSynchronize(M.ctx.stream));
         return GMGS_OK;
     });
@@ -597,14 +580,7 @@ int gmgs_apply_preconditioner_dev(gmgs_handle* h, const double* r, double* z) {
         if (!h || !r || !z) fail(GMGS_ERR_INVALID_ARGUMENT, "NULL argument");
         gmgs::Model& M = h->M;
         ensure_coarse(h);
-        gmgs::Level& lv = M.levels[0];
-        const int64_t nn = lv.n_node, S = lv.g.slots;
-        gmgs::DevBuf xd = gmgs::dalloc(3 * S * sizeof(double)), yd = gmgs::dalloc(3 * S * sizeof(double));
-        GMGS_CUDA(cudaMemsetAsync(xd.p, 0, 3 * S * sizeof(double), M.ctx.stream));
-        GMGS_CUDA(cudaMemsetAsync(yd.p, 0, 3 * S * sizeof(double), M.ctx.stream));
-        gmgs::launch_compact_to_dense<double>(M.ctx, nn, S, lv.node_slot.as<int32_t>(), r, xd.as<double>());
-        gmgs::vcycle_apply(M, xd.as<double>(), yd.as<double>());
-        gmgs::launch_dense_to_compact<double>(M.ctx, nn, S, lv.node_slot.as<int32_t>(), yd.as<double>(), z);
+        gmgs::vcycle_apply(M, r, z);
         GMGS_CUDA(cudaStreamSynchronize(M.ctx.stream));
         return GMGS_OK;
     });

@@ -327,10 +327,6 @@ struct Ctx {
 // ---------------------------------------------------------------------------
 constexpr int KE = 576;
 
-// conversion copy out = a
-template <typename T, typename U>
-void launch_copy(Ctx& c, int64_t n, T* out, const U* a);
-
 // restriction r_c = P^T r_f (RestrictResidual.m)
 template <typename T>
 void launch_restrict(Ctx& c, const Grid& gf, const Grid& gc, const uint8_t* nflag_c,

@@ -11,27 +11,11 @@ static dim3 node_grid(const Grid& g, dim3 blk) {
     return dim3((g.ny + 1 + blk.x - 1) / blk.x, (g.nx + 1 + blk.y - 1) / blk.y, g.nz + 1);
 }
 
-// ---------------------------------------------------------------------------
-// elementwise helpers
-// ---------------------------------------------------------------------------
 static int ew_blocks(const Ctx& c, int64_t n) {
     int64_t b = (n + 255) / 256;
     int64_t cap = (int64_t)c.num_sms * 16;
     return (int)(b < cap ? (b < 1 ? 1 : b) : cap);
 }
-
-template <typename T, typename U>
-__global__ void k_copy(int64_t n, T* __restrict__ x, const U* __restrict__ a) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        x[i] = (T)a[i];
-}
-template <typename T, typename U>
-void launch_copy(Ctx& c, int64_t n, T* x, const U* a) {
-    k_copy<T, U><<<ew_blocks(c, n), 256, 0, c.stream>>>(n, x, a);
-    GMGS_LAUNCHED(c);
-}
-template void launch_copy<float, double>(Ctx&, int64_t, float*, const double*);
-template void launch_copy<double, float>(Ctx&, int64_t, double*, const float*);
 
 // ---------------------------------------------------------------------------
 // trilinear transfers (RestrictResidual.m, InterpolationDeviation.m)

@@ -80,8 +80,9 @@ void set_density_dev(Model& M, const double* rho_dev);
 void alloc_work(Model& M);
 void reset_graphs(Model& M);   // destroy the captured PCG iteration graphs
 int pcg_solve(Model& M, const double* b_dense, double* x_dense, int32_t* iters, double* relres, double* hist);
-void vcycle_apply(Model& M, const double* r_dense, double* z_dense);
-void apply_operator_dense(Model& M, int level, const double* x_dense, double* y_dense);
+// on compact interleaved device vectors (in place allowed); level 0-based
+void vcycle_apply(Model& M, const double* r, double* z);
+void operator_apply(Model& M, int level, const double* x, double* y);
 
 // post.cu
 void stress_dev(Model& M, const double* U_dense, double* nodal_compact, float* per_voxel_compact);
