@@ -305,7 +305,7 @@ struct StepJobs {
 // up to 512) are loaded while that kernel finishes, then the hardware grid
 // dependency is waited for, and only then are vectors read or written.
 __global__ void __launch_bounds__(32 * STEP_ROWS) k_rows(int B, const __grid_constant__ StepJobs jobs) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    pdl_begin();
     const StepJob& J = jobs.j[blockIdx.y];
     const int lane = threadIdx.x & 31, row = blockIdx.x * STEP_ROWS + (threadIdx.x >> 5);
     constexpr int PRE = 8;        // double2 per lane
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(32 * STEP_ROWS) k_rows(int B, const __grid_con
             for (int q = 0; q < PRE; ++q)
                 if (64 * q < B) m[s][q] = r[32 * q + lane];
         }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_wait();
     const double b = (lane == 0 && J.base) ? J.base[row] : 0.0;
     double s0 = 0.0, s1 = 0.0;
 #pragma unroll
@@ -347,17 +347,7 @@ __global__ void __launch_bounds__(32 * STEP_ROWS) k_rows(int B, const __grid_con
 
 void launch_step(Ctx& c, int B, const StepJobs& jobs) {
     if (jobs.n == 0) return;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(B / STEP_ROWS, jobs.n, 1);
-    cfg.blockDim = dim3(32 * STEP_ROWS, 1, 1);
-    cfg.stream = c.stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    GMGS_CUDA(cudaLaunchKernelEx(&cfg, k_rows, B, jobs));
-    GMGS_LAUNCHED(c);
+    launch_chain(c, k_rows, dim3(B / STEP_ROWS, jobs.n, 1), dim3(32 * STEP_ROWS, 1, 1), 0, B, jobs);
 }
 
 int coarse_middle(int nb) { return (nb - 1) / 2; }

@@ -110,7 +110,6 @@ __device__ __forceinline__ void epi_fetch(const FineArgs& a, int S, int n, EpiDa
 //   c * 256 + 32 * lx + ((((ly >> 2) ^ lx) << 2) | (ly & 3)).
 constexpr int EPI_BOX = 3 * NT;                              // floats per array and plane
 constexpr int EPI_STAGE_BYTES = EPI_ARRAYS * EPI_BOX * 4;
-constexpr size_t EPI_DYN_SMEM = EPI_STAGE_BYTES + 1024;      // + alignment slack
 constexpr uint64_t EPI_WAIT_NS = 5000000ull;                 // a plane's copies take microseconds
 // the thread that arms the stage: lane 0 of the last warp, which stages no
 // halo points (threads 0..83 do), so the copies do not lengthen the warp the
@@ -161,6 +160,81 @@ __device__ __forceinline__ void epi_from_stage(const float* st, int sidx, bool f
     }
 }
 
+// ---------------------------------------------------------------------------
+// V-cycle down-sweep at nodes that touch elements with their own Galerkin
+// matrix: eight lanes per node (four nodes per warp).  For each of the
+// node's 8 elements, lane j multiplies the node's three rows of the element
+// matrix at columns 3j..3j+2 (the coupling to element node j) with node j's
+// Jacobi step w r; each lane keeps the three row sums across the elements and
+// a shuffle reduction over the 8 lanes (xor 1, 2, 4) adds them up.  The
+// per-lane sums and the reduction order are those of a lane per (row,
+// column group), so the result does not depend on the lane layout.
+// out = r - A (w r) with fixed rows zeroed (AtX.m:57).
+// The work is a few dependent loads per node (list, element types, operands):
+// they are issued for all elements before the first is used, and on levels
+// with other nodes as well these nodes are blocks of the streaming launch, so
+// their latency runs beside the tiles (11 to 24 us per level as a launch of
+// its own after them).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void perel_node(const FineLevel& L, const Coef32& cf, const FineArgs& a, int node, int j) {
+    const int count = a.n_perel;
+    const bool active = node < count;          // whole 8-lane groups; idle groups still shuffle
+    const Grid& g = L.g;
+    const int S = (int)g.slots, sx = g.py, sz = g.py * g.px;
+    const int n = active ? chk::ld(a.perel, node, count, chk::PEREL_NODE) : 0;
+    const long long n3 = 3ll * S;
+    constexpr int V = chk::PEREL_VEC;
+    float acc[3] = {0.f, 0.f, 0.f};
+    int type[8];                               // -1 void, 0 uniform, k the stored matrix k - 1
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const int es = n - (e & 1) - ((e >> 1) & 1) * sx - (e >> 2) * sz;
+        type[e] = -1;
+        if (active && chk::ld(L.emask, es, S, chk::PEREL_ELEM)) {
+            type[e] = L.etype ? chk::ld(L.etype, es, S, chk::PEREL_ELEM) : 0;
+            if (type[e] > 0 && !chk::ok(type[e] - 1, L.nK, chk::PEREL_KS)) type[e] = -1;
+        }
+    }
+    pdl_wait();
+#pragma unroll
+    for (int h = 0; h < 8; h += 2) {           // two elements' loads in flight
+        float d[2][3], K[2][9];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int e = h + q, es = n - (e & 1) - ((e >> 1) & 1) * sx - (e >> 2) * sz;
+            const int nj = es + corner_y(j) + corner_x(j) * sx + corner_z(j) * sz;
+            const bool on = type[e] >= 0;      // uniform across the node's lanes
+            const float* Ke = (type[e] > 0 ? L.Ks + (int64_t)(type[e] - 1) * KE : cf.K) +
+                              3 * corner_of(e & 1, (e >> 1) & 1, e >> 2) * 24 + 3 * j;
+#pragma unroll
+            for (int b = 0; b < 3; ++b)
+                d[q][b] = on ? chk::ld(a.r32, nj + b * S, n3, V) * chk::ld(a.wdinv, nj + b * S, n3, V) : 0.f;
+#pragma unroll
+            for (int b = 0; b < 9; ++b) K[q][b] = on ? Ke[24 * (b / 3) + b % 3] : 0.f;
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            if (type[h + q] < 0) continue;
+            const float k = type[h + q] > 0 ? 1.f : L.kscale;
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                acc[c] = fmaf(k * K[q][3 * c], d[q][0], fmaf(k * K[q][3 * c + 1], d[q][1], fmaf(k * K[q][3 * c + 2], d[q][2], acc[c])));
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 1);
+        acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 2);
+        acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 4);
+    }
+    if (active && j < 3) {
+        const uint32_t f = chk::ld(L.nflag, n, S, chk::PEREL_ELEM);
+        const float y = j == 0 ? acc[0] : (j == 1 ? acc[1] : acc[2]);
+        const int i = n + j * S;
+        chk::st(a.out32, i, n3, chk::PEREL_OUT, chk::ld(a.r32, i, n3, V) - ((f & (NF_FIX_X << j)) ? 0.f : y));
+    }
+}
+
 // 48 registers (5 CTAs per SM) for the stencil-only modes, 40 (6 CTAs) for
 // the CG direction with its field staged by TMA (1.073 -> 1.063 ms; the
 // down-sweep, which also holds r for its output, spills at 40); the CG update
@@ -182,15 +256,22 @@ __global__ void __launch_bounds__(NT, MODE == FM_CG_UPDATE_JACOBI ? ((STG & 1) ?
     const int S = (int)g.slots;
     const int sz = g.py * g.px;
     const int y0 = blockIdx.x * TY, x0 = blockIdx.y * TX;
-    const int zb = blockIdx.z * zc;
+    pdl_begin();
+    if (MODE == FM_VCYCLE_DOWN && (int)blockIdx.z < a.perel_z) {   // the first grid layers: nodes on stored matrices
+        const int t = threadIdx.x + threadIdx.y * TY;
+        const int blk = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+        perel_node(L, cf, a, blk * (NT / 8) + t / 8, t & 7);
+        return;
+    }
+    const int zb = ((int)blockIdx.z - (MODE == FM_VCYCLE_DOWN ? a.perel_z : 0)) * zc;
     const int ze = min(zb + zc, g.nz + 1);        // node planes [zb, ze)
-    if (L.tile_occ) {                             // no solid node in this column tile: nothing to compute
-        int any = 0;
+    int any = L.tile_occ ? 0 : 1;
+    if (L.tile_occ)
         for (int iz = zb; iz < ze; ++iz) any |= L.tile_occ[((int64_t)iz * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x];
-        if (!any) {
-            if (MODE == FM_CG_DIRECTION || MODE == FM_CG_UPDATE_JACOBI) grid_dot_finish(0.0, a.dot, sh);
-            return;
-        }
+    pdl_wait();
+    if (!any) {                                   // no solid node in this column tile: nothing to compute
+        if (MODE == FM_CG_DIRECTION || MODE == FM_CG_UPDATE_JACOBI) grid_dot_finish(0.0, a.dot, sh);
+        return;
     }
     // warps cover 8 (y) x 4 (x) node patches, so a face of the domain
     // crosses few warps and the boundary path rarely diverges
@@ -213,16 +294,28 @@ __global__ void __launch_bounds__(NT, MODE == FM_CG_UPDATE_JACOBI ? ((STG & 1) ?
         stage = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(fine_dyn) + 1023) & ~uintptr_t(1023));
         sidx = 32 * lx + ((((ly >> 2) ^ lx) << 2) | (ly & 3));
     }
+    auto issue_epi = [&](int iz) {
+        const int na = a.first ? 4 : EPI_ARRAYS;
+        mbar_expect_tx(&ebar, (uint32_t)(na * EPI_BOX * 4));
+        for (int j = 0; j < na; ++j)
+            tma_load_plane(stage + j * EPI_BOX, &em.m[j], y0 + Grid::YOFF, x0 + 1, iz + 1, &ebar);
+    };
     if constexpr (FTMA) {
         fstage = TMA ? stage + EPI_ARRAYS * EPI_BOX
                      : reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(fine_dyn) + 127) & ~uintptr_t(127));
     }
     if constexpr (TMA || FTMA) {
-        if (tid == 0) {
+        if (tid == EPI_ISSUER) {
             if (TMA) tc::mbar_init(&ebar, 1);
             if (FTMA) tc::mbar_init(&fbar, 1);
             efail = 0;
             tc::mbar_fence_init();
+            // the first plane's operands, beside the prologue's field loads (the
+            // first step's barrier shows the initialised barriers to the waiters)
+            if constexpr (TMA) {
+                issue_epi(zb);
+                last_phase = 0;
+            }
         }
     }
 
@@ -270,12 +363,17 @@ __global__ void __launch_bounds__(NT, MODE == FM_CG_UPDATE_JACOBI ? ((STG & 1) ?
         }
     };
 
+    // the first three planes' loads all in flight before the first is used: on
+    // small grids a CTA has few planes and this latency is most of its time
     float vc[3], vh[3];
-    fetch(zb - 1, vc, vh);
-    store(ring[(zb - 1 + RING) % RING], vc, vh);
-    fetch(zb, vc, vh);
-    store(ring[zb % RING], vc, vh);
-    fetch(zb + 1, vc, vh);
+    {
+        float va[3], ha[3], vb[3], hb[3];
+        fetch(zb - 1, va, ha);
+        fetch(zb, vb, hb);
+        fetch(zb + 1, vc, vh);
+        store(ring[(zb - 1 + RING) % RING], va, ha);
+        store(ring[zb % RING], vb, hb);
+    }
 
     const bool own = cy <= g.ny && cx <= g.nx;
     uint32_t f_next = 0, e8_next = 0;
@@ -337,16 +435,13 @@ __global__ void __launch_bounds__(NT, MODE == FM_CG_UPDATE_JACOBI ? ((STG & 1) ?
             }
         }
         if constexpr (TMA) {
-            if (tid == EPI_ISSUER && !efail) {
+            if (tid == EPI_ISSUER && !efail && iz > zb) {
                 // the previous plane's copies have landed long ago; waiting for
                 // them keeps one phase of the barrier in flight at a time
                 const int k = iz - zb;
-                if (k == 0 || tc::mbar_wait_bounded(&ebar, (k - 1) & 1, EPI_WAIT_NS)) {
-                    const int na = a.first ? 4 : EPI_ARRAYS;
+                if (tc::mbar_wait_bounded(&ebar, (k - 1) & 1, EPI_WAIT_NS)) {
                     fence_proxy_async_cta();
-                    mbar_expect_tx(&ebar, (uint32_t)(na * EPI_BOX * 4));
-                    for (int j = 0; j < na; ++j)
-                        tma_load_plane(stage + j * EPI_BOX, &em.m[j], y0 + Grid::YOFF, x0 + 1, iz + 1, &ebar);
+                    issue_epi(iz);
                     last_phase = k;
                 } else {
                     efail = 1;
@@ -449,18 +544,21 @@ static int pick_zc(const Grid& g, const Ctx& c, int per_sm = 3) {
     int64_t zc = (cols * (g.nz + 1) + want - 1) / want;
     // at least 6 planes per CTA where that still leaves four CTAs per SM (each
     // chunk stages two planes beyond its own: coarse levels 22.17 -> 21.96 ms
-    // per solve against 4; 8 was slower), else at least 4 (small grids keep
-    // their CTAs spread over all SMs)
-    // (the 42x37x64 model: 31.9 ms with 6 everywhere, 30.1 ms so)
-    const int64_t zmin = cols * ((g.nz + 1 + 5) / 6) < 4 * (int64_t)c.num_sms ? 4 : 6;
+    // per solve against 4; 8 was slower), else at least 4 where that does;
+    // smaller grids take one plane per CTA: there a CTA's chain of planes is
+    // the launch's time, not the planes staged twice (42 x 37 x 64 solve, the
+    // chunks of its three levels at 4 / 3 / 2 / 1 planes: 22.4 / 20.3 / 19.2 /
+    // 18.5 ms)
+    const int64_t full = 4 * (int64_t)c.num_sms;
+    const int64_t zmin = cols * ((g.nz + 1 + 5) / 6) >= full ? 6 : (cols * ((g.nz + 1 + 3) / 4) >= full ? 4 : 1);
     if (zc < zmin) zc = zmin;
     if (zc > 64) zc = 64;
     return (int)zc;
 }
 
 int fine_grid_blocks(const Grid& g) {
-    // upper bound over the z-chunk choices (zc >= 4)
-    return ((g.ny + 1 + TY - 1) / TY) * ((g.nx + 1 + TX - 1) / TX) * ((g.nz + 1 + 3) / 4);
+    // upper bound over the z-chunk choices
+    return ((g.ny + 1 + TY - 1) / TY) * ((g.nx + 1 + TX - 1) / TX) * (g.nz + 1);
 }
 
 // true when cf holds exactly the compiled-in default-material tables (then
@@ -540,16 +638,22 @@ static void launch_stg(Ctx& c, dim3 grid, const FineLevel& L, const Coef32& cf, 
             opted.fetch_or(bit);
         }
     }
-    k_fine<MODE, DEF, STG><<<grid, dim3(TY, TX, 1), dyn, c.stream>>>(L, cf, a, zc, em);
+    launch_chain(c, k_fine<MODE, DEF, STG>, grid, dim3(TY, TX, 1), dyn, L, cf, a, zc, em);
 }
 
 template <int MODE>
-void launch_fine(Ctx& c, const FineLevel& L, const Coef32& cf, const FineArgs& a) {
+void launch_fine(Ctx& c, const FineLevel& L, const Coef32& cf, const FineArgs& args) {
+    FineArgs a = args;
     // the CG update with its staged operands: longer z-chunks (2 instead of 3
     // in the wave count: 1.820 -> 1.792 ms, 1 gave 1.820 ms; the other modes
     // were slower with 2)
     const int zc = pick_zc(L.g, c, MODE == FM_CG_UPDATE_JACOBI ? 2 : 3);
     dim3 grid((L.g.ny + 1 + TY - 1) / TY, (L.g.nx + 1 + TX - 1) / TX, (L.g.nz + 1 + zc - 1) / zc);
+    if (MODE == FM_VCYCLE_DOWN && a.n_perel > 0) {
+        const int per = (NT / 8) * (int)(grid.x * grid.y);
+        a.perel_z = (a.n_perel + per - 1) / per;
+        grid.z += a.perel_z;
+    }
     const bool def = coef_is_default(cf);
     EpiMaps em;
     std::memset(&em, 0, sizeof(em));
@@ -582,7 +686,6 @@ void launch_fine(Ctx& c, const FineLevel& L, const Coef32& cf, const FineArgs& a
         if (ftma) go(std::integral_constant<int, 2>{});
         else go(std::integral_constant<int, 0>{});
     }
-    GMGS_LAUNCHED(c);
 }
 template void launch_fine<FM_PLAIN>(Ctx&, const FineLevel&, const Coef32&, const FineArgs&);
 template void launch_fine<FM_VCYCLE_DOWN>(Ctx&, const FineLevel&, const Coef32&, const FineArgs&);
@@ -610,10 +713,10 @@ __device__ __forceinline__ float up_post(float w, float r, float rp, float wp, f
 template <bool DOT>
 __global__ void __launch_bounds__(256, 4) k_up32(Grid gf, Grid gc, const uint8_t* __restrict__ nflag,
                                               const uint8_t* __restrict__ tile_occ, int zc,
-                                              const float* __restrict__ wdinv, const float* __restrict__ r,
-                                              const float* __restrict__ rp, const float* __restrict__ xc,
-                                              float* __restrict__ xf, int zero_fixed, DotOut dout) {
+                                              const float* __restrict__ wdinv, const float* r, const float* rp,
+                                              const float* xc, float* xf, int zero_fixed, DotOut dout) {
     __shared__ double sh[32];
+    pdl_begin();
     const int Sf = (int)gf.slots, Sc = (int)gc.slots;
     const int csx = gc.py, csz = gc.py * gc.px, fsz = gf.py * gf.px;
     const int iy = blockIdx.x * TY + threadIdx.x, ix = blockIdx.y * TX + threadIdx.y;
@@ -659,6 +762,7 @@ __global__ void __launch_bounds__(256, 4) k_up32(Grid gf, Grid gc, const uint8_t
             }
         };
         bool okc = zb < ze && occ(zb);
+        pdl_wait();
         if (okc) fetch(zb, flc, wdc, rc, rpc);
         for (int iz = zb; iz < ze; ++iz) {
             const bool okn = iz + 1 < ze && occ(iz + 1);
@@ -701,6 +805,7 @@ __global__ void __launch_bounds__(256, 4) k_up32(Grid gf, Grid gc, const uint8_t
             okc = okn;
         }
     }
+    pdl_wait();      // threads outside the grid: before the partial sums are touched
     if (DOT) grid_dot_finish(dot.value(), dout, sh);
 }
 
@@ -716,18 +821,13 @@ void launch_up32(Ctx& c, const Grid& gf, const Grid& gc, const uint8_t* nflag, c
     const int zc = up32_zc(gf, c);
     const dim3 grid((gf.ny + 1 + TY - 1) / TY, (gf.nx + 1 + TX - 1) / TX, (gf.nz + 1 + zc - 1) / zc);
     const dim3 blk(TY, TX, 1);
-    if (dot) {
-        k_up32<true><<<grid, blk, 0, c.stream>>>(gf, gc, nflag, tile_occ, zc, wdinv, r, rp, xc, xf, zero_fixed, *dot);
-    } else {
-        k_up32<false><<<grid, blk, 0, c.stream>>>(gf, gc, nflag, tile_occ, zc, wdinv, r, rp, xc, xf, zero_fixed,
-                                                   DotOut{});
-    }
-    GMGS_LAUNCHED(c);
+    launch_chain(c, dot ? k_up32<true> : k_up32<false>, grid, blk, 0, gf, gc, nflag, tile_occ, zc, wdinv, r, rp, xc, xf,
+                 zero_fixed, dot ? *dot : DotOut{});
 }
 
-// upper bound of the k_up32 grid over the z-chunk choices (zc >= 2)
+// upper bound of the k_up32 grid over the z-chunk choices
 int up32_grid_blocks(const Grid& g) {
-    return ((g.ny + 1 + TY - 1) / TY) * ((g.nx + 1 + TX - 1) / TX) * ((g.nz + 1 + 1) / 2);
+    return ((g.ny + 1 + TY - 1) / TY) * ((g.nx + 1 + TX - 1) / TX) * (g.nz + 1);
 }
 
 // (x_hi, x_lo) -= the last, not yet cancelled Jacobi step dx = fl32(fl32(r32 - alpha q) * w),
@@ -775,76 +875,13 @@ void launch_df_split(Ctx& c, int64_t n, const double* b, float* hi, float* lo) {
     GMGS_LAUNCHED(c);
 }
 
-// ---------------------------------------------------------------------------
-// V-cycle down-sweep at nodes that touch elements with their own Galerkin
-// matrix: eight lanes per node (four nodes per warp).  For each of the
-// node's 8 elements, lane j multiplies the node's three rows of the element
-// matrix at columns 3j..3j+2 (the coupling to element node j) with node j's
-// Jacobi step w r; each lane keeps the three row sums across the elements and
-// a shuffle reduction over the 8 lanes (xor 1, 2, 4) adds them up.  The
-// per-lane sums and the reduction order are those of a lane per (row,
-// column group), so the result does not depend on the lane layout.
-// out = r - A (w r) with fixed rows zeroed (AtX.m:57).
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_perel_vdown(FineLevel L, const __grid_constant__ Coef32 cf,
-                                                     const int32_t* __restrict__ nodes, int count,
-                                                     const float* __restrict__ r, const float* __restrict__ w,
-                                                     float* __restrict__ out) {
-    const int gl = blockIdx.x * blockDim.x + threadIdx.x;
-    const int node = gl >> 3, j = gl & 7;
-    const bool active = node < count;          // whole 8-lane groups; idle groups still shuffle
-    const Grid& g = L.g;
-    const int S = (int)g.slots, sx = g.py, sz = g.py * g.px;
-    const int n = active ? chk::ld(nodes, node, count, chk::PEREL_NODE) : 0;
-    const long long n3 = 3ll * S;
-    float acc[3] = {0.f, 0.f, 0.f};
-    if (active) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const int A = e & 1, B = (e >> 1) & 1, C = e >> 2;
-            const int es = n - A - B * sx - C * sz;
-            if (!chk::ld(L.emask, es, S, chk::PEREL_ELEM)) continue;   // uniform across the node's lanes
-            const int ci = corner_of(A, B, C);
-            const int t = L.etype ? chk::ld(L.etype, es, S, chk::PEREL_ELEM) : 0;
-            const int nj = es + corner_y(j) + corner_x(j) * sx + corner_z(j) * sz;
-            constexpr int V = chk::PEREL_VEC;
-            const float d0 = chk::ld(r, nj, n3, V) * chk::ld(w, nj, n3, V);
-            const float d1 = chk::ld(r, nj + S, n3, V) * chk::ld(w, nj + S, n3, V);
-            const float d2 = chk::ld(r, nj + 2 * S, n3, V) * chk::ld(w, nj + 2 * S, n3, V);
-            if (t > 0 && !chk::ok(t - 1, L.nK, chk::PEREL_KS)) continue;
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                const int off = (3 * ci + a) * 24 + 3 * j;
-                if (t > 0) {
-                    const float* K = L.Ks + (int64_t)(t - 1) * KE + off;
-                    acc[a] = fmaf(K[0], d0, fmaf(K[1], d1, fmaf(K[2], d2, acc[a])));
-                } else {
-                    const float k = L.kscale;
-                    acc[a] = fmaf(k * cf.K[off], d0, fmaf(k * cf.K[off + 1], d1, fmaf(k * cf.K[off + 2], d2, acc[a])));
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        acc[a] += __shfl_xor_sync(0xffffffffu, acc[a], 1);
-        acc[a] += __shfl_xor_sync(0xffffffffu, acc[a], 2);
-        acc[a] += __shfl_xor_sync(0xffffffffu, acc[a], 4);
-    }
-    if (active && j < 3) {
-        const uint32_t f = chk::ld(L.nflag, n, S, chk::PEREL_ELEM);
-        const float y = j == 0 ? acc[0] : (j == 1 ? acc[1] : acc[2]);
-        const int i = n + j * S;
-        chk::st(out, i, n3, chk::PEREL_OUT, chk::ld(r, i, n3, chk::PEREL_VEC) - ((f & (NF_FIX_X << j)) ? 0.f : y));
-    }
+// the down-sweep of a level whose nodes all lie on stored matrices
+__global__ void __launch_bounds__(NT) k_perel_vdown(FineLevel L, const __grid_constant__ Coef32 cf, FineArgs a) {
+    pdl_begin();
+    perel_node(L, cf, a, (int)blockIdx.x * (NT / 8) + (int)threadIdx.x / 8, threadIdx.x & 7);
 }
-
-void launch_perel_vdown(Ctx& c, const FineLevel& L, const Coef32& cf, const int32_t* nodes, int count, const float* r,
-                        const float* w, float* out) {
-    if (count <= 0) return;
-    const int blocks = (int)(((int64_t)count * 8 + 255) / 256);
-    k_perel_vdown<<<blocks, 256, 0, c.stream>>>(L, cf, nodes, count, r, w, out);
-    GMGS_LAUNCHED(c);
+void launch_perel_vdown(Ctx& c, const FineLevel& L, const Coef32& cf, const FineArgs& a) {
+    launch_chain(c, k_perel_vdown, (a.n_perel + NT / 8 - 1) / (NT / 8), NT, 0, L, cf, a);
 }
 
 // occupancy of the streaming kernel's node tiles: one block per (y tile,

@@ -60,6 +60,9 @@ struct FineArgs {
     float* x_lo = nullptr;
     float* r32out = nullptr;         // high part of the updated residual (must not alias r32)
     DotOut dot;
+    const int32_t* perel = nullptr;  // FM_VCYCLE_DOWN: slots of the nodes on stored matrices
+    int n_perel = 0;
+    int perel_z = 0;                 // grid layers that take them (set by the launcher)
     int* err = nullptr;              // set when a bounded wait for staged operands ran out
 };
 
@@ -306,8 +309,8 @@ void launch_up32(Ctx& c, const Grid& gf, const Grid& gc, const uint8_t* nflag, c
                  const float* wdinv, const float* r, const float* rp, const float* xc, float* xf, bool zero_fixed,
                  const DotOut* dot);
 void launch_wdinv(Ctx& c, int64_t n, const double* d, double omega, float* w);
-void launch_perel_vdown(Ctx& c, const FineLevel& L, const Coef32& cf, const int32_t* nodes, int count, const float* r,
-                        const float* w, float* out);
+// the down-sweep of the perel nodes alone
+void launch_perel_vdown(Ctx& c, const FineLevel& L, const Coef32& cf, const FineArgs& a);
 void launch_emask8(Ctx& c, const Grid& g, const uint8_t* emask, uint8_t* e8);
 size_t tile_occ_bytes(const Grid& g);
 void launch_tile_occ(Ctx& c, const Grid& g, const uint8_t* nflag, uint8_t* occ);

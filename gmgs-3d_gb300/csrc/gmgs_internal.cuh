@@ -22,6 +22,7 @@
 #include <functional>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "gmgs.h"
@@ -321,6 +322,37 @@ struct Ctx {
         if (stop) s.bytes += bytes;
     }
 };
+
+// ---------------------------------------------------------------------------
+// programmatic dependent launch
+// ---------------------------------------------------------------------------
+// The kernels of a PCG iteration form one chain in their stream, each reading
+// what the one before wrote.  launch_chain() makes a launch a programmatic
+// dependent of the previous kernel: its CTAs are placed while that kernel
+// drains, and pdl_wait() holds them (the hardware grid dependency) until the
+// previous grid has completed and its writes are visible.  Every kernel
+// launched this way calls pdl_begin() first and touches nothing that an
+// earlier kernel of the chain writes before pdl_wait(); the grid before has
+// waited for its own predecessor, so the order is transitive.  Pointers to
+// such data carry no __restrict__: a load the compiler takes for invariant
+// could move above the wait.
+__device__ __forceinline__ void pdl_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... P, typename... A>
+void launch_chain(Ctx& c, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c.stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    GMGS_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(std::forward<A>(args))...));
+    GMGS_LAUNCHED(c);
+}
 
 // ---------------------------------------------------------------------------
 // kernels and launchers (operators.cu, setup.cu, post.cu)

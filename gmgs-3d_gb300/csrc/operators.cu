@@ -43,15 +43,16 @@ __device__ __forceinline__ double restrict_acc(double acc, double v, bool centre
 }
 
 template <typename T>
-__global__ void k_restrict(Grid gf, Grid gc, const uint8_t* __restrict__ nflag_c, const T* __restrict__ rf,
-                           T* __restrict__ rc) {
+__global__ void k_restrict(Grid gf, Grid gc, const uint8_t* __restrict__ nflag_c, const T* rf, T* rc) {
     const int Iy = blockIdx.x * blockDim.x + threadIdx.x;
     const int Ix = blockIdx.y * blockDim.y + threadIdx.y;
     const int Iz = blockIdx.z;
+    pdl_begin();
     if (Iy > gc.ny || Ix > gc.nx) return;
     const int64_t cs = gc.slot(Iy, Ix, Iz);
     const int64_t Sf = gf.slots, Sc = gc.slots, sx = gf.sx(), sz = gf.sz();
     constexpr int R = chk::RESTRICT;
+    pdl_wait();
     if (!(chk::ld(nflag_c, cs, Sc, R) & NF_SOLID)) {
         chk::st(rc, cs, 3 * Sc, R, 0);
         chk::st(rc, cs + Sc, 3 * Sc, R, 0);
@@ -81,8 +82,7 @@ __global__ void k_restrict(Grid gf, Grid gc, const uint8_t* __restrict__ nflag_c
 template <typename T>
 void launch_restrict(Ctx& c, const Grid& gf, const Grid& gc, const uint8_t* nflag_c, const T* rf, T* rc) {
     dim3 blk(32, 4, 1);
-    k_restrict<T><<<node_grid(gc, blk), blk, 0, c.stream>>>(gf, gc, nflag_c, rf, rc);
-    GMGS_LAUNCHED(c);
+    launch_chain(c, k_restrict<T>, node_grid(gc, blk), blk, 0, gf, gc, nflag_c, rf, rc);
 }
 template void launch_restrict<double>(Ctx&, const Grid&, const Grid&, const uint8_t*, const double*, double*);
 template void launch_restrict<float>(Ctx&, const Grid&, const Grid&, const uint8_t*, const float*, float*);
@@ -146,26 +146,26 @@ template void launch_dot<double, double>(Ctx&, const DotScratch&, int64_t, const
 // coarsest level: free-DOF gather and scatter
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void k_gather(int64_t n, const int32_t* __restrict__ idx, const T* __restrict__ src,
-                         double* __restrict__ dst) {
+__global__ void k_gather(int64_t n, const int32_t* __restrict__ idx, const T* src, double* dst) {
+    pdl_begin();
+    pdl_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         dst[i] = (double)src[idx[i]];
 }
 template <typename T>
-__global__ void k_scatter(int64_t n, const int32_t* __restrict__ idx, const double* __restrict__ src,
-                          T* __restrict__ dst) {
+__global__ void k_scatter(int64_t n, const int32_t* __restrict__ idx, const double* src, T* dst) {
+    pdl_begin();
+    pdl_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         dst[idx[i]] = (T)src[i];
 }
 template <typename T>
 void launch_gather(Ctx& c, int64_t n, const int32_t* idx, const T* src, double* dst) {
-    k_gather<T><<<ew_blocks(c, n), 256, 0, c.stream>>>(n, idx, src, dst);
-    GMGS_LAUNCHED(c);
+    launch_chain(c, k_gather<T>, ew_blocks(c, n), 256, 0, n, idx, src, dst);
 }
 template <typename T>
 void launch_scatter(Ctx& c, int64_t n, const int32_t* idx, const double* src, T* dst) {
-    k_scatter<T><<<ew_blocks(c, n), 256, 0, c.stream>>>(n, idx, src, dst);
-    GMGS_LAUNCHED(c);
+    launch_chain(c, k_scatter<T>, ew_blocks(c, n), 256, 0, n, idx, src, dst);
 }
 template void launch_gather<double>(Ctx&, int64_t, const int32_t*, const double*, double*);
 template void launch_gather<float>(Ctx&, int64_t, const int32_t*, const float*, double*);

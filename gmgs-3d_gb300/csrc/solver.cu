@@ -286,18 +286,18 @@ static void vcycle32(Model& M, const float* r32, float* z, bool with_dot, int do
         }
         if (l == 1) c.mark(PK_COARSE, false);
         const FineLevel fl = fine_level(lv);
+        a.perel = lv.perel_nodes.as<int32_t>();
+        a.n_perel = (int)lv.n_perel;
         if (M.use_tc && lv.n_perel < lv.n_node) {
             FineLevel ft = fl;
             ft.tile_occ = lv.tc_occ.as<uint8_t>();
             launch_tc_vdown(c, ft, M.tcoef, a.r32, a.wdinv, a.out32, M.tc_err.as<int>());
-        } else if (l == 0) {
-            launch_l0<FM_VCYCLE_DOWN>(M, fl, a);
+            if (lv.n_perel > 0) launch_perel_vdown(c, fl, M.coef, a);
         } else if (lv.n_perel < lv.n_node) {
             launch_fine<FM_VCYCLE_DOWN>(c, fl, M.coef, a);
+        } else {
+            launch_perel_vdown(c, fl, M.coef, a);
         }
-        if (lv.n_perel > 0)
-            launch_perel_vdown(c, fl, M.coef, lv.perel_nodes.as<int32_t>(), (int)lv.n_perel, a.r32, a.wdinv,
-                               a.out32);
         if (l == 0) {
             c.mark(PK_FINE_MATVEC, true, bytes);
             c.mark(PK_VDOWN0, true, bytes);
