@@ -187,7 +187,7 @@ int64_t model_bytes(const gmgs::Model& M) {
     for (const auto& lv : M.levels)
         for (const gmgs::DevBuf* d : {&lv.emask, &lv.nflag, &lv.etype, &lv.escale64, &lv.escale32, &lv.Ks64, &lv.Ks32,
                                       &lv.kslot, &lv.diag64, &lv.wdinv32, &lv.wdinv64, &lv.bnd_nodes, &lv.emask8, &lv.perel_nodes, &lv.node_slot, &lv.elem_slot,
-                                      &lv.vr, &lv.vrp, &lv.vx, &lv.tile_occ, &lv.tc_occ})
+                                      &lv.vr, &lv.vrp, &lv.vx, &lv.tile_occ, &lv.tile_occ64, &lv.tc_occ})
             b += (int64_t)d->bytes;
     for (const gmgs::DevBuf* d : {&M.ke0_dev, &M.rho, &M.F, &M.U, &M.free_idx, &M.cb.sinv, &M.cb.g, &M.cb.gt, &M.cvec_in, &M.cvec_out,
                                   &M.cg_x, &M.cg_r, &M.cg_rb, &M.cg_p, &M.cg_p2, &M.cg_q64, &M.cg_z64, &M.mask_stencil, &M.cg_q32,

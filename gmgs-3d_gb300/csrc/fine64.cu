@@ -41,13 +41,14 @@ namespace gmgs {
 
 namespace {
 
-constexpr int TY = 32, TX = 8;
+constexpr int TY = 16, TX = 16;
 constexpr int NT = TY * TX;
 constexpr int HY = TY + 2, HX = TX + 2;
 constexpr int NP = HY * HX;          // points of a tile plane with its one-node halo
 constexpr int NHALO = NP - NT;       // 84
 constexpr int NXP = HY * TX;         // points of the x stage: the tile's columns with the y halo
-constexpr int LANES = 8;             // lanes per list node
+constexpr int BND_LANES = 4;         // lanes per boundary node
+constexpr int ELEM_LANES = 8;        // lanes per node on stored matrices
 
 __host__ __device__ constexpr int field_arrays64(int mode) {
     return mode == M64_PLAIN ? 1 : (mode == M64_CG_UPDATE_JACOBI ? 3 : 2);
@@ -122,58 +123,65 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// sum over the 8 lanes of a list node
+// sum over the N lanes of a list node
+template <int N>
 __device__ __forceinline__ double lanes_sum(double v) {
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    v += __shfl_xor_sync(0xffffffffu, v, 2);
-    v += __shfl_xor_sync(0xffffffffu, v, 4);
+#pragma unroll
+    for (int o = 1; o < N; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 
-// one list node (8 lanes, j = lane): bnd: the assembled stencil of its solid
-// elements, lane j taking the offsets j, j + 8, ...; else the element sum,
-// lane j taking the coupling to element node j
-template <int MODE>
-__device__ void list_node(const Level64& L, const Args64& a, bool bnd, int at, int j, double ab, double& dot) {
+// A boundary node, 4 lanes: the assembled stencil of its solid elements, lane
+// j taking the j-th, j+4-th, ... of the offsets those elements reach (18 of 27
+// on a face).  Fewer lanes per node spend fewer FP64 operations on the sum
+// across them (8 lanes over all 27 offsets: 560 lane operations per node of
+// the update; 4 over the reached ones: 330).
+// A node on stored matrices, 8 lanes: the element sum, lane j taking the
+// coupling to element node j.
+template <int MODE, bool BND>
+__device__ void list_node(const Level64& L, const Args64& a, int at, int j, double ab, double& dot) {
     const Grid& g = L.g;
     const int64_t S = g.slots, n3 = 3 * S, sx = g.sx(), sz = g.sz();
-    const int count = bnd ? L.n_bnd : L.n_perel;
+    const int count = BND ? L.n_bnd : L.n_perel;
     const bool active = at < count;
-    const int64_t n = active ? chk::ld(bnd ? L.bnd : L.perel, at, count, chk::F64_LIST) : 0;
+    const int64_t n = active ? chk::ld(BND ? L.bnd : L.perel, at, count, chk::F64_LIST) : 0;
     double y[3] = {0.0, 0.0, 0.0};
-    if (active && bnd) {
-        uint32_t mask = 0;
+    // the 8 elements around the node, all loads in flight together: -1 void, 0 uniform, k the stored matrix k - 1
+    int type[8];
+    uint32_t mask = 0;
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-            if (chk::ld(L.emask, n - (e & 1) - ((e >> 1) & 1) * sx - (e >> 2) * sz, S, chk::F64_LIST)) mask |= 1u << e;
-        const double* T = L.mask_stencil + (int64_t)mask * MASK_STENCIL;
+    for (int e = 0; e < 8; ++e) {
+        const int64_t es = n - (e & 1) - ((e >> 1) & 1) * sx - (e >> 2) * sz;
+        type[e] = -1;
+        if (active && chk::ld(L.emask, es, S, chk::F64_LIST)) {
+            mask |= 1u << e;
+            type[e] = !BND && L.etype ? chk::ld(L.etype, es, S, chk::F64_LIST) : 0;
+            if (type[e] > 0 && !chk::ok(type[e] - 1, L.nK, chk::F64_LIST)) type[e] = -1;
+        }
+    }
+    if (BND) {
+        const MaskStencil& T = L.mask_stencil[mask];      // mask 0 (idle lanes): no offsets
+        for (int t = j; t < T.n; t += BND_LANES) {
+            const int k = T.k[t];
+            const int64_t m = n + off_y(k) + off_x(k) * sx + off_z(k) * sz;
+            double v[3], s;
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const int k = j + t * LANES;
-            if (k < 27) {
-                const int64_t m = n + off_y(k) + off_x(k) * sx + off_z(k) * sz;
-                double v[3], s;
+            for (int b = 0; b < 3; ++b) form_at<MODE>(a, m + b * S, n3, ab, v[b], s);
 #pragma unroll
-                for (int b = 0; b < 3; ++b) form_at<MODE>(a, m + b * S, n3, ab, v[b], s);
+            for (int c = 0; c < 3; ++c)
 #pragma unroll
-                for (int c = 0; c < 3; ++c)
-#pragma unroll
-                    for (int b = 0; b < 3; ++b) y[c] = fma(T[9 * k + 3 * c + b], v[b], y[c]);
-            }
+                for (int b = 0; b < 3; ++b) y[c] = fma(T.S[t][3 * c + b], v[b], y[c]);
         }
 #pragma unroll
-        for (int c = 0; c < 3; ++c) y[c] *= L.kscale;
-    } else if (active) {
-#pragma unroll 2
+        for (int c = 0; c < 3; ++c) y[c] = L.kscale * lanes_sum<BND_LANES>(y[c]);
+    } else {
+#pragma unroll
         for (int e = 0; e < 8; ++e) {
+            if (type[e] < 0) continue;                    // uniform across the node's lanes
             const int A = e & 1, B = (e >> 1) & 1, C = e >> 2;
-            const int64_t es = n - A - B * sx - C * sz;
-            if (!chk::ld(L.emask, es, S, chk::F64_LIST)) continue;      // uniform across the node's lanes
-            const int t = L.etype ? chk::ld(L.etype, es, S, chk::F64_LIST) : 0;
-            if (t > 0 && !chk::ok(t - 1, L.nK, chk::F64_LIST)) continue;
-            const int64_t m = es + corner_y(j) + corner_x(j) * sx + corner_z(j) * sz;
-            const double* K = (t > 0 ? L.Ks + (int64_t)(t - 1) * KE : L.ke0) + 3 * corner_of(A, B, C) * 24 + 3 * j;
-            const double k = t > 0 ? 1.0 : L.kscale;
+            const int64_t m = n - A - B * sx - C * sz + corner_y(j) + corner_x(j) * sx + corner_z(j) * sz;
+            const double* K = (type[e] > 0 ? L.Ks + (int64_t)(type[e] - 1) * KE : L.ke0) + 3 * corner_of(A, B, C) * 24 + 3 * j;
+            const double k = type[e] > 0 ? 1.0 : L.kscale;
             double v[3], s;
 #pragma unroll
             for (int b = 0; b < 3; ++b) {
@@ -185,9 +193,9 @@ __device__ void list_node(const Level64& L, const Args64& a, bool bnd, int at, i
 #pragma unroll
                 for (int b = 0; b < 3; ++b) y[c] = fma(K[24 * c + b], v[b], y[c]);
         }
-    }
 #pragma unroll
-    for (int c = 0; c < 3; ++c) y[c] = lanes_sum(y[c]);
+        for (int c = 0; c < 3; ++c) y[c] = lanes_sum<ELEM_LANES>(y[c]);
+    }
     if (active && j < 3) {
         const uint32_t f = chk::ld(L.nflag, n, S, chk::F64_LIST);
         const int64_t i = n + j * S;
@@ -254,8 +262,8 @@ constexpr size_t fine64_smem() {
 }
 
 // ---------------------------------------------------------------------------
-// K x with the uniform matrix, axis by axis.  A CTA owns a 32 (y, lanes) x 8
-// (x) column of nodes and walks a chunk of z planes.  Per plane:
+// K x with the uniform matrix, axis by axis.  A CTA owns a 16 (y) x 16 (x)
+// column of nodes and walks a chunk of z planes.  Per plane:
 //   - the field of plane z + 1 is formed from its inputs, which cp.async has
 //     brought to this thread's own places in shared memory one plane ahead
 //     (each thread reads back only what it copied: no barrier)
@@ -265,6 +273,8 @@ constexpr size_t fine64_smem() {
 //     and their y halo                                     (33 operations, 9/8 warps)
 //   - y stage and the mode's vector updates at the interior nodes
 // Two barriers per plane; two CTAs per SM keep the FP64 pipe fed across them.
+// The square tile wastes fewer lanes than 32 x 8 on grids a little over a
+// multiple of 32 (84 x 73 x 128: 82 against 74 % of the tile's nodes used).
 // ---------------------------------------------------------------------------
 template <int MODE>
 __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_constant__ Coef64 cf, Args64 a, int zc, int nb_bnd,
@@ -273,12 +283,16 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
     extern __shared__ double dyn[];
     const int tid = threadIdx.x;
     const Grid& g = L.g;
+    pdl_begin();
+    pdl_wait();
     const double ab = step_length<MODE>(a);
     double dot = 0.0;
     if ((int)blockIdx.x < nb_list) {
-        const bool bnd = (int)blockIdx.x < nb_bnd;
-        const int at = ((int)blockIdx.x - (bnd ? 0 : nb_bnd)) * (NT / LANES) + tid / LANES;
-        list_node<MODE>(L, a, bnd, at, tid % LANES, ab, dot);
+        if ((int)blockIdx.x < nb_bnd)
+            list_node<MODE, true>(L, a, (int)blockIdx.x * (NT / BND_LANES) + tid / BND_LANES, tid % BND_LANES, ab, dot);
+        else
+            list_node<MODE, false>(L, a, ((int)blockIdx.x - nb_bnd) * (NT / ELEM_LANES) + tid / ELEM_LANES, tid % ELEM_LANES,
+                                   ab, dot);
         dot_finish<MODE>(dot, a, sh);
         return;
     }
@@ -378,7 +392,7 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
         Rr[2] = mx(7);
     };
     const int xc = (p.pc % HY) + (tid / TY) * HY;                // own point of the x stage
-    const int hxc = tid & 15, hyy = (hxc & 1) ? HY - 1 : 0;      // the y halo's points: 16 threads
+    const int hxc = tid & (2 * TX - 1), hyy = (hxc & 1) ? HY - 1 : 0;      // the y halo's points: one warp
     const int hz_pt = hyy + ((hxc >> 1) + 1) * HY, hx_pt = hyy + (hxc >> 1) * HY;
 
 #pragma unroll 1
@@ -404,7 +418,7 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
             if (tid < NHALO) z_stage(p.ph, hm, hc, hp);
             __syncthreads();
             double P[3], Q[3], Rr[3];
-            if (tid < 16) {
+            if (tid < 2 * TX) {
                 x_stage(hz_pt, P, Q, Rr);
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
@@ -413,12 +427,15 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
                     chk::st(Xb, (6 + c) * NXP + hx_pt, 9 * NXP, R, Rr[c]);
                 }
             }
-            x_stage(p.pc, P, Q, Rr);
+            // a warp holds whole y columns of the tile, so its x stage is read by its own y stage alone
+            if (__any_sync(0xffffffffu, node)) {
+                x_stage(p.pc, P, Q, Rr);
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                chk::st(Xb, c * NXP + xc, 9 * NXP, R, P[c]);
-                chk::st(Xb, (3 + c) * NXP + xc, 9 * NXP, R, Q[c]);
-                chk::st(Xb, (6 + c) * NXP + xc, 9 * NXP, R, Rr[c]);
+                for (int c = 0; c < 3; ++c) {
+                    chk::st(Xb, c * NXP + xc, 9 * NXP, R, P[c]);
+                    chk::st(Xb, (3 + c) * NXP + xc, 9 * NXP, R, Q[c]);
+                    chk::st(Xb, (6 + c) * NXP + xc, 9 * NXP, R, Rr[c]);
+                }
             }
             __syncthreads();
             if (node) {
@@ -539,6 +556,8 @@ __global__ void __launch_bounds__(NT, 2) k_modal64(Level64 L, const __grid_const
     extern __shared__ double dyn[];
     const int tid = threadIdx.x;
     const Grid& g = L.g;
+    pdl_begin();
+    pdl_wait();
     const double ab = step_length<MODE>(a);
     const int bty = blockIdx.x % tiles_y, btx = blockIdx.x / tiles_y % tiles_x, btz = blockIdx.x / (tiles_y * tiles_x);
     const int y0 = bty * TY, x0 = btx * TX;
@@ -700,14 +719,20 @@ __global__ void __launch_bounds__(NT, 2) k_modal64(Level64 L, const __grid_const
     dot_finish<MODE>(dot, a, sh);
 }
 
-// z planes per CTA: about 12 waves of two resident CTAs per SM on large grids,
-// at least 4 planes there (each chunk forms two planes beyond its own), down
-// to 2 where the grid would otherwise leave SMs without a CTA
+// z planes per CTA: about 12 waves of two resident CTAs per SM on large grids
+// (169 x 147 x 256 solve: 8 planes 161 ms; 4, 6 and 12 planes 162 to 163 ms),
+// at least 2 where that gives every SM two CTAs (each chunk forms two planes
+// beyond its own; 42 x 37 x 64 solve with 1 / 2 / 3 / 4 / 6 planes on its
+// finest level: 39.1 / 38.3 / 42 / 50 / 60 ms), else zmin: a plane per CTA for
+// the factorised form (its coarse levels at 1 / 2 / 3 / 4 planes: 39.1 / 40.3 /
+// 42.6 / 44.5 ms), 2 for the modal one, whose chunks compute a layer more
+// (density gradient at 42 x 37 x 64 with 2 / 3 / 4 / 5 planes: 22.0 / 23.3 /
+// 24.0 / 26.6 ms)
 int pick_zc64(const Grid& g, const Ctx& c, int zmin) {
     const int64_t cols = (int64_t)((g.ny + 1 + TY - 1) / TY) * ((g.nx + 1 + TX - 1) / TX);
     const int64_t want = (int64_t)c.num_sms * 2 * 12;
     int64_t zc = (cols * (g.nz + 1) + want - 1) / want;
-    if (zc < 4) zc = cols * ((g.nz + 1 + 3) / 4) >= 4 * (int64_t)c.num_sms ? 4 : zmin;
+    if (zc < 2) zc = cols * ((g.nz + 1 + 1) / 2) >= 2 * (int64_t)c.num_sms ? 2 : zmin;
     return (int)std::min<int64_t>(zc, 32);
 }
 
@@ -747,23 +772,52 @@ Coef64 make_coef64(double E, double nu, const double ele[3]) {
     return c;
 }
 
-__global__ void k_mask_stencils(const double* __restrict__ ke0, double* __restrict__ table) {
-    const int mask = blockIdx.x;
-    for (int i = threadIdx.x; i < MASK_STENCIL; i += blockDim.x) {
-        const int k = i / 9, a = i % 9 / 3, b = i % 3;
+// occupied tiles: one block per (y tile, x tile, z plane)
+__global__ void k_tile_occ64(Grid g, const uint8_t* __restrict__ nflag, uint8_t* __restrict__ occ) {
+    const int iy = blockIdx.x * TY + threadIdx.x % TY, ix = blockIdx.y * TX + threadIdx.x / TY, iz = blockIdx.z;
+    const bool solid = iy <= g.ny && ix <= g.nx && (nflag[g.slot(iy, ix, iz)] & NF_SOLID);
+    const int any = __syncthreads_or(solid);
+    if (threadIdx.x == 0) occ[((int64_t)iz * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = any ? 1 : 0;
+}
+size_t tile_occ64_bytes(const Grid& g) {
+    return (size_t)((g.ny + 1 + TY - 1) / TY) * ((g.nx + 1 + TX - 1) / TX) * (g.nz + 1);
+}
+void launch_tile_occ64(Ctx& c, const Grid& g, const uint8_t* nflag, uint8_t* occ) {
+    const dim3 grid((g.ny + 1 + TY - 1) / TY, (g.nx + 1 + TX - 1) / TX, g.nz + 1);
+    k_tile_occ64<<<grid, NT, 0, c.stream>>>(g, nflag, occ);
+    GMGS_LAUNCHED(c);
+}
+
+__global__ void k_mask_stencils(const double* __restrict__ ke0, MaskStencil* __restrict__ table) {
+    MaskStencil& T = table[blockIdx.x];
+    const int mask = blockIdx.x, k = threadIdx.x;          // one warp, lane = offset
+    // the solid elements that hold both the node and its neighbour at offset k
+    auto holds = [&](int e, int& cn, int& cm) {
+        const int A = e & 1, B = (e >> 1) & 1, C = e >> 2;                  // node = element origin + (A, B, C)
+        const int my = A + off_y(k), mx = B + off_x(k), mz = C + off_z(k);  // neighbour relative to the origin
+        if (!((mask >> e) & 1) || my < 0 || my > 1 || mx < 0 || mx > 1 || mz < 0 || mz > 1) return false;
+        cn = corner_of(A, B, C);
+        cm = corner_of(my, mx, mz);
+        return true;
+    };
+    int cn = 0, cm = 0;
+    bool any = false;
+    if (k < 27)
+        for (int e = 0; e < 8; ++e) any = holds(e, cn, cm) || any;
+    const unsigned reach = __ballot_sync(0xffffffffu, any);
+    if (k == 0) T.n = __popc(reach);
+    if (!any) return;
+    const int t = __popc(reach & ((1u << k) - 1u));
+    T.k[t] = k;
+    for (int i = 0; i < 9; ++i) {
         double v = 0.0;
-        for (int e = 0; e < 8; ++e) {
-            if (!((mask >> e) & 1)) continue;
-            const int A = e & 1, B = (e >> 1) & 1, C = e >> 2;                  // node = element origin + (A, B, C)
-            const int my = A + off_y(k), mx = B + off_x(k), mz = C + off_z(k);  // neighbour relative to the origin
-            if (my < 0 || my > 1 || mx < 0 || mx > 1 || mz < 0 || mz > 1) continue;
-            v += ke0[(3 * corner_of(A, B, C) + a) * 24 + 3 * corner_of(my, mx, mz) + b];
-        }
-        table[(int64_t)mask * MASK_STENCIL + i] = v;
+        for (int e = 0; e < 8; ++e)
+            if (holds(e, cn, cm)) v += ke0[(3 * cn + i / 3) * 24 + 3 * cm + i % 3];
+        T.S[t][i] = v;
     }
 }
-void launch_mask_stencils(Ctx& c, const double* ke0, double* table) {
-    k_mask_stencils<<<256, 256, 0, c.stream>>>(ke0, table);
+void launch_mask_stencils(Ctx& c, const double* ke0, MaskStencil* table) {
+    k_mask_stencils<<<256, 32, 0, c.stream>>>(ke0, table);
     GMGS_LAUNCHED(c);
 }
 
@@ -773,10 +827,9 @@ void launch_fine64(Ctx& c, const Level64& L, const Coef64& cf0, const Args64& a)
     static std::atomic<unsigned long long> opted_m{0}, opted_f{0};
     if (L.escale) {
         opt_in_smem(k_modal64<MODE>, MODAL_SMEM, opted_m);
-        const int zc = pick_zc64(L.g, c, 3);
+        const int zc = pick_zc64(L.g, c, 2);
         const int blocks = ty * tx * ((L.g.nz + 1 + zc - 1) / zc);
-        k_modal64<MODE><<<blocks, NT, MODAL_SMEM, c.stream>>>(L, cf0, a, zc, ty, tx);
-        GMGS_LAUNCHED(c);
+        launch_chain(c, k_modal64<MODE>, blocks, NT, MODAL_SMEM, L, cf0, a, zc, ty, tx);
         return;
     }
     Coef64 cf = cf0;
@@ -789,46 +842,42 @@ void launch_fine64(Ctx& c, const Level64& L, const Coef64& cf0, const Args64& a)
     cf.gxz *= L.kscale;
     cf.gyz *= L.kscale;
     opt_in_smem(k_fine64<MODE>, fine64_smem<MODE>(), opted_f);
-    const int per = NT / LANES;
-    const int nb_bnd = (L.n_bnd + per - 1) / per, nb_list = nb_bnd + (L.n_perel + per - 1) / per;
-    const int zc = pick_zc64(L.g, c, 2);
+    constexpr int per_b = NT / BND_LANES, per_e = NT / ELEM_LANES;
+    const int nb_bnd = (L.n_bnd + per_b - 1) / per_b, nb_list = nb_bnd + (L.n_perel + per_e - 1) / per_e;
+    const int zc = pick_zc64(L.g, c, 1);
     // a level whose nodes are all on the lists has no tiles to walk
     const int tiles = L.n_bnd + (int64_t)L.n_perel < L.n_node ? ty * tx * ((L.g.nz + 1 + zc - 1) / zc) : 0;
-    k_fine64<MODE><<<nb_list + tiles, NT, fine64_smem<MODE>(), c.stream>>>(L, cf, a, zc, nb_bnd, nb_list, ty, tx);
-    GMGS_LAUNCHED(c);
+    launch_chain(c, k_fine64<MODE>, nb_list + tiles, NT, fine64_smem<MODE>(), L, cf, a, zc, nb_bnd, nb_list, ty, tx);
 }
 template void launch_fine64<M64_PLAIN>(Ctx&, const Level64&, const Coef64&, const Args64&);
 template void launch_fine64<M64_VCYCLE_DOWN>(Ctx&, const Level64&, const Coef64&, const Args64&);
 template void launch_fine64<M64_CG_UPDATE_JACOBI>(Ctx&, const Level64&, const Coef64&, const Args64&);
 template void launch_fine64<M64_CG_DIRECTION>(Ctx&, const Level64&, const Coef64&, const Args64&);
 
-int dot64_blocks(const Grid& g, int64_t n_list) {
-    const int64_t tiles = (int64_t)((g.ny + 1 + TY - 1) / TY) * ((g.nx + 1 + TX - 1) / TX) * ((g.nz + 1 + 1) / 2);
-    return (int)(tiles + n_list / (NT / LANES) + 2);
-}
 
 // ---------------------------------------------------------------------------
-// up-sweep (Vcycle.m:27-32): one thread per (y, x) column of a 32 x 8 tile,
+// up-sweep (Vcycle.m:27-32): one thread per (y, x) column of a 32 x 8 tile
+// (a warp holds one x, so the parity of x is uniform in it),
 // walking a chunk of z planes.  The trilinear sum adds the coarse planes
 // first, then x, then y (3.5 additions per DOF on average instead of up to 7
 // weighted terms), and omega / diagonal is stored, so no division is left.
 // ---------------------------------------------------------------------------
+constexpr int UY = 32, UX = 8;
 template <bool DOT>
-__global__ void __launch_bounds__(NT, 2) k_up64(Grid gf, Grid gc, const uint8_t* __restrict__ nflag,
-                                                const uint8_t* __restrict__ tile_occ, int zc, const double* __restrict__ w,
-                                                const double* __restrict__ r, const double* __restrict__ rp,
-                                                const double* __restrict__ xc, double* __restrict__ xf, int zero_fixed,
-                                                DotOut64 dout) {
+__global__ void __launch_bounds__(UY * UX, 2) k_up64(Grid gf, Grid gc, const uint8_t* __restrict__ nflag, int zc,
+                                                const double* __restrict__ w, const double* r, const double* rp, const double* xc, double* xf,
+                                                int zero_fixed, DotOut64 dout) {
     __shared__ double sh[32];
+    pdl_begin();
+    pdl_wait();
     const int64_t Sf = gf.slots, Sc = gc.slots, csx = gc.sx(), csz = gc.sz(), fsz = gf.sz();
-    const int iy = blockIdx.x * TY + threadIdx.x, ix = blockIdx.y * TX + threadIdx.y;
+    const int iy = blockIdx.x * UY + threadIdx.x, ix = blockIdx.y * UX + threadIdx.y;
     const int zb = blockIdx.z * zc, ze = min(zb + zc, gf.nz + 1);
     double dot = 0.0;
     if (iy <= gf.ny && ix <= gf.nx) {
         const bool oy = iy & 1, ox = ix & 1;            // ox is uniform across a warp
         const double wyx = (oy ? 0.5 : 1.0) * (ox ? 0.5 : 1.0);
         const int64_t fcol = gf.slot(iy, ix, 0), ccol = gc.slot(iy >> 1, ix >> 1, 0);
-        const int64_t trow = (int64_t)gridDim.y * gridDim.x, tcol = (int64_t)blockIdx.y * gridDim.x + blockIdx.x;
         constexpr int U = chk::UP_FINE, UC = chk::UP_COARSE;
         double qa[3][4], qb[3][4];
         int qa_z = -1;
@@ -843,7 +892,6 @@ __global__ void __launch_bounds__(NT, 2) k_up64(Grid gf, Grid gc, const uint8_t*
             }
         };
         for (int iz = zb; iz < ze; ++iz) {
-            if (tile_occ && !tile_occ[iz * trow + tcol]) continue;
             const int64_t fs = fcol + iz * fsz;
             const uint32_t fl = chk::ld(nflag, fs, Sf, U);
             if (!(fl & NF_SOLID)) continue;
@@ -887,14 +935,23 @@ __global__ void __launch_bounds__(NT, 2) k_up64(Grid gf, Grid gc, const uint8_t*
     if (DOT) grid_dot_finish(dot, DotOut{dout.partials, dout.ticket, dout.out}, sh);
 }
 
-void launch_up64(Ctx& c, const Grid& gf, const Grid& gc, const uint8_t* nflag, const uint8_t* tile_occ, const double* w,
-                 const double* r, const double* rp, const double* xc, double* xf, bool zero_fixed, const DotOut64* dot) {
-    const int zc = pick_zc64(gf, c, 2);
-    const dim3 grid((gf.ny + 1 + TY - 1) / TY, (gf.nx + 1 + TX - 1) / TX, (gf.nz + 1 + zc - 1) / zc);
-    const dim3 blk(TY, TX, 1);
-    if (dot) k_up64<true><<<grid, blk, 0, c.stream>>>(gf, gc, nflag, tile_occ, zc, w, r, rp, xc, xf, zero_fixed, *dot);
-    else k_up64<false><<<grid, blk, 0, c.stream>>>(gf, gc, nflag, tile_occ, zc, w, r, rp, xc, xf, zero_fixed, DotOut64{});
-    GMGS_LAUNCHED(c);
+void launch_up64(Ctx& c, const Grid& gf, const Grid& gc, const uint8_t* nflag, const double* w, const double* r,
+                 const double* rp, const double* xc, double* xf, bool zero_fixed, const DotOut64* dot) {
+    const int ty = (gf.ny + 1 + UY - 1) / UY, tx = (gf.nx + 1 + UX - 1) / UX;
+    const int64_t want = (int64_t)c.num_sms * 2 * 12;
+    const int zc = (int)std::min<int64_t>(32, std::max<int64_t>(2, ((int64_t)ty * tx * (gf.nz + 1) + want - 1) / want));
+    const dim3 grid(ty, tx, (gf.nz + 1 + zc - 1) / zc);
+    const dim3 blk(UY, UX, 1);
+    launch_chain(c, dot ? k_up64<true> : k_up64<false>, grid, blk, 0, gf, gc, nflag, zc, w, r, rp, xc, xf,
+                 zero_fixed ? 1 : 0, dot ? *dot : DotOut64{});
+}
+
+// upper bound over the z-chunk choices
+int dot64_blocks(const Grid& g, int64_t n_list) {
+    const int64_t a = (int64_t)((g.ny + 1 + TY - 1) / TY) * ((g.nx + 1 + TX - 1) / TX);
+    const int64_t b = (int64_t)((g.ny + 1 + UY - 1) / UY) * ((g.nx + 1 + UX - 1) / UX);
+    const int64_t tiles = std::max(a, b) * (g.nz + 1);
+    return (int)(tiles + n_list / (NT / ELEM_LANES) + 2);
 }
 
 // x -= dx, dx = w (r - alpha q) as the fused update added it

@@ -20,10 +20,14 @@ struct Coef64 {
     double hx, hy, hz;
 };
 Coef64 make_coef64(double E, double nu, const double ele[3]);
-// 3 x 3 blocks of the stencil (27 offsets) for each of the 256 sets of solid
-// elements around a node, on the uniform element matrix: 256 x 243 doubles
-constexpr int MASK_STENCIL = 243;
-void launch_mask_stencils(Ctx& c, const double* ke0, double* table);
+// The assembled stencil of one set of solid elements around a node, on the
+// uniform element matrix: the offsets the elements reach and their 3 x 3 blocks
+struct MaskStencil {
+    int n;
+    int k[27];
+    double S[27][9];
+};
+void launch_mask_stencils(Ctx& c, const double* ke0, MaskStencil* table);   // for the 256 sets
 
 // one level as the FP64 kernels see it
 struct Level64 {
@@ -37,7 +41,7 @@ struct Level64 {
     const double* ke0;            // Ke0, row = output DOF
     double kscale;
     const double* escale;         // finest-level element scale or null
-    const double* mask_stencil;   // launch_mask_stencils
+    const MaskStencil* mask_stencil;   // one per set of solid elements
     const int32_t* bnd;           // solid nodes with a void element around them and no stored matrix
     int n_bnd;
     const int32_t* perel;         // nodes touching an element with its own stored matrix
@@ -76,13 +80,15 @@ struct Args64 {
 
 template <int MODE>
 void launch_fine64(Ctx& c, const Level64& L, const Coef64& cf, const Args64& a);
+size_t tile_occ64_bytes(const Grid& g);
+void launch_tile_occ64(Ctx& c, const Grid& g, const uint8_t* nflag, uint8_t* occ);
 // upper bound of the blocks (dot partials) of launch_fine64 and launch_up64
 int dot64_blocks(const Grid& g, int64_t n_list);
 
 // z = w (r + r') + P x_c on solid nodes (Vcycle.m:27-32), optionally the fixed
 // DOFs zeroed and the dot r . z accumulated
-void launch_up64(Ctx& c, const Grid& gf, const Grid& gc, const uint8_t* nflag, const uint8_t* tile_occ, const double* w,
-                 const double* r, const double* rp, const double* xc, double* xf, bool zero_fixed, const DotOut64* dot);
+void launch_up64(Ctx& c, const Grid& gf, const Grid& gc, const uint8_t* nflag, const double* w, const double* r,
+                 const double* rp, const double* xc, double* xf, bool zero_fixed, const DotOut64* dot);
 // x -= the last Jacobi step w (r - alpha q)
 void launch_drop_last_dx64(Ctx& c, int64_t n, double* x, const double* r, const double* q, const double* w,
                            const double* scal, int cur);

@@ -260,7 +260,8 @@ struct Level {
     DevBuf elem_slot;         // compact element id -> slot (int32), eleMapBack order
     // V-cycle work vectors (3 planes each), precision of the V-cycle
     DevBuf vr, vrp, vx;
-    DevBuf tile_occ;          // per 32x8 node tile and z plane, 1 if it holds a solid node
+    DevBuf tile_occ;          // mixed path: per 32x8 node tile and z plane, 1 if it holds a solid node
+    DevBuf tile_occ64;        // FP64 operator: the same for its 16x16 tiles
     DevBuf wdinv64;           // FP64 path: omega / diag
     DevBuf bnd_nodes;         // FP64 operator: slots of solid nodes with void elements around them and no stored matrix
     int64_t n_bnd = -1;       // -1: the list is not built yet

@@ -28,12 +28,12 @@ static void prepare_fp64_level(Model& M, int l) {
     Ctx& c = M.ctx;
     Level& lv = M.levels[l];
     if (!M.mask_stencil.p) {
-        M.mask_stencil = dalloc(256 * MASK_STENCIL * sizeof(double));
-        launch_mask_stencils(c, M.ke0_dev.as<double>(), M.mask_stencil.as<double>());
+        M.mask_stencil = dalloc(256 * sizeof(MaskStencil));
+        launch_mask_stencils(c, M.ke0_dev.as<double>(), M.mask_stencil.as<MaskStencil>());
     }
     if (lv.n_bnd >= 0) return;
-    if (lv.tile_occ.bytes < tile_occ_bytes(lv.g)) lv.tile_occ = dalloc(tile_occ_bytes(lv.g));
-    launch_tile_occ(c, lv.g, lv.nflag.as<uint8_t>(), lv.tile_occ.as<uint8_t>());
+    if (lv.tile_occ64.bytes < tile_occ64_bytes(lv.g)) lv.tile_occ64 = dalloc(tile_occ64_bytes(lv.g));
+    launch_tile_occ64(c, lv.g, lv.nflag.as<uint8_t>(), lv.tile_occ64.as<uint8_t>());
     if (l == 0 && lv.escale64.p) lv.n_bnd = 0;   // every node takes the scaled elements
     else build_boundary_list(M, l);
 }
@@ -43,14 +43,14 @@ static Level64 level64(const Model& M, const Level& lv) {
     f.g = lv.g;
     f.emask = lv.emask.as<uint8_t>();
     f.nflag = lv.nflag.as<uint8_t>();
-    f.tile_occ = lv.tile_occ.as<uint8_t>();
+    f.tile_occ = lv.tile_occ64.as<uint8_t>();
     f.etype = lv.etype.as<int32_t>();
     f.Ks = lv.Ks64.as<double>();
     f.nK = lv.Ks64.p ? lv.nK : 0;
     f.ke0 = M.ke0_dev.as<double>();
     f.kscale = lv.kscale;
     f.escale = lv.escale64.as<double>();
-    f.mask_stencil = M.mask_stencil.as<double>();
+    f.mask_stencil = M.mask_stencil.as<MaskStencil>();
     f.bnd = lv.bnd_nodes.as<int32_t>();
     f.n_bnd = (int)lv.n_bnd;
     f.perel = lv.perel_nodes.as<int32_t>();
@@ -177,7 +177,7 @@ static void vcycle64(Model& M, const double* r0, double* z, bool with_dot, int d
     for (int l = L - 2; l >= 0; --l) {
         Level& lv = M.levels[l];
         const DotOut64 d = dot_out64(M, dot_slot);
-        launch_up64(c, lv.g, M.levels[l + 1].g, lv.nflag.as<uint8_t>(), lv.tile_occ.as<uint8_t>(), lv.wdinv64.as<double>(),
+        launch_up64(c, lv.g, M.levels[l + 1].g, lv.nflag.as<uint8_t>(), lv.wdinv64.as<double>(),
                     l == 0 ? r0 : lv.vr.as<double>(), lv.vrp.as<double>(), M.levels[l + 1].vx.as<double>(),
                     l == 0 ? z : lv.vx.as<double>(), l == 0, (l == 0 && with_dot) ? &d : nullptr);
     }
