@@ -13,7 +13,9 @@
 // the 576 of the element form.  The 1-D second differences annihilate
 // constants exactly, so the result is also more accurate than the assembled
 // sum (2.6e-14 against 3.8e-14 relative on a smooth field, where |K x| is
-// small against |K||x|).
+// small against |K||x|).  The integer units do those operations on 96-bit fixed
+// point, exactly and four times as fast, wherever that is the more accurate
+// form (fixed96.cuh, k_fine64); FP64 arithmetic remains for the rest.
 //
 // Solid nodes with void elements around them take the assembled stencil of
 // their own set of solid elements (256 precomputed sets), nodes on elements
@@ -26,16 +28,19 @@
 // residuals, dot products) are fused into it as in the mixed path (fine.cu).
 //
 // Measured at 6.4M nodes (169 x 147 x 256 elements): K x alone took 4.1 ms as
-// a thread per node on the assembled pairs and eight element rows; with the
-// Jacobi step and the residual in the same launch it takes 1.44 ms, with the
-// CG direction 1.54 ms, with the CG update 1.80 ms, at 78 to 83 % of the FP64
-// pipe (12 % of the issue slots).  A PCG iteration went from 16.9 to 6.2 ms.
+// a thread per node on the assembled pairs and eight element rows.  Axis by
+// axis in FP64, with the Jacobi step and the residual in the same launch, it
+// took 1.44 ms, with the CG update 1.80 ms, at 80 % of the FP64 unit; with the
+// stencil on integers 0.70 and 1.14 ms (FP64 unit 32 and 36 %, issue slots 44
+// and 31 %, shared-memory pipe 57 and 41 %: no one unit bounds them, two CTAs
+// of 128 registers per SM do).  A PCG iteration went from 16.9 to 3.8 ms.
 #include <algorithm>
 #include <atomic>
 
 #include "element_host.h"
 #include "fine.cuh"
 #include "fine64.cuh"
+#include "fixed96.cuh"
 
 namespace gmgs {
 
@@ -256,10 +261,24 @@ struct Points {
     }
 };
 
+// the z and x stages' fields (9 each, three words a value), the field inputs of two planes
 template <int MODE>
 constexpr size_t fine64_smem() {
-    return sizeof(double) * (9 * NP + 9 * NXP + 2 * 3 * field_arrays64(MODE) * NP);
+    return 12 * (9 * NP + 9 * NXP) + sizeof(double) * (2 * 3 * field_arrays64(MODE) * NP);
 }
+
+// The three stages run on 96-bit integers (fixed96.cuh) where that is at least
+// as accurate as FP64 arithmetic at every node: the values of the three planes
+// on the scale of their largest exponent E, unit 2^(E - 1105), are exact down
+// to 2^-30 of the largest value, all sums are exact, and the products with the
+// coefficients (exact as fractions) drop less than 3 units each, 2^-76 of the
+// largest value in all.  FP64 rounds each operation at 2^-53 of the values
+// around a node, so the integers are the more accurate form at every node whose
+// neighbours reach 2^-23 of the window's largest value.  Windows with smaller
+// non-zero points, with infinities or NaN, or near the ends of the exponent
+// range take the same stages in FP64, as do voxels so flat that a coefficient
+// is below 2^-11 of the largest one.
+constexpr int FIXED_RANGE = 23;
 
 // ---------------------------------------------------------------------------
 // K x with the uniform matrix, axis by axis.  A CTA owns a 16 (y) x 16 (x)
@@ -314,9 +333,11 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
     const bool own = p.cy <= g.ny && p.cx <= g.nx;
     constexpr int NA = field_arrays64(MODE);
     constexpr int R = chk::F64_TILE;
-    double* const Zb = dyn;                       // 9 fields of the z stage: m, k, d of the three components
-    double* const Xb = Zb + 9 * NP;               // 9 fields of the x stage: P, Q, R
-    double* const stage = Xb + 9 * NXP;           // [2][NA * 3][NP] field inputs of two planes
+    double* const stage = dyn;                    // [2][NA * 3][NP] field inputs of two planes
+    double* const Zb = stage + 2 * NA * 3 * NP;   // 9 fields of the z stage: m, k, d of the three components
+    double* const Xb = Zb + 9 * NP * 3 / 2;       // 9 fields of the x stage: P, Q, R
+    uint32_t* const Zw = reinterpret_cast<uint32_t*>(Zb);      // the same as three words a value
+    uint32_t* const Xw = reinterpret_cast<uint32_t*>(Xb);
     const int narr = ((MODE == M64_CG_UPDATE_JACOBI || MODE == M64_CG_DIRECTION) && a.first) ? NA - 1 : NA;
 
     // field inputs of plane iz to this thread's places of buffer iz & 1
@@ -349,6 +370,30 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
         }
     };
     double vm[3], vc[3], vp[3], hm[3], hc[3], hp[3], sc[3], sp[3], unused[3];
+    // of a formed plane, over the CTA: the largest biased exponent, and 2047
+    // minus the smallest of its points' largest ones (points that are zero in
+    // all components left out)
+    __shared__ int s_exp[2][2][NT / 32];
+    auto put_exp = [&](int par, const double* u, const double* h) {
+        int e = 0, g = 0;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            e = max(e, (__double2hiint(u[c]) >> 20) & 0x7ff);
+            g = max(g, (__double2hiint(h[c]) >> 20) & 0x7ff);
+        }
+        const int top = __reduce_max_sync(0xffffffffu, max(e, g));
+        const int low = __reduce_max_sync(0xffffffffu, max(e ? 2047 - e : 0, g ? 2047 - g : 0));
+        if ((tid & 31) == 0) {
+            s_exp[par][0][tid >> 5] = top;
+            s_exp[par][1][tid >> 5] = low;
+        }
+    };
+    auto get_exp = [&](int par, int k) {
+        int e = s_exp[par][k][0];
+#pragma unroll
+        for (int w = 1; w < NT / 32; ++w) e = max(e, s_exp[par][k][w]);
+        return e;
+    };
     issue(zb - 1);
     cp_async_commit();
     issue(zb);
@@ -361,6 +406,11 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
     cp_async_wait<1>();
     formed(zb, p.pc, p.cok, vc, sc);
     formed(zb, p.ph, p.hok, hc, unused);
+    put_exp(0, vm, hm);
+    put_exp(1, vc, hc);
+    __syncthreads();
+    int em = get_exp(0, 0), ec = get_exp(1, 0), lm = get_exp(0, 1), lc = get_exp(1, 1);
+    __syncthreads();
 
     auto z_stage = [&](int pt, const double* um, const double* u, const double* up) {
 #pragma unroll
@@ -391,6 +441,49 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
         Rr[1] = fma(cf.gyz, mx(8), cf.gxy * dM[0]);
         Rr[2] = mx(7);
     };
+    // the same stages on 96-bit integers, all values multiples of 2^(E - 1105)
+    auto put_w = [](uint32_t* w, int n, int k, int pt, const I96& x) {
+        chk::st(w, (3 * k + 0) * n + pt, 27 * n, R, x.a);
+        chk::st(w, (3 * k + 1) * n + pt, 27 * n, R, x.b);
+        chk::st(w, (3 * k + 2) * n + pt, 27 * n, R, x.c);
+    };
+    auto get_w = [](const uint32_t* w, int n, int k, int pt) {
+        return I96{chk::ld(w, (3 * k + 0) * n + pt, 27 * n, R), chk::ld(w, (3 * k + 1) * n + pt, 27 * n, R),
+                   chk::ld(w, (3 * k + 2) * n + pt, 27 * n, R)};
+    };
+    auto z_stage_i = [&](int pt, const double* um, const double* u, const double* up, int E) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const I96 l = to_fixed(um[c], E), m = to_fixed(u[c], E), r = to_fixed(up[c], E), t = l + r;
+            put_w(Zw, NP, c, pt, t + shl<2>(m));
+            put_w(Zw, NP, 3 + c, pt, shl<1>(m) - t);
+            put_w(Zw, NP, 6 + c, pt, r - l);
+        }
+    };
+    auto x_stage_i = [&](int pt, I96 P[3], I96 Q[3], I96 Rr[3]) {
+        auto zf = [&](int k, int o) { return get_w(Zw, NP, k, pt + o * HY); };
+        auto mx = [&](int k) { return zf(k, -1) + zf(k, 1) + shl<2>(zf(k, 0)); };
+        {
+            const I96 l = zf(0, -1), u = zf(0, 0), r = zf(0, 1), t = l + r;
+            Q[0] = t + shl<2>(u);
+            P[0] = mul_frac(shl<1>(u) - t, cf.fax[0]);
+            Rr[1] = mul_frac(r - l, cf.fgxy);
+        }
+        {
+            const I96 l = zf(1, -1), u = zf(1, 0), r = zf(1, 1), t = l + r;
+            Q[1] = t + shl<2>(u);
+            P[1] = mul_frac(shl<1>(u) - t, cf.fax[1]) + mul_frac(mx(4), cf.faz[1]);
+            Rr[0] = r - l;
+        }
+        {
+            const I96 l = zf(2, -1), u = zf(2, 0), r = zf(2, 1), t = l + r;
+            Q[2] = t + shl<2>(u);
+            P[2] = mul_frac(shl<1>(u) - t, cf.fax[2]) + mul_frac(mx(5), cf.faz[2]) - mul_frac(zf(6, 1) - zf(6, -1), cf.fgxz);
+        }
+        P[0] = P[0] + mul_frac(mx(3), cf.faz[0]) - mul_frac(zf(8, 1) - zf(8, -1), cf.fgxz);
+        Rr[1] = Rr[1] + mul_frac(mx(8), cf.fgyz);
+        Rr[2] = mx(7);
+    };
     const int xc = (p.pc % HY) + (tid / TY) * HY;                // own point of the x stage
     const int hxc = tid & (2 * TX - 1), hyy = (hxc & 1) ? HY - 1 : 0;      // the y halo's points: one warp
     const int hz_pt = hyy + ((hxc >> 1) + 1) * HY, hx_pt = hyy + (hxc >> 1) * HY;
@@ -413,7 +506,55 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
         cp_async_wait<1>();
         formed(iz + 1, p.pc, p.cok, vp, sp);
         formed(iz + 1, p.ph, p.hok, hp, unused);
-        if (occ(iz)) {                                           // uniform across the CTA
+        put_exp((iz - zb) & 1, vp, hp);
+        __syncthreads();
+        const int ep = get_exp((iz - zb) & 1, 0), lp = get_exp((iz - zb) & 1, 1);
+        const int E = max(em, max(ec, ep)), range = E - 2047 + max(lm, max(lc, lp));
+        em = ec;
+        ec = ep;
+        lm = lc;
+        lc = lp;
+        if (!occ(iz)) {                                          // uniform across the CTA, as the next one
+        } else if (cf.fixed && range <= FIXED_RANGE && E > 1023 - 700 && E < 1023 + 700) {
+            z_stage_i(p.pc, vm, vc, vp, E);
+            if (tid < NHALO) z_stage_i(p.ph, hm, hc, hp, E);
+            __syncthreads();
+            I96 P[3], Q[3], Rr[3];
+            if (tid < 2 * TX) {
+                x_stage_i(hz_pt, P, Q, Rr);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    put_w(Xw, NXP, c, hx_pt, P[c]);
+                    put_w(Xw, NXP, 3 + c, hx_pt, Q[c]);
+                    put_w(Xw, NXP, 6 + c, hx_pt, Rr[c]);
+                }
+            }
+            // a warp holds whole y columns of the tile, so its x stage is read by its own y stage alone
+            if (__any_sync(0xffffffffu, node)) {
+                x_stage_i(p.pc, P, Q, Rr);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    put_w(Xw, NXP, c, xc, P[c]);
+                    put_w(Xw, NXP, 3 + c, xc, Q[c]);
+                    put_w(Xw, NXP, 6 + c, xc, Rr[c]);
+                }
+            }
+            __syncthreads();
+            if (node) {
+                const int ex = E - 1105 + cf.cexp + 1023 + 95;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    auto xf = [&](int k, int o) { return get_w(Xw, NXP, 3 * k + c, xc + o); };
+                    const I96 mP = xf(0, -1) + xf(0, 1) + shl<2>(P[c]);
+                    const I96 kQ = shl<1>(Q[c]) - (xf(1, -1) + xf(1, 1));
+                    I96 dR = xf(2, 1) - xf(2, -1);
+                    if (c != 1) dR = mul_frac(dR, c == 0 ? cf.fgxy : cf.fgyz);
+                    double y = to_double(mP + mul_frac(kQ, cf.fay[c]) + dR, ex);
+                    if (f & (NF_FIX_X << c)) y = 0.0;
+                    finish_dof<MODE>(a, n + c * S, n3, y, vc[c], sc[c], px[c], xx[c], ab, dot);
+                }
+            }
+        } else {
             z_stage(p.pc, vm, vc, vp);
             if (tid < NHALO) z_stage(p.ph, hm, hc, hp);
             __syncthreads();
@@ -821,6 +962,24 @@ void launch_mask_stencils(Ctx& c, const double* ke0, MaskStencil* table) {
     GMGS_LAUNCHED(c);
 }
 
+void set_fixed_coefs(Coef64& c) {
+    const double g[12] = {c.ax[0], c.ax[1], c.ax[2], c.ay[0], c.ay[1], c.ay[2],
+                          c.az[0], c.az[1], c.az[2], c.gxy, -c.gxz, c.gyz};
+    uint2* f[12] = {&c.fax[0], &c.fax[1], &c.fax[2], &c.fay[0], &c.fay[1], &c.fay[2],
+                    &c.faz[0], &c.faz[1], &c.faz[2], &c.fgxy, &c.fgxz, &c.fgyz};
+    const double big = *std::max_element(g, g + 12), small = *std::min_element(g, g + 12);
+    c.fixed = 0;
+    if (!(small > 0) || !std::isfinite(big)) return;
+    std::frexp(big, &c.cexp);                       // big < 2^cexp
+    // below 2^-11 of the largest a coefficient's 53 bits would not fit the fraction
+    if (small < std::ldexp(big, -11) || c.cexp < -100 || c.cexp > 100) return;
+    for (int k = 0; k < 12; ++k) {
+        const uint64_t C = (uint64_t)std::ldexp(g[k], 64 - c.cexp);
+        *f[k] = make_uint2((uint32_t)C, (uint32_t)(C >> 32));
+    }
+    c.fixed = 1;
+}
+
 template <int MODE>
 void launch_fine64(Ctx& c, const Level64& L, const Coef64& cf0, const Args64& a) {
     const int ty = (L.g.ny + 1 + TY - 1) / TY, tx = (L.g.nx + 1 + TX - 1) / TX;
@@ -841,6 +1000,7 @@ void launch_fine64(Ctx& c, const Level64& L, const Coef64& cf0, const Args64& a)
     cf.gxy *= L.kscale;
     cf.gxz *= L.kscale;
     cf.gyz *= L.kscale;
+    set_fixed_coefs(cf);
     opt_in_smem(k_fine64<MODE>, fine64_smem<MODE>(), opted_f);
     constexpr int per_b = NT / BND_LANES, per_e = NT / ELEM_LANES;
     const int nb_bnd = (L.n_bnd + per_b - 1) / per_b, nb_list = nb_bnd + (L.n_perel + per_e - 1) / per_e;

@@ -18,7 +18,12 @@ struct Coef64 {
     // modal form of one element (fine64.cu): diagonal and coupling coefficients
     double lam, mu;             // Lame constants
     double hx, hy, hz;
+    // the stencil's coefficients as fractions C / 2^64 of 2^cexp (Coef64's
+    // signs: gxz is negative, the others positive); fixed: they are exact
+    uint2 fax[3], fay[3], faz[3], fgxy, fgxz, fgyz;
+    int cexp = 0, fixed = 0;
 };
+void set_fixed_coefs(Coef64& c);   // from ax .. gyz
 Coef64 make_coef64(double E, double nu, const double ele[3]);
 // The assembled stencil of one set of solid elements around a node, on the
 // uniform element matrix: the offsets the elements reach and their 3 x 3 blocks

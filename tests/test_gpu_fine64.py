@@ -72,3 +72,51 @@ def test_operator_on_a_mixed_handle_matches_the_fp64_one():
     for level in (1, 2, 3):
         x = rng.standard_normal(3 * handles[0].num_nodes(level))
         assert np.array_equal(handles[0].apply_operator(x, level), handles[1].apply_operator(x, level))
+
+
+# The stages of the factorised stencil run on 96-bit integers where the values of
+# a window stay within 2^23 of each other, on FP64 elsewhere.  Elementwise bound:
+# every row's terms are rounded at most 100 times at 2^-53 (FP64 stages, 3 x 3 x 3
+# weights on three components in sequence), so |y - K x| <= 100 * 2^-53 |K| |x|.
+@pytest.mark.parametrize("spread", [0, 10, 22, 24, 60, 200], ids=lambda s: f"2^{s}")
+@pytest.mark.parametrize("scale", [1.0, 1e-200, 1e-290, 1e250])
+def test_operator_elementwise_over_dynamic_ranges(spread, scale):
+    import scipy.sparse as sp
+    o, s = pair((18, 17, 12), 1, 2, (1.0, 1.0, 1.0), None, 9)
+    o.setup()
+    K = sp.csr_matrix(o.assemble_level(0))
+    rng = np.random.default_rng(spread)
+    n = o.levels[0].numDOFs
+    x = rng.choice([-1.0, 1.0], n) * np.repeat(np.exp2(rng.uniform(-spread, 0, n // 3)), 3) * rng.uniform(0.5, 1, n) * scale
+    free = np.ones(n, bool)
+    free[o.levels[0].fixedDOFs] = False
+    with np.errstate(under="ignore"):
+        err, bound = np.abs(s.apply_operator(x, 1) - K @ x), 100 * 2.0 ** -53 * (abs(K) @ abs(x))
+    assert np.all(err[free] <= 2 * bound[free] + 1e-322)     # the reference product rounds as well
+
+
+@pytest.mark.parametrize("ele", [(1.0, 1.0, 30.0), (1.0, 40.0, 1.0), (0.02, 1.0, 1.0), (1.0, 6.0, 0.5)])
+def test_operator_on_flat_voxels(ele):
+    """Coefficients far apart: within 2^11 of each other on integers, beyond on FP64."""
+    o, s = pair((18, 17, 12), 1, 2, ele, None, 9)
+    o.setup()
+    x = np.random.default_rng(1).standard_normal(o.levels[0].numDOFs)
+    assert rel(s.apply_operator(x, 1), o.atx(x, 0)) < TOL
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_operator_keeps_non_finite_values(bad):
+    """A NaN or infinity reaches the rows coupled to it and no others."""
+    o, s = pair((18, 17, 20), 0, 2, (1.0, 1.0, 1.0), None, 9)
+    o.setup()
+    n = o.levels[0].numDOFs
+    x = np.random.default_rng(1).standard_normal(n)
+    clean = s.apply_operator(x, 1)
+    at = 3 * (19 * 18 * 10 + 19 * 8 + 9)          # an interior node
+    x[at] = bad
+    y = s.apply_operator(x, 1)
+    node = np.arange(n // 3)
+    iy, ix, iz = node % 19, node // 19 % 18, node // (19 * 18)
+    near = (abs(iy - iy[at // 3]) <= 1) & (abs(ix - ix[at // 3]) <= 1) & (abs(iz - iz[at // 3]) <= 1)
+    assert not np.isfinite(y.reshape(-1, 3)[near]).all(axis=1).any()
+    assert np.all(np.abs(y - clean).reshape(-1, 3)[~near] <= 1e-13)
