@@ -18,237 +18,190 @@
 // so both sequential sweeps run as two independent chains of about nb/2
 // steps, and the two halves of the factorisation run on two streams.
 //
-// Everything runs in FP64 (about 2 lanes per clock per SM on GB300), so the
-// factorisation is organised to do few operations on many SMs:
-//   - each D_i^-1 by symmetric block sweeps (Gauss-Jordan on the lower
-//     triangle, 32 pivots at a time, no pivoting: every D_i is SPD), B^3 / 2
-//     multiply-adds in B/32 pairs of launches.  A recursive Cholesky with the
-//     inverse factor and L^-T L^-1 took B^3 and spent 43 us in each of its
-//     B/32 single-CTA leaves: 1.45 ms per block of order 448
+// Each D_i^-1 comes from a recursive blocked Cholesky that also forms L^-1 (no
+// pivoting: every D_i is SPD), then D^-1 = L^-T L^-1.
+//
+// Every sum is a chain of multiply-adds in ascending order from zero, grouped
+// by the recursion and, in the solve, by 16 columns and 64-column tiles: the
+// results do not depend on how the launches tile the work.  The mixed path
+// rounds the solution to FP32 each V-cycle, and on an ill-conditioned coarsest
+// level another order changes some of those roundings and through them the
+// stresses in the eighth digit (an inverse by Gauss-Jordan block sweeps, with
+// half the operations, was as accurate and 0.1 ms per block faster, and is not
+// used for that reason).
+//
+// A warp's FP64 instruction takes the SM's one FP64 unit for 19 clocks (64 for
+// a single warp) however many of its lanes are active (measured), so the work
+// is spread over many SMs and small launches, and operations are avoided:
 //   - the couplings A_(i,i-1) hold about 20 non-zeros per row (27-point
-//     coupling), so the products with them are sparse: 5 % of the dense ones'
-//     operations (172 and 118 us per block)
-// Measured for 15 blocks of order 448: factorisation 14 -> 5.7 ms, solve 15
-// launches of a 64 x 64-tile product with partial sums and arrival counters
-// (about 8 us each in the stream) -> 15 launches of a warp per row.
-// The errors of the solve are the same (5.9e-15 for both on a 6315-DOF
-// coarsest level, 1.5e-10 against 2.2e-10 on a long column of condition 2e7).
+//     coupling); the products with them skip the zeros (172 and 118 us per
+//     block of order 448 as dense products, 14 and 13 us so)
+//   - the 32 x 32 Cholesky leaf spent two thirds of its 43 us in the square
+//     root and the division of each column; it forms both from one FP32
+//     reciprocal square root, while the other warps update
+//   - L^-T L^-1 is symmetric: half of its tiles are computed
+// Measured for 15 blocks of order 448: factorisation 14 -> FACT_MS ms; the solve's
+// launches 8 -> 4 us each (a warp per row instead of 64 x 64 tiles with partial
+// sums in memory and arrival counters).
 #include "setup.cuh"
 
 namespace gmgs {
 
 namespace {
 
-constexpr int PB = 32;       // pivots per panel
-constexpr int PH = 16;       // pivots swept one by one
-constexpr int PR = 8;        // rows per panel CTA
+enum : int { TRI_A_LOWER = 1, TRI_A_UPPER = 2, TRI_B_LOWER = 4, TRI_B_UPPER = 8 };
+enum : int { OUT_ALL = 0, OUT_LOWER = 1, OUT_MIRROR = 2 };
 
-// 1 / d of a positive normal d from an FP32 reciprocal by one third-order step
-// (Halley's iteration for the reciprocal: relative error e -> e^3, 2^-24 ->
-// rounding): three FP64 operations instead of the division's dozen; outside
-// the FP32 range the division.
-__device__ __forceinline__ double reciprocal(double d) {
-    const int e = (__double2hiint(d) >> 20) - 1023;
-    if (e < -120 || e > 120) return 1.0 / d;
-    const double r = f2d_int(__frcp_rn(d2f_int(d)));
-    const double h = fma(-d, r, 1.0);
-    return fma(r, fma(h, h, h), r);
-}
-
-// Sweeps of the 16 x 16 SPD block at (o, o) of A (lower triangle) one pivot at
-// a time; its inverse into the same place of Pm, both triangles.  256 threads;
-// ends with a barrier.  A pivot that is not positive sets *info and is replaced
-// by 1 so the arithmetic stays finite.
-struct SweepShared {
-    double col[2][PH], rp[2], ws[PH];
-};
-__device__ __forceinline__ void invert16(const double (*A)[PB + 1], double (*Pm)[PB + 1], int o, SweepShared& sh, int* info) {
-    constexpr int NO = PH * (PH - 1) / 2;                // elements below the diagonal: threads 0..119
-    const int t = threadIdx.x;
-    int i = -1, j = -1;
-    if (t >= 128 && t < 128 + PH) {
-        i = j = t - 128;
-    } else if (t < NO) {                                 // i > j: t = i (i - 1) / 2 + j
-        i = (int)((sqrtf(8.f * (float)t + 1.f) + 1.f) * 0.5f);
-        while (i * (i + 1) / 2 <= t) ++i;
-        while (i * (i - 1) / 2 > t) --i;
-        j = t - i * (i - 1) / 2;
-    }
-    double a = i >= 0 ? A[o + i][o + j] : 0.0;
-    auto publish = [&](int s) {     // the pivot column of sweep s and the reciprocal of its pivot
-        if (i == s || j == s) sh.col[s & 1][i == s ? j : i] = a;
-        if (i == s && j == s) {
-            const int hi = __double2hiint(a);
-            const bool ok = hi >= 0x00100000 && hi < 0x7ff00000;      // positive, normal, finite
-            if (!ok) atomicExch(info, 1);
-            sh.rp[s & 1] = ok ? reciprocal(a) : 1.0;
-        }
-    };
-    publish(0);
-#pragma unroll 1
-    for (int s = 0; s < PH; ++s) {
-        __syncthreads();
-        const double r = sh.rp[s & 1];
-        if (t < PH) sh.ws[t] = sh.col[s & 1][t] * r;
-        __syncthreads();
-        if (i == s || j == s) a = i == j ? -r : sh.ws[i == s ? j : i];
-        else if (i >= 0) a = fma(-sh.ws[i], sh.col[s & 1][j], a);
-        if (s + 1 < PH) publish(s + 1);
-    }
-    if (i >= 0) Pm[o + i][o + j] = Pm[o + j][o + i] = -a;
-    __syncthreads();
-}
-
-// Inverse P of the 32 x 32 pivot block and W = C P for 8 rows of the panel C
-// (the pivot columns of the symmetric matrix, of which D holds the lower
-// triangle).  Every CTA inverts the pivot block for itself: that is a
-// dependent chain, so sharing one inverse would only add a launch between it
-// and the panel.  A warp's FP64 instruction takes the SM's FP64 unit for 19
-// clocks (64 for a single warp) however many of its lanes are active
-// (measured), so the cost of a sweep is its number of warp instructions: 17
-// warps for one element per thread of a 32 x 32 triangle, 5 for 16 x 16.  The
-// block is therefore inverted by halves, each half swept pivot by pivot and
-// the rest products with one output per thread:
-//   P22 = (A22 - W A21^T)^-1,  W = A21 A11^-1,  P21 = -P22 W,  P11 = A11^-1 + W^T P22 W
-// (32 sweeps of the whole block took 32 to 43 us per launch: a division per
-// sweep, 2 x 2 pivots, or a common factor in place of the divisions.)
-constexpr int PT = 256;
-__global__ void __launch_bounds__(PT) k_sweep_panel(int B, const double* D, int k0, double* W, double* C, double* P,
-                                                    int* __restrict__ info) {
-    __shared__ double A[PB][PB + 1], Ps[PB][PB + 1], Wh[PH][PH + 1], Xh[PH][PH + 1], Cs[PR][PB + 1];
-    __shared__ SweepShared sh;
-    const int t = threadIdx.x;
-    const int r0 = blockIdx.x * PR;
-    const bool pivot_rows = r0 >= k0 && r0 < k0 + PB, below = r0 > k0;
-#pragma unroll
-    for (int q = 0; q < PB * PB / PT; ++q) {
-        const int r = t % PB, c = t / PB + q * (PT / PB);
-        if (r >= c) A[r][c] = D[(int64_t)(k0 + c) * B + k0 + r];
-    }
-    // above the pivot block the column is held as a row of the lower triangle
-    const int rr = below ? t % PR : t / PB, cc = below ? t / PR : t % PB;
-    if (!pivot_rows) Cs[rr][cc] = below ? D[(int64_t)(k0 + cc) * B + r0 + rr] : D[(int64_t)(r0 + rr) * B + k0 + cc];
-    __syncthreads();
-    invert16(A, Ps, 0, sh, info);
-    const int x = t / PH, y = t % PH;
-    {
-        double w0 = 0.0, w1 = 0.0;
-#pragma unroll
-        for (int m = 0; m < PH; m += 2) {
-            w0 = fma(A[PH + x][m], Ps[m][y], w0);
-            w1 = fma(A[PH + x][m + 1], Ps[m + 1][y], w1);
-        }
-        Wh[x][y] = w0 + w1;
-    }
-    __syncthreads();
-    if (x >= y) {
-        double s0 = A[PH + x][PH + y], s1 = 0.0;
-#pragma unroll
-        for (int m = 0; m < PH; m += 2) {
-            s0 = fma(-Wh[x][m], A[PH + y][m], s0);
-            s1 = fma(-Wh[x][m + 1], A[PH + y][m + 1], s1);
-        }
-        A[PH + x][PH + y] = s0 + s1;
-    }
-    __syncthreads();
-    invert16(A, Ps, PH, sh, info);
-    {
-        double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-        for (int m = 0; m < PH; m += 2) {
-            s0 = fma(Ps[PH + x][PH + m], Wh[m][y], s0);
-            s1 = fma(Ps[PH + x][PH + m + 1], Wh[m + 1][y], s1);
-        }
-        Xh[x][y] = s0 + s1;
-        Ps[PH + x][y] = Ps[y][PH + x] = -(s0 + s1);
-    }
-    __syncthreads();
-    {
-        double s0 = Ps[x][y], s1 = 0.0;
-#pragma unroll
-        for (int m = 0; m < PH; m += 2) {
-            s0 = fma(Wh[m][x], Xh[m][y], s0);
-            s1 = fma(Wh[m + 1][x], Xh[m + 1][y], s1);
-        }
-        Ps[x][y] = s0 + s1;
-    }
-    __syncthreads();
-    const int r = t % PR, c = t / PR;
-    if (pivot_rows) {
-        P[(r + r0 - k0) * PB + c] = Ps[r + r0 - k0][c];
-        return;
-    }
-    double w0 = 0.0, w1 = 0.0;
-#pragma unroll 8
-    for (int m = 0; m < PB; m += 2) {
-        w0 = fma(Cs[r][m], Ps[m][c], w0);
-        w1 = fma(Cs[r][m + 1], Ps[m + 1][c], w1);
-    }
-    W[(int64_t)c * B + r0 + r] = w0 + w1;
-    C[(int64_t)c * B + r0 + r] = Cs[r][c];
-}
-
-// The sweep's update of a 32 x 16 half of a tile of the lower triangle: A_ij -=
-// W_i C_j^T off the pivots, A_ik = W_i, A_kk = -P.  After the last pivots the
-// matrix is -D^-1: that launch changes the sign and fills both triangles.
-// (Half tiles: the two chains' 420 CTAs of 4 us balance over the SMs where 210
-// of 8 us leave some of them a round behind.)
-constexpr int UT = 128, UC = 16;
-__global__ void __launch_bounds__(UT) k_sweep_update(int B, double* D, int k0, const double* W, const double* C,
-                                                     const double* P, int last) {
-    __shared__ double Ws[PB][PB + 1], Cs[PB][UC + 1];   // [pivot][row], [pivot][column]
-    const int tile = (int)blockIdx.x >> 1, half = (int)blockIdx.x & 1;
-    int ti = (int)((sqrtf(8.f * (float)tile + 1.f) - 1.f) * 0.5f);
-    while ((ti + 1) * (ti + 2) / 2 <= tile) ++ti;
-    while (ti * (ti + 1) / 2 > tile) --ti;
-    const int tj = tile - ti * (ti + 1) / 2, kt = k0 / PB;
-    const int t = threadIdx.x, x = t & 15, y = t >> 4, ri = ti * PB, cj = tj * PB + half * UC;
-    double v[2][2];
-    if (ti == kt || tj == kt) {
-#pragma unroll
-        for (int p = 0; p < 2; ++p)
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const int r = x + 16 * p, c = half * UC + y + 8 * q;
-                v[p][q] = ti == tj ? -P[r * PB + c] : (tj == kt ? W[(int64_t)c * B + ri + r] : W[(int64_t)r * B + tj * PB + c]);
-            }
-    } else {
-#pragma unroll
-        for (int q = 0; q < PB * PB / UT; ++q) {
-            const int e = t + q * UT, m = e / PB, r = e % PB;
-            Ws[m][r] = W[(int64_t)m * B + ri + r];
-        }
-#pragma unroll
-        for (int q = 0; q < PB * UC / UT; ++q) {
-            const int e = t + q * UT, m = e / UC, c = e % UC;
-            Cs[m][c] = C[(int64_t)m * B + cj + c];
-        }
-#pragma unroll
-        for (int p = 0; p < 2; ++p)
-#pragma unroll
-            for (int q = 0; q < 2; ++q) v[p][q] = D[(int64_t)(cj + y + 8 * q) * B + ri + x + 16 * p];
-        __syncthreads();
-#pragma unroll 8
-        for (int m = 0; m < PB; ++m) {
-            const double w0 = Ws[m][x], w1 = Ws[m][x + 16], c0 = Cs[m][y], c1 = Cs[m][y + 8];
-            v[0][0] = fma(-w0, c0, v[0][0]);
-            v[1][0] = fma(-w1, c0, v[1][0]);
-            v[0][1] = fma(-w0, c1, v[0][1]);
-            v[1][1] = fma(-w1, c1, v[1][1]);
-        }
-    }
-#pragma unroll
-    for (int p = 0; p < 2; ++p)
+// C = alpha op(A) op(B) + beta C, column-major, m, n, k multiples of 16, one
+// output per thread on 16 x 8 tiles (the smallest products of the recursion are
+// 32^3: small tiles put them on more SMs).  TRI marks operands known to be
+// triangular so the k-loop skips their zero tiles (exact zeros).  OUT_LOWER
+// skips output tiles strictly above the diagonal (their values are never
+// read), OUT_MIRROR computes a symmetric product's lower half and stores both.
+constexpr int GR = 16, GC = 8, GK = 16, GT = GR * GC;
+template <bool TA, bool TB, int TRI, int OUT>
+__global__ void __launch_bounds__(GT) k_dgemm(int k, double alpha, const double* __restrict__ A, int lda,
+                                              const double* __restrict__ B, int ldb, double beta, double* __restrict__ C,
+                                              int ldc) {
+    const int r0 = blockIdx.x * GR, c0 = blockIdx.y * GC;
+    if (OUT != OUT_ALL && r0 + GR <= c0) return;
+    __shared__ double As[2][GK][GR + 1];   // As[.][l][i] = op(A)(r0 + i, k0 + l)
+    __shared__ double Bs[2][GK][GC + 1];   // Bs[.][l][j] = op(B)(k0 + l, c0 + j)
+    const int t = threadIdx.x, tx = t % GR, ty = t / GR;
+    int kb = 0, ke = k;
+    if (TRI & TRI_A_LOWER) ke = min(ke, r0 + GR);
+    if (TRI & TRI_A_UPPER) kb = max(kb, r0);
+    if (TRI & TRI_B_LOWER) kb = max(kb, c0 & ~(GK - 1));
+    if (TRI & TRI_B_UPPER) ke = min(ke, (c0 & ~(GK - 1)) + GK);
+    double ra[2], rb;
+    auto load = [&](int k0) {
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-            const int r = ri + x + 16 * p, c = cj + y + 8 * q;
-            if (!last) {
-                D[(int64_t)c * B + r] = v[p][q];
-            } else if (ti != tj || r >= c) {        // a diagonal tile's lower half, mirrored
-                D[(int64_t)c * B + r] = -v[p][q];
-                D[(int64_t)r * B + c] = -v[p][q];
-            }
+            const int e = t + q * GT;
+            ra[q] = TA ? A[(int64_t)(r0 + e / GK) * lda + k0 + e % GK] : A[(int64_t)(k0 + e / GR) * lda + r0 + e % GR];
         }
+        rb = TB ? B[(int64_t)(k0 + t / GC) * ldb + c0 + t % GC] : B[(int64_t)(c0 + t / GK) * ldb + k0 + t % GK];
+    };
+    double acc = 0.0;
+    if (kb < ke) load(kb);
+    int buf = 0;
+    for (int k0 = kb; k0 < ke; k0 += GK, buf ^= 1) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int e = t + q * GT;
+            if (TA) As[buf][e % GK][e / GK] = ra[q];
+            else As[buf][e / GR][e % GR] = ra[q];
+        }
+        if (TB) Bs[buf][t / GC][t % GC] = rb;
+        else Bs[buf][t % GK][t / GK] = rb;
+        __syncthreads();
+        if (k0 + GK < ke) load(k0 + GK);
+#pragma unroll
+        for (int l = 0; l < GK; ++l) acc = fma(As[buf][l][tx], Bs[buf][l][ty], acc);
+    }
+    const int r = r0 + tx, c = c0 + ty;
+    if (OUT == OUT_MIRROR) {
+        if (r < c) return;
+        C[(int64_t)c * ldc + r] = alpha * acc;
+        C[(int64_t)r * ldc + c] = alpha * acc;
+        return;
+    }
+    double* cp = C + (int64_t)c * ldc + r;
+    *cp = beta == 0.0 ? alpha * acc : fma(alpha, acc, beta * *cp);
+}
+template <bool TA, bool TB, int TRI, int OUT>
+void gemm(Ctx& c, int m, int n, int k, double alpha, const double* A, int lda, const double* B, int ldb, double beta,
+          double* C, int ldc) {
+    if (m <= 0 || n <= 0) return;
+    k_dgemm<TA, TB, TRI, OUT><<<dim3(m / GR, n / GC), GT, 0, c.stream>>>(k, alpha, A, lda, B, ldb, beta, C, ldc);
+    GMGS_LAUNCHED(c);
+}
+
+// sqrt(d) and 1 / sqrt(d)'s rounded value's reciprocal, both correctly rounded,
+// for a positive normal d: an FP32 reciprocal square root y, one third-order
+// step (y (1 + h / 2 + 3 h^2 / 8), h = 1 - d y^2, error h^3), then Markstein's
+// final steps: s = RN(s0 + (d - s0^2) y / 2) and RN(y + y (1 - s y)) with exact
+// FMA residuals.  Ten dependent FP64 operations; the library's square root and
+// division of a lane take about 25.  Outside the FP32 range: the library's.
+__device__ __forceinline__ void sqrt_and_reciprocal(double d, double& s, double& r) {
+    const int e = (__double2hiint(d) >> 20) - 1023;
+    if (e < -120 || e > 120) {
+        s = sqrt(d);
+        r = 1.0 / s;
+        return;
+    }
+    double y = f2d_int(rsqrtf(d2f_int(d)));
+    const double h = fma(-(d * y), y, 1.0);
+    y = fma(y, h * fma(0.375, h, 0.5), y);
+    const double s0 = d * y;
+    s = fma(fma(-s0, s0, d), 0.5 * y, s0);
+    r = fma(y, fma(-s, y, 1.0), y);
+}
+
+// Cholesky of a 32 x 32 SPD tile (lower triangle of A, in place) and the
+// inverse of its factor into Li (zeros above the diagonal), one column per
+// step: the pivot's square root and reciprocal, column j of L, row j of L^-1
+// (forward substitution of L X = I carried along: X(j, c) is final once
+// scaled by 1 / L(j,j)), then the rank-1 updates of the rows below j of A and
+// of X.  Warp 0 updates row j + 1 first and goes on to its square root while
+// the other warps update the rest.  A pivot that is not positive sets *info and
+// is replaced by 1 so the arithmetic stays finite.
+__global__ void __launch_bounds__(256) k_chol_inv32(double* __restrict__ A, int lda, double* __restrict__ Li, int ldl,
+                                                    int* __restrict__ info) {
+    __shared__ double a[32][33];   // a[c][r] = A(r, c), becomes L
+    __shared__ double x[32][33];   // x[c][r] = X(r, c), becomes L^-1
+    __shared__ double s_piv, s_inv;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    for (int e = t; e < 1024; e += 256) {
+        const int cc = e >> 5, r = e & 31;
+        a[cc][r] = A[(int64_t)cc * lda + r];
+        x[cc][r] = r == cc ? 1.0 : 0.0;
+    }
+    auto pivot = [&](double d) {
+        const bool ok = d > 0.0 && d < INFINITY;
+        if (!ok) atomicExch(info, 1);
+        double s = 1.0, r = 1.0;
+        if (ok) sqrt_and_reciprocal(d, s, r);
+        s_piv = s;
+        s_inv = r;
+    };
+    __syncthreads();
+    if (t == 0) pivot(a[0][0]);
+#pragma unroll 1
+    for (int j = 0; j < 32; ++j) {
+        __syncthreads();
+        const double dinv = s_inv;
+        if (w == 0) {
+            if (lane == j) a[j][j] = s_piv;
+            if (lane > j) a[j][lane] *= dinv;               // L(r, j)
+        } else if (w == 1 && lane <= j) {
+            x[lane][j] *= dinv;                             // X(j, c), c <= j
+        }
+        __syncthreads();
+        auto row = [&](int r) {
+            double v = 0.0;
+            if (lane > j) {
+                if (r >= lane) a[lane][r] = v = fma(-a[j][r], a[j][lane], a[lane][r]);
+            } else {
+                x[lane][r] = fma(-a[j][r], x[lane][j], x[lane][r]);
+            }
+            return v;
+        };
+        if (w == 0) {
+            if (j + 1 < 32) {
+                const double d = row(j + 1);
+                if (lane == j + 1) pivot(d);
+            }
+        } else {
+            for (int r = j + 1 + w; r < 32; r += 7) row(r);
+        }
+    }
+    __syncthreads();
+    for (int e = t; e < 1024; e += 256) {
+        const int cc = e >> 5, r = e & 31;
+        if (r >= cc) A[(int64_t)cc * lda + r] = a[cc][r];
+        Li[(int64_t)cc * ldl + r] = x[cc][r];
+    }
 }
 
 // The non-zeros E'(row, c0 .. c0 + 255) of one row of E' (E, or its transpose)
@@ -315,27 +268,40 @@ __global__ void __launch_bounds__(256) k_sparse_update(int B, const double* __re
 
 // scratch of one chain of the factorisation
 struct Chain {
-    DevBuf w, c, p, g;      // panels W and C (PB columns), pivot inverse, G column-major
+    DevBuf li, l, t, g;      // L^-1, the off-diagonal parts of L, a product, G column-major (B x B each)
     void alloc(int B) {
-        w = dalloc((size_t)PB * B * sizeof(double));
-        c = dalloc((size_t)PB * B * sizeof(double));
-        p = dalloc((size_t)PB * PB * sizeof(double));
-        g = dalloc((size_t)B * B * sizeof(double));
+        for (DevBuf* d : {&li, &l, &t, &g}) *d = dalloc((size_t)B * B * sizeof(double));
     }
 };
 
-// D^-1 of the SPD block D (lower triangle in, both triangles out).  Plain
-// launches: as programmatic dependents the two chains hold each other up (8.4
-// instead of 5.7 ms for 15 blocks of order 448).
-void inv_spd(Ctx& c, double* D, int B, Chain& s, int* info) {
-    const int tiles = B / PB;
-    for (int k0 = 0; k0 < B; k0 += PB) {
-        k_sweep_panel<<<B / PR, PT, 0, c.stream>>>(B, D, k0, s.w.as<double>(), s.c.as<double>(), s.p.as<double>(), info);
+// L^-1 (into Li, whose part above the diagonal must be zero on entry) of the
+// n x n SPD matrix A (overwritten), n a multiple of 32, by halves:
+// L11 = chol(A11), L21 = A21 L11^-T, L22 = chol(A22 - L21 L21^T),
+// L^-1_21 = -L22^-1 L21 L11^-1.  L21 goes to the same place of Lo; T: scratch.
+void chol_inv(Ctx& c, double* A, double* Li, double* Lo, int n, int ld, double* T, int* info) {
+    if (n == 32) {
+        k_chol_inv32<<<1, 256, 0, c.stream>>>(A, ld, Li, ld, info);
         GMGS_LAUNCHED(c);
-        k_sweep_update<<<tiles * (tiles + 1), UT, 0, c.stream>>>(B, D, k0, s.w.as<double>(), s.c.as<double>(),
-                                                                 s.p.as<double>(), k0 + PB == B ? 1 : 0);
-        GMGS_LAUNCHED(c);
+        return;
     }
+    const int n1 = 32 * ((n / 32) / 2), n2 = n - n1;
+    const int64_t at22 = (int64_t)n1 * ld + n1;
+    double* L21 = Lo + n1;
+    chol_inv(c, A, Li, Lo, n1, ld, T, info);
+    gemm<false, true, TRI_B_UPPER, OUT_ALL>(c, n2, n1, n1, 1.0, A + n1, ld, Li, ld, 0.0, L21, ld);
+    gemm<false, true, 0, OUT_LOWER>(c, n2, n2, n1, -1.0, L21, ld, L21, ld, 1.0, A + at22, ld);
+    chol_inv(c, A + at22, Li + at22, Lo + at22, n2, ld, T, info);
+    gemm<false, false, TRI_B_LOWER, OUT_ALL>(c, n2, n1, n1, 1.0, L21, ld, Li, ld, 0.0, T, n2);          // L21 L11^-1
+    gemm<false, false, TRI_A_LOWER, OUT_ALL>(c, n2, n1, n2, -1.0, Li + at22, ld, T, n2, 0.0, Li + n1, ld);
+}
+
+// D^-1 of the SPD block D (lower triangle in, both triangles out).  Plain
+// launches: as programmatic dependents the two chains hold each other up.
+void inv_spd(Ctx& c, double* D, int B, Chain& s, int* info) {
+    double* li = s.li.as<double>();
+    GMGS_CUDA(cudaMemsetAsync(li, 0, (size_t)B * B * sizeof(double), c.stream));
+    chol_inv(c, D, li, s.l.as<double>(), B, B, s.t.as<double>(), info);
+    gemm<true, false, TRI_A_UPPER | TRI_B_LOWER, OUT_MIRROR>(c, B, B, B, 1.0, li, B, li, B, 0.0, D, B);
 }
 void sparse_left(Ctx& c, int B, const double* E, bool trans, const double* X, double* gt, double* gc) {
     k_sparse_left<<<dim3(B, (B + 255) / 256), 256, 0, c.stream>>>(B, E, trans, X, gt, gc);
@@ -350,7 +316,9 @@ void sparse_update(Ctx& c, int B, const double* E, bool trans, const double* gc,
 // the solve: launches of independent jobs y = base - sum_s M_s v_s (base null:
 // the sum itself), M_s B x B with its rows contiguous
 // ---------------------------------------------------------------------------
-constexpr int STEP_ROWS = 4;      // rows (warps) per CTA
+constexpr int STEP_ROWS = 8;      // rows (warps) per CTA
+constexpr int CH = 16;            // columns per lane: the sums' first grouping
+constexpr int PART = 32 * CH;     // columns a warp takes at a time
 constexpr int MAX_JOBS = 4;
 struct StepJob {
     const double* M[2];
@@ -368,51 +336,80 @@ struct StepJobs {
     }
 };
 
-// One warp per row, four rows per CTA: at 2 FP64 lanes per clock per SM a
-// matrix-vector product has to be spread over all SMs, and a row per warp
-// needs no partial sums through memory.  Launched as a programmatic dependent
-// of the previous kernel in the stream: the first 16 entries per lane (rows of
-// up to 512) are loaded while that kernel finishes, then the hardware grid
-// dependency is waited for, and only then are vectors read or written.
+// Rows in the order k_rows reads them: of each 512 columns lane L takes the
+// columns 16 L .. 16 L + 15, stored as pairs, pair u of all lanes together.  In
+// place, one CTA per row; z: the three families of matrices.
+__global__ void __launch_bounds__(128) k_order_rows(int B, double* m0, double* m1, double* m2) {
+    __shared__ double part[PART];
+    double* m = (blockIdx.z == 0 ? m0 : (blockIdx.z == 1 ? m1 : m2)) + ((int64_t)blockIdx.y * B + blockIdx.x) * B;
+    for (int p0 = 0; p0 < B; p0 += PART, m += PART) {
+        const int n = min(PART, B - p0), nl = n / CH;
+        __syncthreads();
+        for (int i = threadIdx.x; i < n; i += blockDim.x) part[i] = m[i];
+        __syncthreads();
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            const int u = i / (2 * nl), l = i % (2 * nl) / 2;
+            m[i] = part[CH * l + 2 * u + (i & 1)];
+        }
+    }
+}
+
+// One warp per row, eight rows per CTA: a matrix-vector product has to be
+// spread over all SMs (an SM does 1.7 FP64 multiply-adds per clock), and a row
+// per warp needs no partial sums through memory.  Launched as a programmatic
+// dependent of the previous kernel in the stream: a row's first 512 entries are
+// loaded while that kernel finishes, then the hardware grid dependency is
+// waited for, and only then are vectors read or written.
+// Order of a row's sum: 16 columns in sequence, (s0 + s1) + (s2 + s3) of four
+// such groups, then the 64-column tiles (of both segments) in sequence; the
+// tiles of the CTA's rows are summed by one warp, a lane per row.
 __global__ void __launch_bounds__(32 * STEP_ROWS) k_rows(int B, const __grid_constant__ StepJobs jobs) {
     pdl_begin();
+    __shared__ double vs[17 * 32];                        // 512 entries of v, 17 places per 16
+    __shared__ double tile[8][STEP_ROWS];
     const StepJob& J = jobs.j[blockIdx.y];
-    const int lane = threadIdx.x & 31, row = blockIdx.x * STEP_ROWS + (threadIdx.x >> 5);
-    constexpr int PRE = 8;        // double2 per lane
-    double2 m[2][PRE];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5, row = blockIdx.x * STEP_ROWS + w;
+    const int nl0 = min(32, B / CH);
+    double2 m[2][CH / 2];
 #pragma unroll
     for (int s = 0; s < 2; ++s)
-        if (s < J.nseg) {
+        if (s < J.nseg && lane < nl0) {
             const double2* r = reinterpret_cast<const double2*>(J.M[s] + (int64_t)row * B);
 #pragma unroll
-            for (int q = 0; q < PRE; ++q)
-                if (64 * q < B) m[s][q] = r[32 * q + lane];
+            for (int u = 0; u < CH / 2; ++u) m[s][u] = r[u * nl0 + lane];
         }
     pdl_wait();
-    const double b = (lane == 0 && J.base) ? J.base[row] : 0.0;
-    double s0 = 0.0, s1 = 0.0;
+    double sum = 0.0;                                     // lanes of warp 0: the row's tiles so far
 #pragma unroll
-    for (int s = 0; s < 2; ++s)
-        if (s < J.nseg) {
-            const double2* v = reinterpret_cast<const double2*>(J.v[s]);
+    for (int s = 0; s < 2; ++s) {
+        if (s >= J.nseg) break;
+        for (int p0 = 0; p0 < B; p0 += PART) {
+            const int n = min(PART, B - p0), nl = n / CH;
+            for (int i = t; i < n; i += 32 * STEP_ROWS) vs[i + i / CH] = J.v[s][p0 + i];
+            __syncthreads();                              // also: the tile sums before these are taken
+            double acc = 0.0;
+            if (lane < nl) {
+                const double2* r = reinterpret_cast<const double2*>(J.M[s] + (int64_t)row * B + p0);
+                const double* v = vs + 17 * lane;
 #pragma unroll
-            for (int q = 0; q < PRE; ++q)
-                if (64 * q < B) {
-                    const double2 u = v[32 * q + lane];
-                    s0 = fma(m[s][q].x, u.x, s0);
-                    s1 = fma(m[s][q].y, u.y, s1);
+                for (int u = 0; u < CH / 2; ++u) {
+                    const double2 e = p0 == 0 ? m[s][u] : r[u * nl + lane];
+                    acc = fma(e.x, v[2 * u], acc);
+                    acc = fma(e.y, v[2 * u + 1], acc);
                 }
-            const double2* r = reinterpret_cast<const double2*>(J.M[s] + (int64_t)row * B);
-            for (int q = PRE; 64 * q < B; ++q) {
-                const double2 u = v[32 * q + lane], w = r[32 * q + lane];
-                s0 = fma(w.x, u.x, s0);
-                s1 = fma(w.y, u.y, s1);
             }
+            acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+            acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+            if ((lane & 3) == 0 && lane < nl) tile[lane / 4][w] = acc;
+            __syncthreads();
+            if (w == 0 && lane < STEP_ROWS)
+                for (int k = 0; k < n / 64; ++k) sum += tile[k][lane];
         }
-    double s = s0 + s1;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) J.y[row] = J.base ? b - s : s;
+    }
+    if (w == 0 && lane < STEP_ROWS) {
+        const int r = blockIdx.x * STEP_ROWS + lane;
+        J.y[r] = J.base ? J.base[r] - sum : sum;
+    }
 }
 
 void launch_step(Ctx& c, int B, const StepJobs& jobs) {
@@ -425,7 +422,7 @@ int coarse_middle(int nb) { return (nb - 1) / 2; }
 }  // namespace
 
 int coarse_block_order(int n, int half_bandwidth) {
-    constexpr int Q = 64;         // a lane of k_rows reads double2: rows of 64 entries
+    constexpr int Q = 64;         // the solve's tiles
     const int want = std::max(half_bandwidth, 1);
     return std::max(Q, (std::min(want, n) + Q - 1) / Q * Q);
 }
@@ -515,6 +512,9 @@ void factor_coarse(Ctx& c, CoarseBlocks& cb, const std::function<void()>& overla
         keep_g(c, chain[1], k + 1);
     }
     inv_spd(c, Db(k), B, chain[0], inf);
+    // rows into the solve's order: D^-1 (symmetric), G^T (the columns of G) and G
+    k_order_rows<<<dim3(B, nb, 3), 128, 0, c.stream>>>(B, D, E, cb.gt.as<double>());
+    GMGS_LAUNCHED(c);
     c.trace_point("bc: coarsest block LDL^T");
     int h_info[2] = {0, 0};
     GMGS_CUDA(cudaMemcpyAsync(h_info, info.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
@@ -526,7 +526,7 @@ void launch_coarse_solve(Ctx& c, const CoarseBlocks& cb, double* cvec, double* x
     const int B = cb.B, nb = cb.nb, k = coarse_middle(nb);
     if (nb <= 0) return;
     const int64_t B2 = (int64_t)B * B;
-    auto Db = [&](int i) { return cb.sinv.as<double>() + i * B2; };    // symmetric
+    auto Db = [&](int i) { return cb.sinv.as<double>() + i * B2; };    // symmetric; rows in k_rows' order
     auto G = [&](int i) { return cb.gt.as<double>() + i * B2; };       // rows of G
     auto GT = [&](int i) { return cb.g.as<double>() + i * B2; };       // rows of G^T
     auto cv = [&](int i) { return cvec + (int64_t)i * B; };

@@ -535,7 +535,7 @@ __global__ void __launch_bounds__(NT, MODE == FM_CG_UPDATE_JACOBI ? ((STG & 1) ?
     if (MODE == FM_CG_DIRECTION || MODE == FM_CG_UPDATE_JACOBI) grid_dot_finish(dot.value(), a.dot, sh);
 }
 
-static int pick_zc(const Grid& g, const Ctx& c, int per_sm = 3) {
+static int pick_zc(const Grid& g, const Ctx& c, int per_sm, bool dot) {
     const int64_t cols = (int64_t)((g.ny + 1 + TY - 1) / TY) * ((g.nx + 1 + TX - 1) / TX);
     // ~24 waves of 3 resident CTAs: shorter z-chunks balance the tail and let
     // empty column tiles of real geometry skip more (12 waves: 214 -> 208 ms
@@ -544,13 +544,15 @@ static int pick_zc(const Grid& g, const Ctx& c, int per_sm = 3) {
     int64_t zc = (cols * (g.nz + 1) + want - 1) / want;
     // at least 6 planes per CTA where that still leaves four CTAs per SM (each
     // chunk stages two planes beyond its own: coarse levels 22.17 -> 21.96 ms
-    // per solve against 4; 8 was slower), else at least 4 where that does;
-    // smaller grids take one plane per CTA: there a CTA's chain of planes is
-    // the launch's time, not the planes staged twice (42 x 37 x 64 solve, the
-    // chunks of its three levels at 4 / 3 / 2 / 1 planes: 22.4 / 20.3 / 19.2 /
-    // 18.5 ms)
+    // per solve against 4; 8 was slower), else at least 4.  On grids where 4
+    // planes leave fewer, the down-sweep takes one plane per CTA: there a CTA's
+    // chain of planes is the launch's time, not the planes staged twice.  The
+    // modes with a dot product keep 4: a thread's compensated FP32 sum runs over
+    // its chunk, p.q cancels to a small part of |p||q|, and another grouping
+    // changes alpha's FP32 rounding often enough to move a solve's result in
+    // the ninth digit
     const int64_t full = 4 * (int64_t)c.num_sms;
-    const int64_t zmin = cols * ((g.nz + 1 + 5) / 6) >= full ? 6 : (cols * ((g.nz + 1 + 3) / 4) >= full ? 4 : 1);
+    const int64_t zmin = cols * ((g.nz + 1 + 5) / 6) >= full ? 6 : (dot || cols * ((g.nz + 1 + 3) / 4) >= full ? 4 : 1);
     if (zc < zmin) zc = zmin;
     if (zc > 64) zc = 64;
     return (int)zc;
@@ -647,7 +649,8 @@ void launch_fine(Ctx& c, const FineLevel& L, const Coef32& cf, const FineArgs& a
     // the CG update with its staged operands: longer z-chunks (2 instead of 3
     // in the wave count: 1.820 -> 1.792 ms, 1 gave 1.820 ms; the other modes
     // were slower with 2)
-    const int zc = pick_zc(L.g, c, MODE == FM_CG_UPDATE_JACOBI ? 2 : 3);
+    const int zc = pick_zc(L.g, c, MODE == FM_CG_UPDATE_JACOBI ? 2 : 3,
+                           MODE == FM_CG_UPDATE_JACOBI || MODE == FM_CG_DIRECTION);
     dim3 grid((L.g.ny + 1 + TY - 1) / TY, (L.g.nx + 1 + TX - 1) / TX, (L.g.nz + 1 + zc - 1) / zc);
     if (MODE == FM_VCYCLE_DOWN && a.n_perel > 0) {
         const int per = (NT / 8) * (int)(grid.x * grid.y);
