@@ -189,7 +189,7 @@ int64_t model_bytes(const gmgs::Model& M) {
                                       &lv.kslot, &lv.diag64, &lv.wdinv32, &lv.wdinv64, &lv.bnd_nodes, &lv.emask8, &lv.perel_nodes, &lv.node_slot, &lv.elem_slot,
                                       &lv.vr, &lv.vrp, &lv.vx, &lv.tile_occ, &lv.tile_occ64, &lv.tc_occ})
             b += (int64_t)d->bytes;
-    for (const gmgs::DevBuf* d : {&M.ke0_dev, &M.rho, &M.F, &M.U, &M.free_idx, &M.cb.sinv, &M.cb.g, &M.cb.gt, &M.cvec_in, &M.cvec_out,
+    for (const gmgs::DevBuf* d : {&M.ke0_dev, &M.galerkin_child, &M.galerkin_grand, &M.rho, &M.F, &M.U, &M.free_idx, &M.cb.sinv, &M.cb.g, &M.cb.gt, &M.cvec_in, &M.cvec_out,
                                   &M.cg_x, &M.cg_r, &M.cg_rb, &M.cg_p, &M.cg_p2, &M.cg_q64, &M.cg_z64, &M.mask_stencil, &M.cg_q32,
                                   &M.cg_z32, &M.cg_r32, &M.cg_r32b, &M.cg_pa, &M.cg_pb, &M.scal, &M.dot_partials, &M.dot_ticket, &M.tc_err})
         b += (int64_t)d->bytes;
@@ -395,27 +395,45 @@ int gmgs_set_bc(gmgs_handle* h, const int32_t* fixed, int64_t nfixed, const doub
     });
 }
 
+static void density_impl(gmgs_handle* h, const double* rho_dev, double penal) {
+    gmgs::Model& M = h->M;
+    gmgs::set_density_dev(M, rho_dev, penal);
+    if (M.bc_set)
+        gmgs::apply_bc(M, h->fixed_host.data(), (int64_t)h->fixed_host.size(), h->loads_host.data(),
+                       (int64_t)h->loads_host.size() / 4);
+}
+
 int gmgs_set_density(gmgs_handle* h, const double* rho, double penal) {
     return guarded(h, [&]() -> int {
         if (!h || !rho) fail(GMGS_ERR_INVALID_ARGUMENT, "NULL argument");
         if (!std::isfinite(penal) || penal < 0) fail(GMGS_ERR_INVALID_ARGUMENT, "invalid penalty");
         gmgs::Model& M = h->M;
         const int64_t ne = M.levels[0].n_elem;
-        for (int64_t i = 0; i < ne; ++i)
-            if (!(rho[i] > 0) || !std::isfinite(rho[i])) fail(GMGS_ERR_INVALID_ARGUMENT, "density must be positive");
         gmgs::DevBuf d = gmgs::dalloc(ne * sizeof(double));
         {
             HostPin pin(rho, ne * sizeof(double), true);
             GMGS_CUDA(cudaMemcpyAsync(d.p, rho, ne * sizeof(double), cudaMemcpyHostToDevice, M.ctx.stream));
             GMGS_CUDA(cudaStreamSynchronize(M.ctx.stream));
         }
-        M.penal = penal;
-        gmgs::set_density_dev(M, d.as<double>());
-        M.coarse_ready = false;
-        M.solved = false;
-        if (M.bc_set)
-            gmgs::apply_bc(M, h->fixed_host.data(), (int64_t)h->fixed_host.size(), h->loads_host.data(),
-                           (int64_t)h->loads_host.size() / 4);
+        density_impl(h, d.as<double>(), penal);
+        return GMGS_OK;
+    });
+}
+
+int gmgs_set_density_dev(gmgs_handle* h, const double* rho_dev, double penal) {
+    return guarded(h, [&]() -> int {
+        if (!h || !rho_dev) fail(GMGS_ERR_INVALID_ARGUMENT, "NULL argument");
+        if (!std::isfinite(penal) || penal < 0) fail(GMGS_ERR_INVALID_ARGUMENT, "invalid penalty");
+        density_impl(h, rho_dev, penal);
+        return GMGS_OK;
+    });
+}
+
+int gmgs_load_work(gmgs_handle* h, double* result) {
+    return guarded(h, [&]() -> int {
+        if (!h || !result) fail(GMGS_ERR_INVALID_ARGUMENT, "NULL argument");
+        if (!h->M.solved) fail(GMGS_ERR_NO_SOLUTION, "No Deformation Field Available, compute the deformation first");
+        *result = gmgs::load_work(h->M);
         return GMGS_OK;
     });
 }

@@ -432,7 +432,7 @@ void factor_coarse(Ctx& c, CoarseBlocks& cb, const std::function<void()>& overla
     const int64_t B2 = (int64_t)B * B;
     double* D = cb.sinv.as<double>();   // A_ii on entry
     double* E = cb.g.as<double>();      // E_i = A_(i,i-1) on entry (i >= 1)
-    cb.gt = dalloc((size_t)nb * B2 * sizeof(double));
+    if (cb.gt.bytes < (size_t)nb * B2 * sizeof(double)) cb.gt = dalloc((size_t)nb * B2 * sizeof(double));
     auto Db = [&](int i) { return D + i * B2; };
     auto Eb = [&](int i) { return E + i * B2; };
     auto Gt = [&](int i) { return cb.gt.as<double>() + i * B2; };

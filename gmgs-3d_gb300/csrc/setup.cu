@@ -745,27 +745,58 @@ __global__ void k_escale(int64_t ne, const int32_t* __restrict__ elem_slot, cons
     GRID_STRIDE(e, ne) esc[elem_slot[e]] = pow(rho[e], penal);
 }
 
+static void ensure(DevBuf& b, size_t bytes) {
+    if (b.bytes < bytes) b = dalloc(bytes);
+}
+
+__global__ void k_check_density(int64_t n, const double* __restrict__ rho, int* __restrict__ bad) {
+    int b = 0;
+    GRID_STRIDE(i, n) b |= !(rho[i] > 0.0) || !(rho[i] < INFINITY);
+    if (__any_sync(0xffffffffu, b) && (threadIdx.x & 31) == 0) atomicOr(bad, 1);
+}
+
 // Extension: finest element scale rho^penal; every coarse level then stores
-// one Galerkin matrix per element.
-void set_density_dev(Model& M, const double* rho_dev) {
+// one Galerkin matrix per element.  The levels, element types and node lists
+// follow from the occupancy alone: the first density builds them, later ones
+// only the scales, matrices and diagonals, in the same buffers.
+void set_density_dev(Model& M, const double* rho_dev, double penal) {
     Ctx& c = M.ctx;
     Level& l0 = M.levels[0];
-    M.rho = dalloc(l0.n_elem * sizeof(double));
+    {
+        DevBuf bad = dalloc(sizeof(int));
+        int h = 0;
+        GMGS_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), c.stream));
+        k_check_density<<<blocks_for(c, l0.n_elem), 256, 0, c.stream>>>(l0.n_elem, rho_dev, bad.as<int>());
+        GMGS_LAUNCHED(c);
+        GMGS_CUDA(cudaMemcpyAsync(&h, bad.p, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+        GMGS_CUDA(cudaStreamSynchronize(c.stream));
+        if (h) throw Error(GMGS_ERR_INVALID_ARGUMENT, "density must be positive");
+    }
+    const bool again = M.density_built;
+    M.density_built = false;
+    M.coarse_ready = false;
+    M.solved = false;
+    M.penal = penal;
+    ensure(M.rho, l0.n_elem * sizeof(double));
     GMGS_CUDA(cudaMemcpyAsync(M.rho.p, rho_dev, l0.n_elem * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
-    l0.escale64 = dalloc(l0.g.slots * sizeof(double));
-    GMGS_CUDA(cudaMemsetAsync(l0.escale64.p, 0, l0.g.slots * sizeof(double), c.stream));
+    if (!again) {
+        l0.escale64 = dalloc(l0.g.slots * sizeof(double));
+        GMGS_CUDA(cudaMemsetAsync(l0.escale64.p, 0, l0.g.slots * sizeof(double), c.stream));
+        l0.bnd_nodes.release();
+        l0.n_bnd = -1;
+    }
     k_escale<<<blocks_for(c, l0.n_elem), 256, 0, c.stream>>>(l0.n_elem, l0.elem_slot.as<int32_t>(), M.rho.as<double>(),
                                                              M.penal, l0.escale64.as<double>());
     GMGS_LAUNCHED(c);
-    l0.escale32.release();
-    l0.bnd_nodes.release();
-    l0.n_bnd = -1;
     M.has_density = true;
-    build_levels(M, nullptr);
-    build_operators(M);
+    if (!again) build_levels(M, nullptr);
+    build_operators(M, again);
+    M.density_built = true;
 }
 
-void build_operators(Model& M) {
+// matrices that depend on the material and the hierarchy alone, interior
+// flags and the lists of nodes on stored matrices
+static void build_structure(Model& M) {
     Ctx& c = M.ctx;
     const int L = M.num_levels;
     double Ke[KE], KeT[KE];
@@ -806,7 +837,6 @@ void build_operators(Model& M) {
                          (long long)M.levels[l].nK, (long long)M.levels[l].n_perel);
     M.ke0_dev = dalloc(KE * sizeof(double));
     GMGS_CUDA(cudaMemcpyAsync(M.ke0_dev.p, KeT, KE * sizeof(double), cudaMemcpyHostToDevice, c.stream));
-    const double* ke0 = M.ke0_dev.as<double>();
     // G_j = P_j^T Ke0 P_j for the 8 child positions j (SetupSolver.m:53-66 applied to one solid child)
     static_assert(KE == 576, "24x24 element matrices");
     auto child_product = [](const double* K, int j, double* out) {     // out = P_j^T K P_j
@@ -839,23 +869,33 @@ void build_operators(Model& M) {
     // Mixed precision with a density field: the level-2 matrices are kept in
     // FP32 only and level 3 is built from the 64 finest descendants
     // (about 60 % less device memory on large models).
-    const bool lean = M.has_density && M.prm.precision == GMGS_MIXED && L >= 3;
-    DevBuf G2;
-    if (lean) {
+    M.lean_level1 = M.has_density && M.prm.precision == GMGS_MIXED && L >= 3;
+    if (M.lean_level1) {
         std::vector<double> G2h(64 * KE);
         for (int cc = 0; cc < 8; ++cc)
             for (int j = 0; j < 8; ++j) child_product(&Gh[j * KE], cc, &G2h[(cc * 8 + j) * KE]);
-        G2 = dalloc(64 * KE * sizeof(double));
-        GMGS_CUDA(cudaMemcpyAsync(G2.p, G2h.data(), 64 * KE * sizeof(double), cudaMemcpyHostToDevice, c.stream));
+        M.galerkin_grand = dalloc(64 * KE * sizeof(double));
+        GMGS_CUDA(cudaMemcpyAsync(M.galerkin_grand.p, G2h.data(), 64 * KE * sizeof(double), cudaMemcpyHostToDevice, c.stream));
     }
-    M.lean_level1 = lean;
+    GMGS_CUDA(cudaStreamSynchronize(c.stream));   // the host tables go out of scope
+}
+
+// values_only: the hierarchy and the structure are unchanged, only the finest
+// element scales are new
+void build_operators(Model& M, bool values_only) {
+    Ctx& c = M.ctx;
+    const int L = M.num_levels;
+    if (!values_only) build_structure(M);
+    const bool lean = M.lean_level1;
+    const double* ke0 = M.ke0_dev.as<double>();
+    const DevBuf& G2 = M.galerkin_grand;
     // Galerkin matrices level by level
     for (int l = 1; l < L; ++l) {
         Level& lv = M.levels[l];
         Level& fv = M.levels[l - 1];
         if (lean && l == 1) {
             lv.Ks64.release();
-            lv.Ks32 = dalloc(std::max<int64_t>(1, lv.nK) * KE * sizeof(float));
+            ensure(lv.Ks32, std::max<int64_t>(1, lv.nK) * KE * sizeof(float));
             if (lv.nK > 0) {
                 k_galerkin<<<(unsigned)lv.nK, 192, 0, c.stream>>>(
                     lv.g, fv.g, lv.kslot.as<int32_t>(), fv.emask.as<uint8_t>(), fv.etype.as<int32_t>(), nullptr,
@@ -864,7 +904,7 @@ void build_operators(Model& M) {
             }
             continue;
         }
-        lv.Ks64 = dalloc(std::max<int64_t>(1, lv.nK) * KE * sizeof(double));
+        ensure(lv.Ks64, std::max<int64_t>(1, lv.nK) * KE * sizeof(double));
         if (lv.nK > 0 && lean && l == 2) {
             Level& l0 = M.levels[0];
             k_galerkin_grand<<<(unsigned)lv.nK, 192, 0, c.stream>>>(
@@ -884,7 +924,7 @@ void build_operators(Model& M) {
     for (int l = 0; l < L; ++l) {
         Level& lv = M.levels[l];
         if (l < L - 1) {
-            lv.diag64 = dalloc(3 * lv.g.slots * sizeof(double));
+            ensure(lv.diag64, 3 * lv.g.slots * sizeof(double));
             if (lean && l == 1) {
                 Level& l0 = M.levels[0];
                 k_diag_children<<<blocks_for(c, lv.g.slots), 256, 0, c.stream>>>(
@@ -907,13 +947,13 @@ void build_operators(Model& M) {
         }
         if (M.prm.precision == GMGS_MIXED) {
             if (lv.nK > 0 && l < L - 1 && !(lean && l == 1)) {
-                lv.Ks32 = dalloc(lv.nK * KE * sizeof(float));
+                ensure(lv.Ks32, lv.nK * KE * sizeof(float));
                 k_to_float<<<blocks_for(c, lv.nK * KE), 256, 0, c.stream>>>(lv.nK * KE, lv.Ks64.as<double>(),
                                                                              lv.Ks32.as<float>());
                 GMGS_LAUNCHED(c);
             }
             if (l == 0 && lv.escale64.p) {
-                lv.escale32 = dalloc(lv.g.slots * sizeof(float));
+                ensure(lv.escale32, lv.g.slots * sizeof(float));
                 k_to_float<<<blocks_for(c, lv.g.slots), 256, 0, c.stream>>>(lv.g.slots, lv.escale64.as<double>(),
                                                                              lv.escale32.as<float>());
                 GMGS_LAUNCHED(c);
@@ -1039,7 +1079,6 @@ void build_coarse_bc(Model& M, const std::function<void()>& overlap) {
         GMGS_CUDA(cudaStreamSynchronize(c.stream));
     }
     CoarseBlocks& cb = M.cb;
-    cb = CoarseBlocks();
     cb.n = n;
     cb.B = coarse_block_order(n, bw);
     cb.nb = (n + cb.B - 1) / cb.B;
@@ -1047,8 +1086,8 @@ void build_coarse_bc(Model& M, const std::function<void()>& overlap) {
     const size_t blk_bytes = (size_t)cb.nb * cb.B * cb.B * sizeof(double);
     if (blk_bytes > ((size_t)16 << 30))
         throw Error(GMGS_ERR_RESOLUTION, "coarsest level too large for the block factorisation; use more levels");
-    cb.sinv = dalloc(blk_bytes);
-    cb.g = dalloc(blk_bytes);
+    ensure(cb.sinv, blk_bytes);
+    ensure(cb.g, blk_bytes);
     GMGS_CUDA(cudaMemsetAsync(cb.sinv.p, 0, blk_bytes, c.stream));
     GMGS_CUDA(cudaMemsetAsync(cb.g.p, 0, blk_bytes, c.stream));
     k_assemble_blocks<<<blocks_for(c, (int64_t)n * 81), 256, 0, c.stream>>>(
@@ -1062,8 +1101,8 @@ void build_coarse_bc(Model& M, const std::function<void()>& overlap) {
     }
     c.trace_point("bc: coarsest free DOFs + block assembly");
     factor_coarse(c, cb, overlap);
-    M.cvec_in = dalloc(npad * sizeof(double));
-    M.cvec_out = dalloc(npad * sizeof(double));
+    ensure(M.cvec_in, npad * sizeof(double));
+    ensure(M.cvec_out, npad * sizeof(double));
     GMGS_CUDA(cudaMemsetAsync(M.cvec_in.p, 0, npad * sizeof(double), c.stream));
     GMGS_CUDA(cudaMemsetAsync(M.cvec_out.p, 0, npad * sizeof(double), c.stream));
     GMGS_CUDA(cudaStreamSynchronize(c.stream));

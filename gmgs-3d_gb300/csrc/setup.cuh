@@ -15,6 +15,7 @@ struct Model {
     double ele[3] = {1, 1, 1};
     int num_levels = 0;
     bool has_density = false;
+    bool density_built = false;   // levels and operators stand for a density field
     double penal = 3.0;
     std::vector<Level> levels;
     Ctx ctx;
@@ -22,6 +23,7 @@ struct Model {
     double ke0_rows[KE];   // Ke0 with row = output DOF
     DevBuf ke0_dev;
     DevBuf galerkin_child; // 8 x 24x24: P_j^T Ke0 P_j per child position j
+    DevBuf galerkin_grand; // 64 x 24x24: the same over two levels (mixed precision + density)
     bool lean_level1 = false; // level-2 (index 1) matrices kept in FP32 only (mixed precision + density)
     Coef64 coef64{};       // factorised FP64 stencil of this handle's material and voxel
     DevBuf mask_stencil;   // its 256 boundary stencils
@@ -69,12 +71,12 @@ void stress_coefficients(double E, double nu, const double ele[3], double c[6]);
 
 // setup.cu
 void build_levels(Model& M, const int32_t* occ_dev);
-void build_operators(Model& M);
+void build_operators(Model& M, bool values_only = false);
 void build_boundary_list(Model& M, int l);
 void apply_bc(Model& M, const int32_t* fixed, int64_t nfixed, const double* loads, int64_t nload);
 // overlap: see factor_coarse
 void build_coarse_bc(Model& M, const std::function<void()>& overlap = {});
-void set_density_dev(Model& M, const double* rho_dev);
+void set_density_dev(Model& M, const double* rho_dev, double penal);
 
 // solver.cu
 void alloc_work(Model& M);
@@ -86,6 +88,7 @@ void operator_apply(Model& M, int level, const double* x, double* y);
 
 // post.cu
 void stress_dev(Model& M, const double* U_dense, double* nodal_compact, float* per_voxel_compact);
+double load_work(Model& M);   // F . U of the last solve
 void grad_dev(Model& M, const double* U_dense, const double* lam_dense, double* dJdrho_compact);
 
 }  // namespace gmgs

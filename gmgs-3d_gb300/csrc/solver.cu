@@ -664,6 +664,16 @@ static int pcg_fp64(Model& M, const double* b, double* x, int32_t* iters_out, do
     return status;
 }
 
+double load_work(Model& M) {
+    Ctx& c = M.ctx;
+    double* out = M.scal.as<double>() + SC_N - 1;
+    launch_dot<double, double>(c, dots(M), 3 * M.levels[0].g.slots, M.F.as<double>(), M.U.as<double>(), out);
+    double v = 0;
+    GMGS_CUDA(cudaMemcpyAsync(&v, out, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    GMGS_CUDA(cudaStreamSynchronize(c.stream));
+    return v;
+}
+
 int pcg_solve(Model& M, const double* b, double* x, int32_t* iters_out, double* relres_out, double* hist) {
     return M.prm.precision == GMGS_MIXED ? pcg_mixed(M, b, x, iters_out, relres_out, hist)
                                          : pcg_fp64(M, b, x, iters_out, relres_out, hist);

@@ -57,6 +57,8 @@ SIGNATURES = {
     "gmgs_create": (C.c_int, [_i32p, _i32, _i32, _i32, _dp, C.POINTER(Params), C.POINTER(_p)]),
     "gmgs_set_bc": (C.c_int, [_p, _i32p, _i64, _dp, _i64]),
     "gmgs_set_density": (C.c_int, [_p, _dp, _d]),
+    "gmgs_set_density_dev": (C.c_int, [_p, _p, _d]),
+    "gmgs_load_work": (C.c_int, [_p, _dp]),
     "gmgs_solve": (C.c_int, [_p, _dp, _i32p, _dp, _dp]),
     "gmgs_solve_dev": (C.c_int, [_p, _p, _i32p, _dp, _dp]),
     "gmgs_stress": (C.c_int, [_p, _dp, _fp]),

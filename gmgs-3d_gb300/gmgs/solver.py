@@ -178,9 +178,9 @@ class Solver:
     def load_vector(self):
         """F (3*num_nodes, interleaved) as ApplyBoundaryCondition.m:7-10 builds it."""
         F = np.zeros(3 * self.num_nodes(1))
-        for row in self._loads:               # a later duplicate id wins
-            i = 3 * (int(row[0]) - 1)
-            F[i:i + 3] = row[1:4]
+        ids = self._loads[:, 0].astype(np.int64) - 1
+        last = len(ids) - 1 - np.unique(ids[::-1], return_index=True)[1]   # a later duplicate id wins
+        F.reshape(-1, 3)[ids[last]] = self._loads[last, 1:4]
         return F
 
     def set_density(self, rho, penal: float = 3.0):
@@ -188,6 +188,16 @@ class Solver:
         if r.size != self.num_elements(1):
             raise ValueError("rho must have one entry per solid voxel")
         self._check(self._lib.gmgs_set_density(self._h, _dptr(r), penal))
+
+    def set_density_dev(self, rho_ptr: int, penal: float = 3.0):
+        """set_density from device memory (num_elements float64)."""
+        self._check(self._lib.gmgs_set_density_dev(self._h, C.c_void_p(rho_ptr), penal))
+
+    def load_work(self) -> float:
+        """F^T U of the last solve (the compliance), formed on the device."""
+        out = C.c_double()
+        self._check(self._lib.gmgs_load_work(self._h, C.byref(out)))
+        return out.value
 
     def solve(self, with_history=False, out=None):
         """Return U (3*num_nodes, interleaved); raise on divergence.

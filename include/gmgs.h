@@ -112,6 +112,8 @@ int gmgs_set_bc(gmgs_handle* h, const int32_t* fixed_nodes, int64_t nfixed,
  * on the finest level, in the compact element order (eleMapBack,
  * DiscretizeDesignDomain.m:68).  Rebuilds every coarse operator. */
 int gmgs_set_density(gmgs_handle* h, const double* rho, double penal);
+/* The same from device memory (num_elements doubles, ready when called). */
+int gmgs_set_density_dev(gmgs_handle* h, const double* rho_dev, double penal);
 
 /* Solve K U = F.  Replaces GetDeformation() / CG_solver(@AtX,@Vcycle,...)
  * (src/kernel/GetDeformation.m:1-22, src/kernel/CG_solver.m:1-56).
@@ -135,6 +137,8 @@ int gmgs_stress_dev(gmgs_handle* h, double* nodal_dev, float* per_voxel_dev);
  * interleaved vector (an adjoint solve K lambda = ell with the same PCG).
  * dJdrho: num_elements doubles in the compact element order. */
 int gmgs_grad(gmgs_handle* h, const double* ell, double* dJdrho);
+/* Extension: the compliance F^T U of the last solve, formed on the device. */
+int gmgs_load_work(gmgs_handle* h, double* result);
 int gmgs_grad_dev(gmgs_handle* h, const double* ell_dev, double* dJdrho_dev);
 
 /* Operator handles of CG_solver: AtX(x, level) (src/kernel/AtX.m:1-58) and

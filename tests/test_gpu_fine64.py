@@ -120,3 +120,47 @@ def test_operator_keeps_non_finite_values(bad):
     near = (abs(iy - iy[at // 3]) <= 1) & (abs(ix - ix[at // 3]) <= 1) & (abs(iz - iz[at // 3]) <= 1)
     assert not np.isfinite(y.reshape(-1, 3)[near]).all(axis=1).any()
     assert np.all(np.abs(y - clean).reshape(-1, 3)[~near] <= 1e-13)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_later_densities_equal_a_fresh_handle(precision):
+    """The second density of a handle reuses the hierarchy of the first; device and
+    host densities give the same bits, and what was refused is refused."""
+    torch = pytest.importorskip("torch")
+    from gmgs import GMGSError
+    from gmgs.autograd import compliance
+    vox = synthetic.sphere_voids(20, 18, 28, 2, 6)
+    fixed, loads = synthetic.boundary_conditions(vox, 3)
+    first, second = (synthetic.density(int(vox.sum()), (0.2, 1.0), k) for k in (1, 2))
+
+    def handle():
+        s = Solver(vox, omega=0.4, num_levels=3, precision=precision)
+        s.set_bc(fixed, loads)
+        return s
+
+    fresh, kept = handle(), handle()
+    fresh.set_density(second, 2.0)
+    u_ref, g_ref = fresh.solve(), fresh.grad()
+    kept.set_density(first, 3.0)
+    kept.solve()
+    kept.set_bc(fixed, loads)
+    with pytest.raises(GMGSError):
+        kept.set_density(np.where(np.arange(len(second)) == 7, -1.0, second), 2.0)
+    on_gpu = torch.tensor(second, device="cuda")
+    torch.cuda.synchronize()
+    kept.set_density_dev(on_gpu.data_ptr(), 2.0)
+    u = kept.solve()
+    assert np.array_equal(u, u_ref) and np.array_equal(kept.grad(), g_ref)
+    assert abs(kept.load_work() - kept.load_vector() @ u) <= 1e-12 * abs(kept.load_work())
+    for bad in (np.nan, np.inf, 0.0):
+        wrong = on_gpu.clone()
+        wrong[3] = bad
+        torch.cuda.synchronize()
+        with pytest.raises(GMGSError):
+            kept.set_density_dev(wrong.data_ptr(), 2.0)
+    for device in ("cpu", "cuda"):
+        rho = torch.tensor(second, device=device, requires_grad=True)
+        j = compliance(rho, kept, 2.0)
+        (2 * j).backward()
+        assert abs(j.item() - kept.load_vector() @ u_ref) <= 1e-12 * abs(j.item())
+        assert np.array_equal(rho.grad.cpu().numpy(), 2 * g_ref)
