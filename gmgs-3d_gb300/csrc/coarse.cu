@@ -40,7 +40,7 @@
 //     root and the division of each column; it forms both from one FP32
 //     reciprocal square root, while the other warps update
 //   - L^-T L^-1 is symmetric: half of its tiles are computed
-// Measured for 15 blocks of order 448: factorisation 14 -> FACT_MS ms; the solve's
+// Measured for 15 blocks of order 448: factorisation 14 -> 8.0 ms; the solve's
 // launches 8 -> 4 us each (a warp per row instead of 64 x 64 tiles with partial
 // sums in memory and arrival counters).
 #include "setup.cuh"
@@ -60,9 +60,10 @@ enum : int { OUT_ALL = 0, OUT_LOWER = 1, OUT_MIRROR = 2 };
 // read), OUT_MIRROR computes a symmetric product's lower half and stores both.
 constexpr int GR = 16, GC = 8, GK = 16, GT = GR * GC;
 template <bool TA, bool TB, int TRI, int OUT>
-__global__ void __launch_bounds__(GT) k_dgemm(int k, double alpha, const double* __restrict__ A, int lda,
-                                              const double* __restrict__ B, int ldb, double beta, double* __restrict__ C,
-                                              int ldc) {
+__global__ void __launch_bounds__(GT) k_dgemm(int k, double alpha, const double* A, int lda, const double* B, int ldb, double beta,
+                                              double* C, int ldc) {
+    pdl_begin();
+    pdl_wait();
     const int r0 = blockIdx.x * GR, c0 = blockIdx.y * GC;
     if (OUT != OUT_ALL && r0 + GR <= c0) return;
     __shared__ double As[2][GK][GR + 1];   // As[.][l][i] = op(A)(r0 + i, k0 + l)
@@ -113,15 +114,14 @@ template <bool TA, bool TB, int TRI, int OUT>
 void gemm(Ctx& c, int m, int n, int k, double alpha, const double* A, int lda, const double* B, int ldb, double beta,
           double* C, int ldc) {
     if (m <= 0 || n <= 0) return;
-    k_dgemm<TA, TB, TRI, OUT><<<dim3(m / GR, n / GC), GT, 0, c.stream>>>(k, alpha, A, lda, B, ldb, beta, C, ldc);
-    GMGS_LAUNCHED(c);
+    launch_chain(c, k_dgemm<TA, TB, TRI, OUT>, dim3(m / GR, n / GC), GT, 0, k, alpha, A, lda, B, ldb, beta, C, ldc);
 }
 
 // sqrt(d) and 1 / sqrt(d)'s rounded value's reciprocal, both correctly rounded,
 // for a positive normal d: an FP32 reciprocal square root y, one third-order
 // step (y (1 + h / 2 + 3 h^2 / 8), h = 1 - d y^2, error h^3), then Markstein's
 // final steps: s = RN(s0 + (d - s0^2) y / 2) and RN(y + y (1 - s y)) with exact
-// FMA residuals.  Ten dependent FP64 operations; the library's square root and
+// FMA residuals.  Ten dependent FP64 operations of 64 clocks; the library's square root and
 // division of a lane take about 25.  Outside the FP32 range: the library's.
 __device__ __forceinline__ void sqrt_and_reciprocal(double d, double& s, double& r) {
     const int e = (__double2hiint(d) >> 20) - 1023;
@@ -134,7 +134,8 @@ __device__ __forceinline__ void sqrt_and_reciprocal(double d, double& s, double&
     const double h = fma(-(d * y), y, 1.0);
     y = fma(y, h * fma(0.375, h, 0.5), y);
     const double s0 = d * y;
-    s = fma(fma(-s0, s0, d), 0.5 * y, s0);
+    const double half = __hiloint2double(__double2hiint(y) - (1 << 20), __double2loint(y));
+    s = fma(fma(-s0, s0, d), half, s0);
     r = fma(y, fma(-s, y, 1.0), y);
 }
 
@@ -144,10 +145,12 @@ __device__ __forceinline__ void sqrt_and_reciprocal(double d, double& s, double&
 // (forward substitution of L X = I carried along: X(j, c) is final once
 // scaled by 1 / L(j,j)), then the rank-1 updates of the rows below j of A and
 // of X.  Warp 0 updates row j + 1 first and goes on to its square root while
-// the other warps update the rest.  A pivot that is not positive sets *info and
+// the warps of the other three quarters of the SM update the rest (warp 4
+// shares warp 0's quarter and would hold its chain up).  A pivot that is not positive sets *info and
 // is replaced by 1 so the arithmetic stays finite.
-__global__ void __launch_bounds__(256) k_chol_inv32(double* __restrict__ A, int lda, double* __restrict__ Li, int ldl,
-                                                    int* __restrict__ info) {
+__global__ void __launch_bounds__(256) k_chol_inv32(double* A, int lda, double* Li, int ldl, int* __restrict__ info) {
+    pdl_begin();
+    pdl_wait();
     __shared__ double a[32][33];   // a[c][r] = A(r, c), becomes L
     __shared__ double x[32][33];   // x[c][r] = X(r, c), becomes L^-1
     __shared__ double s_piv, s_inv;
@@ -158,7 +161,8 @@ __global__ void __launch_bounds__(256) k_chol_inv32(double* __restrict__ A, int 
         x[cc][r] = r == cc ? 1.0 : 0.0;
     }
     auto pivot = [&](double d) {
-        const bool ok = d > 0.0 && d < INFINITY;
+        const int hi = __double2hiint(d);
+        const bool ok = hi >= 0x00100000 && hi < 0x7ff00000;    // positive, normal, finite
         if (!ok) atomicExch(info, 1);
         double s = 1.0, r = 1.0;
         if (ok) sqrt_and_reciprocal(d, s, r);
@@ -192,8 +196,8 @@ __global__ void __launch_bounds__(256) k_chol_inv32(double* __restrict__ A, int 
                 const double d = row(j + 1);
                 if (lane == j + 1) pivot(d);
             }
-        } else {
-            for (int r = j + 1 + w; r < 32; r += 7) row(r);
+        } else if (w != 4) {
+            for (int r = j + 1 + (w < 4 ? w : w - 1); r < 32; r += 6) row(r);
         }
     }
     __syncthreads();
@@ -280,8 +284,7 @@ struct Chain {
 // L^-1_21 = -L22^-1 L21 L11^-1.  L21 goes to the same place of Lo; T: scratch.
 void chol_inv(Ctx& c, double* A, double* Li, double* Lo, int n, int ld, double* T, int* info) {
     if (n == 32) {
-        k_chol_inv32<<<1, 256, 0, c.stream>>>(A, ld, Li, ld, info);
-        GMGS_LAUNCHED(c);
+        launch_chain(c, k_chol_inv32, 1, 256, 0, A, ld, Li, ld, info);
         return;
     }
     const int n1 = 32 * ((n / 32) / 2), n2 = n - n1;
@@ -295,8 +298,9 @@ void chol_inv(Ctx& c, double* A, double* Li, double* Lo, int n, int ld, double* 
     gemm<false, false, TRI_A_LOWER, OUT_ALL>(c, n2, n1, n2, -1.0, Li + at22, ld, T, n2, 0.0, Li + n1, ld);
 }
 
-// D^-1 of the SPD block D (lower triangle in, both triangles out).  Plain
-// launches: as programmatic dependents the two chains hold each other up.
+// D^-1 of the SPD block D (lower triangle in, both triangles out): 68 dependent
+// launches per block of order 448, as programmatic dependents of each other (15
+// blocks 8.0 ms, as plain launches 8.7 ms)
 void inv_spd(Ctx& c, double* D, int B, Chain& s, int* info) {
     double* li = s.li.as<double>();
     GMGS_CUDA(cudaMemsetAsync(li, 0, (size_t)B * B * sizeof(double), c.stream));
