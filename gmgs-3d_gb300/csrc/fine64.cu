@@ -128,6 +128,17 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// beta = r.z / r_old.z_old of the direction, alpha = r.z / p.q of the update:
+// one division per CTA
+template <int MODE>
+__device__ __forceinline__ double step_length(const Args64& a) {
+    if (!has_dot(MODE) || a.first) return 0.0;
+    __shared__ double s_ab;
+    if (threadIdx.x == 0) s_ab = a.scal[a.cur] / a.scal[MODE == M64_CG_DIRECTION ? (a.cur ^ 1) : 2];
+    __syncthreads();
+    return s_ab;
+}
+
 // sum over the N lanes of a list node
 template <int N>
 __device__ __forceinline__ double lanes_sum(double v) {
@@ -144,7 +155,7 @@ __device__ __forceinline__ double lanes_sum(double v) {
 // A node on stored matrices, 8 lanes: the element sum, lane j taking the
 // coupling to element node j.
 template <int MODE, bool BND>
-__device__ void list_node(const Level64& L, const Args64& a, int at, int j, double ab, double& dot) {
+__device__ void list_node(const Level64& L, const Args64& a, int at, int j, double& dot) {
     const Grid& g = L.g;
     const int64_t S = g.slots, n3 = 3 * S, sx = g.sx(), sz = g.sz();
     const int count = BND ? L.n_bnd : L.n_perel;
@@ -164,6 +175,8 @@ __device__ void list_node(const Level64& L, const Args64& a, int at, int j, doub
             if (type[e] > 0 && !chk::ok(type[e] - 1, L.nK, chk::F64_LIST)) type[e] = -1;
         }
     }
+    pdl_wait();                      // the lists, masks and types above do not change during a solve
+    const double ab = step_length<MODE>(a);
     if (BND) {
         const MaskStencil& T = L.mask_stencil[mask];      // mask 0 (idle lanes): no offsets
         for (int t = j; t < T.n; t += BND_LANES) {
@@ -216,21 +229,18 @@ __device__ void list_node(const Level64& L, const Args64& a, int at, int j, doub
     }
 }
 
-// beta = r.z / r_old.z_old of the direction, alpha = r.z / p.q of the update:
-// one division per CTA
-template <int MODE>
-__device__ __forceinline__ double step_length(const Args64& a) {
-    if (!has_dot(MODE) || a.first) return 0.0;
-    __shared__ double s_ab;
-    if (threadIdx.x == 0) s_ab = a.scal[a.cur] / a.scal[MODE == M64_CG_DIRECTION ? (a.cur ^ 1) : 2];
-    __syncthreads();
-    return s_ab;
-}
-
 template <int MODE>
 __device__ __forceinline__ void dot_finish(double dot, const Args64& a, double* sh) {
     if (has_dot(MODE)) grid_dot_finish(dot, DotOut{a.dot.partials, a.dot.ticket, a.dot.out}, sh);
 }
+
+// A warp holds the y columns x and x + 8 of the tile: at the planes' pitch of
+// 18 their 16 words each fall into opposite halves of the 32 banks (columns x
+// and x + 1 would share two banks, a second pass for every access: 44 M of 100 M
+// shared-memory wavefronts of a down-sweep at 6.4M nodes).
+__device__ __forceinline__ int tile_y(int tid) { return tid & (TY - 1); }
+__device__ __forceinline__ int tile_x(int tid) { return (tid >> 5) + 8 * ((tid >> 4) & 1); }
+static_assert(TY == 16 && TX == 16 && HY == 18, "two columns 8 apart are 16 banks apart");
 
 // this thread's points of a tile plane: its own node and, for the first
 // NHALO threads, one point of the one-node halo
@@ -240,7 +250,7 @@ struct Points {
     bool cok, hok;          // inside the allocated grid
     int cy, cx;
     __device__ Points(const Grid& g, int y0, int x0, int tid) {
-        const int ly = tid & (TY - 1), lx = tid / TY;
+        const int ly = tile_y(tid), lx = tile_x(tid);
         cy = y0 + ly;
         cx = x0 + lx;
         pc = (ly + 1) + (lx + 1) * HY;
@@ -303,15 +313,13 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
     const int tid = threadIdx.x;
     const Grid& g = L.g;
     pdl_begin();
-    pdl_wait();
-    const double ab = step_length<MODE>(a);
     double dot = 0.0;
     if ((int)blockIdx.x < nb_list) {
         if ((int)blockIdx.x < nb_bnd)
-            list_node<MODE, true>(L, a, (int)blockIdx.x * (NT / BND_LANES) + tid / BND_LANES, tid % BND_LANES, ab, dot);
+            list_node<MODE, true>(L, a, (int)blockIdx.x * (NT / BND_LANES) + tid / BND_LANES, tid % BND_LANES, dot);
         else
             list_node<MODE, false>(L, a, ((int)blockIdx.x - nb_bnd) * (NT / ELEM_LANES) + tid / ELEM_LANES, tid % ELEM_LANES,
-                                   ab, dot);
+                                   dot);
         dot_finish<MODE>(dot, a, sh);
         return;
     }
@@ -319,18 +327,19 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
     const int bty = bid % tiles_y, btx = bid / tiles_y % tiles_x, btz = bid / (tiles_y * tiles_x);
     const int y0 = bty * TY, x0 = btx * TX;
     const int zb = btz * zc, ze = min(zb + zc, g.nz + 1);       // node planes [zb, ze)
-    auto occ = [&](int iz) { return L.tile_occ[((int64_t)iz * tiles_x + btx) * tiles_y + bty] != 0; };
-    {
-        bool any = false;
-        for (int iz = zb; iz < ze; ++iz) any |= occ(iz);
-        if (!any) {                                             // uniform across the CTA
-            dot_finish<MODE>(0.0, a, sh);
-            return;
-        }
-    }
+    uint32_t occ = 0;                                           // planes of the chunk (at most 32) with a solid node in the tile
+    for (int iz = zb; iz < ze; ++iz)
+        occ |= L.tile_occ[((int64_t)iz * tiles_x + btx) * tiles_y + bty] != 0 ? 1u << (iz - zb) : 0u;
     const int64_t S = g.slots, n3 = 3 * S, sz = g.sz();
     const Points p(g, y0, x0, tid);
     const bool own = p.cy <= g.ny && p.cx <= g.nx;
+    uint32_t f_next = own ? chk::ld(L.nflag, p.cbase + zb * sz, S, chk::F64_FIELD) : 0u;
+    pdl_wait();                                                 // occupancy and flags do not change during a solve
+    if (!occ) {                                                 // uniform across the CTA
+        dot_finish<MODE>(0.0, a, sh);
+        return;
+    }
+    const double ab = step_length<MODE>(a);
     constexpr int NA = field_arrays64(MODE);
     constexpr int R = chk::F64_TILE;
     double* const stage = dyn;                    // [2][NA * 3][NP] field inputs of two planes
@@ -484,7 +493,7 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
         Rr[1] = Rr[1] + mul_frac(mx(8), cf.fgyz);
         Rr[2] = mx(7);
     };
-    const int xc = (p.pc % HY) + (tid / TY) * HY;                // own point of the x stage
+    const int xc = p.pc - HY;                // own point of the x stage
     const int hxc = tid & (2 * TX - 1), hyy = (hxc & 1) ? HY - 1 : 0;      // the y halo's points: one warp
     const int hz_pt = hyy + ((hxc >> 1) + 1) * HY, hx_pt = hyy + (hxc >> 1) * HY;
 
@@ -493,7 +502,8 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
         if (iz + 1 < ze) issue(iz + 2);
         cp_async_commit();
         const int64_t n = p.cbase + iz * sz;
-        const uint32_t f = own ? chk::ld(L.nflag, n, S, chk::F64_FIELD) : 0u;
+        const uint32_t f = f_next;              // loaded a plane ahead: the x and p loads below depend on it
+        if (own && iz + 1 < ze) f_next = chk::ld(L.nflag, n + sz, S, chk::F64_FIELD);
         const bool node = (f & NF_INTERIOR) != 0;
         double xx[3] = {0.0, 0.0, 0.0}, px[3] = {0.0, 0.0, 0.0};
         if (MODE == M64_CG_UPDATE_JACOBI && node) {
@@ -514,7 +524,7 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
         ec = ep;
         lm = lc;
         lc = lp;
-        if (!occ(iz)) {                                          // uniform across the CTA, as the next one
+        if (!((occ >> (iz - zb)) & 1u)) {                        // uniform across the CTA, as the next one
         } else if (cf.fixed && range <= FIXED_RANGE && E > 1023 - 700 && E < 1023 + 700) {
             z_stage_i(p.pc, vm, vc, vp, E);
             if (tid < NHALO) z_stage_i(p.ph, hm, hc, hp, E);
@@ -827,7 +837,7 @@ __global__ void __launch_bounds__(NT, 2) k_modal64(Level64 L, const __grid_const
                 }
             }
             __syncthreads();
-            const int ly = tid & (TY - 1), lx = tid / TY;
+            const int ly = tile_y(tid), lx = tile_x(tid);
             const int e00 = ly + lx * EY;      // the element with this node at its (1, 1) corner
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
