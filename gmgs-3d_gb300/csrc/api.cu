@@ -189,9 +189,9 @@ int64_t model_bytes(const gmgs::Model& M) {
                                       &lv.kslot, &lv.diag64, &lv.wdinv32, &lv.wdinv64, &lv.bnd_nodes, &lv.emask8, &lv.perel_nodes, &lv.node_slot, &lv.elem_slot,
                                       &lv.vr, &lv.vrp, &lv.vx, &lv.tile_occ, &lv.tile_occ64, &lv.tc_occ})
             b += (int64_t)d->bytes;
-    for (const gmgs::DevBuf* d : {&M.ke0_dev, &M.galerkin_child, &M.galerkin_grand, &M.rho, &M.F, &M.U, &M.free_idx, &M.cb.sinv, &M.cb.g, &M.cb.gt, &M.cvec_in, &M.cvec_out,
+    for (const gmgs::DevBuf* d : {&M.ke0_dev, &M.galerkin_child, &M.galerkin_grand, &M.rho, &M.F, &M.U, &M.free_idx, &M.free_rank, &M.cb.sinv, &M.cb.g, &M.cb.gt, &M.cvec_in, &M.cvec_out,
                                   &M.cg_x, &M.cg_r, &M.cg_rb, &M.cg_p, &M.cg_p2, &M.cg_q64, &M.cg_z64, &M.mask_stencil, &M.cg_q32,
-                                  &M.cg_z32, &M.cg_r32, &M.cg_r32b, &M.cg_pa, &M.cg_pb, &M.scal, &M.dot_partials, &M.dot_ticket, &M.tc_err})
+                                  &M.cg_z32, &M.cg_r32, &M.cg_r32b, &M.cg_pa, &M.cg_pb, &M.scal, &M.dot_partials, &M.dot_ticket})
         b += (int64_t)d->bytes;
     return b;
 }

@@ -330,13 +330,19 @@ struct StepJob {
     const double* base;
     double* y;
     int nseg;
+    int out;             // y is final: its first row in the solution, else -1
 };
 struct StepJobs {
     StepJob j[MAX_JOBS];
+    CoarseOut out;
     int n = 0;
     void add(double* y, const double* base, const double* M0, const double* v0, const double* M1 = nullptr,
              const double* v1 = nullptr) {
-        j[n++] = {{M0, M1}, {v0, v1}, base, y, M1 ? 2 : 1};
+        j[n++] = {{M0, M1}, {v0, v1}, base, y, M1 ? 2 : 1, -1};
+    }
+    void add_final(int row, double* y, const double* base, const double* M0, const double* v0) {
+        add(y, base, M0, v0);
+        j[n - 1].out = row;
     }
 };
 
@@ -412,7 +418,13 @@ __global__ void __launch_bounds__(32 * STEP_ROWS) k_rows(int B, const __grid_con
     }
     if (w == 0 && lane < STEP_ROWS) {
         const int r = blockIdx.x * STEP_ROWS + lane;
-        J.y[r] = J.base ? J.base[r] - sum : sum;
+        const double y = J.base ? J.base[r] - sum : sum;
+        J.y[r] = y;
+        if (J.out >= 0 && J.out + r < jobs.out.n) {         // to the level's vector (a scatter launch less)
+            const int32_t slot = jobs.out.idx[J.out + r];
+            if (jobs.out.f) jobs.out.f[slot] = (float)y;
+            else jobs.out.d[slot] = y;
+        }
     }
 }
 
@@ -526,7 +538,7 @@ void factor_coarse(Ctx& c, CoarseBlocks& cb, const std::function<void()>& overla
     if (h_info[0] || h_info[1]) throw Error(GMGS_ERR_NOT_SPD, "coarsest-level matrix is not positive definite");
 }
 
-void launch_coarse_solve(Ctx& c, const CoarseBlocks& cb, double* cvec, double* x) {
+void launch_coarse_solve(Ctx& c, const CoarseBlocks& cb, double* cvec, double* x, const CoarseOut& out) {
     const int B = cb.B, nb = cb.nb, k = coarse_middle(nb);
     if (nb <= 0) return;
     const int64_t B2 = (int64_t)B * B;
@@ -543,6 +555,7 @@ void launch_coarse_solve(Ctx& c, const CoarseBlocks& cb, double* cvec, double* x
     const int steps = std::max(top, bot);
     for (int step = 0; step < steps; ++step) {
         StepJobs J;
+        J.out = out;
         if (step == steps - 1) {              // the middle block's right-hand side: both chains have ended
             if (top > 0 && bot > 0) J.add(cv(k), cv(k), G(k), cv(k - 1), G(k + 1), cv(k + 1));
             else J.add(cv(k), cv(k), G(bot > 0 ? k + 1 : k), cv(bot > 0 ? k + 1 : k - 1));
@@ -560,14 +573,16 @@ void launch_coarse_solve(Ctx& c, const CoarseBlocks& cb, double* cvec, double* x
     }
     {
         StepJobs J;
-        J.add(xv(k), nullptr, Db(k), cv(k));
+        J.out = out;
+        J.add_final(k * B, xv(k), nullptr, Db(k), cv(k));
         launch_step(c, B, J);
     }
     // backward chains, in place on x: top i = k-1..0, bottom i = k+1..nb-1
     for (int s = 0; s < steps; ++s) {
         StepJobs J;
-        if (s < top) J.add(xv(k - 1 - s), xv(k - 1 - s), GT(k - s), xv(k - s));
-        if (s < bot) J.add(xv(k + 1 + s), xv(k + 1 + s), GT(k + 1 + s), xv(k + s));
+        J.out = out;
+        if (s < top) J.add_final((k - 1 - s) * B, xv(k - 1 - s), xv(k - 1 - s), GT(k - s), xv(k - s));
+        if (s < bot) J.add_final((k + 1 + s) * B, xv(k + 1 + s), xv(k + 1 + s), GT(k + 1 + s), xv(k + s));
         launch_step(c, B, J);
     }
 }

@@ -369,11 +369,10 @@ struct DotScratch { double* partials; unsigned int* ticket; int blocks; };
 template <typename Ta, typename Tb>
 void launch_dot(Ctx& c, const DotScratch& s, int64_t n, const Ta* a, const Tb* b, double* out);
 
-// coarsest level: gather free DOFs, scatter back
+// the same onto the coarsest level's free DOFs: cvec[rank[slot]] (rank -1: fixed)
 template <typename T>
-void launch_gather(Ctx& c, int64_t n, const int32_t* idx, const T* src, double* dst);
-template <typename T>
-void launch_scatter(Ctx& c, int64_t n, const int32_t* idx, const double* src, T* dst);
+void launch_restrict_free(Ctx& c, const Grid& gf, const Grid& gc, const uint8_t* nflag_c, const T* rf, const int32_t* rank,
+                          double* cvec);
 // coarsest level: block-tridiagonal LDL^T of the free-DOF matrix, factored
 // from both ends towards the middle block (coarse.cu)
 struct CoarseBlocks {
@@ -388,8 +387,16 @@ int coarse_block_order(int n, int half_bandwidth);
 // overlap: host work run while the two halves factor on their own streams
 // (it may enqueue on c.stream); may be empty
 void factor_coarse(Ctx& c, CoarseBlocks& cb, const std::function<void()>& overlap);
+// where the solution goes besides x: slot idx[i] of the level's dense vector,
+// in FP32 or FP64
+struct CoarseOut {
+    const int32_t* idx;
+    float* f;
+    double* d;
+    int n;
+};
 // x = A^-1 r: r in cvec (overwritten), both nb*B long with zero padding
-void launch_coarse_solve(Ctx& c, const CoarseBlocks& cb, double* cvec, double* x);
+void launch_coarse_solve(Ctx& c, const CoarseBlocks& cb, double* cvec, double* x, const CoarseOut& out);
 
 // compact <-> dense (interleaved 3-vectors)
 template <typename T>

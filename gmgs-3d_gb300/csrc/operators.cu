@@ -1,6 +1,5 @@
 // Per-level helpers of the V-cycle PCG: trilinear restriction, deterministic
-// dot products, coarsest-level gather / scatter and the compact <-> dense
-// conversions (K*x, the prolongation and the CG updates are in fine.cu and
+// dot products and the compact <-> dense conversions (K*x, the prolongation and the CG updates are in fine.cu and
 // fine64.cu).  All kernels work on the dense slot grids described in
 // gmgs_internal.cuh and are free of atomics on data (reruns are bitwise equal).
 #include "gmgs_internal.cuh"
@@ -42,8 +41,11 @@ __device__ __forceinline__ double restrict_acc(double acc, double v, bool centre
     return centre ? __dadd_rn(acc, v) : __fma_rn(0.5, v, acc);
 }
 
-template <typename T>
-__global__ void k_restrict(Grid gf, Grid gc, const uint8_t* __restrict__ nflag_c, const T* rf, T* rc) {
+// FREE: onto the coarsest level's free DOFs, cvec[rank of the DOF] in FP64,
+// instead of its dense vector (a gather launch less per V-cycle)
+template <typename T, bool FREE>
+__global__ void k_restrict(Grid gf, Grid gc, const uint8_t* __restrict__ nflag_c, const T* rf, T* rc,
+                           const int32_t* __restrict__ rank, double* cvec) {
     const int Iy = blockIdx.x * blockDim.x + threadIdx.x;
     const int Ix = blockIdx.y * blockDim.y + threadIdx.y;
     const int Iz = blockIdx.z;
@@ -54,6 +56,7 @@ __global__ void k_restrict(Grid gf, Grid gc, const uint8_t* __restrict__ nflag_c
     constexpr int R = chk::RESTRICT;
     pdl_wait();
     if (!(chk::ld(nflag_c, cs, Sc, R) & NF_SOLID)) {
+        if (FREE) return;
         chk::st(rc, cs, 3 * Sc, R, 0);
         chk::st(rc, cs + Sc, 3 * Sc, R, 0);
         chk::st(rc, cs + 2 * Sc, 3 * Sc, R, 0);
@@ -75,17 +78,32 @@ __global__ void k_restrict(Grid gf, Grid gc, const uint8_t* __restrict__ nflag_c
             }
             accz = restrict_acc(accz, accx, c == 0);
         }
-        chk::st(rc, cs + comp * Sc, 3 * Sc, R, accz);
+        if (FREE) {
+            const int at = chk::ld(rank, cs + comp * Sc, 3 * Sc, R);
+            if (at >= 0) cvec[at] = (double)accz;
+        } else {
+            chk::st(rc, cs + comp * Sc, 3 * Sc, R, accz);
+        }
     }
 }
 
 template <typename T>
 void launch_restrict(Ctx& c, const Grid& gf, const Grid& gc, const uint8_t* nflag_c, const T* rf, T* rc) {
     dim3 blk(32, 4, 1);
-    launch_chain(c, k_restrict<T>, node_grid(gc, blk), blk, 0, gf, gc, nflag_c, rf, rc);
+    launch_chain(c, k_restrict<T, false>, node_grid(gc, blk), blk, 0, gf, gc, nflag_c, rf, rc, nullptr, nullptr);
+}
+template <typename T>
+void launch_restrict_free(Ctx& c, const Grid& gf, const Grid& gc, const uint8_t* nflag_c, const T* rf, const int32_t* rank,
+                          double* cvec) {
+    dim3 blk(32, 4, 1);
+    launch_chain(c, k_restrict<T, true>, node_grid(gc, blk), blk, 0, gf, gc, nflag_c, rf, nullptr, rank, cvec);
 }
 template void launch_restrict<double>(Ctx&, const Grid&, const Grid&, const uint8_t*, const double*, double*);
 template void launch_restrict<float>(Ctx&, const Grid&, const Grid&, const uint8_t*, const float*, float*);
+template void launch_restrict_free<double>(Ctx&, const Grid&, const Grid&, const uint8_t*, const double*, const int32_t*,
+                                           double*);
+template void launch_restrict_free<float>(Ctx&, const Grid&, const Grid&, const uint8_t*, const float*, const int32_t*,
+                                          double*);
 
 // ---------------------------------------------------------------------------
 // deterministic dot product: fixed grid-stride partition, fixed-order block
@@ -141,36 +159,6 @@ void launch_dot(Ctx& c, const DotScratch& s, int64_t n, const Ta* a, const Tb* b
     GMGS_LAUNCHED(c);
 }
 template void launch_dot<double, double>(Ctx&, const DotScratch&, int64_t, const double*, const double*, double*);
-
-// ---------------------------------------------------------------------------
-// coarsest level: free-DOF gather and scatter
-// ---------------------------------------------------------------------------
-template <typename T>
-__global__ void k_gather(int64_t n, const int32_t* __restrict__ idx, const T* src, double* dst) {
-    pdl_begin();
-    pdl_wait();
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        dst[i] = (double)src[idx[i]];
-}
-template <typename T>
-__global__ void k_scatter(int64_t n, const int32_t* __restrict__ idx, const double* src, T* dst) {
-    pdl_begin();
-    pdl_wait();
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        dst[idx[i]] = (T)src[i];
-}
-template <typename T>
-void launch_gather(Ctx& c, int64_t n, const int32_t* idx, const T* src, double* dst) {
-    launch_chain(c, k_gather<T>, ew_blocks(c, n), 256, 0, n, idx, src, dst);
-}
-template <typename T>
-void launch_scatter(Ctx& c, int64_t n, const int32_t* idx, const double* src, T* dst) {
-    launch_chain(c, k_scatter<T>, ew_blocks(c, n), 256, 0, n, idx, src, dst);
-}
-template void launch_gather<double>(Ctx&, int64_t, const int32_t*, const double*, double*);
-template void launch_gather<float>(Ctx&, int64_t, const int32_t*, const float*, double*);
-template void launch_scatter<double>(Ctx&, int64_t, const int32_t*, const double*, double*);
-template void launch_scatter<float>(Ctx&, int64_t, const int32_t*, const double*, float*);
 
 // ---------------------------------------------------------------------------
 // compact interleaved <-> dense planes

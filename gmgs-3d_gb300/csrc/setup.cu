@@ -1058,7 +1058,8 @@ void build_coarse_bc(Model& M, const std::function<void()>& overlap) {
     k_free_list<<<blocks_for(c, 3 * S), 256, 0, c.stream>>>(S, lc.nflag.as<uint8_t>(), cnt.as<int32_t>(),
                                                              M.free_idx.as<int32_t>());
     GMGS_LAUNCHED(c);
-    DevBuf rank = dalloc(3 * S * sizeof(int32_t));
+    ensure(M.free_rank, 3 * S * sizeof(int32_t));
+    const DevBuf& rank = M.free_rank;
     k_rank_fill<<<blocks_for(c, 3 * S), 256, 0, c.stream>>>(3 * S, rank.as<int32_t>());
     GMGS_LAUNCHED(c);
     k_rank_set<<<blocks_for(c, nf), 256, 0, c.stream>>>(nf, M.free_idx.as<int32_t>(), rank.as<int32_t>());

@@ -32,7 +32,8 @@ struct Model {
     DevBuf F, U;
     // coarsest level
     int nfree = 0;
-    DevBuf free_idx, cvec_in, cvec_out;   // free DOF slots; coarse vectors (cb.nb * cb.B long)
+    DevBuf free_idx, free_rank;           // free DOF -> slot and slot -> free DOF (-1: none)
+    DevBuf cvec_in, cvec_out;             // coarse vectors (cb.nb * cb.B long)
     CoarseBlocks cb;
     // outer CG work vectors
     DevBuf cg_x, cg_r;                                         // mixed path: hi / lo parts; cg_r also FP64
@@ -41,7 +42,6 @@ struct Model {
     DevBuf cg_r32b, cg_pa, cg_pb;                              // mixed path double buffers
     Coef32 coef{};                                             // FP32 stencil + element matrix
     TcCoef tcoef{};                                            // Ke as the tensor cores' B operand
-    DevBuf tc_err;         // int: set when a tensor-core wait ran out
     bool use_tc = false;   // V-cycle down-sweeps on the tensor cores (environment GMGS_TC)
     DevBuf scal;           // device scalars (see solver.cu)
     DevBuf dot_partials, dot_ticket;

@@ -14,7 +14,7 @@
 
 namespace gmgs {
 
-enum { SC_RZ0 = 0, SC_RZ1 = 1, SC_PQ = 2, SC_RR = 3, SC_BB = 4, SC_TC = 5, SC_N = 8 };   // SC_TC: host copy of the device wait-error flag
+enum { SC_RZ0 = 0, SC_RZ1 = 1, SC_PQ = 2, SC_RR = 3, SC_BB = 5, SC_TC = 4, SC_N = 8 };   // SC_TC: the wait-error flag (an int), beside SC_RR: one copy fetches both
 
 static void zalloc(Ctx& c, DevBuf& b, size_t bytes) {
     if (b.bytes < bytes) b = dalloc(bytes);
@@ -106,7 +106,6 @@ void alloc_work(Model& M) {
         zalloc(c, M.cg_z64, n3 * 8);
     }
     zalloc(c, M.scal, SC_N * sizeof(double));
-    if (mixed) zalloc(c, M.tc_err, sizeof(int));
     M.dot_blocks = M.ctx.num_sms * 4;
     const Level& l0 = M.levels[0];
     const int maxb = mixed ? std::max({M.dot_blocks, fine_grid_blocks(l0.g), up32_grid_blocks(l0.g)})
@@ -116,6 +115,8 @@ void alloc_work(Model& M) {
     if (!M.scal_host) GMGS_CUDA(cudaMallocHost(&M.scal_host, SC_N * sizeof(double)));
     GMGS_CUDA(cudaStreamSynchronize(c.stream));
 }
+
+static int* wait_error(Model& M) { return reinterpret_cast<int*>(M.scal.as<double>() + SC_TC); }
 
 static DotScratch dots(Model& M) {
     return DotScratch{M.dot_partials.as<double>(), M.dot_ticket.as<unsigned int>(), M.dot_blocks};
@@ -132,12 +133,11 @@ static bool tc_enabled() {
 // flag; the solve reports it instead of returning a result computed without
 // the data it waited for.
 static void check_tc(Model& M) {
-    if (!M.tc_err.p) return;
     int flag = 0;
-    GMGS_CUDA(cudaMemcpyAsync(&flag, M.tc_err.p, sizeof(int), cudaMemcpyDeviceToHost, M.ctx.stream));
+    GMGS_CUDA(cudaMemcpyAsync(&flag, wait_error(M), sizeof(int), cudaMemcpyDeviceToHost, M.ctx.stream));
     GMGS_CUDA(cudaStreamSynchronize(M.ctx.stream));
     if (flag) {
-        GMGS_CUDA(cudaMemsetAsync(M.tc_err.p, 0, sizeof(int), M.ctx.stream));
+        GMGS_CUDA(cudaMemsetAsync(wait_error(M), 0, sizeof(int), M.ctx.stream));
         throw Error(GMGS_ERR_CUDA, "a kernel's bounded wait for its tensor-core MMA or staged operands timed out");
     }
 }
@@ -168,12 +168,13 @@ static void vcycle64(Model& M, const double* r0, double* z, bool with_dot, int d
         if (l == 0) c.mark(PK_FINE_MATVEC, false);
         launch_fine64<M64_VCYCLE_DOWN>(c, level64(M, lv), M.coef64, a);
         if (l == 0) c.mark(PK_FINE_MATVEC, true, (double)lv.n_node * 3 * 24 + (double)lv.n_elem);
-        launch_restrict<double>(c, lv.g, lc.g, lc.nflag.as<uint8_t>(), lv.vrp.as<double>(), lc.vr.as<double>());
+        if (l + 1 < L - 1) launch_restrict<double>(c, lv.g, lc.g, lc.nflag.as<uint8_t>(), lv.vrp.as<double>(), lc.vr.as<double>());
+        else launch_restrict_free<double>(c, lv.g, lc.g, lc.nflag.as<uint8_t>(), lv.vrp.as<double>(), M.free_rank.as<int32_t>(),
+                                         M.cvec_in.as<double>());
     }
     Level& lc = M.levels[L - 1];
-    launch_gather<double>(c, M.nfree, M.free_idx.as<int32_t>(), lc.vr.as<double>(), M.cvec_in.as<double>());
-    launch_coarse_solve(c, M.cb, M.cvec_in.as<double>(), M.cvec_out.as<double>());
-    launch_scatter<double>(c, M.nfree, M.free_idx.as<int32_t>(), M.cvec_out.as<double>(), lc.vx.as<double>());
+    launch_coarse_solve(c, M.cb, M.cvec_in.as<double>(), M.cvec_out.as<double>(),
+                        CoarseOut{M.free_idx.as<int32_t>(), nullptr, lc.vx.as<double>(), M.nfree});
     for (int l = L - 2; l >= 0; --l) {
         Level& lv = M.levels[l];
         const DotOut64 d = dot_out64(M, dot_slot);
@@ -291,7 +292,7 @@ static void vcycle32(Model& M, const float* r32, float* z, bool with_dot, int do
         if (M.use_tc && lv.n_perel < lv.n_node) {
             FineLevel ft = fl;
             ft.tile_occ = lv.tc_occ.as<uint8_t>();
-            launch_tc_vdown(c, ft, M.tcoef, a.r32, a.wdinv, a.out32, M.tc_err.as<int>());
+            launch_tc_vdown(c, ft, M.tcoef, a.r32, a.wdinv, a.out32, wait_error(M));
             if (lv.n_perel > 0) launch_perel_vdown(c, fl, M.coef, a);
         } else if (lv.n_perel < lv.n_node) {
             launch_fine<FM_VCYCLE_DOWN>(c, fl, M.coef, a);
@@ -302,13 +303,14 @@ static void vcycle32(Model& M, const float* r32, float* z, bool with_dot, int do
             c.mark(PK_FINE_MATVEC, true, bytes);
             c.mark(PK_VDOWN0, true, bytes);
         }
-        launch_restrict<float>(c, lv.g, lc.g, lc.nflag.as<uint8_t>(), lv.vrp.as<float>(), lc.vr.as<float>());
+        if (l + 1 < L - 1) launch_restrict<float>(c, lv.g, lc.g, lc.nflag.as<uint8_t>(), lv.vrp.as<float>(), lc.vr.as<float>());
+        else launch_restrict_free<float>(c, lv.g, lc.g, lc.nflag.as<uint8_t>(), lv.vrp.as<float>(), M.free_rank.as<int32_t>(),
+                                         M.cvec_in.as<double>());
     }
     if (L == 2) c.mark(PK_COARSE, false);
     Level& lc = M.levels[L - 1];
-    launch_gather<float>(c, M.nfree, M.free_idx.as<int32_t>(), lc.vr.as<float>(), M.cvec_in.as<double>());
-    launch_coarse_solve(c, M.cb, M.cvec_in.as<double>(), M.cvec_out.as<double>());
-    launch_scatter<float>(c, M.nfree, M.free_idx.as<int32_t>(), M.cvec_out.as<double>(), lc.vx.as<float>());
+    launch_coarse_solve(c, M.cb, M.cvec_in.as<double>(), M.cvec_out.as<double>(),
+                        CoarseOut{M.free_idx.as<int32_t>(), lc.vx.as<float>(), nullptr, M.nfree});
     for (int l = L - 2; l >= 0; --l) {
         Level& lv = M.levels[l];
         const DotOut d = dot_out(M, dot_slot);
@@ -434,7 +436,7 @@ static int pcg_mixed(Model& M, const double* b, double* x, int32_t* iters_out, d
         a.cur = cur;
         a.first = first;
         a.dot = dot_out(M, SC_RR);
-        a.err = M.tc_err.as<int>();
+        a.err = wait_error(M);
         c.mark(PK_FINE_MATVEC, false);
         c.mark(PK_UPDATE_JACOBI, false);
         launch_l0<FM_CG_UPDATE_JACOBI>(M, f0, a);
@@ -503,9 +505,8 @@ static int pcg_mixed(Model& M, const double* b, double* x, int32_t* iters_out, d
             body(its);
         }
         c.mark(PK_CG_ITER, true);
-        GMGS_CUDA(cudaMemcpyAsync(M.scal_host + SC_RR, scal + SC_RR, sizeof(double), cudaMemcpyDeviceToHost,
-                                  c.stream));
-        GMGS_CUDA(cudaMemcpyAsync(M.scal_host + SC_TC, M.tc_err.p, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+        static_assert(SC_TC == SC_RR + 1, "the residual and the flag in one copy");
+        GMGS_CUDA(cudaMemcpyAsync(M.scal_host + SC_RR, scal + SC_RR, 2 * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
         GMGS_CUDA(cudaStreamSynchronize(c.stream));
         if (*reinterpret_cast<const int*>(M.scal_host + SC_TC)) break;   // check_tc reports it
         resnorm = std::sqrt(M.scal_host[SC_RR]) / normB;
