@@ -191,7 +191,7 @@ int64_t model_bytes(const gmgs::Model& M) {
             b += (int64_t)d->bytes;
     for (const gmgs::DevBuf* d : {&M.ke0_dev, &M.galerkin_child, &M.galerkin_grand, &M.rho, &M.F, &M.U, &M.free_idx, &M.free_rank, &M.cb.sinv, &M.cb.g, &M.cb.gt, &M.cvec_in, &M.cvec_out,
                                   &M.cg_x, &M.cg_r, &M.cg_rb, &M.cg_p, &M.cg_p2, &M.cg_q64, &M.cg_z64, &M.mask_stencil, &M.cg_q32,
-                                  &M.cg_z32, &M.cg_r32, &M.cg_r32b, &M.cg_pa, &M.cg_pb, &M.scal, &M.dot_partials, &M.dot_ticket})
+                                  &M.cg_z32, &M.cg_r32, &M.cg_r32b, &M.cg_pa, &M.cg_pb, &M.scal, &M.dot_partials, &M.dot_ticket, &M.dot_prod, &M.dot_chunk})
         b += (int64_t)d->bytes;
     return b;
 }

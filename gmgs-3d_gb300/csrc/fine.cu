@@ -235,6 +235,44 @@ __device__ __forceinline__ void perel_node(const FineLevel& L, const Coef32& cf,
     }
 }
 
+// The dot product of a split launch (one plane per CTA): each CTA stores its
+// plane's products, and the last of a chunk's CTAs to arrive forms every
+// thread's compensated sum over the chunk's planes in order, so the sum is that
+// of one CTA walking the chunk, bit for bit, without its latency.  A node that
+// does not count is marked by a bit pattern no product has (the hardware's NaN
+// is 0x7fffffff).
+__device__ __forceinline__ void split_dot_finish(const FineArgs& a, bool counted, const float* prod, int iz, int nplane,
+                                                 double* sh) {
+    __shared__ bool last;
+    constexpr uint32_t NONE = 0xffffffffu;
+    const int tid = threadIdx.x + threadIdx.y * TY;
+    const unsigned tile = blockIdx.x + gridDim.x * blockIdx.y, tiles = gridDim.x * gridDim.y;
+    const int chunk = iz / DOT_CHUNK, first = chunk * DOT_CHUNK, n = min(DOT_CHUNK, nplane - first);
+    uint32_t* const at = reinterpret_cast<uint32_t*>(a.prod) + ((int64_t)tile * nplane + first) * DOT_PLANE + tid;
+#pragma unroll
+    for (int b = 0; b < 3; ++b) at[(iz - first) * DOT_PLANE + b * NT] = counted ? __float_as_uint(prod[b]) : NONE;
+    __threadfence();
+    __syncthreads();
+    unsigned int* const count = a.chunk + chunk * tiles + tile;
+    if (tid == 0) last = atomicAdd(count, 1u) == (unsigned)(n - 1);
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    uint32_t v[DOT_CHUNK][3];
+#pragma unroll
+    for (int q = 0; q < DOT_CHUNK; ++q)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) v[q][b] = q < n ? __ldcg(at + q * DOT_PLANE + b * NT) : NONE;
+    Kahan dot;
+#pragma unroll
+    for (int q = 0; q < DOT_CHUNK; ++q)
+#pragma unroll
+        for (int b = 0; b < 3; ++b)
+            if (v[q][b] != NONE) dot.add(__uint_as_float(v[q][b]));
+    if (tid == 0) *count = 0;
+    grid_dot_finish(dot.value(), a.dot, sh, tile + tiles * chunk, tiles * (unsigned)((nplane + DOT_CHUNK - 1) / DOT_CHUNK));
+}
+
 // 48 registers (5 CTAs per SM) for the stencil-only modes, 40 (6 CTAs) for
 // the CG direction with its field staged by TMA (1.073 -> 1.063 ms; the
 // down-sweep, which also holds r for its output, spills at 40); the CG update
@@ -245,8 +283,10 @@ __device__ __forceinline__ void perel_node(const FineLevel& L, const Coef32& cf,
 // 1.13 ms and the direction kernel from 1.26 to 1.22 ms against 4 CTAs/SM.
 // STG bit 0: the CG update's operands staged by TMA; bit 1: the field inputs
 // staged by TMA (else loaded per thread into registers one plane ahead)
-template <int MODE, bool DEF = false, int STG = 0>
-__global__ void __launch_bounds__(NT, MODE == FM_CG_UPDATE_JACOBI ? ((STG & 1) ? 4 : 3) : ((MODE == FM_CG_DIRECTION && (STG & 2)) ? 6 : 5))
+// SPLIT: one plane per CTA, the dot product's sums left to split_dot_finish (a
+// kernel of its own: its registers would spill the 40 of the CG direction)
+template <int MODE, bool DEF = false, int STG = 0, bool SPLIT = false>
+__global__ void __launch_bounds__(NT, MODE == FM_CG_UPDATE_JACOBI ? ((STG & 1) ? 4 : 3) : ((MODE == FM_CG_DIRECTION && (STG & 2) && !SPLIT) ? 6 : 5))
     k_fine(FineLevel L, const __grid_constant__ Coef32 cf, FineArgs a, int zc, const __grid_constant__ EpiMaps em) {
     constexpr bool TMA = (STG & 1) != 0, FTMA = (STG & 2) != 0;
     static_assert(!TMA || MODE == FM_CG_UPDATE_JACOBI, "operand staging is for the CG update");
@@ -269,8 +309,14 @@ __global__ void __launch_bounds__(NT, MODE == FM_CG_UPDATE_JACOBI ? ((STG & 1) ?
     if (L.tile_occ)
         for (int iz = zb; iz < ze; ++iz) any |= L.tile_occ[((int64_t)iz * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x];
     pdl_wait();
+    constexpr bool HAS_DOT = MODE == FM_CG_DIRECTION || MODE == FM_CG_UPDATE_JACOBI;
     if (!any) {                                   // no solid node in this column tile: nothing to compute
-        if (MODE == FM_CG_DIRECTION || MODE == FM_CG_UPDATE_JACOBI) grid_dot_finish(0.0, a.dot, sh);
+        if constexpr (SPLIT) {
+            const float none[3] = {0.f, 0.f, 0.f};
+            split_dot_finish(a, false, none, zb, g.nz + 1, sh);
+        } else if constexpr (HAS_DOT) {
+            grid_dot_finish(0.0, a.dot, sh);
+        }
         return;
     }
     // warps cover 8 (y) x 4 (x) node patches, so a face of the domain
@@ -382,6 +428,8 @@ __global__ void __launch_bounds__(NT, MODE == FM_CG_UPDATE_JACOBI ? ((STG & 1) ?
         e8_next = chk::ld(L.emask8, cbase + zb * sz, g.slots, chk::FINE_FLAGS);
     }
     Kahan dot;
+    float prod[3] = {0.f, 0.f, 0.f};              // SPLIT: this thread's products, if its node counts
+    bool counted = false;
     // FTMA: the field of plane z from the field stage (ring point p is box element p + 3)
     int nfa = field_arrays(MODE);                 // the first CG iteration has no q / p term
     if (a.first && (MODE == FM_CG_DIRECTION || MODE == FM_CG_UPDATE_JACOBI)) --nfa;
@@ -509,13 +557,16 @@ __global__ void __launch_bounds__(NT, MODE == FM_CG_UPDATE_JACOBI ? ((STG & 1) ?
                     chk::st(a.x_lo, i, n3, O, xl);
                     chk::st(a.r_lo, i, n3, O, rl);
                     chk::st(a.r32out, i, n3, O, rh);
-                    dot.add(__fmul_rn(rm32, rm32));
+                    if constexpr (SPLIT) prod[b] = __fmul_rn(rm32, rm32);
+                    else dot.add(__fmul_rn(rm32, rm32));
                 } else {
                     chk::st(a.pout, i, n3, O, v);
                     chk::st(a.out32, i, n3, O, y[b]);                   // q = A p
-                    dot.add(__fmul_rn(v, y[b]));
+                    if constexpr (SPLIT) prod[b] = __fmul_rn(v, y[b]);
+                    else dot.add(__fmul_rn(v, y[b]));
                 }
             }
+            if constexpr (SPLIT) counted = true;
         }
         if constexpr (TMA) {
             // every thread sees each phase complete within its step, so no
@@ -532,30 +583,37 @@ __global__ void __launch_bounds__(NT, MODE == FM_CG_UPDATE_JACOBI ? ((STG & 1) ?
         // (every earlier phase completed before the next one was armed)
         if (tid == EPI_ISSUER && last_phase >= 0) tc::mbar_wait_bounded(&ebar, last_phase & 1, EPI_WAIT_NS);
     }
-    if (MODE == FM_CG_DIRECTION || MODE == FM_CG_UPDATE_JACOBI) grid_dot_finish(dot.value(), a.dot, sh);
+    if constexpr (SPLIT) split_dot_finish(a, counted, prod, zb, g.nz + 1, sh);
+    else if constexpr (HAS_DOT) grid_dot_finish(dot.value(), a.dot, sh);
 }
 
-static int pick_zc(const Grid& g, const Ctx& c, int per_sm, bool dot) {
+static int pick_zc(const Grid& g, int num_sms, int per_sm) {
     const int64_t cols = (int64_t)((g.ny + 1 + TY - 1) / TY) * ((g.nx + 1 + TX - 1) / TX);
     // ~24 waves of 3 resident CTAs: shorter z-chunks balance the tail and let
     // empty column tiles of real geometry skip more (12 waves: 214 -> 208 ms
     // on the 153M-DOF block, 286 -> 271 ms on kitten 512; 48 waves: slower)
-    const int64_t want = (int64_t)c.num_sms * per_sm * 24;
+    const int64_t want = (int64_t)num_sms * per_sm * 24;
     int64_t zc = (cols * (g.nz + 1) + want - 1) / want;
     // at least 6 planes per CTA where that still leaves four CTAs per SM (each
     // chunk stages two planes beyond its own: coarse levels 22.17 -> 21.96 ms
     // per solve against 4; 8 was slower), else at least 4.  On grids where 4
-    // planes leave fewer, the down-sweep takes one plane per CTA: there a CTA's
-    // chain of planes is the launch's time, not the planes staged twice.  The
-    // modes with a dot product keep 4: a thread's compensated FP32 sum runs over
-    // its chunk, p.q cancels to a small part of |p||q|, and another grouping
-    // changes alpha's FP32 rounding often enough to move a solve's result in
-    // the ninth digit
-    const int64_t full = 4 * (int64_t)c.num_sms;
-    const int64_t zmin = cols * ((g.nz + 1 + 5) / 6) >= full ? 6 : (dot || cols * ((g.nz + 1 + 3) / 4) >= full ? 4 : 1);
+    // planes leave fewer, a CTA's chain of planes is the launch's time, not the
+    // planes staged twice: one plane per CTA.  The modes with a dot product
+    // then leave its sums over 4 planes to split_dot_finish: p.q cancels to a
+    // small part of |p||q|, and another grouping of the compensated FP32 sums
+    // changes alpha's rounding often enough to move a solve's result in the
+    // ninth digit.
+    const int64_t full = 4 * (int64_t)num_sms;
+    const int64_t zmin = cols * ((g.nz + 1 + 5) / 6) >= full ? 6 : (cols * ((g.nz + 1 + 3) / 4) >= full ? 4 : 1);
     if (zc < zmin) zc = zmin;
     if (zc > 64) zc = 64;
     return (int)zc;
+}
+
+size_t dot_split_planes(const Grid& g, int num_sms) {
+    // (the update's and the direction's chunks reach one plane on the same grids)
+    if (pick_zc(g, num_sms, 2) > 1 && pick_zc(g, num_sms, 3) > 1) return 0;
+    return (size_t)((g.ny + 1 + TY - 1) / TY) * ((g.nx + 1 + TX - 1) / TX) * (g.nz + 1);
 }
 
 int fine_grid_blocks(const Grid& g) {
@@ -620,7 +678,7 @@ static bool env_on(const char* name) {
     return !(e && e[0] == '0');
 }
 
-template <int MODE, bool DEF, int STG>
+template <int MODE, bool DEF, int STG, bool SPLIT>
 static void launch_stg(Ctx& c, dim3 grid, const FineLevel& L, const Coef32& cf, const FineArgs& a, int zc,
                        const EpiMaps& em) {
     size_t dyn = 0;
@@ -635,12 +693,12 @@ static void launch_stg(Ctx& c, dim3 grid, const FineLevel& L, const Coef32& cf, 
         GMGS_CUDA(cudaGetDevice(&dev));
         const unsigned long long bit = 1ull << (dev & 63);
         if (!(opted.load() & bit)) {
-            GMGS_CUDA(cudaFuncSetAttribute(k_fine<MODE, DEF, STG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            GMGS_CUDA(cudaFuncSetAttribute(k_fine<MODE, DEF, STG, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)dyn));
             opted.fetch_or(bit);
         }
     }
-    launch_chain(c, k_fine<MODE, DEF, STG>, grid, dim3(TY, TX, 1), dyn, L, cf, a, zc, em);
+    launch_chain(c, k_fine<MODE, DEF, STG, SPLIT>, grid, dim3(TY, TX, 1), dyn, L, cf, a, zc, em);
 }
 
 template <int MODE>
@@ -649,14 +707,6 @@ void launch_fine(Ctx& c, const FineLevel& L, const Coef32& cf, const FineArgs& a
     // the CG update with its staged operands: longer z-chunks (2 instead of 3
     // in the wave count: 1.820 -> 1.792 ms, 1 gave 1.820 ms; the other modes
     // were slower with 2)
-    const int zc = pick_zc(L.g, c, MODE == FM_CG_UPDATE_JACOBI ? 2 : 3,
-                           MODE == FM_CG_UPDATE_JACOBI || MODE == FM_CG_DIRECTION);
-    dim3 grid((L.g.ny + 1 + TY - 1) / TY, (L.g.nx + 1 + TX - 1) / TX, (L.g.nz + 1 + zc - 1) / zc);
-    if (MODE == FM_VCYCLE_DOWN && a.n_perel > 0) {
-        const int per = (NT / 8) * (int)(grid.x * grid.y);
-        a.perel_z = (a.n_perel + per - 1) / per;
-        grid.z += a.perel_z;
-    }
     const bool def = coef_is_default(cf);
     EpiMaps em;
     std::memset(&em, 0, sizeof(em));
@@ -675,19 +725,41 @@ void launch_fine(Ctx& c, const FineLevel& L, const Coef32& cf, const FineArgs& a
     }
     // the per-node operand stage exists for the CG update only
     const int stg = (etma ? 1 : 0) | (ftma ? 2 : 0);
-    auto go = [&](auto tag) {
+    int zc = pick_zc(L.g, c.num_sms, MODE == FM_CG_UPDATE_JACOBI ? 2 : 3);
+    // one plane per CTA: a mode with a dot product keeps its sums over
+    // DOT_CHUNK planes, in a split launch where everything is staged by TMA,
+    // else by walking them
+    constexpr bool HAS_DOT = MODE == FM_CG_UPDATE_JACOBI || MODE == FM_CG_DIRECTION;
+    constexpr int FULL = MODE == FM_CG_UPDATE_JACOBI ? 3 : 2;
+    const bool split = HAS_DOT && zc == 1 && stg == FULL && a.prod && a.chunk;
+    if (HAS_DOT && zc == 1 && !split) zc = DOT_CHUNK;
+    dim3 grid((L.g.ny + 1 + TY - 1) / TY, (L.g.nx + 1 + TX - 1) / TX, (L.g.nz + 1 + zc - 1) / zc);
+    if (MODE == FM_VCYCLE_DOWN && a.n_perel > 0) {
+        const int per = (NT / 8) * (int)(grid.x * grid.y);
+        a.perel_z = (a.n_perel + per - 1) / per;
+        grid.z += a.perel_z;
+    }
+    auto go = [&](auto tag, auto sp) {
         constexpr int G = decltype(tag)::value;
-        if (def) launch_stg<MODE, true, G>(c, grid, L, cf, a, zc, em);
-        else launch_stg<MODE, false, G>(c, grid, L, cf, a, zc, em);
+        constexpr bool SP = decltype(sp)::value;
+        if (def) launch_stg<MODE, true, G, SP>(c, grid, L, cf, a, zc, em);
+        else launch_stg<MODE, false, G, SP>(c, grid, L, cf, a, zc, em);
     };
+    const std::false_type whole{};
+    if constexpr (HAS_DOT) {
+        if (split) {
+            go(std::integral_constant<int, FULL>{}, std::true_type{});
+            return;
+        }
+    }
     if constexpr (MODE == FM_CG_UPDATE_JACOBI) {
-        if (stg == 3) go(std::integral_constant<int, 3>{});
-        else if (stg == 1) go(std::integral_constant<int, 1>{});
-        else if (stg == 2) go(std::integral_constant<int, 2>{});
-        else go(std::integral_constant<int, 0>{});
+        if (stg == 3) go(std::integral_constant<int, 3>{}, whole);
+        else if (stg == 1) go(std::integral_constant<int, 1>{}, whole);
+        else if (stg == 2) go(std::integral_constant<int, 2>{}, whole);
+        else go(std::integral_constant<int, 0>{}, whole);
     } else {
-        if (ftma) go(std::integral_constant<int, 2>{});
-        else go(std::integral_constant<int, 0>{});
+        if (ftma) go(std::integral_constant<int, 2>{}, whole);
+        else go(std::integral_constant<int, 0>{}, whole);
     }
 }
 template void launch_fine<FM_PLAIN>(Ctx&, const FineLevel&, const Coef32&, const FineArgs&);

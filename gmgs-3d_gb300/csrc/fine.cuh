@@ -44,6 +44,10 @@ enum FineMode {
     FM_CG_DIRECTION = 3       // v = fl32(z + beta p_old), p = v, q = A v, p.q  (CG_solver.m:23-31)
 };
 
+constexpr int DOT_CHUNK = 4;              // planes of a thread's compensated sum on small grids
+constexpr int DOT_PLANE = 3 * 256;        // products of a tile plane: component, thread
+size_t dot_split_planes(const Grid& g, int num_sms);   // tile planes of a split launch, 0 where none is split
+
 struct FineArgs {
     const float* v = nullptr;        // FM_PLAIN input
     const float* r32 = nullptr;      // FM_VCYCLE_DOWN residual; FM_CG_UPDATE_JACOBI: its high part (read on the halo)
@@ -63,6 +67,8 @@ struct FineArgs {
     const int32_t* perel = nullptr;  // FM_VCYCLE_DOWN: slots of the nodes on stored matrices
     int n_perel = 0;
     int perel_z = 0;                 // grid layers that take them (set by the launcher)
+    float* prod = nullptr;           // modes with a dot on small grids: the products of every tile plane (DOT_PLANE each)
+    unsigned int* chunk = nullptr;   // and an arrival counter per chunk of DOT_CHUNK planes (zero between launches)
     int* err = nullptr;              // set when a bounded wait for staged operands ran out
 };
 
@@ -123,14 +129,12 @@ __device__ __forceinline__ double block_sum_d(double v, double* sh) {
     return v;   // valid in thread 0
 }
 
-// deterministic grid reduction: partial per block, the last block sums them in order
-__device__ inline void grid_dot_finish(double v, const DotOut& d, double* sh) {
+// deterministic grid reduction: partial b of nb, the last block to arrive sums them in order
+__device__ inline void grid_dot_finish(double v, const DotOut& d, double* sh, unsigned b, unsigned nb) {
     __shared__ bool last;
     v = block_sum_d(v, sh);
     const int nthr = blockDim.x * blockDim.y;
     const int tid = threadIdx.x + threadIdx.y * blockDim.x;
-    const unsigned nb = gridDim.x * gridDim.y * gridDim.z;
-    const unsigned b = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
     if (tid == 0) {
         d.partials[b] = v;
         __threadfence();
@@ -147,6 +151,12 @@ __device__ inline void grid_dot_finish(double v, const DotOut& d, double* sh) {
             *d.ticket = 0;
         }
     }
+}
+
+// one partial per block
+__device__ inline void grid_dot_finish(double v, const DotOut& d, double* sh) {
+    grid_dot_finish(v, d, sh, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z),
+                    gridDim.x * gridDim.y * gridDim.z);
 }
 
 // input field at one point (3 components) from the kernel's inputs

@@ -45,6 +45,7 @@ struct Model {
     bool use_tc = false;   // V-cycle down-sweeps on the tensor cores (environment GMGS_TC)
     DevBuf scal;           // device scalars (see solver.cu)
     DevBuf dot_partials, dot_ticket;
+    DevBuf dot_prod, dot_chunk;   // split dot products of small grids (mixed path)
     // CUDA graphs of the mixed PCG iteration body (one per parity), valid for
     // the solution buffer and the work-buffer generation they were captured with
     cudaGraphExec_t cg_graph[2] = {nullptr, nullptr};

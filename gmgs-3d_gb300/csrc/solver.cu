@@ -112,6 +112,10 @@ void alloc_work(Model& M) {
                            : std::max(M.dot_blocks, dot64_blocks(l0.g, l0.n_bnd + l0.n_perel));
     zalloc(c, M.dot_partials, (size_t)maxb * sizeof(double));
     zalloc(c, M.dot_ticket, sizeof(unsigned int));
+    if (const size_t planes = mixed ? dot_split_planes(l0.g, c.num_sms) : 0) {
+        if (M.dot_prod.bytes < planes * DOT_PLANE * sizeof(float)) M.dot_prod = dalloc(planes * DOT_PLANE * sizeof(float));
+        zalloc(c, M.dot_chunk, planes * sizeof(unsigned int));
+    }
     if (!M.scal_host) GMGS_CUDA(cudaMallocHost(&M.scal_host, SC_N * sizeof(double)));
     GMGS_CUDA(cudaStreamSynchronize(c.stream));
 }
@@ -436,6 +440,8 @@ static int pcg_mixed(Model& M, const double* b, double* x, int32_t* iters_out, d
         a.cur = cur;
         a.first = first;
         a.dot = dot_out(M, SC_RR);
+        a.prod = M.dot_prod.as<float>();
+        a.chunk = M.dot_chunk.as<unsigned int>();
         a.err = wait_error(M);
         c.mark(PK_FINE_MATVEC, false);
         c.mark(PK_UPDATE_JACOBI, false);
@@ -460,6 +466,8 @@ static int pcg_mixed(Model& M, const double* b, double* x, int32_t* iters_out, d
             a.first = its == 1;
             a.out32 = q;
             a.dot = dot_out(M, SC_PQ);
+            a.prod = M.dot_prod.as<float>();
+            a.chunk = M.dot_chunk.as<unsigned int>();
             c.mark(PK_FINE_MATVEC, false);
             c.mark(PK_DIRECTION, false);
             launch_l0<FM_CG_DIRECTION>(M, f0, a);
