@@ -1028,9 +1028,13 @@ template void launch_fine64<M64_CG_DIRECTION>(Ctx&, const Level64&, const Coef64
 // ---------------------------------------------------------------------------
 // up-sweep (Vcycle.m:27-32): one thread per (y, x) column of a 32 x 8 tile
 // (a warp holds one x, so the parity of x is uniform in it),
-// walking a chunk of z planes.  The trilinear sum adds the coarse planes
-// first, then x, then y (3.5 additions per DOF on average instead of up to 7
-// weighted terms), and omega / diagonal is stored, so no division is left.
+// walking a chunk of z planes.  omega / diagonal is stored, so no division is
+// left, and the trilinear sum (in FP64: coarse planes first, then x, then y, 3.5
+// additions per DOF on average) is one of 64-bit integers (fixed96.cuh): FP64
+// operations bound the kernel (7.5 per DOF with the dot product, 3 now) and one
+// of them costs the issue slots of 75 integer ones.  At 6.4M nodes 414 -> 264 us;
+// on small grids the shorter chain of 64-clock operations counts as well (solve
+// 42 x 37 x 64 35.1 -> 25.5 ms together with k_restrict).
 // ---------------------------------------------------------------------------
 constexpr int UY = 32, UX = 8;
 template <bool DOT>
@@ -1047,6 +1051,7 @@ __global__ void __launch_bounds__(UY * UX, 2) k_up64(Grid gf, Grid gc, const uin
     if (iy <= gf.ny && ix <= gf.nx) {
         const bool oy = iy & 1, ox = ix & 1;            // ox is uniform across a warp
         const double wyx = (oy ? 0.5 : 1.0) * (ox ? 0.5 : 1.0);
+        const int kyx = (oy ? 1 : 0) + (ox ? 1 : 0), drop_y = oy ? 0 : SUM64_DROP;
         const int64_t fcol = gf.slot(iy, ix, 0), ccol = gc.slot(iy >> 1, ix >> 1, 0);
         constexpr int U = chk::UP_FINE, UC = chk::UP_COARSE;
         double qa[3][4], qb[3][4];
@@ -1079,15 +1084,32 @@ __global__ void __launch_bounds__(UY * UX, 2) k_up64(Grid gf, Grid gc, const uin
             const double wt = wyx * (oz ? 0.5 : 1.0);
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                double e0 = qa[c][0], e1 = qa[c][1], e2 = qa[c][2], e3 = qa[c][3];
+                double e0 = qa[c][0], e1 = qa[c][1], e2 = qa[c][2], e3 = qa[c][3], t;
+                int h = max(abs_hi(e0), oy ? abs_hi(e1) : 0);
+                if (ox) h = max(h, max(abs_hi(e2), oy ? abs_hi(e3) : 0));
                 if (oz) {
-                    e0 += qb[c][0];
-                    e1 += qb[c][1];
-                    if (ox) { e2 += qb[c][2]; e3 += qb[c][3]; }
+                    h = max(h, max(abs_hi(qb[c][0]), oy ? abs_hi(qb[c][1]) : 0));
+                    if (ox) h = max(h, max(abs_hi(qb[c][2]), oy ? abs_hi(qb[c][3]) : 0));
                 }
-                if (ox) { e0 += e2; e1 += e3; }
-                const double t = oy ? e0 + e1 : e0;
-                double out = fma(wt, t, wv[c] * (rv[c] + pv[c]));
+                const int E = h >> 20;
+                if (sum64_holds(E)) {
+                    long long n = sum64_term(e0, E, 0) + sum64_term(e1, E, drop_y);
+                    if (ox) n += sum64_term(e2, E, 0) + sum64_term(e3, E, drop_y);
+                    if (oz) {
+                        n += sum64_term(qb[c][0], E, 0) + sum64_term(qb[c][1], E, drop_y);
+                        if (ox) n += sum64_term(qb[c][2], E, 0) + sum64_term(qb[c][3], E, drop_y);
+                    }
+                    t = sum64_value(n, E, kyx + (oz ? 1 : 0));
+                } else {                                // zeros, infinities, NaN, the ends of the range
+                    if (oz) {
+                        e0 += qb[c][0];
+                        e1 += qb[c][1];
+                        if (ox) { e2 += qb[c][2]; e3 += qb[c][3]; }
+                    }
+                    if (ox) { e0 += e2; e1 += e3; }
+                    t = wt * (oy ? e0 + e1 : e0);
+                }
+                double out = fma(wv[c], rv[c] + pv[c], t);
                 if (zero_fixed && (fl & (NF_FIX_X << c))) out = 0.0;
                 chk::st(xf, fs + c * Sf, 3 * Sf, chk::UP_OUT, out);
                 if (DOT) dot = fma(rv[c], out, dot);

@@ -1,4 +1,5 @@
-// 96-bit fixed-point numbers for the FP64 operator (fine64.cu).
+// Fixed-point sums for the FP64 kernels: 96 bits for the operator (fine64.cu),
+// 64 bits for the transfers (k_up64, k_restrict).
 //
 // GB300's FP64 unit takes 19 clocks of the SM per warp instruction; the integer
 // units take a quarter of a clock.  Sums of a few FP64 values on a common scale
@@ -98,6 +99,47 @@ __device__ __forceinline__ double to_double(I96 x, int ex) {
     }
     const uint32_t dh = ((uint32_t)(ex - 1) << 20) + (h >> 11);   // the leading one adds 1 to the exponent
     return __hiloint2double((int)(dh | (sg & 0x80000000u)), (int)__funnelshift_r(l2, h, 11));
+}
+
+// Weighted sums of a few values as 64-bit integers: value v weighs 2^-k and
+// counts in units of 2^(E - 1083), E the largest biased exponent of the sum's
+// values.  |v| 2^-k < 2^60 units, so the weights may add up to 8.  A value is
+// exact down to E - 7, below that its last bits are cut off: at most 2^-60 of
+// the largest value, where an FP64 sum rounds by up to 2^-53 at each addition.
+// E within SUM64_MIN .. SUM64_MAX only (no zeros, subnormals, infinities, NaN).
+constexpr int SUM64_MIN = 128, SUM64_MAX = 2000;
+constexpr int SUM64_DROP = 4096;      // a k that drops the value, whatever it is
+
+__device__ __forceinline__ int abs_hi(double v) { return __double2hiint(v) & 0x7fffffff; }
+__device__ __forceinline__ bool sum64_holds(int E) { return E >= SUM64_MIN && E <= SUM64_MAX; }
+
+// k: 2^-k, or SUM64_DROP
+__device__ __forceinline__ long long sum64_term(double v, int E, int k) {
+    const uint32_t hi = (uint32_t)__double2hiint(v), lo = (uint32_t)__double2loint(v);
+    const int t = min(E - (int)((hi >> 20) & 0x7ffu) + k, 63);        // zeros and subnormals: below the unit
+    const uint32_t m = (hi & 0xfffffu) | 0x100000u;
+    const unsigned long long M = ((unsigned long long)__funnelshift_l(lo, m, 7) << 32) | (lo << 7);
+    const long long x = (long long)(M >> t), sg = (long long)((int32_t)hi >> 31);
+    return (x ^ sg) - sg;
+}
+// x 2^-k units in FP64, rounded to nearest
+__device__ __forceinline__ double sum64_value(long long x, int E, int k) {
+    const long long sg = x >> 63;
+    const unsigned long long u = (unsigned long long)((x ^ sg) - sg);
+    if (u == 0) return 0.0;
+    const int z = __clzll((long long)u);
+    unsigned long long n = u << z;                                    // 2^63 <= n < 2^64
+    int ex = E + 3 - z - k;                                           // z = 4: |v| in [2^(E - 1023), 2^(E - 1022))
+    const unsigned long long n2 = n + 0x400u;                         // round at bit 10
+    if (n2 < n) {
+        n = 1ull << 63;
+        ++ex;
+    } else {
+        n = n2;
+    }
+    const uint32_t h = (uint32_t)(n >> 32), l = (uint32_t)n;
+    const uint32_t dh = ((uint32_t)ex << 20) + (h >> 11);             // the leading one adds 1 to the exponent
+    return __hiloint2double((int)(dh | ((uint32_t)(int32_t)sg & 0x80000000u)), (int)__funnelshift_r(l, h, 11));
 }
 
 }  // namespace gmgs

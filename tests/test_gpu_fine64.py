@@ -164,3 +164,38 @@ def test_later_densities_equal_a_fresh_handle(precision):
         (2 * j).backward()
         assert abs(j.item() - kept.load_vector() @ u_ref) <= 1e-12 * abs(j.item())
         assert np.array_equal(rho.grad.cpu().numpy(), 2 * g_ref)
+
+
+# The transfers sum as 64-bit integers on the exponent of the largest value, in
+# FP64 for zeros, non-finite values and near the ends of the range.
+def vcycle_inputs():
+    o, s = pair((20, 18, 26), 3, 3, (1.0, 1.0, 1.0), None, 5)
+    r = np.random.default_rng(8).standard_normal(o.levels[0].numDOFs)
+    r[o.levels[0].fixedDOFs] = 0
+    return o, s, r
+
+
+@pytest.mark.parametrize("power", [-600, -40, 40, 600])
+def test_vcycle_scales_by_powers_of_two(power):
+    """All steps are linear, and exact in a power of two while nothing leaves the range."""
+    o, s, r = vcycle_inputs()
+    assert np.array_equal(s.apply_preconditioner(np.ldexp(r, power)), np.ldexp(s.apply_preconditioner(r), power))
+
+
+@pytest.mark.parametrize("spread", [0, 6, 8, 30, 52, 70, 300], ids=lambda s: f"2^{s}")
+def test_vcycle_over_dynamic_ranges(spread):
+    o, s, r = vcycle_inputs()
+    o.setup()
+    r *= np.exp2(np.random.default_rng(spread).uniform(-spread, 0, r.size))
+    r[::7] = 0
+    assert rel(s.apply_preconditioner(r), o.vcycle(r)) < 1e-10
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_vcycle_keeps_non_finite_values(bad):
+    o, s, r = vcycle_inputs()
+    assert np.array_equal(s.apply_preconditioner(0.0 * r), 0.0 * r)
+    at = np.flatnonzero(r)[r.size // 2]
+    r[at] = bad
+    z = s.apply_preconditioner(r)
+    assert not np.isfinite(z[at]) and np.isnan(z).any()
