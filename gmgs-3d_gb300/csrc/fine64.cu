@@ -50,7 +50,7 @@ constexpr int TY = 16, TX = 16;
 constexpr int NT = TY * TX;
 constexpr int HY = TY + 2, HX = TX + 2;
 constexpr int NP = HY * HX;          // points of a tile plane with its one-node halo
-constexpr int NHALO = NP - NT;       // 84
+constexpr int NHALO = NP - NT;       // 68
 constexpr int NXP = HY * TX;         // points of the x stage: the tile's columns with the y halo
 constexpr int BND_LANES = 4;         // lanes per boundary node
 constexpr int ELEM_LANES = 8;        // lanes per node on stored matrices
@@ -242,14 +242,14 @@ __device__ __forceinline__ int tile_y(int tid) { return tid & (TY - 1); }
 __device__ __forceinline__ int tile_x(int tid) { return (tid >> 5) + 8 * ((tid >> 4) & 1); }
 static_assert(TY == 16 && TX == 16 && HY == 18, "two columns 8 apart are 16 banks apart");
 
-// this thread's points of a tile plane: its own node and, for the first
-// NHALO threads, one point of the one-node halo
+// this thread's points of a tile plane: its own node and point k of the
+// one-node halo (none for k >= NHALO)
 struct Points {
     int pc, ph;             // index in the (HX x HY) plane
     int64_t cbase, hbase;   // slot at z = 0
     bool cok, hok;          // inside the allocated grid
     int cy, cx;
-    __device__ Points(const Grid& g, int y0, int x0, int tid) {
+    __device__ Points(const Grid& g, int y0, int x0, int tid, int k) {
         const int ly = tile_y(tid), lx = tile_x(tid);
         cy = y0 + ly;
         cx = x0 + lx;
@@ -259,10 +259,10 @@ struct Points {
         ph = 0;
         hbase = 0;
         hok = false;
-        if (tid < NHALO) {
+        if (k < NHALO) {
             int hy, hx;
-            if (tid < 2 * TY) { hx = tid < TY ? 0 : HX - 1; hy = 1 + (tid & (TY - 1)); }      // x faces: whole rows
-            else { const int k = tid - 2 * TY; hy = (k & 1) ? HY - 1 : 0; hx = k >> 1; }      // y faces with the corners
+            if (k < 2 * TY) { hx = k < TY ? 0 : HX - 1; hy = 1 + (k & (TY - 1)); }            // x faces: whole rows
+            else { hy = (k & 1) ? HY - 1 : 0; hx = (k - 2 * TY) >> 1; }                       // y faces with the corners
             ph = hy + hx * HY;
             const int gy = y0 - 1 + hy, gx = x0 - 1 + hx;
             hok = gy <= g.ny + 1 && gx <= g.nx + 1;
@@ -297,9 +297,14 @@ constexpr int FIXED_RANGE = 23;
 //     brought to this thread's own places in shared memory one plane ahead
 //     (each thread reads back only what it copied: no barrier)
 //   - z stage: m, k and d along z at the tile's nodes and halo, from the three
-//     planes in registers                                  (12 operations, 11/8 warps)
+//     planes in registers                                  (12 operations)
 //   - x stage: sums P, Q, R of the y operators m, k, d at the tile's columns
-//     and their y halo                                     (33 operations, 9/8 warps)
+//     and their y halo                                     (33 operations)
+//   - both halos by components: a thread holds one component of one point of
+//     the z halo (10 points a warp), three warps one component each of the x
+//     stage's.  With all three components on the first threads, their warps did
+//     twice the work of the others between two barriers (K x at 6.4M nodes 683
+//     -> 639 us)
 //   - y stage and the mode's vector updates at the interior nodes
 // Two barriers per plane; two CTAs per SM keep the FP64 pipe fed across them.
 // The square tile wastes fewer lanes than 32 x 8 on grids a little over a
@@ -331,7 +336,10 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
     for (int iz = zb; iz < ze; ++iz)
         occ |= L.tile_occ[((int64_t)iz * tiles_x + btx) * tiles_y + bty] != 0 ? 1u << (iz - zb) : 0u;
     const int64_t S = g.slots, n3 = 3 * S, sz = g.sz();
-    const Points p(g, y0, x0, tid);
+    const int lane = tid & 31, hcmp = lane % 3, hk = lane < 30 ? (tid >> 5) * 10 + lane / 3 : NHALO;
+    const int h_nxt = lane < 30 ? lane - hcmp + (hcmp + 1) % 3 : lane, h_prv = lane < 30 ? lane - hcmp + (hcmp + 2) % 3 : lane;
+    const Points p(g, y0, x0, tid, hk);                         // one component of a halo point per thread
+    const int64_t hbase = p.hbase + hcmp * S;
     const bool own = p.cy <= g.ny && p.cx <= g.nx;
     uint32_t f_next = own ? chk::ld(L.nflag, p.cbase + zb * sz, S, chk::F64_FIELD) : 0u;
     pdl_wait();                                                 // occupancy and flags do not change during a solve
@@ -358,38 +366,38 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
             const double* src = field_array<MODE>(a, j);
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const int64_t ic = p.cbase + iz * sz + c * S, ih = p.hbase + iz * sz + c * S;
+                const int64_t ic = p.cbase + iz * sz + c * S;
                 if (p.cok && chk::ok(ic, n3, chk::F64_FIELD)) cp_async8(st + (j * 3 + c) * NP + p.pc, src + ic);
-                if (p.hok && chk::ok(ih, n3, chk::F64_FIELD)) cp_async8(st + (j * 3 + c) * NP + p.ph, src + ih);
             }
+            const int64_t ih = hbase + iz * sz;
+            if (p.hok && chk::ok(ih, n3, chk::F64_FIELD)) cp_async8(st + (j * 3 + hcmp) * NP + p.ph, src + ih);
         }
     };
-    auto formed = [&](int iz, int pt, bool ok, double v[3], double s[3]) {
+    auto formed_one = [&](int iz, int pt, int c, bool ok, double& v, double& s) {
         const double* st = stage + ((iz + 1) & 1) * (NA * 3 * NP);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            v[c] = s[c] = 0.0;
-            if (ok) {
-                const double f0 = chk::ld(st, c * NP + pt, NA * 3 * NP, R);
-                double f1 = 0.0, f2 = 0.0;
-                if (NA > 1 && narr > 1) f1 = chk::ld(st, (3 + c) * NP + pt, NA * 3 * NP, R);
-                if (NA > 2 && narr > 2) f2 = chk::ld(st, (6 + c) * NP + pt, NA * 3 * NP, R);
-                form<MODE>(f0, f1, f2, ab, a.first, v[c], s[c]);
-            }
+        v = s = 0.0;
+        if (ok) {
+            const double f0 = chk::ld(st, c * NP + pt, NA * 3 * NP, R);
+            double f1 = 0.0, f2 = 0.0;
+            if (NA > 1 && narr > 1) f1 = chk::ld(st, (3 + c) * NP + pt, NA * 3 * NP, R);
+            if (NA > 2 && narr > 2) f2 = chk::ld(st, (6 + c) * NP + pt, NA * 3 * NP, R);
+            form<MODE>(f0, f1, f2, ab, a.first, v, s);
         }
     };
-    double vm[3], vc[3], vp[3], hm[3], hc[3], hp[3], sc[3], sp[3], unused[3];
+    auto formed = [&](int iz, double v[3], double s[3]) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) formed_one(iz, p.pc, c, p.cok, v[c], s[c]);
+    };
+    double vm[3], vc[3], vp[3], hm, hc, hp, sc[3], sp[3], unused[3], unused_h;
     // of a formed plane, over the CTA: the largest biased exponent, and 2047
     // minus the smallest of its points' largest ones (points that are zero in
     // all components left out)
     __shared__ int s_exp[2][2][NT / 32];
-    auto put_exp = [&](int par, const double* u, const double* h) {
-        int e = 0, g = 0;
+    auto put_exp = [&](int par, const double* u, double h) {
+        int e = 0, g = (__double2hiint(h) >> 20) & 0x7ff;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            e = max(e, (__double2hiint(u[c]) >> 20) & 0x7ff);
-            g = max(g, (__double2hiint(h[c]) >> 20) & 0x7ff);
-        }
+        for (int c = 0; c < 3; ++c) e = max(e, (__double2hiint(u[c]) >> 20) & 0x7ff);
+        g = max(g, max(__shfl_sync(0xffffffffu, g, h_nxt), __shfl_sync(0xffffffffu, g, h_prv)));
         const int top = __reduce_max_sync(0xffffffffu, max(e, g));
         const int low = __reduce_max_sync(0xffffffffu, max(e ? 2047 - e : 0, g ? 2047 - g : 0));
         if ((tid & 31) == 0) {
@@ -408,47 +416,35 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
     issue(zb);
     cp_async_commit();
     cp_async_wait<1>();
-    formed(zb - 1, p.pc, p.cok, vm, unused);
-    formed(zb - 1, p.ph, p.hok, hm, unused);
+    formed(zb - 1, vm, unused);
+    formed_one(zb - 1, p.ph, hcmp, p.hok, hm, unused_h);
     issue(zb + 1);
     cp_async_commit();
     cp_async_wait<1>();
-    formed(zb, p.pc, p.cok, vc, sc);
-    formed(zb, p.ph, p.hok, hc, unused);
+    formed(zb, vc, sc);
+    formed_one(zb, p.ph, hcmp, p.hok, hc, unused_h);
     put_exp(0, vm, hm);
     put_exp(1, vc, hc);
     __syncthreads();
     int em = get_exp(0, 0), ec = get_exp(1, 0), lm = get_exp(0, 1), lc = get_exp(1, 1);
     __syncthreads();
 
-    auto z_stage = [&](int pt, const double* um, const double* u, const double* up) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const double s = um[c] + up[c];
-            chk::st(Zb, c * NP + pt, 9 * NP, R, fma(4.0, u[c], s));
-            chk::st(Zb, (3 + c) * NP + pt, 9 * NP, R, fma(2.0, u[c], -s));
-            chk::st(Zb, (6 + c) * NP + pt, 9 * NP, R, up[c] - um[c]);
-        }
+    auto z_one = [&](int pt, int c, double um, double u, double up) {
+        const double s = um + up;
+        chk::st(Zb, c * NP + pt, 9 * NP, R, fma(4.0, u, s));
+        chk::st(Zb, (3 + c) * NP + pt, 9 * NP, R, fma(2.0, u, -s));
+        chk::st(Zb, (6 + c) * NP + pt, 9 * NP, R, up - um);
     };
-    // P, Q, R at plane point (yy, x column): operands at pt - HY, pt, pt + HY
-    auto x_stage = [&](int pt, double P[3], double Q[3], double Rr[3]) {
+    // P, Q, R of component c at plane point (yy, x column): operands at pt - HY, pt, pt + HY
+    auto x_one = [&](int pt, int c, double& P, double& Q, double& Rr) {
         auto zf = [&](int f, int o) { return chk::ld((const double*)Zb, f * NP + pt + o * HY, 9 * NP, R); };
         auto mx = [&](int f) { return fma(4.0, zf(f, 0), zf(f, -1) + zf(f, 1)); };
-        double kM[3], dM[2];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const double l = zf(c, -1), u = zf(c, 0), r = zf(c, 1), s = l + r;
-            Q[c] = fma(4.0, u, s);
-            kM[c] = fma(2.0, u, -s);
-            if (c < 2) dM[c] = r - l;
-        }
-        const double dDz = zf(8, 1) - zf(8, -1), dDx = zf(6, 1) - zf(6, -1);
-        P[0] = fma(cf.gxz, dDz, fma(cf.az[0], mx(3), cf.ax[0] * kM[0]));
-        P[1] = fma(cf.az[1], mx(4), cf.ax[1] * kM[1]);
-        P[2] = fma(cf.gxz, dDx, fma(cf.az[2], mx(5), cf.ax[2] * kM[2]));
-        Rr[0] = dM[1];
-        Rr[1] = fma(cf.gyz, mx(8), cf.gxy * dM[0]);
-        Rr[2] = mx(7);
+        auto dx = [&](int f) { return zf(f, 1) - zf(f, -1); };
+        const double u = zf(c, 0), s = zf(c, -1) + zf(c, 1), kM = fma(2.0, u, -s);
+        Q = fma(4.0, u, s);
+        P = fma(cf.az[c], mx(3 + c), cf.ax[c] * kM);
+        if (c != 1) P = fma(cf.gxz, dx(c == 0 ? 8 : 6), P);
+        Rr = c == 0 ? dx(1) : (c == 1 ? fma(cf.gyz, mx(8), cf.gxy * dx(0)) : mx(7));
     };
     // the same stages on 96-bit integers, all values multiples of 2^(E - 1105)
     auto put_w = [](uint32_t* w, int n, int k, int pt, const I96& x) {
@@ -460,42 +456,27 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
         return I96{chk::ld(w, (3 * k + 0) * n + pt, 27 * n, R), chk::ld(w, (3 * k + 1) * n + pt, 27 * n, R),
                    chk::ld(w, (3 * k + 2) * n + pt, 27 * n, R)};
     };
-    auto z_stage_i = [&](int pt, const double* um, const double* u, const double* up, int E) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const I96 l = to_fixed(um[c], E), m = to_fixed(u[c], E), r = to_fixed(up[c], E), t = l + r;
-            put_w(Zw, NP, c, pt, t + shl<2>(m));
-            put_w(Zw, NP, 3 + c, pt, shl<1>(m) - t);
-            put_w(Zw, NP, 6 + c, pt, r - l);
-        }
+    auto z_one_i = [&](int pt, int c, double um, double u, double up, int E) {
+        const I96 l = to_fixed(um, E), m = to_fixed(u, E), r = to_fixed(up, E), t = l + r;
+        put_w(Zw, NP, c, pt, t + shl<2>(m));
+        put_w(Zw, NP, 3 + c, pt, shl<1>(m) - t);
+        put_w(Zw, NP, 6 + c, pt, r - l);
     };
-    auto x_stage_i = [&](int pt, I96 P[3], I96 Q[3], I96 Rr[3]) {
+    auto x_one_i = [&](int pt, int c, I96& P, I96& Q, I96& Rr) {
         auto zf = [&](int k, int o) { return get_w(Zw, NP, k, pt + o * HY); };
         auto mx = [&](int k) { return zf(k, -1) + zf(k, 1) + shl<2>(zf(k, 0)); };
-        {
-            const I96 l = zf(0, -1), u = zf(0, 0), r = zf(0, 1), t = l + r;
-            Q[0] = t + shl<2>(u);
-            P[0] = mul_frac(shl<1>(u) - t, cf.fax[0]);
-            Rr[1] = mul_frac(r - l, cf.fgxy);
-        }
-        {
-            const I96 l = zf(1, -1), u = zf(1, 0), r = zf(1, 1), t = l + r;
-            Q[1] = t + shl<2>(u);
-            P[1] = mul_frac(shl<1>(u) - t, cf.fax[1]) + mul_frac(mx(4), cf.faz[1]);
-            Rr[0] = r - l;
-        }
-        {
-            const I96 l = zf(2, -1), u = zf(2, 0), r = zf(2, 1), t = l + r;
-            Q[2] = t + shl<2>(u);
-            P[2] = mul_frac(shl<1>(u) - t, cf.fax[2]) + mul_frac(mx(5), cf.faz[2]) - mul_frac(zf(6, 1) - zf(6, -1), cf.fgxz);
-        }
-        P[0] = P[0] + mul_frac(mx(3), cf.faz[0]) - mul_frac(zf(8, 1) - zf(8, -1), cf.fgxz);
-        Rr[1] = Rr[1] + mul_frac(mx(8), cf.fgyz);
-        Rr[2] = mx(7);
+        auto dx = [&](int k) { return zf(k, 1) - zf(k, -1); };
+        const I96 u = zf(c, 0), t = zf(c, -1) + zf(c, 1);
+        Q = t + shl<2>(u);
+        P = mul_frac(shl<1>(u) - t, cf.fax[c]) + mul_frac(mx(3 + c), cf.faz[c]);
+        if (c != 1) P = P - mul_frac(dx(c == 0 ? 8 : 6), cf.fgxz);
+        Rr = c == 0 ? dx(1) : (c == 1 ? mul_frac(dx(0), cf.fgxy) + mul_frac(mx(8), cf.fgyz) : mx(7));
     };
     const int xc = p.pc - HY;                // own point of the x stage
-    const int hxc = tid & (2 * TX - 1), hyy = (hxc & 1) ? HY - 1 : 0;      // the y halo's points: one warp
-    const int hz_pt = hyy + ((hxc >> 1) + 1) * HY, hx_pt = hyy + (hxc >> 1) * HY;
+    // the y halo of the x stage: a component to each of the last three warps
+    const int hx_c = (tid >> 5) - (NT / 32 - 3), hyy = (lane & 1) ? HY - 1 : 0;
+    const int hz_pt = hyy + ((lane >> 1) + 1) * HY, hx_pt = hyy + (lane >> 1) * HY;
+    static_assert(2 * TX == 32 && NHALO <= 10 * (NT / 32), "points of the y halo and of the z halo by warps");
 
 #pragma unroll 1
     for (int iz = zb; iz < ze; ++iz) {
@@ -514,8 +495,8 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
             }
         }
         cp_async_wait<1>();
-        formed(iz + 1, p.pc, p.cok, vp, sp);
-        formed(iz + 1, p.ph, p.hok, hp, unused);
+        formed(iz + 1, vp, sp);
+        formed_one(iz + 1, p.ph, hcmp, p.hok, hp, unused_h);
         put_exp((iz - zb) & 1, vp, hp);
         __syncthreads();
         const int ep = get_exp((iz - zb) & 1, 0), lp = get_exp((iz - zb) & 1, 1);
@@ -526,24 +507,26 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
         lc = lp;
         if (!((occ >> (iz - zb)) & 1u)) {                        // uniform across the CTA, as the next one
         } else if (cf.fixed && range <= FIXED_RANGE && E > 1023 - 700 && E < 1023 + 700) {
-            z_stage_i(p.pc, vm, vc, vp, E);
-            if (tid < NHALO) z_stage_i(p.ph, hm, hc, hp, E);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) z_one_i(p.pc, c, vm[c], vc[c], vp[c], E);
+            if (hk < NHALO) z_one_i(p.ph, hcmp, hm, hc, hp, E);
             __syncthreads();
             I96 P[3], Q[3], Rr[3];
-            if (tid < 2 * TX) {
-                x_stage_i(hz_pt, P, Q, Rr);
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    put_w(Xw, NXP, c, hx_pt, P[c]);
-                    put_w(Xw, NXP, 3 + c, hx_pt, Q[c]);
-                    put_w(Xw, NXP, 6 + c, hx_pt, Rr[c]);
+            for (int c = 0; c < 3; ++c) {
+                if (hx_c == c) {                                 // uniform across the warp
+                    I96 hP, hQ, hR;
+                    x_one_i(hz_pt, c, hP, hQ, hR);
+                    put_w(Xw, NXP, c, hx_pt, hP);
+                    put_w(Xw, NXP, 3 + c, hx_pt, hQ);
+                    put_w(Xw, NXP, 6 + c, hx_pt, hR);
                 }
             }
             // a warp holds whole y columns of the tile, so its x stage is read by its own y stage alone
             if (__any_sync(0xffffffffu, node)) {
-                x_stage_i(p.pc, P, Q, Rr);
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
+                    x_one_i(p.pc, c, P[c], Q[c], Rr[c]);
                     put_w(Xw, NXP, c, xc, P[c]);
                     put_w(Xw, NXP, 3 + c, xc, Q[c]);
                     put_w(Xw, NXP, 6 + c, xc, Rr[c]);
@@ -565,24 +548,26 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
                 }
             }
         } else {
-            z_stage(p.pc, vm, vc, vp);
-            if (tid < NHALO) z_stage(p.ph, hm, hc, hp);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) z_one(p.pc, c, vm[c], vc[c], vp[c]);
+            if (hk < NHALO) z_one(p.ph, hcmp, hm, hc, hp);
             __syncthreads();
             double P[3], Q[3], Rr[3];
-            if (tid < 2 * TX) {
-                x_stage(hz_pt, P, Q, Rr);
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    chk::st(Xb, c * NXP + hx_pt, 9 * NXP, R, P[c]);
-                    chk::st(Xb, (3 + c) * NXP + hx_pt, 9 * NXP, R, Q[c]);
-                    chk::st(Xb, (6 + c) * NXP + hx_pt, 9 * NXP, R, Rr[c]);
+            for (int c = 0; c < 3; ++c) {
+                if (hx_c == c) {
+                    double hP, hQ, hR;
+                    x_one(hz_pt, c, hP, hQ, hR);
+                    chk::st(Xb, c * NXP + hx_pt, 9 * NXP, R, hP);
+                    chk::st(Xb, (3 + c) * NXP + hx_pt, 9 * NXP, R, hQ);
+                    chk::st(Xb, (6 + c) * NXP + hx_pt, 9 * NXP, R, hR);
                 }
             }
             // a warp holds whole y columns of the tile, so its x stage is read by its own y stage alone
             if (__any_sync(0xffffffffu, node)) {
-                x_stage(p.pc, P, Q, Rr);
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
+                    x_one(p.pc, c, P[c], Q[c], Rr[c]);
                     chk::st(Xb, c * NXP + xc, 9 * NXP, R, P[c]);
                     chk::st(Xb, (3 + c) * NXP + xc, 9 * NXP, R, Q[c]);
                     chk::st(Xb, (6 + c) * NXP + xc, 9 * NXP, R, Rr[c]);
@@ -608,10 +593,10 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
         for (int c = 0; c < 3; ++c) {
             vm[c] = vc[c];
             vc[c] = vp[c];
-            hm[c] = hc[c];
-            hc[c] = hp[c];
             sc[c] = sp[c];
         }
+        hm = hc;
+        hc = hp;
     }
     cp_async_wait<0>();
     dot_finish<MODE>(dot, a, sh);
@@ -724,7 +709,7 @@ __global__ void __launch_bounds__(NT, 2) k_modal64(Level64 L, const __grid_const
     }
     if (tid == 0) modal_k(cf, mk);
     const int64_t S = g.slots, n3 = 3 * S, sx = g.sx(), sz = g.sz();
-    const Points p(g, y0, x0, tid);
+    const Points p(g, y0, x0, tid, tid);
     const bool own = p.cy <= g.ny && p.cx <= g.nx;
     constexpr int R = chk::F64_TILE;
     double* const Zb = dyn;               // s (0..2) and e (3..5) along z of the three components
