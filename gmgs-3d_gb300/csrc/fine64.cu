@@ -273,10 +273,10 @@ struct Points {
     }
 };
 
-// the z and x stages' fields (9 each, three words a value), the field inputs of two planes
+// the z and x stages' fields (9 each, three words a value), the field inputs of a plane
 template <int MODE>
 constexpr size_t fine64_smem() {
-    return 12 * (9 * NP + 9 * NXP) + sizeof(double) * (2 * 3 * field_arrays64(MODE) * NP);
+    return 12 * (9 * NP + 9 * NXP) + sizeof(double) * (3 * field_arrays64(MODE) * NP);
 }
 
 // The three stages run on 96-bit integers (fixed96.cuh) where that is at least
@@ -308,7 +308,10 @@ constexpr int FIXED_RANGE = 23;
 //     twice the work of the others between two barriers (K x at 6.4M nodes 683
 //     -> 639 us)
 //   - y stage and the mode's vector updates at the interior nodes
-// Two barriers per plane; two CTAs per SM keep the FP64 pipe fed across them.
+// Three barriers per plane; two CTAs per SM keep the FP64 pipe fed across them.
+// One buffer of field inputs, refilled right after it was read: with two, the
+// CG update's CTAs took 112 KB each and left the L1 cache next to nothing (its
+// loads then waited in the memory pipeline; solve 169 x 147 x 256 90.8 -> 83.3 ms).
 // The square tile wastes fewer lanes than 32 x 8 on grids a little over a
 // multiple of 32 (84 x 73 x 128: 82 against 74 % of the tile's nodes used).
 // ---------------------------------------------------------------------------
@@ -352,16 +355,15 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
     const double ab = step_length<MODE>(a);
     constexpr int NA = field_arrays64(MODE);
     constexpr int R = chk::F64_TILE;
-    double* const stage = dyn;                    // [2][NA * 3][NP] field inputs of two planes
-    double* const Zb = stage + 2 * NA * 3 * NP;   // 9 fields of the z stage: m, k, d of the three components
+    double* const stage = dyn;                    // [NA * 3][NP] field inputs of a plane
+    double* const Zb = stage + NA * 3 * NP;   // 9 fields of the z stage: m, k, d of the three components
     double* const Xb = Zb + 9 * NP * 3 / 2;       // 9 fields of the x stage: P, Q, R
     uint32_t* const Zw = reinterpret_cast<uint32_t*>(Zb);      // the same as three words a value
     uint32_t* const Xw = reinterpret_cast<uint32_t*>(Xb);
     const int narr = ((MODE == M64_CG_UPDATE_JACOBI || MODE == M64_CG_DIRECTION) && a.first) ? NA - 1 : NA;
 
-    // field inputs of plane iz to this thread's places of buffer iz & 1
-    auto issue = [&](int iz) {
-        double* st = stage + ((iz + 1) & 1) * (NA * 3 * NP);
+    // field inputs of plane iz to this thread's places of st
+    auto issue = [&](int iz, double* st) {
 #pragma unroll
         for (int j = 0; j < NA; ++j) {
             if (j >= narr) break;
@@ -375,8 +377,7 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
             if (p.hok && chk::ok(ih, n3, chk::F64_FIELD)) cp_async8(st + (j * 3 + hcmp) * NP + p.ph, src + ih);
         }
     };
-    auto formed_one = [&](int iz, int pt, int c, bool ok, double& v, double& s) {
-        const double* st = stage + ((iz + 1) & 1) * (NA * 3 * NP);
+    auto formed_one = [&](const double* st, int pt, int c, bool ok, double& v, double& s) {
         v = s = 0.0;
         if (ok) {
             const double f0 = chk::ld(st, c * NP + pt, NA * 3 * NP, R);
@@ -386,9 +387,9 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
             form<MODE>(f0, f1, f2, ab, a.first, v, s);
         }
     };
-    auto formed = [&](int iz, double v[3], double s[3]) {
+    auto formed = [&](const double* st, double v[3], double s[3]) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) formed_one(iz, p.pc, c, p.cok, v[c], s[c]);
+        for (int c = 0; c < 3; ++c) formed_one(st, p.pc, c, p.cok, v[c], s[c]);
     };
     double vm[3], vc[3], vp[3], hm, hc, hp, sc[3], sp[3], unused[3], unused_h;
     // of a formed plane, over the CTA: the largest biased exponent, and 2047
@@ -413,18 +414,20 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
         for (int w = 1; w < NT / 32; ++w) e = max(e, s_exp[par][k][w]);
         return e;
     };
-    issue(zb - 1);
+    // the first two planes pass through the stages' buffers, all three in flight together
+    static_assert(12 * 9 * NXP >= 8 * 3 * NA * NP && NXP <= NP, "a plane's field inputs fit");
+    issue(zb - 1, Zb);
     cp_async_commit();
-    issue(zb);
+    issue(zb, Xb);
     cp_async_commit();
+    issue(zb + 1, stage);
+    cp_async_commit();
+    cp_async_wait<2>();
+    formed(Zb, vm, unused);
+    formed_one(Zb, p.ph, hcmp, p.hok, hm, unused_h);
     cp_async_wait<1>();
-    formed(zb - 1, vm, unused);
-    formed_one(zb - 1, p.ph, hcmp, p.hok, hm, unused_h);
-    issue(zb + 1);
-    cp_async_commit();
-    cp_async_wait<1>();
-    formed(zb, vc, sc);
-    formed_one(zb, p.ph, hcmp, p.hok, hc, unused_h);
+    formed(Xb, vc, sc);
+    formed_one(Xb, p.ph, hcmp, p.hok, hc, unused_h);
     put_exp(0, vm, hm);
     put_exp(1, vc, hc);
     __syncthreads();
@@ -482,8 +485,6 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
 
 #pragma unroll 1
     for (int iz = zb; iz < ze; ++iz) {
-        if (iz + 1 < ze) issue(iz + 2);
-        cp_async_commit();
         const int64_t n = p.cbase + iz * sz;
         const uint32_t f = f_next;              // loaded a plane ahead: the x and p loads below depend on it
         if (own && iz + 1 < ze) f_next = chk::ld(L.nflag, n + sz, S, chk::F64_FIELD);
@@ -496,11 +497,13 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
                 if (!a.first) px[c] = chk::ld(a.pold, n + c * S, n3, chk::F64_FIELD);
             }
         }
-        cp_async_wait<1>();
-        formed(iz + 1, vp, sp);
-        formed_one(iz + 1, p.ph, hcmp, p.hok, hp, unused_h);
+        cp_async_wait<0>();
+        formed(stage, vp, sp);
+        formed_one(stage, p.ph, hcmp, p.hok, hp, unused_h);
         put_exp((iz - zb) & 1, vp, hp);
         __syncthreads();
+        if (iz + 1 < ze) issue(iz + 2, stage);                   // the places just read
+        cp_async_commit();
         const int ep = get_exp((iz - zb) & 1, 0), lp = get_exp((iz - zb) & 1, 1);
         const int E = max(em, max(ec, ep)), range = E - 2047 + max(lm, max(lc, lp));
         em = ec;
