@@ -33,9 +33,9 @@
 // took 1.44 ms, with the CG update 1.80 ms, at 80 % of the FP64 unit; with the
 // stencil on integers 0.70 and 1.14 ms; K x alone 0.64 ms since the columns of
 // a warp avoid bank conflicts and the halo is spread over all warps.  No one
-// unit bounds them then (FP64 unit about a third, issue slots less than half,
-// shared-memory pipe about half busy): two CTAs of 128 registers per SM do.
-// A PCG iteration went from 16.9 to 3.1 ms.
+// unit bounds them then (FP64 unit about a third, issue slots about half,
+// shared-memory pipe 40 % busy): two CTAs of 128 registers per SM do.
+// A PCG iteration went from 16.9 to 2.9 ms.
 #include <algorithm>
 #include <atomic>
 
