@@ -37,10 +37,13 @@ struct Error : std::runtime_error {
     Error(int s, const std::string& m) : std::runtime_error(m), status(s) {}
 };
 
+// a failed call also leaves its error as the runtime's last one: cleared here, or
+// the next launch of any handle would report it again
 #define GMGS_CUDA(call)                                                              \
     do {                                                                             \
         cudaError_t e_ = (call);                                                     \
         if (e_ != cudaSuccess) {                                                     \
+            (void)cudaGetLastError();                                                \
             throw ::gmgs::Error(e_ == cudaErrorMemoryAllocation ? GMGS_ERR_OUT_OF_MEMORY \
                                                                 : GMGS_ERR_CUDA,     \
                                 std::string(#call) + ": " + cudaGetErrorString(e_)); \
