@@ -735,10 +735,13 @@ void launch_fine(Ctx& c, const FineLevel& L, const Coef32& cf, const FineArgs& a
     const bool split = HAS_DOT && zc == 1 && stg == FULL && a.prod && a.chunk;
     if (HAS_DOT && zc == 1 && !split) zc = DOT_CHUNK;
     dim3 grid((L.g.ny + 1 + TY - 1) / TY, (L.g.nx + 1 + TX - 1) / TX, (L.g.nz + 1 + zc - 1) / zc);
+    // the nodes on stored matrices as grid layers of this launch, or, on a column so
+    // long that the layers exceed a grid's z extent, as a launch of their own
+    bool perel_apart = false;
     if (MODE == FM_VCYCLE_DOWN && a.n_perel > 0) {
-        const int per = (NT / 8) * (int)(grid.x * grid.y);
-        a.perel_z = (a.n_perel + per - 1) / per;
-        grid.z += a.perel_z;
+        const int per = (NT / 8) * (int)(grid.x * grid.y), layers = (a.n_perel + per - 1) / per;
+        perel_apart = grid.z + layers > 65535;
+        if (!perel_apart) grid.z += a.perel_z = layers;
     }
     auto go = [&](auto tag, auto sp) {
         constexpr int G = decltype(tag)::value;
@@ -762,6 +765,7 @@ void launch_fine(Ctx& c, const FineLevel& L, const Coef32& cf, const FineArgs& a
         if (ftma) go(std::integral_constant<int, 2>{}, whole);
         else go(std::integral_constant<int, 0>{}, whole);
     }
+    if (perel_apart) launch_perel_vdown(c, L, cf, a);
 }
 template void launch_fine<FM_PLAIN>(Ctx&, const FineLevel&, const Coef32&, const FineArgs&);
 template void launch_fine<FM_VCYCLE_DOWN>(Ctx&, const FineLevel&, const Coef32&, const FineArgs&);
