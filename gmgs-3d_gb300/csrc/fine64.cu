@@ -280,17 +280,57 @@ constexpr size_t fine64_smem() {
 }
 
 // The three stages run on 96-bit integers (fixed96.cuh) where that is at least
-// as accurate as FP64 arithmetic at every node: the values of the three planes
-// on the scale of their largest exponent E, unit 2^(E - 1105), are exact down
-// to 2^-30 of the largest value, all sums are exact, and the products with the
-// coefficients (exact as fractions) drop less than 3 units each, 2^-76 of the
-// largest value in all.  FP64 rounds each operation at 2^-53 of the values
-// around a node, so the integers are the more accurate form at every node whose
-// neighbours reach 2^-23 of the window's largest value.  Windows with smaller
-// non-zero points, with infinities or NaN, or near the ends of the exponent
-// range take the same stages in FP64, as do voxels so flat that a coefficient
-// is below 2^-11 of the largest one.
-constexpr int FIXED_RANGE = 23;
+// as accurate as FP64 arithmetic at every node.  The values of the three planes
+// are multiples of 2^-82 of the largest one: exact down to 2^-30 of it, all sums
+// are exact, and the products with the coefficients (exact as fractions) drop
+// less than 3 units each, about 70 units of a row in all.  A row of FP64 rounds
+// its terms at 2^-53, so integers lose nothing
+//   - in a window whose non-zero components all reach 2^-23 of its largest value:
+//     every row then has a term of that size or none at all
+//   - elsewhere, if every row's largest term (own component: 27 neighbours;
+//     another one: the 12 whose 3 x 3 block couples the two) reaches 2^-20 of the
+//     largest value or all are zero: what is cut off the smaller values, at most
+//     240 units, is less than that term's rounding.  A component at rounding
+//     level, as on a symmetry plane, fails the first test and passes this one
+//     (rows_hold).
+// Both limits shrink by the spread of the coefficients.  A point's largest
+// component does not do as a test: u = (2^-60, 0, 1) at one node has an x row of
+// 2^-60, which the z component does not couple into.  Other windows, those with
+// infinities or NaN, or near the ends of the exponent range take the same stages in
+// FP64, as do voxels so flat that a coefficient is below 2^-11 of the largest one.
+constexpr int FIXED_RANGE = 23, FIXED_ROW_MARGIN = 3;
+
+// how far a value lies below the largest exponent E, in binary orders; 255: zero
+__device__ __forceinline__ uint32_t below_top(double v, int E) {
+    const int e = (__double2hiint(v) >> 20) & 0x7ff;
+    return e ? (uint32_t)min(E - e, 254) : 255u;
+}
+
+// Whether every row of this node reaches the limit: a component's own term at
+// any of the 27 points, another component's where both axes differ (x and y for
+// the pair of components x, y).  k: below_top of the three components, a byte
+// each, for the planes iz - 1, iz, iz + 1; pc: the node's point.
+__device__ __forceinline__ bool rows_hold(const uint32_t* k, int pc, int limit) {
+    uint32_t best = 0xffffffffu;
+#pragma unroll 1
+    for (int dz = -1; dz <= 1; ++dz)                      // not unrolled: no registers of the walk spill
+#pragma unroll
+        for (int o = 0; o < 9; ++o) {
+            const int dy = o % 3 - 1, dx = o / 3 - 1;
+            const uint32_t w = chk::ld(k, (dz + 1) * NP + pc + dy + dx * HY, 3 * NP, chk::F64_TILE) | 0xff000000u;
+            best = __vminu4(best, w);
+            if (dx && dy) best = __vminu4(best, __byte_perm(w, 0xffffffffu, 0x4401));         // (y, x, -)
+            if (dx && dz) best = __vminu4(best, __byte_perm(w, 0xffffffffu, 0x4042));         // (z, -, x)
+            if (dy && dz) best = __vminu4(best, __byte_perm(w, 0xffffffffu, 0x4124));         // (-, z, y)
+        }
+    bool ok = true;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const int b = (int)((best >> (8 * c)) & 0xffu);
+        ok = ok && (b <= limit || b == 255);
+    }
+    return ok;
+}
 
 // ---------------------------------------------------------------------------
 // K x with the uniform matrix, axis by axis.  A CTA owns a 16 (y) x 16 (x)
@@ -342,7 +382,6 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
         occ |= L.tile_occ[((int64_t)iz * tiles_x + btx) * tiles_y + bty] != 0 ? 1u << (iz - zb) : 0u;
     const int64_t S = g.slots, n3 = 3 * S, sz = g.sz();
     const int lane = tid & 31, hcmp = lane % 3, hk = lane < 30 ? (tid >> 5) * 10 + lane / 3 : NHALO;
-    const int h_nxt = lane < 30 ? lane - hcmp + (hcmp + 1) % 3 : lane, h_prv = lane < 30 ? lane - hcmp + (hcmp + 2) % 3 : lane;
     const Points p(g, y0, x0, tid, hk);                         // one component of a halo point per thread
     const int64_t hbase = p.hbase + hcmp * S;
     const bool own = p.cy <= g.ny && p.cx <= g.nx;
@@ -392,26 +431,25 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
         for (int c = 0; c < 3; ++c) formed_one(st, p.pc, c, p.cok, v[c], s[c]);
     };
     double vm[3], vc[3], vp[3], hm, hc, hp, sc[3], sp[3], unused[3], unused_h;
-    // of a formed plane, over the CTA: the largest biased exponent, and 2047
-    // minus the smallest of its points' largest ones (points that are zero in
-    // all components left out)
-    __shared__ int s_exp[2][2][NT / 32];
+    // of a formed plane, over the CTA: the largest biased exponent, and in the
+    // upper half 2047 minus the smallest one of a non-zero component
+    __shared__ uint32_t s_exp[2][NT / 32];
     auto put_exp = [&](int par, const double* u, double h) {
-        int e = 0, g = (__double2hiint(h) >> 20) & 0x7ff;
+        int e = (__double2hiint(h) >> 20) & 0x7ff, top = e, low = e ? 2047 - e : 0;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) e = max(e, (__double2hiint(u[c]) >> 20) & 0x7ff);
-        g = max(g, max(__shfl_sync(0xffffffffu, g, h_nxt), __shfl_sync(0xffffffffu, g, h_prv)));
-        const int top = __reduce_max_sync(0xffffffffu, max(e, g));
-        const int low = __reduce_max_sync(0xffffffffu, max(e ? 2047 - e : 0, g ? 2047 - g : 0));
-        if ((tid & 31) == 0) {
-            s_exp[par][0][tid >> 5] = top;
-            s_exp[par][1][tid >> 5] = low;
+        for (int c = 0; c < 3; ++c) {
+            e = (__double2hiint(u[c]) >> 20) & 0x7ff;
+            top = max(top, e);
+            low = max(low, e ? 2047 - e : 0);
         }
+        top = __reduce_max_sync(0xffffffffu, top);
+        low = __reduce_max_sync(0xffffffffu, low);
+        if ((tid & 31) == 0) s_exp[par][tid >> 5] = (uint32_t)(top | low << 16);
     };
-    auto get_exp = [&](int par, int k) {
-        int e = s_exp[par][k][0];
+    auto get_exp = [&](int par) {
+        uint32_t e = s_exp[par][0];
 #pragma unroll
-        for (int w = 1; w < NT / 32; ++w) e = max(e, s_exp[par][k][w]);
+        for (int w = 1; w < NT / 32; ++w) e = __vmaxu2(e, s_exp[par][w]);
         return e;
     };
     // the first two planes pass through the stages' buffers, all three in flight together
@@ -431,7 +469,7 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
     put_exp(0, vm, hm);
     put_exp(1, vc, hc);
     __syncthreads();
-    int em = get_exp(0, 0), ec = get_exp(1, 0), lm = get_exp(0, 1), lc = get_exp(1, 1);
+    uint32_t em = get_exp(0), ec = get_exp(1);
     __syncthreads();
 
     auto z_one = [&](int pt, int c, double um, double u, double up) {
@@ -504,14 +542,26 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
         __syncthreads();
         if (iz + 1 < ze) issue(iz + 2, stage);                   // the places just read
         cp_async_commit();
-        const int ep = get_exp((iz - zb) & 1, 0), lp = get_exp((iz - zb) & 1, 1);
-        const int E = max(em, max(ec, ep)), range = E - 2047 + max(lm, max(lc, lp));
+        const uint32_t ep = get_exp((iz - zb) & 1), ew = __vmaxu2(em, __vmaxu2(ec, ep));
+        const int E = (int)(ew & 0xffffu);
         em = ec;
         ec = ep;
-        lm = lc;
-        lc = lp;
-        if (!((occ >> (iz - zb)) & 1u)) {                        // uniform across the CTA, as the next one
-        } else if (cf.fixed && range <= FIXED_RANGE && E > 1023 - 700 && E < 1023 + 700) {
+        const bool here = (occ >> (iz - zb)) & 1u;               // uniform across the CTA, as the next ones
+        bool fixed = here && cf.fixed && E > 1023 - 700 && E < 1023 + 700;
+        if (fixed && E - 2047 + (int)(ew >> 16) > cf.fixed) {
+            auto put_k = [&](int plane, const double* u, double h) {
+                chk::st(Zw, plane * NP + p.pc, 3 * NP, R, below_top(u[0], E) | below_top(u[1], E) << 8 | below_top(u[2], E) << 16);
+                if (hk < NHALO)
+                    chk::st(reinterpret_cast<uint8_t*>(Zw), 4 * (plane * NP + p.ph) + hcmp, 12 * NP, R, below_top(h, E));
+            };
+            put_k(0, vm, hm);
+            put_k(1, vc, hc);
+            put_k(2, vp, hp);
+            __syncthreads();
+            fixed = __syncthreads_and(!node || rows_hold(Zw, p.pc, cf.fixed - FIXED_ROW_MARGIN));
+        }
+        if (!here) {
+        } else if (fixed) {
 #pragma unroll
             for (int c = 0; c < 3; ++c) z_one_i(p.pc, c, vm[c], vc[c], vp[c], E);
             if (hk < NHALO) z_one_i(p.ph, hcmp, hm, hc, hp, E);
@@ -977,7 +1027,10 @@ void set_fixed_coefs(Coef64& c) {
         const uint64_t C = (uint64_t)std::ldexp(g[k], 64 - c.cexp);
         *f[k] = make_uint2((uint32_t)C, (uint32_t)(C >> 32));
     }
-    c.fixed = 1;
+    // the largest coefficient of the row with the smallest terms, against 2^cexp
+    double row = std::min({c.gxy, -c.gxz, c.gyz});
+    for (int k = 0; k < 3; ++k) row = std::min(row, std::max({c.ax[k], c.ay[k], c.az[k]}));
+    c.fixed = FIXED_RANGE - (c.cexp - 1 - std::ilogb(row));
 }
 
 template <int MODE>

@@ -19,7 +19,8 @@ struct Coef64 {
     double lam, mu;             // Lame constants
     double hx, hy, hz;
     // the stencil's coefficients as fractions C / 2^64 of 2^cexp (Coef64's
-    // signs: gxz is negative, the others positive); fixed: they are exact
+    // signs: gxz is negative, the others positive); fixed: 0 if they are not exact,
+    // else the binary orders below its largest value that a window may reach
     uint2 fax[3], fay[3], faz[3], fgxy, fgxz, fgyz;
     int cexp = 0, fixed = 0;
 };
