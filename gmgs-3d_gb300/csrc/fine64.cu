@@ -301,9 +301,10 @@ constexpr size_t fine64_smem() {
 constexpr int FIXED_RANGE = 23, FIXED_ROW_MARGIN = 3;
 
 // how far a value lies below the largest exponent E, in binary orders; 255: zero
+// (a subnormal, which to_fixed drops, lies at the exponent 0)
 __device__ __forceinline__ uint32_t below_top(double v, int E) {
-    const int e = (__double2hiint(v) >> 20) & 0x7ff;
-    return e ? (uint32_t)min(E - e, 254) : 255u;
+    const int h = abs_hi(v);
+    return h | __double2loint(v) ? (uint32_t)min(E - (h >> 20), 254) : 255u;
 }
 
 // Whether every row of this node reaches the limit: a component's own term at
@@ -435,13 +436,15 @@ __global__ void __launch_bounds__(NT, 2) k_fine64(Level64 L, const __grid_consta
     // upper half 2047 minus the smallest one of a non-zero component
     __shared__ uint32_t s_exp[2][NT / 32];
     auto put_exp = [&](int par, const double* u, double h) {
-        int e = (__double2hiint(h) >> 20) & 0x7ff, top = e, low = e ? 2047 - e : 0;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            e = (__double2hiint(u[c]) >> 20) & 0x7ff;
+        int top = 0, low = 0;
+        auto take = [&](double v) {
+            const int a = abs_hi(v), e = a >> 20;
             top = max(top, e);
-            low = max(low, e ? 2047 - e : 0);
-        }
+            low = max(low, a | __double2loint(v) ? 2047 - e : 0);
+        };
+        take(h);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) take(u[c]);
         top = __reduce_max_sync(0xffffffffu, top);
         low = __reduce_max_sync(0xffffffffu, low);
         if ((tid & 31) == 0) s_exp[par][tid >> 5] = (uint32_t)(top | low << 16);

@@ -1,5 +1,5 @@
 """Where the FP64 operator may use its integer stages (fine64.cu): rows whose
-components lie far apart.
+components lie far apart, and subnormal patches beside normal values.
 
 The reference is the interior stencil of the box element as sums of products of
 the 1-D operators m = [1 4 1], k = [-1 2 -1], d = [-1 0 1], with exact zeros
@@ -102,3 +102,16 @@ def test_component_that_is_noise_on_a_plane_or_everywhere(component):
         check(s, S, u)
         u[[c for c in range(3) if c != component]] = 0.25     # no differences left in the others
         check(s, S, u)
+
+
+# A row of subnormal values: every product and sum may round to a multiple of
+# 2^-1074, at most 100 times on either side.
+def test_subnormal_patch_beside_normal_values():
+    s, S = block(), stencil((1.0, 1.0, 1.0))
+    rng = np.random.default_rng(4)
+    u = np.zeros((3, NZ + 1, NX + 1, NY + 1))
+    u[:, :, :6, :] = rng.uniform(0.5, 1, u[:, :, :6, :].shape)
+    u[:, :, 9:14, 4:12] = rng.uniform(0.5, 1, (3, NZ + 1, 5, 8)) * 2.0 ** -1024
+    y = apply_interior(S, u)
+    assert np.abs(y[:, 2, 10, 6]).max() > 1e6 * 200 * 2.0 ** -1074
+    check(s, S, u, floor=200 * 2.0 ** -1074)
