@@ -118,7 +118,7 @@ void gemm(Ctx& c, int m, int n, int k, double alpha, const double* A, int lda, c
 }
 
 // sqrt(d) and 1 / sqrt(d)'s rounded value's reciprocal, both correctly rounded,
-// for a positive normal d: an FP32 reciprocal square root y, one third-order
+// for a positive d: an FP32 reciprocal square root y, one third-order
 // step (y (1 + h / 2 + 3 h^2 / 8), h = 1 - d y^2, error h^3), then Markstein's
 // final steps: s = RN(s0 + (d - s0^2) y / 2) and RN(y + y (1 - s y)) with exact
 // FMA residuals.  Ten dependent FP64 operations of 64 clocks; the library's square root and
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(256) k_chol_inv32(double* A, int lda, double* 
     }
     auto pivot = [&](double d) {
         const int hi = __double2hiint(d);
-        const bool ok = hi >= 0x00100000 && hi < 0x7ff00000;    // positive, normal, finite
+        const bool ok = hi >= 0 && hi < 0x7ff00000 && (hi | __double2loint(d)) != 0;    // positive and finite
         if (!ok) atomicExch(info, 1);
         double s = 1.0, r = 1.0;
         if (ok) sqrt_and_reciprocal(d, s, r);
