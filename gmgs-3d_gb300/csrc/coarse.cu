@@ -44,6 +44,7 @@
 // launches 8 -> 4 us each (a warp per row instead of 64 x 64 tiles with partial
 // sums in memory and arrival counters).
 #include "setup.cuh"
+#include "sqrt_reciprocal.h"
 
 namespace gmgs {
 
@@ -117,26 +118,16 @@ void gemm(Ctx& c, int m, int n, int k, double alpha, const double* A, int lda, c
     launch_chain(c, k_dgemm<TA, TB, TRI, OUT>, dim3(m / GR, n / GC), GT, 0, k, alpha, A, lda, B, ldb, beta, C, ldc);
 }
 
-// sqrt(d) and 1 / sqrt(d)'s rounded value's reciprocal, both correctly rounded,
-// for a positive d: an FP32 reciprocal square root y, one third-order
-// step (y (1 + h / 2 + 3 h^2 / 8), h = 1 - d y^2, error h^3), then Markstein's
-// final steps: s = RN(s0 + (d - s0^2) y / 2) and RN(y + y (1 - s y)) with exact
-// FMA residuals.  Ten dependent FP64 operations of 64 clocks; the library's square root and
-// division of a lane take about 25.  Outside the FP32 range: the library's.
-__device__ __forceinline__ void sqrt_and_reciprocal(double d, double& s, double& r) {
+// sqrt(d) and its reciprocal, both correctly rounded, for a positive d: from one
+// FP32 reciprocal square root, outside the FP32 range by the library
+__device__ __forceinline__ void pivot_root(double d, double& s, double& r) {
     const int e = (__double2hiint(d) >> 20) - 1023;
     if (e < -120 || e > 120) {
         s = sqrt(d);
         r = 1.0 / s;
         return;
     }
-    double y = f2d_int(rsqrtf(d2f_int(d)));
-    const double h = fma(-(d * y), y, 1.0);
-    y = fma(y, h * fma(0.375, h, 0.5), y);
-    const double s0 = d * y;
-    const double half = __hiloint2double(__double2hiint(y) - (1 << 20), __double2loint(y));
-    s = fma(fma(-s0, s0, d), half, s0);
-    r = fma(y, fma(-s, y, 1.0), y);
+    sqrt_reciprocal(d, f2d_int(rsqrtf(d2f_int(d))), s, r);
 }
 
 // Cholesky of a 32 x 32 SPD tile (lower triangle of A, in place) and the
@@ -165,7 +156,7 @@ __global__ void __launch_bounds__(256) k_chol_inv32(double* A, int lda, double* 
         const bool ok = hi >= 0 && hi < 0x7ff00000 && (hi | __double2loint(d)) != 0;    // positive and finite
         if (!ok) atomicExch(info, 1);
         double s = 1.0, r = 1.0;
-        if (ok) sqrt_and_reciprocal(d, s, r);
+        if (ok) pivot_root(d, s, r);
         s_piv = s;
         s_inv = r;
     };
