@@ -205,10 +205,11 @@ int solve_impl(gmgs_handle* h, double* U_host, double* U_dev, int32_t* iters, do
     const auto t0 = Clock::now();
     HostPrefault pf(U_host, 3 * (size_t)l0.n_node * sizeof(double));
     M.ctx.trace_point("solve: start");
+    M.loads_solved = false;
     const int st = gmgs::pcg_solve(M, M.F.as<double>(), M.U.as<double>(), iters, relres, hist);
     M.ctx.trace_point("solve: PCG (incl. work buffers)");
     if (st == GMGS_ERR_NONFINITE) fail(st, "CG residual is not finite (diverged)");
-    M.solved = true;
+    M.solved = M.loads_solved = true;
     const int64_t nn = l0.n_node;
     if (U_host || U_dev) {
         gmgs::DevBuf tmp;
@@ -384,6 +385,7 @@ int gmgs_set_bc(gmgs_handle* h, const int32_t* fixed, int64_t nfixed, const doub
         if (nfixed <= 0 || !fixed) fail(GMGS_ERR_NO_FIXINGS, "No Constraints! Unable to Perform Static FEA!");
         h->M.ctx.trace_point("set_bc: start");
         gmgs::apply_bc(h->M, fixed, nfixed, loads, nload);
+        h->M.loads_solved = false;
         h->M.ctx.trace_point("set_bc: fixed nodes + loads");
         h->fixed_host.assign(fixed, fixed + nfixed);
         h->loads_host.assign(loads, loads + 4 * nload);
@@ -433,6 +435,7 @@ int gmgs_load_work(gmgs_handle* h, double* result) {
     return guarded(h, [&]() -> int {
         if (!h || !result) fail(GMGS_ERR_INVALID_ARGUMENT, "NULL argument");
         if (!h->M.solved) fail(GMGS_ERR_NO_SOLUTION, "No Deformation Field Available, compute the deformation first");
+        if (!h->M.loads_solved) fail(GMGS_ERR_STATE, "the loads were set after the last solve");
         *result = gmgs::load_work(h->M);
         return GMGS_OK;
     });

@@ -55,6 +55,7 @@ struct Model {
     double* scal_host = nullptr;   // pinned
     int dot_blocks = 0;
     bool bc_set = false, coarse_ready = false, solved = false, ops_ready = false;
+    bool loads_solved = false;   // U belongs to the loads in F (set_bc replaces them)
     // diagnostics
     double t_create_ms = 0, t_bc_ms = 0, t_solve_ms = 0, t_stress_ms = 0;
     int last_iters = 0;

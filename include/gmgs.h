@@ -137,7 +137,8 @@ int gmgs_stress_dev(gmgs_handle* h, double* nodal_dev, float* per_voxel_dev);
  * interleaved vector (an adjoint solve K lambda = ell with the same PCG).
  * dJdrho: num_elements doubles in the compact element order. */
 int gmgs_grad(gmgs_handle* h, const double* ell, double* dJdrho);
-/* Extension: the compliance F^T U of the last solve, formed on the device. */
+/* Extension: the compliance F^T U of the last solve, formed on the device.
+ * GMGS_ERR_STATE once gmgs_set_bc has replaced the loads of that solve. */
 int gmgs_load_work(gmgs_handle* h, double* result);
 int gmgs_grad_dev(gmgs_handle* h, const double* ell_dev, double* dJdrho_dev);
 
