@@ -179,6 +179,8 @@ class Solver:
         """F (3*num_nodes, interleaved) as ApplyBoundaryCondition.m:7-10 builds it."""
         F = np.zeros(3 * self.num_nodes(1))
         ids = self._loads[:, 0].astype(np.int64) - 1
+        if np.any((ids < 0) | (ids >= len(F) // 3)):       # rows that set_bc refused
+            raise ValueError("load node id out of range")
         last = len(ids) - 1 - np.unique(ids[::-1], return_index=True)[1]   # a later duplicate id wins
         F.reshape(-1, 3)[ids[last]] = self._loads[last, 1:4]
         return F
