@@ -170,12 +170,17 @@ __device__ __forceinline__ void epi_from_stage(const float* st, int sidx, bool f
 // per-lane sums and the reduction order are those of a lane per (row,
 // column group), so the result does not depend on the lane layout.
 // out = r - A (w r) with fixed rows zeroed (AtX.m:57).
-// The work is a few dependent loads per node (list, element types, operands):
-// they are issued for all elements before the first is used, and on levels
-// with other nodes as well these nodes are blocks of the streaming launch, so
-// their latency runs beside the tiles (11 to 24 us per level as a launch of
-// its own after them).
+// AHEAD: where these nodes are blocks of the streaming launch, or no more than one
+// wave of a launch of their own, their chain of dependent loads (list, element
+// types, operands) is their time: all types before the dependency, then two
+// elements' loads in flight (as a launch of its own after the tiles, 11 to 24 us
+// per level; the smallest level of the 169 x 147 x 256 model alone 4 us more the
+// other way).  A larger level whose nodes all lie on stored matrices reads
+// gigabytes of them: there one element at a time at 32 registers (8 CTAs per SM)
+// is faster (density model of 428 x 373 x 650: solve 1345 -> 1294 ms, of 214 x 187
+// x 325: 413 -> 403 ms; equal at 84 x 73 x 128).
 // ---------------------------------------------------------------------------
+template <bool AHEAD>
 __device__ __forceinline__ void perel_node(const FineLevel& L, const Coef32& cf, const FineArgs& a, int node, int j) {
     const int count = a.n_perel;
     const bool active = node < count;          // whole 8-lane groups; idle groups still shuffle
@@ -185,40 +190,51 @@ __device__ __forceinline__ void perel_node(const FineLevel& L, const Coef32& cf,
     const long long n3 = 3ll * S;
     constexpr int V = chk::PEREL_VEC;
     float acc[3] = {0.f, 0.f, 0.f};
-    int type[8];                               // -1 void, 0 uniform, k the stored matrix k - 1
+    auto slot_of = [&](int e) { return n - (e & 1) - ((e >> 1) & 1) * sx - (e >> 2) * sz; };
+    auto type_of = [&](int e) {                // -1 void, 0 uniform, k the stored matrix k - 1; uniform across the node's lanes
+        const int es = slot_of(e);
+        if (!active || !chk::ld(L.emask, es, S, chk::PEREL_ELEM)) return -1;
+        const int t = L.etype ? chk::ld(L.etype, es, S, chk::PEREL_ELEM) : 0;
+        return t > 0 && !chk::ok(t - 1, L.nK, chk::PEREL_KS) ? -1 : t;
+    };
+    auto load = [&](int e, int t, float (&d)[3], float (&K)[9]) {
+        const int nj = slot_of(e) + corner_y(j) + corner_x(j) * sx + corner_z(j) * sz;
+        const float* Ke = (t > 0 ? L.Ks + (int64_t)(t - 1) * KE : cf.K) + 3 * corner_of(e & 1, (e >> 1) & 1, e >> 2) * 24 + 3 * j;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        const int es = n - (e & 1) - ((e >> 1) & 1) * sx - (e >> 2) * sz;
-        type[e] = -1;
-        if (active && chk::ld(L.emask, es, S, chk::PEREL_ELEM)) {
-            type[e] = L.etype ? chk::ld(L.etype, es, S, chk::PEREL_ELEM) : 0;
-            if (type[e] > 0 && !chk::ok(type[e] - 1, L.nK, chk::PEREL_KS)) type[e] = -1;
+        for (int b = 0; b < 3; ++b)
+            d[b] = t >= 0 ? chk::ld(a.r32, nj + b * S, n3, V) * chk::ld(a.wdinv, nj + b * S, n3, V) : 0.f;
+#pragma unroll
+        for (int b = 0; b < 9; ++b) K[b] = t >= 0 ? Ke[24 * (b / 3) + b % 3] : 0.f;
+    };
+    auto add = [&](int t, const float (&d)[3], const float (&K)[9]) {
+        const float k = t > 0 ? 1.f : L.kscale;
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            acc[c] = fmaf(k * K[3 * c], d[0], fmaf(k * K[3 * c + 1], d[1], fmaf(k * K[3 * c + 2], d[2], acc[c])));
+    };
+    if constexpr (AHEAD) {
+        int type[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) type[e] = type_of(e);
+        pdl_wait();
+#pragma unroll
+        for (int h = 0; h < 8; h += 2) {
+            float d[2][3], K[2][9];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) load(h + q, type[h + q], d[q], K[q]);
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                if (type[h + q] >= 0) add(type[h + q], d[q], K[q]);
         }
-    }
-    pdl_wait();
+    } else {
+        pdl_wait();
 #pragma unroll
-    for (int h = 0; h < 8; h += 2) {           // two elements' loads in flight
-        float d[2][3], K[2][9];
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const int e = h + q, es = n - (e & 1) - ((e >> 1) & 1) * sx - (e >> 2) * sz;
-            const int nj = es + corner_y(j) + corner_x(j) * sx + corner_z(j) * sz;
-            const bool on = type[e] >= 0;      // uniform across the node's lanes
-            const float* Ke = (type[e] > 0 ? L.Ks + (int64_t)(type[e] - 1) * KE : cf.K) +
-                              3 * corner_of(e & 1, (e >> 1) & 1, e >> 2) * 24 + 3 * j;
-#pragma unroll
-            for (int b = 0; b < 3; ++b)
-                d[q][b] = on ? chk::ld(a.r32, nj + b * S, n3, V) * chk::ld(a.wdinv, nj + b * S, n3, V) : 0.f;
-#pragma unroll
-            for (int b = 0; b < 9; ++b) K[q][b] = on ? Ke[24 * (b / 3) + b % 3] : 0.f;
-        }
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            if (type[h + q] < 0) continue;
-            const float k = type[h + q] > 0 ? 1.f : L.kscale;
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-                acc[c] = fmaf(k * K[q][3 * c], d[q][0], fmaf(k * K[q][3 * c + 1], d[q][1], fmaf(k * K[q][3 * c + 2], d[q][2], acc[c])));
+        for (int e = 0; e < 8; ++e) {
+            const int t = type_of(e);
+            if (t < 0) continue;
+            float d[3], K[9];
+            load(e, t, d, K);
+            add(t, d, K);
         }
     }
 #pragma unroll
@@ -300,7 +316,7 @@ __global__ void __launch_bounds__(NT, MODE == FM_CG_UPDATE_JACOBI ? ((STG & 1) ?
     if (MODE == FM_VCYCLE_DOWN && (int)blockIdx.z < a.perel_z) {   // the first grid layers: nodes on stored matrices
         const int t = threadIdx.x + threadIdx.y * TY;
         const int blk = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-        perel_node(L, cf, a, blk * (NT / 8) + t / 8, t & 7);
+        perel_node<true>(L, cf, a, blk * (NT / 8) + t / 8, t & 7);
         return;
     }
     const int zb = ((int)blockIdx.z - (MODE == FM_VCYCLE_DOWN ? a.perel_z : 0)) * zc;
@@ -956,12 +972,15 @@ void launch_df_split(Ctx& c, int64_t n, const double* b, float* hi, float* lo) {
 }
 
 // the down-sweep of a level whose nodes all lie on stored matrices
-__global__ void __launch_bounds__(NT) k_perel_vdown(FineLevel L, const __grid_constant__ Coef32 cf, FineArgs a) {
+template <bool AHEAD>
+__global__ void __launch_bounds__(NT, AHEAD ? 5 : 6) k_perel_vdown(FineLevel L, const __grid_constant__ Coef32 cf, FineArgs a) {
     pdl_begin();
-    perel_node(L, cf, a, (int)blockIdx.x * (NT / 8) + (int)threadIdx.x / 8, threadIdx.x & 7);
+    perel_node<AHEAD>(L, cf, a, (int)blockIdx.x * (NT / 8) + (int)threadIdx.x / 8, threadIdx.x & 7);
 }
 void launch_perel_vdown(Ctx& c, const FineLevel& L, const Coef32& cf, const FineArgs& a) {
-    launch_chain(c, k_perel_vdown, (a.n_perel + NT / 8 - 1) / (NT / 8), NT, 0, L, cf, a);
+    // one wave of CTAs takes as long as its chain of loads, more are bound by bandwidth
+    const int blocks = (a.n_perel + NT / 8 - 1) / (NT / 8);
+    launch_chain(c, blocks <= 5 * c.num_sms ? k_perel_vdown<true> : k_perel_vdown<false>, blocks, NT, 0, L, cf, a);
 }
 
 // occupancy of the streaming kernel's node tiles: one block per (y tile,
