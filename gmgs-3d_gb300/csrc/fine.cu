@@ -124,7 +124,7 @@ constexpr int FLD_BOX = 3 * PLANE;                            // 1200 floats
 constexpr int FLD_PITCH = (FLD_BOX * 4 + 127) / 128 * 32;     // 1216 floats
 static_assert(RP == 40 && HX == 10, "the field box and the ring share their pitch");
 __host__ __device__ constexpr int field_arrays(int mode) {
-    return mode == FM_PLAIN ? 1 : (mode == FM_CG_UPDATE_JACOBI ? 3 : 2);
+    return mode == FM_CG_UPDATE_JACOBI ? 3 : 2;
 }
 
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* mbar, uint32_t bytes) {
@@ -456,9 +456,7 @@ __global__ void __launch_bounds__(NT, MODE == FM_CG_UPDATE_JACOBI ? ((STG & 1) ?
         for (int c = 0; c < 3; ++c) {
             const int i = c * PLANE + p + 3;
             const float f0 = chk::ld(fstage, i, N, R);
-            if (MODE == FM_PLAIN) {
-                v[c] = f0;
-            } else if (MODE == FM_VCYCLE_DOWN) {
+            if (MODE == FM_VCYCLE_DOWN) {
                 v[c] = f0 * chk::ld(fstage, FLD_PITCH + i, N, R);                      // r * omega/diag
             } else if (MODE == FM_CG_UPDATE_JACOBI) {
                 const float rm = a.first ? f0 : fmaf(-alpha, chk::ld(fstage, 2 * FLD_PITCH + i, N, R), f0);
@@ -550,9 +548,7 @@ __global__ void __launch_bounds__(NT, MODE == FM_CG_UPDATE_JACOBI ? ((STG & 1) ?
             for (int b = 0; b < 3; ++b) {
                 const int i = n + b * S;
                 const float v = chk::ld(P1, pc + b * PLANE, 3 * PLANE, chk::FINE_RING);
-                if (MODE == FM_PLAIN) {
-                    chk::st(a.out32, i, n3, O, y[b]);
-                } else if (MODE == FM_VCYCLE_DOWN) {
+                if (MODE == FM_VCYCLE_DOWN) {
                     chk::st(a.out32, i, n3, O, ed.r[b] - y[b]);         // r' = r - A (omega D^-1 r)
                 } else if (MODE == FM_CG_UPDATE_JACOBI) {
                     // previous iteration's update x += alpha p, r -= alpha q (CG_solver.m:32-33),
@@ -728,7 +724,6 @@ void launch_fine(Ctx& c, const FineLevel& L, const Coef32& cf, const FineArgs& a
     EpiMaps em;
     std::memset(&em, 0, sizeof(em));
     const float* fld[FIELD_ARRAYS] = {nullptr, nullptr, nullptr};
-    if (MODE == FM_PLAIN) fld[0] = a.v;
     if (MODE == FM_VCYCLE_DOWN) { fld[0] = a.r32; fld[1] = a.wdinv; }
     if (MODE == FM_CG_UPDATE_JACOBI) { fld[0] = a.r32; fld[1] = a.wdinv; fld[2] = a.q32; }
     if (MODE == FM_CG_DIRECTION) { fld[0] = a.z32; fld[1] = a.pold; }
@@ -783,7 +778,6 @@ void launch_fine(Ctx& c, const FineLevel& L, const Coef32& cf, const FineArgs& a
     }
     if (perel_apart) launch_perel_vdown(c, L, cf, a);
 }
-template void launch_fine<FM_PLAIN>(Ctx&, const FineLevel&, const Coef32&, const FineArgs&);
 template void launch_fine<FM_VCYCLE_DOWN>(Ctx&, const FineLevel&, const Coef32&, const FineArgs&);
 template void launch_fine<FM_CG_UPDATE_JACOBI>(Ctx&, const FineLevel&, const Coef32&, const FineArgs&);
 template void launch_fine<FM_CG_DIRECTION>(Ctx&, const FineLevel&, const Coef32&, const FineArgs&);

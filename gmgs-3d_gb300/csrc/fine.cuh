@@ -36,7 +36,6 @@ struct DotOut {
 };
 
 enum FineMode {
-    FM_PLAIN = 0,             // y = A v
     FM_VCYCLE_DOWN = 1,       // v = w r, out = r - A v               (Vcycle.m:14, JacobiSmoother.m:5-9)
     FM_CG_UPDATE_JACOBI = 2,  // previous CG update r_m = r - alpha q, x += alpha p, r_m.r_m;
                               // then the Jacobi step v = fl32(w r_m), x += v, r = r_m - A v
@@ -49,7 +48,6 @@ constexpr int DOT_PLANE = 3 * 256;        // products of a tile plane: component
 size_t dot_split_planes(const Grid& g, int num_sms);   // tile planes of a split launch, 0 where none is split
 
 struct FineArgs {
-    const float* v = nullptr;        // FM_PLAIN input
     const float* r32 = nullptr;      // FM_VCYCLE_DOWN residual; FM_CG_UPDATE_JACOBI: its high part (read on the halo)
     float* r_lo = nullptr;           // FM_CG_UPDATE_JACOBI residual, low part (owned nodes, updated in place)
     const float* wdinv = nullptr;    // omega / diag (3 planes)
@@ -76,7 +74,7 @@ struct FineArgs {
 // tensor over the dense slot grid:
 //  m: FM_CG_UPDATE_JACOBI's per-node operands (r high, r low, x high, x low,
 //     q, p), a 32 x 8 x 1 x 3 box: one tile plane of all three components;
-//  f: the field inputs of the mode (FM_PLAIN v; FM_VCYCLE_DOWN r, omega/diag;
+//  f: the field inputs of the mode (FM_VCYCLE_DOWN r, omega/diag;
 //     FM_CG_UPDATE_JACOBI r high, omega/diag, q; FM_CG_DIRECTION z, p), a
 //     40 x 10 x 1 x 3 box: the tile plane with its one-node halo, from y - 4
 //     so that the box starts on a 16-byte boundary.
@@ -167,9 +165,7 @@ __device__ __forceinline__ void field_at(const FineArgs& a, int S, int s, float 
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const int i = s + c * S;
-        if (MODE == FM_PLAIN) {
-            v[c] = chk::ld(a.v, i, n3, F);
-        } else if (MODE == FM_VCYCLE_DOWN) {
+        if (MODE == FM_VCYCLE_DOWN) {
             v[c] = chk::ld(a.r32, i, n3, F) * chk::ld(a.wdinv, i, n3, F);
         } else if (MODE == FM_CG_UPDATE_JACOBI) {
             const float r = chk::ld(a.r32, i, n3, F);

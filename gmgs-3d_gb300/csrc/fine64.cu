@@ -18,9 +18,9 @@
 // form (fixed96.cuh, k_fine64); FP64 arithmetic remains for the rest.
 //
 // Solid nodes with void elements around them take the assembled stencil of
-// their own set of solid elements (256 precomputed sets), nodes on elements
-// with stored matrices the element sum, both from compact node lists, 8 lanes
-// per node; a level with an element scale (density) takes the element form in
+// their own set of solid elements (256 precomputed sets, 4 lanes per node), nodes
+// on elements with stored matrices the element sum (8 lanes per node), both from
+// compact node lists; a level with an element scale (density) takes the element form in
 // modal coordinates (k_modal64).  All parts of one K x run in one launch: the
 // list blocks first, then the tiles.
 //
@@ -292,7 +292,7 @@ constexpr size_t fine64_smem() {
 //     largest value or all are zero: what is cut off the smaller values, at most
 //     240 units, is less than that term's rounding.  A component at rounding
 //     level, as on a symmetry plane, fails the first test and passes this one
-//     (rows_hold).
+//     (rows_hold: 27 loads of packed exponents a node, in such windows only).
 // Both limits shrink by the spread of the coefficients.  A point's largest
 // component does not do as a test: u = (2^-60, 0, 1) at one node has an x row of
 // 2^-60, which the z component does not couple into.  Other windows, those with
@@ -865,10 +865,8 @@ __global__ void __launch_bounds__(NT, 2) k_modal64(Level64 L, const __grid_const
                             const double m0 = zm ? sc_e * t[c][4] : 0.0, m1 = sc_e * t[c][4 * zm + 1],
                                          m2 = sc_e * t[c][4 * zm + 2], m3 = sc_e * t[c][4 * zm + 3];
                             const double s0 = m0 - m1, s1 = m0 + m1, e0 = m2 - m3, e1 = m2 + m3;   // x = 0, 1
-                            double* o = Eb + ((c * 2 + zm) * 4) * NE + e;
                             constexpr int N = 24 * NE;
                             const int b = ((c * 2 + zm) * 4) * NE + e;
-                            (void)o;
                             chk::st(Eb, b, N, R, s0 - e0);                // (y, x) = (0, 0)
                             chk::st(Eb, b + NE, N, R, s0 + e0);           // (1, 0)
                             chk::st(Eb, b + 2 * NE, N, R, s1 - e1);       // (0, 1)
@@ -914,14 +912,14 @@ __global__ void __launch_bounds__(NT, 2) k_modal64(Level64 L, const __grid_const
 }
 
 // z planes per CTA: about 12 waves of two resident CTAs per SM on large grids
-// (169 x 147 x 256 solve: 8 planes 161 ms; 4, 6 and 12 planes 162 to 163 ms),
-// at least 2 where that gives every SM two CTAs (each chunk forms two planes
-// beyond its own; 42 x 37 x 64 solve with 1 / 2 / 3 / 4 / 6 planes on its
-// finest level: 39.1 / 38.3 / 42 / 50 / 60 ms), else zmin: a plane per CTA for
-// the factorised form (its coarse levels at 1 / 2 / 3 / 4 planes: 39.1 / 40.3 /
-// 42.6 / 44.5 ms), 2 for the modal one, whose chunks compute a layer more
-// (density gradient at 42 x 37 x 64 with 2 / 3 / 4 / 5 planes: 22.0 / 23.3 /
-// 24.0 / 26.6 ms)
+// (169 x 147 x 256 solve with 12 / 8 / 6 / 4 planes, 8 of them by this rule: 84.3 /
+// 84.0 / 85.6 / 87.6 ms), at least 2 where that gives every SM two CTAs (each
+// chunk forms two planes beyond its own; 42 x 37 x 64 solve with 1 / 2 / 3 / 4 / 6
+// planes on its finest level: 23.3 / 22.1 / 22.9 / 24.5 / 27.2 ms), else zmin: a
+// plane per CTA for the factorised form (its coarse levels at 1 / 2 / 3 / 4 planes:
+// 22.1 / 21.6 / 21.3 / 21.9 ms), 2 for the modal one, whose chunks compute a layer
+// more (density gradient at 42 x 37 x 64 with 2 / 3 / 4 / 5 planes: 20.7 / 22.9 /
+// 23.6 / 25.6 ms)
 int pick_zc64(const Grid& g, const Ctx& c, int zmin) {
     const int64_t cols = (int64_t)((g.ny + 1 + TY - 1) / TY) * ((g.nx + 1 + TX - 1) / TX);
     const int64_t want = (int64_t)c.num_sms * 2 * 12;

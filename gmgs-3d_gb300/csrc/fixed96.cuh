@@ -106,6 +106,8 @@ __device__ __forceinline__ double to_double(I96 x, int ex) {
 // values.  |v| 2^-k < 2^60 units, so the weights may add up to 8.  A value is
 // exact down to E - 7, below that its last bits are cut off: at most 2^-60 of
 // the largest value, where an FP64 sum rounds by up to 2^-53 at each addition.
+// (Only where large values cancel exactly can FP64 keep more of the small ones:
+// its rounding errors may all be zero there.)
 // E within SUM64_MIN .. SUM64_MAX only (no zeros, subnormals, infinities, NaN).
 constexpr int SUM64_MIN = 128, SUM64_MAX = 2000;
 constexpr int SUM64_DROP = 4096;      // a k that drops the value, whatever it is
