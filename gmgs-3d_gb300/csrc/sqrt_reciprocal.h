@@ -45,12 +45,12 @@ GMGS_HD void sqrt_reciprocal(double d, double y, double& s, double& r) {
     const double s0 = d * y;
     s = std::fma(std::fma(-s0, s0, d), of_bits(bits_of(y) - (1ull << 52)), s0);
     r = std::fma(y, std::fma(-s, y, 1.0), y);
+    // (a power of two s has a power of two r, S R = 2^104 and rest 0 as well)
     constexpr uint64_t ONE = 1ull << 52;
     const uint64_t sb = bits_of(s), rb = bits_of(r);
-    const int up = (int)(sb >> 52) + (int)(rb >> 52) - 2 * 1023 + 1;       // 1 if r reached the next power of two, else 0
-    const uint64_t S = (sb & (ONE - 1)) | ONE, R = ((rb & (ONE - 1)) | ONE) << up;
-    const int64_t rest = -(int64_t)(S * R);                                // 2^105 - S R: 2^105 is 0 modulo 2^64
-    r = of_bits(rb + (2 * rest > (int64_t)S) - (2 * rest < -(int64_t)S));
+    const uint64_t S = (sb & (ONE - 1)) | ONE, R = (rb & (ONE - 1)) | ONE;
+    const uint64_t twice = 0 - 2 * (S * R);                                // 2 (2^105 - S R): 2^105 is 0 modulo 2^64
+    r = of_bits(rb + ((S - twice) >> 63) - ((S + twice) >> 63));           // the sign bits of S - twice, S + twice
 }
 
 }  // namespace gmgs
